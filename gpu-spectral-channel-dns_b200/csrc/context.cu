@@ -31,6 +31,7 @@
 #include "setup.cuh"
 #include "wallsolve.h"
 #include "ypass.cuh"
+#include "zpass.cuh"
 #include "zxpass.cuh"
 
 namespace {
@@ -75,6 +76,12 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
       if ((e = cudaMemcpy(f.wt[i], t.data(), sizeof(C) * n, cudaMemcpyHostToDevice))) return e;
     }
   }
+  std::vector<C> t;
+  const int n = ztw_table<C>(L, t);
+  if (n > 0) {
+    if ((e = cudaMalloc(&f.zt, sizeof(C) * n))) return e;
+    if ((e = cudaMemcpy(f.zt, t.data(), sizeof(C) * n, cudaMemcpyHostToDevice))) return e;
+  }
   return cudaSuccess;
 }
 template <typename C> void free_fft(DevFft<C>& f) {
@@ -86,6 +93,8 @@ template <typename C> void free_fft(DevFft<C>& f) {
     cudaFree(f.wt[i]);
     f.wt[i] = nullptr;
   }
+  cudaFree(f.zt);
+  f.zt = nullptr;
 }
 
 bool fft_len_ok(int L) {
@@ -327,9 +336,9 @@ void default_variants(dns_ctx* c) {
   }
 }
 // the spanwise variant of the FP64 per-function entries: the context's own
-// in the FP64 form, else the block form
+// in the FP64 form, else the first that the length allows
 int zvar64(const dns_ctx* c, int pass) {
-  return c->P.precision == DNS_PREC_FP64 ? c->variant[pass] : DNS_Z_BLOCK;
+  return c->P.precision == DNS_PREC_FP64 ? c->variant[pass] : VAR_AUTO;
 }
 
 dns_status need_scratch(dns_ctx* c) {

@@ -13,12 +13,14 @@ template <typename C> struct DevFft {
   C* tw = nullptr;
   short* drev = nullptr;
   C* wt[3] = {nullptr, nullptr, nullptr};
+  C* zt = nullptr;
   FftTab<C> tab() const {
     FftTab<C> t;
     t.plan = plan;
     t.tw = tw;
     t.drev = drev;
     for (int i = 0; i < 3; ++i) t.wt[i] = wt[i];
+    t.zt = zt;
     return t;
   }
 };

@@ -95,6 +95,43 @@ template <> struct CodeletConst<6> {
   }
 };
 
+// odd multiples of 9: half-wave tables (correctly rounded) and symmetry
+template <int R> struct CodeletHalf;
+template <> struct CodeletHalf<9> {
+  DNS_HD static double c(int m) {
+    const double t[5] = {1.0, 0.766044443118978, 0.17364817766693036, -0.5, -0.9396926207859084};
+    return t[m];
+  }
+  DNS_HD static double s(int m) {
+    const double t[5] = {0.0, 0.6427876096865394, 0.984807753012208, 0.8660254037844386, 0.3420201433256687};
+    return t[m];
+  }
+};
+template <> struct CodeletHalf<18> {
+  DNS_HD static double c(int m) {
+    const double t[10] = {1.0, 0.9396926207859084, 0.766044443118978, 0.5, 0.17364817766693036,
+                          -0.17364817766693036, -0.5, -0.766044443118978, -0.9396926207859084, -1.0};
+    return t[m];
+  }
+  DNS_HD static double s(int m) {
+    const double t[10] = {0.0, 0.3420201433256687, 0.6427876096865394, 0.8660254037844386, 0.984807753012208,
+                          0.984807753012208, 0.8660254037844386, 0.6427876096865394, 0.3420201433256687, 0.0};
+    return t[m];
+  }
+};
+template <int R> struct CodeletConstH {
+  DNS_HD static double c(int m) {
+    m %= R;
+    return CodeletHalf<R>::c(m <= R / 2 ? m : R - m);
+  }
+  DNS_HD static double s(int m) {
+    m %= R;
+    return m <= R / 2 ? CodeletHalf<R>::s(m) : -CodeletHalf<R>::s(R - m);
+  }
+};
+template <> struct CodeletConst<9> : CodeletConstH<9> {};
+template <> struct CodeletConst<18> : CodeletConstH<18> {};
+
 // radices 24, 32, 48: quarter-wave tables (correctly rounded) and symmetry
 template <int R> struct CodeletQuarter;
 template <> struct CodeletQuarter<24> {
@@ -329,6 +366,12 @@ template <bool INV, typename C> struct Codelet<6, INV, C> {
 };
 template <bool INV, typename C> struct Codelet<8, INV, C> {
   DNS_HD static void run(C* v) { codelet_split<2, 4, 8, INV, C>(v); }
+};
+template <bool INV, typename C> struct Codelet<9, INV, C> {
+  DNS_HD static void run(C* v) { codelet_split<3, 3, 9, INV, C>(v); }
+};
+template <bool INV, typename C> struct Codelet<18, INV, C> {
+  DNS_HD static void run(C* v) { codelet_split<2, 9, 18, INV, C>(v); }
 };
 template <bool INV, typename C> struct Codelet<12, INV, C> {
   DNS_HD static void run(C* v) { codelet_split<4, 3, 12, INV, C>(v); }

@@ -21,6 +21,7 @@ template <typename C> struct FftTab {
   const C* tw;          // W_L^j, j < L
   const short* drev;    // digit-reversed position of natural index n
   const C* wt[3];       // FP32 warp-FFT twiddle tables of the plans with 1, 2, 4 lines per warp
+  const C* zt;          // twiddles of the two-pass spanwise form (zpass.cuh), null for lengths without one
 };
 
 // twiddles of a warp-FFT plan: FP32, the plan's own table (lines per warp

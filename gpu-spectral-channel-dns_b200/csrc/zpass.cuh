@@ -1,0 +1,183 @@
+// Spanwise (z) passes as two register butterflies around one exchange.
+//
+// A CTA owns TX streamwise modes x TY wall-normal points, NL = TX TY lines of
+// length L = RA RB.  Pass A reads its RA inputs of a line straight from
+// global memory (zero padding and the zeroed Nyquist modes are skipped
+// there), pass B stores its RB outputs straight to global memory, and the
+// lines cross shared memory once in between, [position][line]: the lanes of
+// a warp cover whole positions, so every shared access is a run of
+// consecutive addresses without padding.  Neither pass works in place, so a
+// thread may take any number of butterflies of a pass, with one block barrier
+// in all.
+//
+// What bounds it: the pass is a transpose with a transform on the way, so HBM
+// should; warp-synchronous in-place lines moved each value through shared
+// memory eight times (FP64, three passes and the staging), which at 128 bytes
+// a clock and SM was the bound.  TY elements of a pencil and TX of a row are
+// the contiguous runs, whole 32-byte sectors on both sides.
+#pragma once
+#include <cmath>
+#include <vector>
+
+#include "fft2.cuh"
+#include "kernels.cuh"
+
+// radices of a length: two factors, both small enough for registers (FP64: a
+// butterfly of radix R holds 4 R of them), the larger first
+template <int L> struct ZPlan { enum { ok = 0, A = 1, B = 1 }; };
+#define ZPLAN(L, RA, RB) \
+  template <> struct ZPlan<L> { enum { ok = 1, A = RA, B = RB }; static_assert(RA * RB == L, "plan"); };
+ZPLAN(24, 6, 4)
+ZPLAN(32, 8, 4)
+ZPLAN(36, 6, 6)
+ZPLAN(48, 8, 6)
+ZPLAN(54, 9, 6)
+ZPLAN(64, 8, 8)
+ZPLAN(72, 9, 8)
+ZPLAN(96, 12, 8)
+ZPLAN(108, 12, 9)
+ZPLAN(128, 16, 8)
+ZPLAN(144, 12, 12)
+ZPLAN(162, 18, 9)
+ZPLAN(192, 16, 12)
+ZPLAN(216, 18, 12)
+ZPLAN(256, 16, 16)
+ZPLAN(288, 18, 16)
+ZPLAN(324, 18, 18)
+ZPLAN(384, 24, 16)
+ZPLAN(432, 24, 18)
+ZPLAN(512, 32, 16)
+ZPLAN(576, 24, 24)
+ZPLAN(768, 32, 24)
+#undef ZPLAN
+#define ZPLAN_LENGTHS(X) \
+  X(24) X(32) X(36) X(48) X(54) X(64) X(72) X(96) X(108) X(128) X(144) X(162) X(192) X(216) X(256) X(288) \
+  X(324) X(384) X(432) X(512) X(576) X(768)
+
+// Pass-B twiddles W_L^{r k}, r = 1..RB-1, k < RA, stored [r - 1][k].
+template <typename C> int ztw_table(int L, std::vector<C>& out) {
+  int ra = 0, rb = 0;
+#define ZCASE(n) \
+  case n: ra = ZPlan<n>::A; rb = ZPlan<n>::B; break;
+  switch (L) { ZPLAN_LENGTHS(ZCASE) default: return -1; }
+#undef ZCASE
+  const long double PI = 3.141592653589793238462643383279502884L;
+  out.resize((size_t)(rb - 1) * ra);
+  for (int r = 1; r < rb; ++r)
+    for (int k = 0; k < ra; ++k) {
+      const long double a = -2.0L * PI * (long double)(r * k) / (long double)L;
+      out[(size_t)(r - 1) * ra + k] = cmk<C>((double)cosl(a), (double)sinl(a));
+    }
+  return (int)out.size();
+}
+
+// butterfly (line li, j) of pass A after its inputs: the RA-point transform,
+// outputs to positions j RA + r
+template <typename C, int RA, int NL, bool INV>
+__device__ __forceinline__ void zpass_a(C* v, C* buf, int li, int j) {
+  Codelet<RA, INV, C>::run(v);
+  C* o = buf + j * (RA * NL) + li;
+#pragma unroll
+  for (int r = 0; r < RA; ++r) o[r * NL] = v[r];
+}
+// butterfly (li, k) of pass B: positions k + r RA in and out, v on return
+template <typename C, int RA, int RB, int NL, bool INV>
+__device__ __forceinline__ void zpass_b(C* v, const C* buf, const C* __restrict__ tw, int li, int k) {
+  const C* x = buf + k * NL + li;
+#pragma unroll
+  for (int r = 0; r < RB; ++r) v[r] = x[r * (RA * NL)];
+#pragma unroll
+  for (int r = 1; r < RB; ++r) {
+    const C w = tw[(r - 1) * RA + k];
+    v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
+  }
+  Codelet<RB, INV, C>::run(v);
+}
+
+// spanwise inverse: pencils [f][kz Kx + kx][y] -> rows [f][y][zp][kx]
+template <typename C, int L, int TX, int TY, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_zb2(PencilArr in, RowArr out, DnsGeom g, const C* __restrict__ tw) {
+  constexpr int RA = ZPlan<L>::A, RB = ZPlan<L>::B, NL = TX * TY;
+  constexpr int Nz = L / 3 * 2, hz = Nz / 2;  // the launcher checks g.Nz
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf = (C*)smem_raw;
+  const int Kx = g.Kx, Py = g.Py;
+  const int kx0 = blockIdx.x * TX, y0 = blockIdx.y * TY, f = blockIdx.z;
+  const long long kzs = (long long)Kx * in.ps;
+  for (int t = threadIdx.x; t < NL * RB; t += NT) {
+    const int li = t % NL, j = t / NL;  // li = kxl TY + yl: TY neighbours of a pencil
+    const int kx = kx0 + li / TY, y = y0 + li % TY;
+    // the streamwise Nyquist column (kx = Kx - 1) and rows beyond Py are zero
+    const bool ok = kx < Kx - 1 && y < Py;
+    const C* src = (const C*)in.base + (long long)f * in.fs + (long long)kx * in.ps + y + (long long)j * kzs;
+    C v[RA];
+#pragma unroll
+    for (int r = 0; r < RA; ++r) {
+      // element n = j + r RB: modes kz < Nz/2, zeros, modes kz - Nz > -Nz/2
+      const int n = j + r * RB;
+      v[r] = cmk<C>(0.0, 0.0);
+      if (r * RB < hz) {
+        if (ok && n < hz) v[r] = src[(long long)(r * RB) * kzs];
+      }
+      if (r * RB + RB - 1 > L - hz) {
+        if (ok && n > L - hz) v[r] = src[(long long)(r * RB - (L - Nz)) * kzs];
+      }
+    }
+    zpass_a<C, RA, NL, true>(v, buf, li, j);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < NL * RA; t += NT) {
+    const int li = t % NL, k = t / NL;
+    C v[RB];
+    zpass_b<C, RA, RB, NL, true>(v, buf, tw, li, k);
+    const int kx = kx0 + li / TY, y = y0 + li % TY;
+    if (kx < Kx && y < Py) {
+      C* dst = (C*)out.base + (long long)f * out.fs + ((long long)y * L + k) * out.rs + kx;
+#pragma unroll
+      for (int r = 0; r < RB; ++r) dst[(long long)(r * RA) * out.rs] = v[r];
+    }
+  }
+}
+
+// spanwise forward: rows [f][y][zp][kx] -> pencils [f][kz Kx + kx][y], the
+// Nz kept wavenumbers
+template <typename C, int L, int TX, int TY, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_zf2(RowArr in, PencilArr out, DnsGeom g, const C* __restrict__ tw) {
+  constexpr int RA = ZPlan<L>::A, RB = ZPlan<L>::B, NL = TX * TY;
+  constexpr int Nz = L / 3 * 2, hz = Nz / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* buf = (C*)smem_raw;
+  const int Kx = g.Kx, Py = g.Py;
+  const int kx0 = blockIdx.x * TX, y0 = blockIdx.y * TY, f = blockIdx.z;
+  for (int t = threadIdx.x; t < NL * RB; t += NT) {
+    const int li = t % NL, j = t / NL;
+    const int kx = kx0 + li / TY, y = y0 + li % TY;
+    const bool ok = kx < Kx && y < Py;
+    const C* src = (const C*)in.base + (long long)f * in.fs + ((long long)y * L + j) * in.rs + kx;
+    C v[RA];
+#pragma unroll
+    for (int r = 0; r < RA; ++r) v[r] = ok ? src[(long long)(r * RB) * in.rs] : cmk<C>(0.0, 0.0);
+    zpass_a<C, RA, NL, false>(v, buf, li, j);
+  }
+  __syncthreads();
+  const long long kzs = (long long)Kx * out.ps;
+  for (int t = threadIdx.x; t < NL * RA; t += NT) {
+    const int li = t % NL, k = t / NL;
+    C v[RB];
+    zpass_b<C, RA, RB, NL, false>(v, buf, tw, li, k);
+    const int kx = kx0 + li / TY, y = y0 + li % TY;
+    if (kx < Kx && y < Py) {
+      C* dst = (C*)out.base + (long long)f * out.fs + (long long)kx * out.ps + y + (long long)k * kzs;
+#pragma unroll
+      for (int r = 0; r < RB; ++r) {
+        const int n = k + r * RA;  // kept: n <= Nz/2 and n > L - Nz/2
+        if (r * RA <= hz) {
+          if (n <= hz) dst[(long long)(r * RA) * kzs] = v[r];
+        }
+        if (r * RA + RA - 1 > L - Nz + hz) {
+          if (n > L - Nz + hz) dst[(long long)(r * RA - (L - Nz)) * kzs] = v[r];
+        }
+      }
+    }
+  }
+}

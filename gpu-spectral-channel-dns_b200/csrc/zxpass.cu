@@ -23,6 +23,7 @@
 
 #include "mbar.cuh"
 #include "wfft.cuh"
+#include "zpass.cuh"
 #include "zxpass.cuh"
 
 namespace {
@@ -122,12 +123,10 @@ __global__ void __launch_bounds__(256, 3) k_zf(RowArr in, PencilArr out, DnsGeom
   }
 }
 
-// Same spanwise passes with warp FFTs: a TX x TY tile of 16 lines
-// (streamwise modes x wall-normal points), NW warps with 16/NW lines each,
-// no block barrier inside the transforms.  The kernels below that read
-// through L1 (k_zbw, k_zfw) use 4 x 4 tiles: 32-byte runs, whole sectors, on
-// both sides; the tensor-staged ones (k_zbt 8 x 2, k_zft 4 x 4) are chosen
-// for their row side.
+// Same spanwise passes in FP32 with warp FFTs on tensor-staged tiles: a TX x TY
+// tile of 16 lines (streamwise modes x wall-normal points), NW warps with
+// 16/NW lines each, no block barrier inside the transforms; the tiles (k_zbt
+// 8 x 2, k_zft 4 x 4) are chosen for their row side.
 //
 // Index arithmetic: on the pencil side a thread keeps one line (its kx and
 // y) and walks the spanwise wavenumbers kz = t/16 + 16 m; on the row side it
@@ -145,76 +144,7 @@ struct SpanTile {
 };
 }  // namespace
 
-template <typename C, int L, int NW, int TX, int TY>
-__global__ void __launch_bounds__(32 * NW) k_zbw(PencilArr in, RowArr out, DnsGeom g, FftTab<C> tab) {
-  typedef SpanTile<C, L, TX, TY, 32 * NW> ST;
-  constexpr int NL = ST::NL, LS = ST::LS, Pz = L;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* lines = (C*)smem_raw;
-  constexpr int Nz = L / 3 * 2;  // my / 3 * 2 (the launcher checks g.Nz)
-  const int Kx = g.Kx, Py = g.Py;
-  const int kx0 = blockIdx.x * TX;
-  const int y0 = blockIdx.y * TY;
-  const int f = blockIdx.z;
-  constexpr int hz = Nz / 2;
-  // pencil side: line li = (kxl, yl) of this thread
-  {
-    const int li = threadIdx.x % NL;
-    const int kx = kx0 + li / TY, y = y0 + li % TY;
-    C* dst = lines + li * LS;
-    // zero band [Nz/2, Pz - Nz/2] (Nyquist and padding)
-    for (int n = hz + threadIdx.x / NL; n <= Pz - hz; n += ST::KS) dst[wsw<C>(n)] = cmk<C>(0.0, 0.0);
-    // the streamwise Nyquist column (kx = Kx - 1) and rows beyond Py stay zero
-    const bool ok = kx < Kx - 1 && y < Py;
-    const C* src = ppen<C>(in, f, ok ? kx : 0) + (ok ? y : 0);
-    const long long kzs = (long long)Kx * in.ps;
-    // loads in batches of ZB independent requests per thread before their stores
-    constexpr int ZB = 8;
-    for (int kz0 = threadIdx.x / NL; kz0 < Nz; kz0 += ZB * ST::KS) {
-      C v[ZB];
-#pragma unroll
-      for (int u = 0; u < ZB; ++u) {
-        const int kz = kz0 + u * ST::KS;
-        v[u] = (ok && kz < Nz && kz != hz) ? src[kz * kzs] : cmk<C>(0.0, 0.0);
-      }
-#pragma unroll
-      for (int u = 0; u < ZB; ++u) {
-        const int kz = kz0 + u * ST::KS;
-        if (kz < Nz && kz != hz) dst[wsw<C>(kz < hz ? kz : kz + (Pz - Nz))] = v[u];
-      }
-    }
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5;
-  constexpr int NLW = NL / NW;  // lines per warp
-  wfft<C, L, NLW, true>(lines + (size_t)NLW * warp * LS, wtw_of(tab, 1), LS);
-  __syncthreads();
-  // row side: this thread's kx, flat index i = yl * Pz + zp
-  const int kxl = threadIdx.x % TX;
-  const int kx = kx0 + kxl;
-  if (kx >= Kx || y0 >= Py) return;
-  const int ni = min(TY, Py - y0) * Pz;
-  C* rowb = prow<C>(out, f, (long long)y0 * Pz) + kx;
-  const C* lb = lines + kxl * TY * LS;
-  constexpr int ZB = 8;
-  for (int i0 = threadIdx.x / TX; i0 < ni; i0 += ZB * ST::IS) {
-    C v[ZB];
-#pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int i = i0 + u * ST::IS;
-      const int yl = i / Pz, zp = i - yl * Pz;
-      v[u] = (i < ni) ? lb[yl * LS + wsw<C>(zp)] : cmk<C>(0.0, 0.0);
-    }
-#pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int i = i0 + u * ST::IS;
-      if (i < ni) rowb[(long long)i * out.rs] = v[u];
-    }
-  }
-}
-
-// The same inverse pass with the pencils staged by the tensor-memory
-// accelerator: warp w owns lines 2w, 2w+1 (one kx, two consecutive y) and
+// Inverse pass with the pencils staged by the tensor-memory accelerator: warp w owns lines 2w, 2w+1 (one kx, two consecutive y) and
 // loads their Nz spanwise values with one tiled 4-D copy (box y 2 x kx 1 x
 // kz Nz x field 1, 4 KB at Nz = 256) into its own line buffer; the first FFT
 // pass reads them there (padding, Nyquist and streamwise-Nyquist zeros
@@ -292,71 +222,7 @@ __global__ void __launch_bounds__(32 * NW, 3) k_zbt(const __grid_constant__ CUte
   }
 }
 
-template <typename C, int L, int NW, int TX, int TY>
-__global__ void __launch_bounds__(32 * NW) k_zfw(RowArr in, PencilArr out, DnsGeom g, FftTab<C> tab) {
-  typedef SpanTile<C, L, TX, TY, 32 * NW> ST;
-  constexpr int NL = ST::NL, LS = ST::LS, Pz = L;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* lines = (C*)smem_raw;
-  constexpr int Nz = L / 3 * 2;  // my / 3 * 2 (the launcher checks g.Nz)
-  const int Kx = g.Kx, Py = g.Py;
-  const int kx0 = blockIdx.x * TX;
-  const int y0 = blockIdx.y * TY;
-  const int f = blockIdx.z;
-  constexpr int ZB = 8;
-  // row side: this thread's kx, flat index i = yl * Pz + zp; rows beyond
-  // Py and columns beyond Kx read as zero
-  {
-    const int kxl = threadIdx.x % TX;
-    const int kx = kx0 + kxl;
-    const int ni = TY * Pz;
-    const int nv = (kx < Kx && y0 < Py) ? min(TY, Py - y0) * Pz : 0;
-    const C* rowb = prow<C>(in, f, (long long)y0 * Pz) + kx;
-    C* lb = lines + kxl * TY * LS;
-    for (int i0 = threadIdx.x / TX; i0 < ni; i0 += ZB * ST::IS) {
-      C v[ZB];
-#pragma unroll
-      for (int u = 0; u < ZB; ++u) {
-        const int i = i0 + u * ST::IS;
-        v[u] = (i < nv) ? rowb[(long long)i * in.rs] : cmk<C>(0.0, 0.0);
-      }
-#pragma unroll
-      for (int u = 0; u < ZB; ++u) {
-        const int i = i0 + u * ST::IS;
-        const int yl = i / Pz, zp = i - yl * Pz;
-        if (i < ni) lb[yl * LS + wsw<C>(zp)] = v[u];
-      }
-    }
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5;
-  constexpr int NLW = NL / NW;  // lines per warp
-  wfft<C, L, NLW, false>(lines + (size_t)NLW * warp * LS, wtw_of(tab, 1), LS);
-  __syncthreads();
-  // pencil side: line li = (kxl, yl) of this thread, wavenumbers kz
-  constexpr int hz = Nz / 2;
-  const int li = threadIdx.x % NL;
-  const int kx = kx0 + li / TY, y = y0 + li % TY;
-  if (kx >= Kx || y >= Py) return;
-  const C* lsrc = lines + li * LS;
-  C* dst = ppen<C>(out, f, kx) + y;
-  const long long kzs = (long long)Kx * out.ps;
-  for (int kz0 = threadIdx.x / NL; kz0 < Nz; kz0 += ZB * ST::KS) {
-    C v[ZB];
-#pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int kz = kz0 + u * ST::KS;
-      v[u] = (kz < Nz) ? lsrc[wsw<C>(kz <= hz ? kz : kz + (Pz - Nz))] : cmk<C>(0.0, 0.0);
-    }
-#pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int kz = kz0 + u * ST::KS;
-      if (kz < Nz) dst[kz * kzs] = v[u];
-    }
-  }
-}
-
-// The same forward pass with the rows staged by tensor copies: lines are
+// Forward pass with the rows staged by tensor copies: lines are
 // numbered y-major (li = yl * 4 + kxl), warp w owns lines 2w, 2w+1 (one y,
 // a kx pair) and loads their Pz values with two tiled 4-D copies (box kx 2
 // x zp Pz/2 x y 1 x field 1) into its own line buffer, [zp][kx pair]; the
@@ -824,55 +690,91 @@ bool row_tmap(const RowArr& in, int nf, const DnsGeom& g, size_t esz, CUtensorMa
 }
 }  // namespace
 
-// warp-FFT tiles gathered through L1: FP32 4 x 4 lines on 8 warps (whole
-// 32-byte sectors on both sides, three CTAs per SM); FP64 4 x 2 lines on 4
-// warps (64-byte runs on the row side, 32-byte runs of y pairs on the
-// pencil side, four CTAs per SM)
-template <typename C> struct ZWarpTile;
-template <> struct ZWarpTile<float2> { enum { NW = 8, TX = 4, TY = 4 }; };
-template <> struct ZWarpTile<double2> { enum { NW = 4, TX = 4, TY = 2 }; };
+// Tiles of the two-pass forms (zpass.cuh), measured at 384 x 384 x 512
+// (inverse / forward, us): FP64 4 x 2 lines on 128 threads, three CTAs per SM
+// 466 / 240, four CTAs (no registers to keep a radix-24 butterfly's loads in
+// flight) 511 / 246, 4 x 4 lines on 256 threads 476 / 246; at 192 x 192 x 256
+// 4 x 4 lines on 128 threads 64 / 36, 4 x 2 on 64 96 / 50, 8 x 2 71 / 34.
+// FP32 at 384: 4 x 4 lines on 256 threads 270 / 130, on 128 288 / 150, 8 x 4
+// 293 / 138 (the tensor-staged form 230 / 124 comes first there).
+template <typename C, int L> struct ZTwo {
+  enum {
+    TX = 4, TY = (sizeof(C) == 8 || L <= 192) ? 4 : 2,
+    NT = (sizeof(C) == 8 && L >= 256) ? 256 : 128,
+    MB = sizeof(C) == 8 ? 2 : (L <= 192 ? 4 : (ZPlan<L>::A > 24 ? 2 : 3))
+  };
+};
+#define DNS_ZCASE(n) case n: return f(std::integral_constant<int, n>());
+template <typename F> cudaError_t with_len_z(int L, F&& f) {
+  switch (L) { ZPLAN_LENGTHS(DNS_ZCASE) }
+  return cudaErrorNotSupported;
+}
+template <typename C>
+cudaError_t launch_zb2(PencilArr in, RowArr out, int nf, DnsGeom g, FftTab<C> tab, cudaStream_t st, bool probe) {
+  return with_len_z(g.Pz, [&](auto LL) -> cudaError_t {
+    constexpr int L = decltype(LL)::value;
+    typedef ZTwo<C, L> T;
+    if (!tab.zt || g.Nz != L / 3 * 2) return cudaErrorNotSupported;
+    if (probe) return cudaSuccess;
+    auto k = k_zb2<C, L, T::TX, T::TY, T::NT, T::MB>;
+    const size_t sm = (size_t)L * T::TX * T::TY * sizeof(C);
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k<<<dim3((g.Kx + T::TX - 1) / T::TX, (g.Py + T::TY - 1) / T::TY, nf), T::NT, sm, st>>>(in, out, g, tab.zt);
+    return cudaGetLastError();
+  });
+}
+template <typename C>
+cudaError_t launch_zf2(RowArr in, PencilArr out, int nf, DnsGeom g, FftTab<C> tab, cudaStream_t st, bool probe) {
+  return with_len_z(g.Pz, [&](auto LL) -> cudaError_t {
+    constexpr int L = decltype(LL)::value;
+    typedef ZTwo<C, L> T;
+    if (!tab.zt || g.Nz != L / 3 * 2) return cudaErrorNotSupported;
+    if (probe) return cudaSuccess;
+    auto k = k_zf2<C, L, T::TX, T::TY, T::NT, T::MB>;
+    const size_t sm = (size_t)L * T::TX * T::TY * sizeof(C);
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k<<<dim3((g.Kx + T::TX - 1) / T::TX, (g.Py + T::TY - 1) / T::TY, nf), T::NT, sm, st>>>(in, out, g, tab.zt);
+    return cudaGetLastError();
+  });
+}
 
 template <typename C>
 cudaError_t launch_zb(PencilArr in, RowArr out, int nf, DnsGeom g, FftTab<C> tab, cudaStream_t st,
                       int* status, int variant, bool probe) {
   const int TX = ZTile<C>::TX, TY = ZTile<C>::TY;
   const bool any = variant == VAR_AUTO;
+  if constexpr (sizeof(C) == 8) {
+    if (any || variant == DNS_Z_TENSOR_COPY) {
+      const cudaError_t e = with_len_xz(g.Pz, [&](auto LL) -> cudaError_t {
+        constexpr int L = decltype(LL)::value;
+        if constexpr (L > 0 && WPlan<L, 2, FftMaxRadix<C>::v>::ok) {
+          constexpr int LS = wlen<C>(L) + 1;
+          CUtensorMap tm;
+          if (status && g.Nz == L / 3 * 2 && wtw_of(tab, 1) &&
+              (size_t)g.Nz * 16 + 128 <= (size_t)2 * LS * sizeof(C) && pencil_tmap(in, nf, g, sizeof(C), &tm)) {
+            if (probe) return cudaSuccess;
+            // pencils staged by tensor copies (a y pair per line pair), 8 x 2
+            // tile: 64-byte runs on the row side
+            const size_t sm = ((size_t)16 * LS) * sizeof(C);
+            cudaFuncSetAttribute(k_zbt<C, L, 8, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            dim3 grid((g.Kx + 7) / 8, (g.Py + 1) / 2, nf);
+            k_zbt<C, L, 8, 8, 2><<<grid, 256, sm, st>>>(tm, out, g, tab, status);
+            return cudaGetLastError();
+          }
+        }
+        return cudaErrorNotSupported;
+      });
+      if (e != cudaErrorNotSupported) return e;
+    }
+  }
+  if (any || variant == DNS_Z_WARP) {
+    const cudaError_t e = launch_zb2<C>(in, out, nf, g, tab, st, probe);
+    if (e != cudaErrorNotSupported) return e;
+  }
+  if (!any && variant != DNS_Z_BLOCK) return cudaErrorNotSupported;
+  if (probe) return cudaSuccess;
   return with_len_xz(g.Pz, [&](auto LL) -> cudaError_t {
     constexpr int L = decltype(LL)::value;
-    if constexpr (L > 0 && WPlan<L, 2, FftMaxRadix<C>::v>::ok) {
-     const C* tw = wtw_of(tab, 1);
-     constexpr int LS = wlen<C>(L) + 1;
-     if constexpr (sizeof(C) == 8) {
-      CUtensorMap tm;
-      if ((any || variant == DNS_Z_TENSOR_COPY) && status && g.Nz == L / 3 * 2 && tw &&
-          (size_t)g.Nz * 16 + 128 <= (size_t)2 * LS * sizeof(C) && pencil_tmap(in, nf, g, sizeof(C), &tm)) {
-       if (probe) return cudaSuccess;
-       // pencils staged by tensor copies (a y pair per line pair), 8 x 2
-       // tile: 64-byte runs on the row side
-       const size_t sm = ((size_t)16 * LS) * sizeof(C);
-       cudaFuncSetAttribute(k_zbt<C, L, 8, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-       dim3 grid((g.Kx + 7) / 8, (g.Py + 1) / 2, nf);
-       k_zbt<C, L, 8, 8, 2><<<grid, 256, sm, st>>>(tm, out, g, tab, status);
-       return cudaGetLastError();
-      }
-     }
-     if ((any || variant == DNS_Z_WARP) && g.Nz == L / 3 * 2 && tw) {
-      if (probe) return cudaSuccess;
-      typedef ZWarpTile<C> WT;
-      const size_t sm = ((size_t)WT::TX * WT::TY * LS) * sizeof(C);
-      // the rest of the SM's memory as L1: the pencil-side gathers of
-      // neighbouring threads share sectors (measured in FP32: a quarter
-      // faster than four CTAs with a small L1)
-      auto k = k_zbw<C, L, WT::NW, WT::TX, WT::TY>;
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 75);
-      dim3 grid((g.Kx + WT::TX - 1) / WT::TX, (g.Py + WT::TY - 1) / WT::TY, nf);
-      k<<<grid, 32 * WT::NW, sm, st>>>(in, out, g, tab);
-      return cudaGetLastError();
-     }
-    }
-    if (!any && variant != DNS_Z_BLOCK) return cudaErrorNotSupported;
-    if (probe) return cudaSuccess;
     const size_t sm = (size_t)TX * TY * FLine<C, L>::stride(g.Pz) * sizeof(C);
     cudaFuncSetAttribute(k_zb<C, TX, TY, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     dim3 grid((g.Kx + TX - 1) / TX, (g.Py + TY - 1) / TY, nf);
@@ -885,38 +787,37 @@ cudaError_t launch_zf(RowArr in, PencilArr out, int nf, DnsGeom g, FftTab<C> tab
                       int* status, int variant, bool probe) {
   const int TX = ZTile<C>::TX, TY = ZTile<C>::TY;
   const bool any = variant == VAR_AUTO;
+  if constexpr (sizeof(C) == 8) {
+    if (any || variant == DNS_Z_TENSOR_COPY) {
+      const cudaError_t e = with_len_xz(g.Pz, [&](auto LL) -> cudaError_t {
+        constexpr int L = decltype(LL)::value;
+        if constexpr (L > 0 && WPlan<L, 2, FftMaxRadix<C>::v>::ok) {
+          constexpr int LS = wlen<C>(L) + 1;
+          CUtensorMap tm;
+          if (status && g.Nz == L / 3 * 2 && wtw_of(tab, 1) &&
+              (size_t)L * 16 + 128 <= (size_t)2 * LS * sizeof(C) && row_tmap(in, nf, g, sizeof(C), &tm)) {
+            if (probe) return cudaSuccess;
+            // rows staged by tensor copies, 4 x 4 tile
+            const size_t sm = ((size_t)16 * LS) * sizeof(C);
+            cudaFuncSetAttribute(k_zft<C, L, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            dim3 grid((g.Kx + 3) / 4, (g.Py + 3) / 4, nf);
+            k_zft<C, L, 8><<<grid, 256, sm, st>>>(tm, out, g, tab, status);
+            return cudaGetLastError();
+          }
+        }
+        return cudaErrorNotSupported;
+      });
+      if (e != cudaErrorNotSupported) return e;
+    }
+  }
+  if (any || variant == DNS_Z_WARP) {
+    const cudaError_t e = launch_zf2<C>(in, out, nf, g, tab, st, probe);
+    if (e != cudaErrorNotSupported) return e;
+  }
+  if (!any && variant != DNS_Z_BLOCK) return cudaErrorNotSupported;
+  if (probe) return cudaSuccess;
   return with_len_xz(g.Pz, [&](auto LL) -> cudaError_t {
     constexpr int L = decltype(LL)::value;
-    if constexpr (L > 0 && WPlan<L, 2, FftMaxRadix<C>::v>::ok) {
-     const C* tw = wtw_of(tab, 1);
-     constexpr int LS = wlen<C>(L) + 1;
-     if constexpr (sizeof(C) == 8) {
-      CUtensorMap tm;
-      if ((any || variant == DNS_Z_TENSOR_COPY) && status && g.Nz == L / 3 * 2 && tw &&
-          (size_t)L * 16 + 128 <= (size_t)2 * LS * sizeof(C) && row_tmap(in, nf, g, sizeof(C), &tm)) {
-       if (probe) return cudaSuccess;
-       // rows staged by tensor copies, 4 x 4 tile
-       const size_t sm = ((size_t)16 * LS) * sizeof(C);
-       cudaFuncSetAttribute(k_zft<C, L, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-       dim3 grid((g.Kx + 3) / 4, (g.Py + 3) / 4, nf);
-       k_zft<C, L, 8><<<grid, 256, sm, st>>>(tm, out, g, tab, status);
-       return cudaGetLastError();
-      }
-     }
-     if ((any || variant == DNS_Z_WARP) && g.Nz == L / 3 * 2 && tw) {
-      if (probe) return cudaSuccess;
-      typedef ZWarpTile<C> WT;
-      const size_t sm = ((size_t)WT::TX * WT::TY * LS) * sizeof(C);
-      auto k = k_zfw<C, L, WT::NW, WT::TX, WT::TY>;
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 75);
-      dim3 grid((g.Kx + WT::TX - 1) / WT::TX, (g.Py + WT::TY - 1) / WT::TY, nf);
-      k<<<grid, 32 * WT::NW, sm, st>>>(in, out, g, tab);
-      return cudaGetLastError();
-     }
-    }
-    if (!any && variant != DNS_Z_BLOCK) return cudaErrorNotSupported;
-    if (probe) return cudaSuccess;
     const size_t sm = (size_t)TX * TY * FLine<C, L>::stride(g.Pz) * sizeof(C);
     cudaFuncSetAttribute(k_zf<C, TX, TY, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     dim3 grid((g.Kx + TX - 1) / TX, (g.Py + TY - 1) / TY, nf);

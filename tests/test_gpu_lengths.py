@@ -1,0 +1,73 @@
+"""GPU: every line length with a compiled transform, in both precisions.
+
+The passes along each direction exist per length (2^a 3^b); grids that are
+short in the other two directions put every length through the drop-in
+transforms (FP64, against the oracle: 1e-13 of the largest value, the parity
+bar of the transforms) and through the time step (the mixed form against FP64:
+1e-6 relative after two steps, the bar of the variants).  The short directions
+leave ragged tiles: 9 streamwise modes, 17 wall-normal points."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from oracle import rpcf_oracle as O  # noqa: E402
+
+SPAN = [24, 32, 36, 48, 54, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 324, 384, 432, 512, 576, 768]
+
+
+@pytest.fixture(autouse=True)
+def _need_gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+def _transform_errors(pkg, mx, my, mz):
+    sz = O.Sizes(mx, my, mz)
+    r = np.random.default_rng(mx * 7 + my * 3 + mz)
+    S = np.zeros((sz.ny, sz.hnx, mz), dtype=np.complex128)
+    S[..., :sz.nz] = r.standard_normal((sz.ny, sz.hnx, sz.nz)) + 1j * r.standard_normal((sz.ny, sz.hnx, sz.nz))
+    pitch = (mx // 2 + 1) * 16
+    c = pkg.Context(pkg.make_params(mx, my, mz, Re=1300.0, dt=0.001))
+    spec = torch.from_numpy(S).cuda()
+    phys = torch.zeros(sz.pz, my, pitch // 8, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    c.transform_3d_one(pkg.BACKWARD, phys.data_ptr(), pitch, spec.data_ptr(), mz * 16)
+    c.synchronize()
+    got = phys.cpu().numpy()[..., :mx]
+    ref = O.transform_backward(S, sz)
+    eb = np.abs(got - ref).max() / np.abs(ref).max()
+    P = r.standard_normal((sz.pz, my, mx))
+    phys[..., :mx] = torch.from_numpy(P)
+    torch.cuda.synchronize()
+    c.transform_3d_one(pkg.FORWARD, phys.data_ptr(), pitch, spec.data_ptr(), mz * 16)
+    c.synchronize()
+    got = spec.cpu().numpy()[..., :sz.pz]
+    ref = O.transform_forward(P, sz)[..., :sz.pz]
+    ef = np.abs(got - ref).max() / np.abs(ref).max()
+    c.close()
+    return eb, ef
+
+
+def _step_error(pkg, mx, my, mz, variants=()):
+    out = []
+    for prec in (pkg.PREC_FP64, pkg.PREC_MIXED):
+        c = pkg.Context(pkg.make_params(mx, my, mz, Re=1300.0, Ro=0.1, dt=0.001, precision=prec))
+        if prec == pkg.PREC_MIXED:
+            for p, v in variants:
+                c.set_variant(p, v)
+        c.set_state(*pkg.seeded_state(c.Nx, c.Ny, c.Nz, amplitude=0.05, seed=1))
+        c.bootstrap()
+        c.step(2)
+        out.append(c.get_state())
+        c.close()
+    return max(np.linalg.norm(a - b) / np.linalg.norm(b) for a, b in zip(out[1], out[0]))
+
+
+@pytest.mark.parametrize("L", SPAN)
+def test_span_length(pkg, L):
+    eb, ef = _transform_errors(pkg, 24, L, 32)
+    assert eb < 1e-13 and ef < 1e-13, (eb, ef)
+    e = _step_error(pkg, 24, L, 32, [(pkg.PASS_ZB, pkg.Z_WARP), (pkg.PASS_ZF, pkg.Z_WARP)])
+    assert e < 1e-6, e
