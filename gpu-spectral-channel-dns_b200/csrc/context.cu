@@ -31,6 +31,7 @@
 #include "setup.cuh"
 #include "wallsolve.h"
 #include "ypass.cuh"
+#include "xpass.cuh"
 #include "zpass.cuh"
 #include "zxpass.cuh"
 
@@ -48,8 +49,16 @@ dns_status fail(dns_status s, const std::string& m) {
     if (e_ != cudaSuccess) return fail(DNS_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// the tables of a length, in one device allocation
 template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
   if (!fft_make_plan(L, &f.plan)) return cudaErrorInvalidValue;
+  std::vector<unsigned char> h;
+  auto put = [&](const void* p, size_t bytes) {
+    const size_t at = (h.size() + 255) & ~(size_t)255;
+    h.resize(at + bytes);
+    std::memcpy(h.data() + at, p, bytes);
+    return at;
+  };
   std::vector<C> tw(L);
   std::vector<short> dr(L);
   const long double PI = 3.141592653589793238462643383279502884L;
@@ -58,43 +67,36 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
     tw[j] = cmk<C>((double)cosl(a), (double)sinl(a));
     dr[j] = (short)fft_digitrev(f.plan, j);
   }
-  cudaError_t e = cudaMalloc(&f.tw, sizeof(C) * L);
-  if (e) return e;
-  e = cudaMalloc(&f.drev, sizeof(short) * L);
-  if (e) return e;
-  e = cudaMemcpy(f.tw, tw.data(), sizeof(C) * L, cudaMemcpyHostToDevice);
-  if (e) return e;
-  e = cudaMemcpy(f.drev, dr.data(), sizeof(short) * L, cudaMemcpyHostToDevice);
-  if (e) return e;
-  // FP32 warp-FFT tables (1, 2, 4 lines per warp) where the length has a plan
-  if (std::is_same<C, float2>::value) {
-    for (int i = 0; i < 3; ++i) {
-      std::vector<C> t;
-      const int n = i == 0 ? wtw_table_any<C, 1>(L, t) : (i == 1 ? wtw_table_any<C, 2>(L, t) : wtw_table_any<C, 4>(L, t));
-      if (n <= 0) continue;
-      if ((e = cudaMalloc(&f.wt[i], sizeof(C) * n))) return e;
-      if ((e = cudaMemcpy(f.wt[i], t.data(), sizeof(C) * n, cudaMemcpyHostToDevice))) return e;
-    }
-  }
+  const size_t otw = put(tw.data(), sizeof(C) * L), odr = put(dr.data(), sizeof(short) * L);
+  // twiddle tables where the length has a plan: FP32 warp FFTs (1, 2 lines
+  // per warp) and the fused streamwise form, both precisions the two-pass
+  // spanwise form
+  const bool f32 = std::is_same<C, float2>::value;
+  const size_t none = ~(size_t)0;
+  size_t off[4] = {none, none, none, none};
   std::vector<C> t;
-  const int n = ztw_table<C>(L, t);
-  if (n > 0) {
-    if ((e = cudaMalloc(&f.zt, sizeof(C) * n))) return e;
-    if ((e = cudaMemcpy(f.zt, t.data(), sizeof(C) * n, cudaMemcpyHostToDevice))) return e;
+  for (int i = 0; i < 4; ++i) {
+    if (i < 3 && !f32) continue;
+    const int n = i == 0 ? wtw_table_any<C, 1>(L, t)
+                : i == 1 ? wtw_table_any<C, 2>(L, t)
+                : i == 2 ? xtw_table<C>(L, t) : ztw_table<C>(L, t);
+    if (n > 0) off[i] = put(t.data(), sizeof(C) * n);
   }
+  cudaError_t e = cudaMalloc(&f.mem, h.size());
+  if (e) return e;
+  if ((e = cudaMemcpy(f.mem, h.data(), h.size(), cudaMemcpyHostToDevice))) return e;
+  auto at = [&](size_t o) { return o == none ? nullptr : (C*)(f.mem + o); };
+  f.tw = at(otw);
+  f.drev = (short*)(f.mem + odr);
+  f.wt[0] = at(off[0]);
+  f.wt[1] = at(off[1]);
+  f.xt = at(off[2]);
+  f.zt = at(off[3]);
   return cudaSuccess;
 }
 template <typename C> void free_fft(DevFft<C>& f) {
-  cudaFree(f.tw);
-  cudaFree(f.drev);
-  f.tw = nullptr;
-  f.drev = nullptr;
-  for (int i = 0; i < 3; ++i) {
-    cudaFree(f.wt[i]);
-    f.wt[i] = nullptr;
-  }
-  cudaFree(f.zt);
-  f.zt = nullptr;
+  cudaFree(f.mem);
+  f = DevFft<C>();
 }
 
 bool fft_len_ok(int L) {
@@ -328,10 +330,16 @@ void default_variants(dns_ctx* c) {
       {DNS_Y3_FFT, DNS_Y3_BLOCK, -1}, {DNS_Y1_WARP, DNS_Y1_BLOCK, -1},
       {DNS_Z_WARP, DNS_Z_BLOCK, -1}, {DNS_Z_WARP, DNS_Z_BLOCK, -1},
       {DNS_Y2_RING3_12K_EF, DNS_Y2_RING2_8K_EF, -1}, {DNS_X_WARP3, DNS_X_BLOCK, -1}};
+  // FP32 spanwise lines: the tensor-staged tiles win once a tile is large
+  // (inverse / forward, us: 384 x 384 x 512 229 / 123 against 273 / 131;
+  // 192 x 192 x 256 41 / 24 against 41 / 23; four 144 x 144 x 256 106 / 51
+  // against 85 / 43)
+  const bool z2 = mixed && c->g.Pz < 256;
   for (int p = 0; p < DNS_NUM_PASSES; ++p) {
     const int* ord = mixed ? order_mixed[p] : order_fp64[p];
     c->variant[p] = ord[0];
-    for (int i = 0; i < 3 && ord[i] >= 0; ++i)
+    const int skip = z2 && (p == DNS_PASS_ZB || p == DNS_PASS_ZF) && variant_available(c, p, ord[1]);
+    for (int i = skip; i < 3 && ord[i] >= 0; ++i)
       if (variant_available(c, p, ord[i])) { c->variant[p] = ord[i]; break; }
   }
 }

@@ -10,16 +10,18 @@
 
 template <typename C> struct DevFft {
   FftPlan plan;
+  unsigned char* mem = nullptr;  // holds the tables below
   C* tw = nullptr;
   short* drev = nullptr;
-  C* wt[3] = {nullptr, nullptr, nullptr};
-  C* zt = nullptr;
+  C* wt[2] = {nullptr, nullptr};
+  C *xt = nullptr, *zt = nullptr;
   FftTab<C> tab() const {
     FftTab<C> t;
     t.plan = plan;
     t.tw = tw;
     t.drev = drev;
-    for (int i = 0; i < 3; ++i) t.wt[i] = wt[i];
+    for (int i = 0; i < 2; ++i) t.wt[i] = wt[i];
+    t.xt = xt;
     t.zt = zt;
     return t;
   }

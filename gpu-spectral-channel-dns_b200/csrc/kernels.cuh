@@ -20,12 +20,13 @@ template <typename C> struct FftTab {
   FftPlan plan;
   const C* tw;          // W_L^j, j < L
   const short* drev;    // digit-reversed position of natural index n
-  const C* wt[3];       // FP32 warp-FFT twiddle tables of the plans with 1, 2, 4 lines per warp
+  const C* wt[2];       // FP32 warp-FFT twiddle tables of the plans with 1, 2 lines per warp
+  const C* xt;          // FP32 twiddles of the fused streamwise form (xpass.cuh)
   const C* zt;          // twiddles of the two-pass spanwise form (zpass.cuh), null for lengths without one
 };
 
 // twiddles of a warp-FFT plan: FP32, the plan's own table (lines per warp
-// 1, 2, 4 -> i = 0, 1, 2); FP64, W_L^j and product recurrences
+// 1, 2 -> i = 0, 1); FP64, W_L^j and product recurrences
 template <typename C> DNS_HD const C* wtw_of(const FftTab<C>& t, int i) {
   return sizeof(C) == 16 ? t.tw : t.wt[i];
 }

@@ -23,6 +23,7 @@
 
 #include "mbar.cuh"
 #include "wfft.cuh"
+#include "xpass.cuh"
 #include "zpass.cuh"
 #include "zxpass.cuh"
 
@@ -420,136 +421,6 @@ __global__ void __launch_bounds__(256, 3) k_x_fused(RowArr in, RowArr out, DnsGe
   }
 }
 
-// Same pass with warp FFTs: a CTA of NW warps (3 or 6) owns four rows of
-// one wall-normal plane.  Warp w inverse-transforms lines LPW w .. LPW w +
-// LPW - 1, LPW = 12 / NW (line 3r+q holds row r's packed pair q), reading
-// the half spectra straight from the row arrays in the first FFT pass;
-// after a block barrier the Lamb vector of the four rows is formed
-// pointwise into lines 0-5 (lines r < 4: lambda_x + i lambda_y of row r;
-// lines 4, 5: lambda_z of rows (0, 1), (2, 3)); each warp forward-transforms
-// 6 / NW of them, and the half spectra are unpacked to the output rows.
-// Six warps hold half the lines each: half the registers per thread, twice
-// the warps per SM.
-template <typename C, int L, int NW>
-__global__ void __launch_bounds__(32 * NW, sizeof(C) == 8 ? 5 : 2) k_xw(RowArr in, RowArr out, DnsGeom g,
-                                                                      FftTab<C> tab, const double* __restrict__ Uy,
-                                                                      double Ro, const double* __restrict__ runs,
-                                                                      int* status) {
-  static_assert(NW == 3 || NW == 6, "three or six warps");
-  constexpr int LPW = 12 / NW;  // inverse lines per warp
-  constexpr int FPW = 6 / NW;   // forward lines per warp
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  typedef T_of<C> T;
-  constexpr int Px = L;
-  constexpr int hx = L / 3;  // Nx / 2 = mx / 3 (the launcher checks it): branches of the packing resolve at compile time
-  constexpr int LW = wlen<C>(L);                        // line stride
-  C* z = (C*)smem_raw;                                  // 12 lines
-  uint64_t* bars = (uint64_t*)(z + (size_t)12 * LW);     // one per warp
-  const long long r0 = (long long)blockIdx.x * 4;
-  const long long nrows = (long long)g.Py * g.Pz * g.nrun;  // a batch: members' rows one after another
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  C* zw = z + (size_t)LPW * warp * LW;
-  // stage this warp's 2 LPW half-spectrum rows (bins 0..hx-1, 16 B aligned)
-  // at the start of its own lines: the first FFT pass reads them all before
-  // it writes its output over them
-  constexpr int SR = (hx + 15) / 16 * 16;  // staged bins per row (>= hx; 128 at L = 384)
-  uint64_t* bar = bars + warp;
-  if (lane == 0) {
-    mbar_init(bar, 1);
-    fence_mbar_init();
-    mbar_expect_tx(bar, 2 * LPW * SR * sizeof(C));
-  }
-  __syncwarp();
-  if (lane < 2 * LPW) {
-    const int line = LPW * warp + (lane >> 1);
-    const int rl = line / 3, q = line - 3 * (line / 3);
-    long long row = r0 + rl;
-    if (row >= nrows) row = nrows - 1;  // duplicate work, not stored
-    // fields of similar magnitude share a transform: (u, v), (ox, oy), (w, oz)
-    const int fa = q == 0 ? 0 : (q == 1 ? 3 : 2), fb = q == 0 ? 1 : (q == 1 ? 4 : 5);
-    bulk_g2s(zw + (size_t)lane * SR, prow<C>(in, (lane & 1) ? fb : fa, row), SR * sizeof(C), bar);
-  }
-  // a wait that runs out is reported and waited once more (bounded); the
-  // warp then goes on, so that every warp reaches the block barriers
-  if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar, 0, 1LL << 31, status))) {
-    if (lane == 0) {
-      atomicOr(status, 1);
-      mbar_wait_bounded(bar, 0, 1LL << 31, nullptr);
-    }
-    __syncwarp();
-  }
-  __syncthreads();
-  {
-    const C* stg = zw;
-    auto ld = [&](int l, int n) -> C { return pack_c2r<C>(stg + (size_t)(2 * l) * SR, stg + (size_t)(2 * l + 1) * SR, n, Px, hx); };
-    auto st = [&](int l, int k, C v) { zw[(size_t)l * LW + wsw<C>(k)] = v; };
-    wfft_io<C, L, LPW, true>(zw, wtw_of(tab, LPW == 4 ? 2 : 1), ld, st);
-  }
-  __syncthreads();
-  // the four rows lie in one wall-normal plane of one member
-  const long long pr = (long long)g.Py * g.Pz;
-  const int run = (int)(r0 / pr);
-  const T ro = (T)(runs ? runs[3 * run + 1] : Ro);
-  const int y = (int)((r0 - run * pr) / g.Pz);
-  const T Ub = (T)Uy[y < g.Py ? y : 0];
-  for (int j = threadIdx.x; j < Px; j += blockDim.x) {
-    const int op = wsw<C>(j);
-    C A[4];
-    T lz[4];
-#pragma unroll
-    for (int rl = 0; rl < 4; ++rl) {
-      const C z0 = z[(size_t)(3 * rl + 0) * LW + op];
-      const C z1 = z[(size_t)(3 * rl + 1) * LW + op];
-      const C z2 = z[(size_t)(3 * rl + 2) * LW + op];
-      const T u = z0.x, v = z0.y, ox = z1.x, oy = z1.y, w = z2.x, oz = z2.y;
-      A[rl].x = oz * v - oy * w - ro * w;
-      A[rl].y = ox * w - oz * u;
-      lz[rl] = oy * u - ox * v + ro * (u + Ub);
-    }
-#pragma unroll
-    for (int rl = 0; rl < 4; ++rl) z[(size_t)rl * LW + op] = A[rl];
-    C B0, B1;
-    B0.x = lz[0]; B0.y = lz[1];
-    B1.x = lz[2]; B1.y = lz[3];
-    z[(size_t)4 * LW + op] = B0;
-    z[(size_t)5 * LW + op] = B1;
-  }
-  __syncthreads();
-  wfft<C, L, FPW, false>(z + (size_t)FPW * warp * LW, wtw_of(tab, FPW - 1));
-  __syncthreads();
-  // unpack: output row o = 3 rl + fl (field fl of row rl) by warp o mod 3,
-  // lanes over the bins k; shared loads of a batch before its stores
-  const int Kx = g.Kx;
-  const T sc = (T)(0.5 / ((double)g.Px * (double)g.Pz));
-  constexpr int XB = 5;
-  for (int o = warp; o < 12; o += NW) {
-    const int rl = o / 3, fl = o - 3 * rl;
-    const long long row = r0 + rl;
-    if (row >= nrows) continue;
-    const C* Z = (fl < 2) ? z + (size_t)rl * LW : z + (size_t)(4 + rl / 2) * LW;
-    const bool im = (fl < 2) ? (fl == 1) : (rl & 1);
-    C* dst = prow<C>(out, fl, row);
-    for (int k0 = lane; k0 < Kx; k0 += 32 * XB) {
-      C zk[XB], zm[XB];
-#pragma unroll
-      for (int u = 0; u < XB; ++u) {
-        const int k = min(k0 + 32 * u, Kx - 1);
-        zk[u] = Z[wsw<C>(k)];
-        zm[u] = Z[wsw<C>(k ? Px - k : 0)];
-      }
-#pragma unroll
-      for (int u = 0; u < XB; ++u) {
-        const int k = k0 + 32 * u;
-        if (k >= Kx) continue;
-        C v;
-        if (!im) { v.x = zk[u].x + zm[u].x; v.y = zk[u].y - zm[u].y; }
-        else { v.x = zk[u].y + zm[u].y; v.y = zm[u].x - zk[u].x; }
-        dst[k] = v * sc;
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // standalone streamwise C2R / R2C (drop-in transform_3d_one pieces)
 // complex rows in [row][kx] (pitch rs) <-> real rows [row][x] (pitch rps)
@@ -825,44 +696,64 @@ cudaError_t launch_zf(RowArr in, PencilArr out, int nf, DnsGeom g, FftTab<C> tab
     return cudaGetLastError();
   });
 }
+// CTAs per SM that k_x2 is compiled for, measured at 384 (FP32 / FP64, us):
+// five 294 / 623, four 312 / 642; FP32 at 216: seven 33.1, five 34.7.  Radix 18
+// in the middle needs the registers of four.
+template <typename C, int L> constexpr int x2_ctas() {
+  typedef XPlan<L, FftMaxRadix<C>::v> P;
+  return P::NW > 3 ? (L > 576 ? 1 : 2) : (P::RF > 16 ? 4 : (sizeof(C) == 8 && L < 256 ? 7 : 5));
+}
+template <typename C, int L, int SC>
+cudaError_t launch_x2(RowArr in, RowArr out, DnsGeom g, FftTab<C> tab, const double* Uy, double Ro, int* status,
+                      cudaStream_t st, const double* runs) {
+  typedef XPlan<L, FftMaxRadix<C>::v> P;
+  constexpr int NR = SC * P::NR;
+  auto k = k_x2<C, L, SC, (x2_ctas<C, L>() / SC > 0 ? x2_ctas<C, L>() / SC : 1)>;
+  const size_t sm = (size_t)3 * NR * xline<C>(L) * sizeof(C);
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const long long nrows = (long long)g.Py * g.Pz * g.nrun;
+  k<<<(unsigned)((nrows + NR - 1) / NR), 32 * SC * P::NW, sm, st>>>(
+      in, out, g, FftMaxRadix<C>::v == 8 ? tab.tw : tab.xt, Uy, Ro, runs, status);
+  return cudaGetLastError();
+}
+#define DNS_XCASE(n) case n: return f(std::integral_constant<int, n>());
+template <typename F> cudaError_t with_len_x(int L, F&& f) {
+  switch (L) { XPLAN_LENGTHS(DNS_XCASE) }
+  return cudaErrorNotSupported;
+}
 template <typename C>
 cudaError_t launch_x_fused(RowArr in, RowArr out, DnsGeom g, FftTab<C> tab, const double* Uy,
                            double Ro, int* status, cudaStream_t st, int variant, bool probe,
                            const double* runs) {
   const bool any = variant == VAR_AUTO;
+  const long long nrows = (long long)g.Py * g.Pz * g.nrun;
+  // the fused form stages half spectra of roundup(Nx/2, 8) bins by bulk
+  // copies; the rows of a pair share a plane where Pz is even
+  const int sr = (g.Nx / 2 + 7) / 8 * 8;
+  const bool ok = g.Pz % 2 == 0 && g.Nx / 2 == g.Px / 3 && in.rs >= sr && (in.rs * sizeof(C)) % 16 == 0 &&
+                  (in.fs * sizeof(C)) % 16 == 0 && aligned16(in.base) && status && nrows < (1LL << 31) &&
+                  (sizeof(C) == 16 || tab.xt);
+  if (ok && (any || variant == DNS_X_WARP3 || variant == DNS_X_WARP6)) {
+    const cudaError_t e = with_len_x(g.Px, [&](auto LL) -> cudaError_t {
+      constexpr int L = decltype(LL)::value;
+      if (variant == DNS_X_WARP6) {
+        // two row groups per CTA, for the lengths of the named grids
+        if constexpr (L == 48 || L == 96 || L == 144 || L == 192 || L == 384) {
+          return probe ? cudaSuccess : launch_x2<C, L, 2>(in, out, g, tab, Uy, Ro, status, st, runs);
+        }
+        return cudaErrorNotSupported;
+      }
+      return probe ? cudaSuccess : launch_x2<C, L, 1>(in, out, g, tab, Uy, Ro, status, st, runs);
+    });
+    if (e != cudaErrorNotSupported) return e;
+  }
+  if (!any && variant != DNS_X_BLOCK) return cudaErrorNotSupported;
+  if (probe) return cudaSuccess;
   return with_len_xz(g.Px, [&](auto LL) -> cudaError_t {
     constexpr int L = decltype(LL)::value;
-    if constexpr (L > 0) {
-      const long long nrows = (long long)g.Py * g.Pz * g.nrun;
-      // four rows per CTA within one wall-normal plane; a warp's staged
-      // rows of SR >= Nx/2 bins (2 SR <= a line) fit in its lines
-      constexpr int SR = (L / 3 + 15) / 16 * 16;
-      const bool ok = g.Pz % 4 == 0 && g.Nx / 2 == L / 3 && 2 * SR <= wlen<C>(L) && in.rs >= SR &&
-                      (in.rs * sizeof(C)) % 16 == 0 && (in.fs * sizeof(C)) % 16 == 0;
-      const size_t sm = ((size_t)12 * wlen<C>(L)) * sizeof(C) + 64;
-      // FP32: the plans' twiddle tables; FP64: W^j with product recurrences
-      if constexpr (WPlan<L, 4, FftMaxRadix<C>::v>::ok && WPlan<L, 2, FftMaxRadix<C>::v>::ok) {
-        if (ok && wtw_of(tab, 1) && wtw_of(tab, 2) && (any || variant == DNS_X_WARP3)) {
-          if (probe) return cudaSuccess;
-          cudaFuncSetAttribute(k_xw<C, L, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-          k_xw<C, L, 3><<<(unsigned)((nrows + 3) / 4), 96, sm, st>>>(in, out, g, tab, Uy, Ro, runs, status);
-          return cudaGetLastError();
-        }
-      }
-      if constexpr (WPlan<L, 2, FftMaxRadix<C>::v>::ok && WPlan<L, 1, FftMaxRadix<C>::v>::ok) {
-        if (ok && wtw_of(tab, 0) && wtw_of(tab, 1) && variant == DNS_X_WARP6) {
-          if (probe) return cudaSuccess;
-          cudaFuncSetAttribute(k_xw<C, L, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-          k_xw<C, L, 6><<<(unsigned)((nrows + 3) / 4), 192, sm, st>>>(in, out, g, tab, Uy, Ro, runs, status);
-          return cudaGetLastError();
-        }
-      }
-    }
-    if (!any && variant != DNS_X_BLOCK) return cudaErrorNotSupported;
-    if (probe) return cudaSuccess;
     const size_t sm = (size_t)(L > 0 ? 6 : 9) * FLine<C, L>::stride(g.Px) * sizeof(C);
     cudaFuncSetAttribute(k_x_fused<C, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    const long long nrows = (long long)g.Py * g.Pz * g.nrun;  // Pz is even: row pairs share a plane
+    // Pz is even: row pairs share a plane
     k_x_fused<C, L><<<(unsigned)((nrows + 1) / 2), 256, sm, st>>>(in, out, g, tab, Uy, Ro, runs);
     return cudaGetLastError();
   });

@@ -4,8 +4,9 @@ The passes along each direction exist per length (2^a 3^b); grids that are
 short in the other two directions put every length through the drop-in
 transforms (FP64, against the oracle: 1e-13 of the largest value, the parity
 bar of the transforms) and through the time step (the mixed form against FP64:
-1e-6 relative after two steps, the bar of the variants).  The short directions
-leave ragged tiles: 9 streamwise modes, 17 wall-normal points."""
+1e-6 relative after two steps, the bar of the variants; the FP64 streamwise
+pass against its block form, 1e-12).  The short directions leave ragged tiles:
+9 streamwise modes, 17 wall-normal points, 54 span points (no multiple of 4)."""
 import numpy as np
 import pytest
 
@@ -50,19 +51,24 @@ def _transform_errors(pkg, mx, my, mz):
     return eb, ef
 
 
+def _state_after(pkg, prec, mx, my, mz, variants=()):
+    c = pkg.Context(pkg.make_params(mx, my, mz, Re=1300.0, Ro=0.1, dt=0.001, precision=prec))
+    for p, v in variants:
+        c.set_variant(p, v)
+    c.set_state(*pkg.seeded_state(c.Nx, c.Ny, c.Nz, amplitude=0.05, seed=1))
+    c.bootstrap()
+    c.step(2)
+    out = c.get_state()
+    c.close()
+    return out
+
+
+def _apart(x, y):
+    return max(np.linalg.norm(a - b) / np.linalg.norm(b) for a, b in zip(x, y))
+
+
 def _step_error(pkg, mx, my, mz, variants=()):
-    out = []
-    for prec in (pkg.PREC_FP64, pkg.PREC_MIXED):
-        c = pkg.Context(pkg.make_params(mx, my, mz, Re=1300.0, Ro=0.1, dt=0.001, precision=prec))
-        if prec == pkg.PREC_MIXED:
-            for p, v in variants:
-                c.set_variant(p, v)
-        c.set_state(*pkg.seeded_state(c.Nx, c.Ny, c.Nz, amplitude=0.05, seed=1))
-        c.bootstrap()
-        c.step(2)
-        out.append(c.get_state())
-        c.close()
-    return max(np.linalg.norm(a - b) / np.linalg.norm(b) for a, b in zip(out[1], out[0]))
+    return _apart(_state_after(pkg, pkg.PREC_MIXED, mx, my, mz, variants), _state_after(pkg, pkg.PREC_FP64, mx, my, mz))
 
 
 @pytest.mark.parametrize("L", SPAN)
@@ -70,4 +76,13 @@ def test_span_length(pkg, L):
     eb, ef = _transform_errors(pkg, 24, L, 32)
     assert eb < 1e-13 and ef < 1e-13, (eb, ef)
     e = _step_error(pkg, 24, L, 32, [(pkg.PASS_ZB, pkg.Z_WARP), (pkg.PASS_ZF, pkg.Z_WARP)])
+    assert e < 1e-6, e
+
+
+@pytest.mark.parametrize("L", SPAN)
+def test_stream_length(pkg, L):
+    fused = _state_after(pkg, pkg.PREC_FP64, L, 54, 32)
+    block = _state_after(pkg, pkg.PREC_FP64, L, 54, 32, [(pkg.PASS_X, pkg.X_BLOCK)])
+    assert _apart(fused, block) < 1e-12
+    e = _step_error(pkg, L, 54, 32, [(pkg.PASS_X, pkg.X_WARP3)])
     assert e < 1e-6, e
