@@ -32,6 +32,7 @@
 #include "wallsolve.h"
 #include "ypass.cuh"
 #include "xpass.cuh"
+#include "ydct.cuh"
 #include "zpass.cuh"
 #include "zxpass.cuh"
 
@@ -70,16 +71,17 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
   const size_t otw = put(tw.data(), sizeof(C) * L), odr = put(dr.data(), sizeof(short) * L);
   // twiddle tables where the length has a plan: FP32 warp FFTs (1, 2 lines
   // per warp) and the fused streamwise form, both precisions the two-pass
-  // spanwise form
+  // spanwise form and the pruned DCT
   const bool f32 = std::is_same<C, float2>::value;
   const size_t none = ~(size_t)0;
-  size_t off[4] = {none, none, none, none};
+  size_t off[5] = {none, none, none, none, none};
   std::vector<C> t;
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < 5; ++i) {
     if (i < 3 && !f32) continue;
     const int n = i == 0 ? wtw_table_any<C, 1>(L, t)
                 : i == 1 ? wtw_table_any<C, 2>(L, t)
-                : i == 2 ? xtw_table<C>(L, t) : ztw_table<C>(L, t);
+                : i == 2 ? xtw_table<C>(L, t)
+                : i == 3 ? ztw_table<C>(L, t) : dtw_table<C>(L, t);
     if (n > 0) off[i] = put(t.data(), sizeof(C) * n);
   }
   cudaError_t e = cudaMalloc(&f.mem, h.size());
@@ -92,6 +94,7 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
   f.wt[1] = at(off[1]);
   f.xt = at(off[2]);
   f.zt = at(off[3]);
+  f.dt = at(off[4]);
   return cudaSuccess;
 }
 template <typename C> void free_fft(DevFft<C>& f) {

@@ -14,13 +14,14 @@ template <typename C> struct DevFft {
   C* tw = nullptr;
   short* drev = nullptr;
   C* wt[2] = {nullptr, nullptr};
-  C *xt = nullptr, *zt = nullptr;
+  C *dt = nullptr, *xt = nullptr, *zt = nullptr;
   FftTab<C> tab() const {
     FftTab<C> t;
     t.plan = plan;
     t.tw = tw;
     t.drev = drev;
     for (int i = 0; i < 2; ++i) t.wt[i] = wt[i];
+    t.dt = dt;
     t.xt = xt;
     t.zt = zt;
     return t;

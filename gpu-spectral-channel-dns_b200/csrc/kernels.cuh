@@ -21,6 +21,7 @@ template <typename C> struct FftTab {
   const C* tw;          // W_L^j, j < L
   const short* drev;    // digit-reversed position of natural index n
   const C* wt[2];       // FP32 warp-FFT twiddle tables of the plans with 1, 2 lines per warp
+  const C* dt;          // twiddles of the pruned DCT (ydct.cuh), null for lengths without one
   const C* xt;          // FP32 twiddles of the fused streamwise form (xpass.cuh)
   const C* zt;          // twiddles of the two-pass spanwise form (zpass.cuh), null for lengths without one
 };

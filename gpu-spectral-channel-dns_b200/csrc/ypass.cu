@@ -21,6 +21,7 @@
 #include "kernels.cuh"
 #include "mbar.cuh"
 #include "wfft.cuh"
+#include "ydct.cuh"
 #include "ypass.cuh"
 
 namespace {
@@ -458,36 +459,32 @@ __global__ void __launch_bounds__(256, 3) k_y3(const double2* __restrict__ V, co
   }
 }
 
-// Same pass with the warp FFT: three warps per pencil, two of the six lines
-// per warp, no block barrier inside the transforms; twiddles from the
-// plan's table through L1.
-template <typename C, int M>
-__global__ void __launch_bounds__(96) k_y3w(const double2* __restrict__ V, const double2* __restrict__ O,
-                                           PencilArr out, DnsGeom g, PhysParams ph, FftTab<C> tab,
-                                           int* status) {
+// Same pass with the six lines as pruned DCTs (ydct.cuh): two warps per
+// pencil.  The FP64 state (by bulk copies), its derivatives and the exchange
+// between the two passes share one region, the six fields' coefficients
+// (halved for n > 0: the even extension) have their own.
+//
+// What bounds it: with whole 3-pass FFTs of the even extensions the pass moved
+// each of 512 values of a line five times through shared memory and spent its
+// issue slots on the redundant half; the two pruned passes move 0.56 of them
+// once.  Measured, FP64: see launch_y3.
+template <typename C, int M, int MB>
+__global__ void __launch_bounds__(64, MB) k_y3d(const double2* __restrict__ V, const double2* __restrict__ O,
+                                               PencilArr out, DnsGeom g, PhysParams ph, const C* __restrict__ dt,
+                                               int* status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int Ny = M / 4 + 1;  // the launcher checks g.Ny, g.Py against M
-  // everything lives in the six line buffers (two per warp): the FP64 state
-  // and derivatives (w, omega_z; D w, D^2 w, D omega_z), then the six
-  // fields in the transform's precision, ready for the even extension
-  // (c_0, c_n / 2), two in the lines of the warp that transforms them
-  // (u, v | w, omega_x | omega_y, omega_z), which its first FFT pass reads
-  // before it writes the lines
-  constexpr int MW = wlen<C>(M);
-  C* lines = (C*)smem_raw;
-  constexpr size_t VS = (Ny * 16 + 15) / 16;             // FP64 vector slot (double2)
-  constexpr size_t FS = (Ny * sizeof(C) + 15) / 16 * 16;  // field slot (bytes)
-  static_assert(2 * VS * 16 + 2 * FS <= (size_t)2 * MW * sizeof(C), "vectors do not fit the lines");
-  unsigned char* rb0 = (unsigned char*)lines;
-  unsigned char* rb1 = (unsigned char*)(lines + (size_t)2 * MW);
-  unsigned char* rb2 = (unsigned char*)(lines + (size_t)4 * MW);
-  double2 *Dw = (double2*)rb0, *D2w = Dw + VS, *w = (double2*)rb1, *Doz = w + VS, *oz = (double2*)rb2;
-  C* fu = (C*)(rb0 + 2 * VS * 16);
-  C* fv = (C*)(rb0 + 2 * VS * 16 + FS);
-  C* fw = (C*)(rb1 + 2 * VS * 16);
-  C* fox = (C*)(rb1 + 2 * VS * 16 + FS);
-  C* foy = (C*)(rb2 + 2 * VS * 16);
-  C* foz = (C*)(rb2 + 2 * VS * 16 + FS);
+  typedef Dct<C, M, 6> D;
+  constexpr int Ny = M / 4 + 1, Py = M / 2 + 1;  // the launcher checks g.Ny, g.Py against M
+  // derivatives in double2, or float2 where they feed FP32 transforms only
+  typedef typename std::conditional<sizeof(C) == 8, float2, double2>::type E;
+  typedef T_of<E> S;
+  constexpr int FS = (Ny + 1) & ~1;  // field stride
+  C* fld = (C*)smem_raw;             // six fields
+  unsigned char* rb = smem_raw + (size_t)6 * FS * sizeof(C);
+  double2 *w = (double2*)rb, *oz = w + FS;
+  E* eDw = (E*)(oz + FS);
+  E *eD2w = eDw + FS, *eDoz = eD2w + FS, *ew = (E*)w, *eoz = (E*)oz;
+  C* X = (C*)rb;
   const long long p = blockIdx.x;
   int run, kx, kz;
   pencil_modes(g, p, run, kx, kz);
@@ -495,7 +492,6 @@ __global__ void __launch_bounds__(96) k_y3w(const double2* __restrict__ V, const
   // the pencil's wavenumbers and 1 / k^2: the FP64 divisions once per CTA
   // (thread 0, under the copies), shared through shared memory
   __shared__ double pen[3];
-  // twiddles and the pencil's state by bulk copies on one barrier
   __shared__ uint64_t bar;
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
@@ -522,46 +518,39 @@ __global__ void __launch_bounds__(96) k_y3w(const double2* __restrict__ V, const
   // linearity, u = i(ia Dw - ib oz)/k^2, v = i(ib Dw + ia oz)/k^2 and their
   // derivatives from D^2 w, D oz (source/velocity.cu:90-170).  The mean
   // mode holds u0, w0 in (w, oz): u = w, v = oz, omega_x = D oz, omega_y = -D w.
-  // The FP32 form takes the state to FP32 first and forms the velocities
-  // and vorticities in FP32: they feed FP32 transforms only.
-  typedef typename std::conditional<sizeof(C) == 8, float2, double2>::type E;
-  typedef T_of<E> S;
-  E *ew = (E*)w, *eDw = (E*)Dw, *eD2w = (E*)D2w, *eoz = (E*)oz, *eDoz = (E*)Doz;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if constexpr (sizeof(C) == 8) {
-    // in place: element n of the FP32 copy lies below element n of the
-    // FP64 vector, so the conversion runs in one pass per warp
-    const int warp0 = threadIdx.x >> 5, lane0 = threadIdx.x & 31;
-    if (warp0 < 2) {
-      const double2* src = warp0 ? oz : w;
-      E* dst = warp0 ? eoz : ew;
-      for (int n0 = 0; n0 < Ny; n0 += 32) {
-        const int n = n0 + lane0;
-        const double2 x = n < Ny ? src[n] : make_double2(0.0, 0.0);
-        __syncwarp();
-        if (n < Ny) dst[n] = make_float2((float)x.x, (float)x.y);
-      }
+    // to FP32 in place: element n of the FP32 copy lies below element n of
+    // the FP64 vector, so the conversion runs in one pass per warp
+    const double2* src = warp ? oz : w;
+    E* dst = warp ? eoz : ew;
+    for (int n0 = 0; n0 < Ny; n0 += 32) {
+      const int n = n0 + lane;
+      const double2 x = n < Ny ? src[n] : make_double2(0.0, 0.0);
+      __syncwarp();
+      if (n < Ny) dst[n] = make_float2((float)x.x, (float)x.y);
     }
-    __syncthreads();
+    __syncwarp();
   }
-  const int warp = threadIdx.x >> 5;
   constexpr int CH = ddz_run(Ny);
   if (warp == 0) {
     ddz_fast<CH, E>(ew, eDw, Ny);
     __syncwarp();
     if (!zero) ddz_fast<CH, E>(eDw, eD2w, Ny);
-  } else if (warp == 1) {
+  } else {
     ddz_fast<CH, E>(eoz, eDoz, Ny);
   }
   __syncthreads();
   const S sia = (S)(ia * kmn1), sib = (S)(ib * kmn1), fia = (S)ia, fib = (S)ib;
-  for (int n = threadIdx.x; n < Ny; n += blockDim.x) {
-    const E wn = ew[n], on = eoz[n], d1 = eDw[n], dz = eDoz[n];
-    E u, v, ox, oy;
+  for (int n = threadIdx.x; n < Ny; n += 64) {
+    E wn = ew[n], on = eoz[n], u, v, ox, oy;
+    const E d1 = eDw[n], dz = eDoz[n];
     if (zero) {
       u = wn;
       v = on;
       ox = dz;
       oy = cmk<E>(-d1.x, -d1.y);
+      wn = on = cmk<E>(0.0, 0.0);  // w and omega_z vanish for the mean mode
     } else {
       const E d2 = eD2w[n];
       u = muli(d1 * sia) - muli(on * sib);
@@ -572,38 +561,20 @@ __global__ void __launch_bounds__(96) k_y3w(const double2* __restrict__ V, const
       oy = muli(wn * fia) - du;
     }
     const S h = n ? (S)0.5 : (S)1.0;  // even extension: c_0, then c_n / 2
-    fu[n] = from_e<C>(u * h);
-    fv[n] = from_e<C>(v * h);
-    fw[n] = from_e<C>(wn * h);
-    fox[n] = from_e<C>(ox * h);
-    foy[n] = from_e<C>(oy * h);
-    foz[n] = from_e<C>(on * h);
+    fld[n] = from_e<C>(u * h);
+    fld[FS + n] = from_e<C>(v * h);
+    fld[2 * FS + n] = from_e<C>(wn * h);
+    fld[3 * FS + n] = from_e<C>(ox * h);
+    fld[4 * FS + n] = from_e<C>(oy * h);
+    fld[5 * FS + n] = from_e<C>(on * h);
   }
   __syncthreads();
-  // this warp's two lines: fields 2 warp, 2 warp + 1; the first FFT pass
-  // reads the even extensions e[0] = c_0, e[n] = e[M-n] = c_n / 2 (n < Ny),
-  // zero elsewhere, the last one writes the Py values
-  C* wl = lines + (size_t)2 * warp * MW;
-  const C* s0 = (warp == 0) ? fu : (warp == 1 ? fw : foy);
-  const C* s1 = (warp == 0) ? fv : (warp == 1 ? fox : foz);
-  // w (line 2) and omega_z (line 5) vanish for the mean mode
-  const bool z0 = zero && warp == 1, z1 = zero && warp == 2;
-  auto ld = [&](int l, int n) -> C {
-    const C* src = l ? s1 : s0;
-    C e = cmk<C>(0.0, 0.0);
-    if (!(l ? z1 : z0)) {
-      if (n < Ny) e = src[n];
-      else if (n > M - Ny) e = src[M - n];
-    }
-    return e;
-  };
-  constexpr int Py = M / 2 + 1;
-  C* d0 = pencil_ptr<C>(out, 2 * warp, p);
-  C* d1 = pencil_ptr<C>(out, 2 * warp + 1, p);
-  auto st = [&](int l, int k, C val) {
-    if (k < Py) (l ? d1 : d0)[k] = val;
-  };
-  wfft_io<C, M, 2, false>(wl, wtw_of(tab, 1), ld, st);
+  for (int i = threadIdx.x; i < D::IA; i += 64)
+    D::template pass_a<Ny>(X, i, [&](int l, int n) { return fld[l * FS + n]; });
+  __syncthreads();
+  C* dst = pencil_ptr<C>(out, 0, p);
+  for (int i = threadIdx.x; i < D::IB; i += 64)
+    D::pass_b(X, dt, i, [&](int l, int k, C v) { dst[l * out.fs + k] = v; });
 }
 
 // ---------------------------------------------------------------------------
@@ -1163,27 +1134,39 @@ cudaError_t launch_solve_eq(const double2* inv, double2* rhs, long long ps, int 
   return cudaGetLastError();
 }
 
+#define DNS_DCASE(n) case n: return f(std::integral_constant<int, n>());
+template <typename F> cudaError_t with_len_d(int M, F&& f) {
+  switch (M) { DPLAN_LENGTHS(DNS_DCASE) }
+  return cudaErrorNotSupported;
+}
+
 template <typename C>
 cudaError_t launch_y3(const double2* V, const double2* O, PencilArr out, DnsGeom g,
                       PhysParams ph, FftTab<C> tab, int* status, cudaStream_t st, int variant, bool probe) {
   const bool any = variant == VAR_AUTO;
   // the warp form stages its inputs by bulk copies (16-byte aligned
   // sources) and takes Ny = M/4 + 1, Py = M/2 + 1 as compile-time constants
-  const bool bulk_ok = aligned16(V) && aligned16(O) && wtw_of(tab, 1) &&
-                       g.Ny == tab.plan.L / 4 + 1 && g.Py == tab.plan.L / 2 + 1;
+  if ((any || variant == DNS_Y3_FFT) && aligned16(V) && aligned16(O) && tab.dt && g.Ny == tab.plan.L / 4 + 1 &&
+      g.Py == tab.plan.L / 2 + 1) {
+    const cudaError_t e = with_len_d(tab.plan.L, [&](auto MM) -> cudaError_t {
+      constexpr int M = decltype(MM)::value;
+      typedef Dct<C, M, 6> D;
+      if (probe) return cudaSuccess;
+      constexpr int FS = (M / 4 + 2) & ~1;
+      constexpr size_t es = sizeof(C) == 8 ? 8 : 16, vec = (size_t)FS * (2 * 16 + 3 * es), ex = D::XN * sizeof(C);
+      const size_t sm = (size_t)6 * FS * sizeof(C) + (vec > ex ? vec : ex);
+      constexpr int MB = sizeof(C) == 8 ? (D::RA > 18 ? 8 : 12) : (D::RA > 24 ? 4 : (D::RA > 18 ? 6 : 8));
+      auto k = k_y3d<C, M, MB>;
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      k<<<(unsigned)g.H, 64, sm, st>>>(V, O, out, g, ph, tab.dt, status);
+      return cudaGetLastError();
+    });
+    if (e != cudaErrorNotSupported) return e;
+  }
+  if (!any && variant != DNS_Y3_BLOCK) return cudaErrorNotSupported;
+  if (probe) return cudaSuccess;
   return with_len_m(tab.plan.L, [&](auto LL) -> cudaError_t {
     constexpr int L = decltype(LL)::value;
-    if constexpr (L > 0 && WPlan<L, 2, FftMaxRadix<C>::v>::ok) {
-     if ((any || variant == DNS_Y3_FFT) && bulk_ok) {
-      if (probe) return cudaSuccess;
-      const size_t sm = (size_t)6 * wlen<C>(L) * sizeof(C);
-      cudaFuncSetAttribute(k_y3w<C, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_y3w<C, L><<<(unsigned)g.H, 96, sm, st>>>(V, O, out, g, ph, tab, status);
-      return cudaGetLastError();
-     }
-    }
-    if (!any && variant != DNS_Y3_BLOCK) return cudaErrorNotSupported;
-    if (probe) return cudaSuccess;
     const size_t sm = y3_smem(g.Ny, FLine<C, L>::stride(tab.plan.L), sizeof(C));
     cudaFuncSetAttribute(k_y3<C, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     k_y3<C, L><<<(unsigned)g.H, 256, sm, st>>>(V, O, out, g, ph, tab);
