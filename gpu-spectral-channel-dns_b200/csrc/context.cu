@@ -69,19 +69,18 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
     dr[j] = (short)fft_digitrev(f.plan, j);
   }
   const size_t otw = put(tw.data(), sizeof(C) * L), odr = put(dr.data(), sizeof(short) * L);
-  // twiddle tables where the length has a plan: FP32 warp FFTs (1, 2 lines
+  // twiddle tables where the length has a plan: FP32 warp FFTs (two lines
   // per warp) and the fused streamwise form, both precisions the two-pass
   // spanwise form and the pruned DCT
   const bool f32 = std::is_same<C, float2>::value;
   const size_t none = ~(size_t)0;
-  size_t off[5] = {none, none, none, none, none};
+  size_t off[4] = {none, none, none, none};
   std::vector<C> t;
-  for (int i = 0; i < 5; ++i) {
-    if (i < 3 && !f32) continue;
-    const int n = i == 0 ? wtw_table_any<C, 1>(L, t)
-                : i == 1 ? wtw_table_any<C, 2>(L, t)
-                : i == 2 ? xtw_table<C>(L, t)
-                : i == 3 ? ztw_table<C>(L, t) : dtw_table<C>(L, t);
+  for (int i = 0; i < 4; ++i) {
+    if (i < 2 && !f32) continue;
+    const int n = i == 0 ? wtw_table_any<C, 2>(L, t)
+                : i == 1 ? xtw_table<C>(L, t)
+                : i == 2 ? ztw_table<C>(L, t) : dtw_table<C>(L, t);
     if (n > 0) off[i] = put(t.data(), sizeof(C) * n);
   }
   cudaError_t e = cudaMalloc(&f.mem, h.size());
@@ -90,11 +89,10 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
   auto at = [&](size_t o) { return o == none ? nullptr : (C*)(f.mem + o); };
   f.tw = at(otw);
   f.drev = (short*)(f.mem + odr);
-  f.wt[0] = at(off[0]);
-  f.wt[1] = at(off[1]);
-  f.xt = at(off[2]);
-  f.zt = at(off[3]);
-  f.dt = at(off[4]);
+  f.wt = at(off[0]);
+  f.xt = at(off[1]);
+  f.zt = at(off[2]);
+  f.dt = at(off[3]);
   return cudaSuccess;
 }
 template <typename C> void free_fft(DevFft<C>& f) {
@@ -248,10 +246,7 @@ cudaError_t enqueue_pipeline(dns_ctx* c, int boot, const DevFft<C>& fz, const De
     return e;
   mark();
   const RhsDims rd{c->wd.nv, c->wd.no, c->wd.gp};
-  const size_t nv = c->wd.nv, no = c->wd.no;
-  const double* t0 = c->rtab;
-  const RhsTabs tb{t0, t0 + 4 * nv, t0 + 4 * nv + 2 * no, t0 + 4 * nv + 2 * no + g.Ny,
-                   t0 + 4 * nv + 2 * no + g.Ny + 5 * nv};
+  const RhsTabs tb = RhsLayout(g.Ny, c->wd.nv, c->wd.no).at(c->rtab);
   if ((e = var(DNS_PASS_Y1, [&](int v) {
          return launch_y1<C>(F3y, b.V, b.O, b.Nvp, b.Nop, c->rv, c->ro, rd, tb, gb, c->ph, fyP.tab(), boot,
                              c->status, c->st, v);
@@ -531,7 +526,7 @@ dns_status ctx_create(const dns_params* p, SlabState* slab, dns_ctx** out, int n
       (e = c->alloc(&c->ro, gn)) || (e = c->alloc(&c->status, 1)) ||
       (e = c->alloc((unsigned char**)&c->F6, c->F6_bytes = f6 * csz)) ||
       (e = c->alloc((unsigned char**)&c->G6, g6 * csz)) ||
-      (e = c->alloc(&c->rtab, 4 * (size_t)c->wd.nv + 2 * (size_t)c->wd.no + Ny + 8 * (size_t)c->wd.nv)) ||
+      (e = c->alloc(&c->rtab, RhsLayout(Ny, c->wd.nv, c->wd.no).end)) ||
       (sl && (e = c->alloc((unsigned char**)&sl->A,
                            std::max((size_t)6 * g.H * sl->nyS, (size_t)3 * sl->ny * g.Pz * c->KxS) * csz))))
     return bail(fail(DNS_ERR_CUDA, std::string("device allocation: ") + cudaGetErrorString(e)));
@@ -543,26 +538,31 @@ dns_status ctx_create(const dns_params* p, SlabState* slab, dns_ctx** out, int n
   cudaMemcpy(c->ddUt, ddU.data(), Ny * 8, cudaMemcpyHostToDevice);
   cudaMemcpy(c->Uy, Uy.data(), g.Py * 8, cudaMemcpyHostToDevice);
   {
-    // y1 tables (integrated cardinal corrections, cos(k pi/N))
+    // y1 tables (integrated cardinal corrections, cos(k pi/N), integration
+    // stencils, wall derivatives)
     const int N = Ny - 1, nv = c->wd.nv, no = c->wd.no;
-    std::vector<double> tab(4 * (size_t)nv + 2 * (size_t)no + Ny + 8 * (size_t)nv);
+    const RhsLayout lay(Ny, nv, no);
+    std::vector<double> tab(lay.end);
     const int mv[4] = {0, 1, N - 1, N};
-    for (int m = 0; m < 4; ++m) wall::cardinal_rows(N, mv[m], 4, nv, &tab[(size_t)m * nv]);
-    wall::cardinal_rows(N, 0, 2, no, &tab[4 * (size_t)nv]);
-    wall::cardinal_rows(N, N, 2, no, &tab[4 * (size_t)nv + no]);
+    for (int m = 0; m < 4; ++m) wall::cardinal_rows(N, mv[m], 4, nv, &tab[lay.bkcv + (size_t)m * nv]);
+    wall::cardinal_rows(N, 0, 2, no, &tab[lay.bkco]);
+    wall::cardinal_rows(N, N, 2, no, &tab[lay.bkco + no]);
     const long double PI = 3.141592653589793238462643383279502884L;
-    for (int k = 0; k <= N; ++k) tab[4 * (size_t)nv + 2 * (size_t)no + k] = (double)cosl(PI * k / N);
-    // rows of B^4 (from row 4) and B^2 (from row 2) as 5- and 3-point
-    // stencils, stored weight-major ([d][r]: a warp's rows read consecutive
-    // entries)
-    std::vector<double> s4((size_t)5 * nv), s2((size_t)3 * nv);
-    wall::integration_stencils(N, nv, s4.data(), s2.data());
-    double* b4 = &tab[4 * (size_t)nv + 2 * (size_t)no + Ny];
-    double* b2 = b4 + 5 * (size_t)nv;
+    for (int k = 0; k <= N; ++k) tab[lay.cosk + k] = (double)cosl(PI * k / N);
+    // rows of B^4 and B^3 (from row 4) and B^2 (from row 2) as 5-, 4- and
+    // 3-point stencils, stored weight-major ([d][r]: a warp's rows read
+    // consecutive entries); columns to N + 2, the degree of U v
+    const int n2 = nv + 2;
+    std::vector<double> s4((size_t)5 * n2), s2((size_t)3 * n2), s3((size_t)4 * nv);
+    wall::integration_stencils(N + 2, n2, s4.data(), s2.data());
+    wall::integration_stencil3(N + 2, nv, s3.data());
+    for (int r = 0; r < n2; ++r)
+      for (int d = 0; d < 3; ++d) tab[lay.b2 + (size_t)d * n2 + r] = s2[(size_t)3 * r + d];
     for (int r = 0; r < nv; ++r) {
-      for (int d = 0; d < 5; ++d) b4[(size_t)d * nv + r] = s4[(size_t)5 * r + d];
-      for (int d = 0; d < 3; ++d) b2[(size_t)d * nv + r] = s2[(size_t)3 * r + d];
+      for (int d = 0; d < 5; ++d) tab[lay.b4 + (size_t)d * nv + r] = s4[(size_t)5 * r + d];
+      for (int d = 0; d < 4; ++d) tab[lay.b3 + (size_t)d * nv + r] = s3[(size_t)4 * r + d];
     }
+    wall::wall_derivatives(N, &tab[lay.tw]);
     cudaMemcpy(c->rtab, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice);
   }
   if (nrun > 1) {
@@ -1180,7 +1180,7 @@ cudaError_t enqueue_solve_wall(dns_ctx* c, const double2* bv, const double2* bo,
   const long long ls = c->P.mz / 2;  // no-padding DCT-I length 2N
   double2* sv = (double2*)c->F6;
   double2* so = sv + g.H * ls;
-  const double* cosk = c->rtab + 4 * (size_t)c->wd.nv + 2 * (size_t)c->wd.no;
+  const double* cosk = c->rtab + RhsLayout(g.Ny, c->wd.nv, c->wd.no).cosk;
   // one kernel where the DCT length has a warp plan, else three
   cudaError_t e = launch_colloc_fused(bv, bo, bp, pbc, cosk, c->Ut, c->ddUt, c->rv, c->ro, c->wd, g, c->ph,
                                       c->fy0_d.tab(), c->status, c->st);

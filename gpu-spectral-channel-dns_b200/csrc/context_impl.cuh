@@ -13,14 +13,13 @@ template <typename C> struct DevFft {
   unsigned char* mem = nullptr;  // holds the tables below
   C* tw = nullptr;
   short* drev = nullptr;
-  C* wt[2] = {nullptr, nullptr};
-  C *dt = nullptr, *xt = nullptr, *zt = nullptr;
+  C *wt = nullptr, *dt = nullptr, *xt = nullptr, *zt = nullptr;
   FftTab<C> tab() const {
     FftTab<C> t;
     t.plan = plan;
     t.tw = tw;
     t.drev = drev;
-    for (int i = 0; i < 2; ++i) t.wt[i] = wt[i];
+    t.wt = wt;
     t.dt = dt;
     t.xt = xt;
     t.zt = zt;
@@ -65,7 +64,7 @@ struct dns_ctx {
   double2* wfac = nullptr;
   double* wQ = nullptr;
   WallDims wd{};
-  double* rtab = nullptr;  // y1 tables: B^4 C_m (4 x nv), B^2 C_m (2 x no), cos(k pi/N)
+  double* rtab = nullptr;  // y1 tables (RhsLayout)
   void* F6 = nullptr;  // also the wall solve's scratch (free while it runs)
   void* G6 = nullptr;
   size_t F6_bytes = 0;

@@ -20,17 +20,11 @@ template <typename C> struct FftTab {
   FftPlan plan;
   const C* tw;          // W_L^j, j < L
   const short* drev;    // digit-reversed position of natural index n
-  const C* wt[2];       // FP32 warp-FFT twiddle tables of the plans with 1, 2 lines per warp
+  const C* wt;          // FP32 warp-FFT twiddles of the plan with two lines per warp
   const C* dt;          // twiddles of the pruned DCT (ydct.cuh), null for lengths without one
   const C* xt;          // FP32 twiddles of the fused streamwise form (xpass.cuh)
   const C* zt;          // twiddles of the two-pass spanwise form (zpass.cuh), null for lengths without one
 };
-
-// twiddles of a warp-FFT plan: FP32, the plan's own table (lines per warp
-// 1, 2 -> i = 0, 1); FP64, W_L^j and product recurrences
-template <typename C> DNS_HD const C* wtw_of(const FftTab<C>& t, int i) {
-  return sizeof(C) == 16 ? t.tw : t.wt[i];
-}
 
 // Pass launchers take a variant (the DNS_Y3_*, DNS_Y1_*, DNS_Z_* values of
 // the public header) or VAR_AUTO, the first form the arguments allow in the

@@ -167,10 +167,7 @@ cudaError_t part_y1(dns_ctx* c, int boot, const void* recv) {
   cudaError_t e = move_segments(c, S.segP, 3, (void*)recv, c->F6, c->PyS, S.np * c->PyS, true, false);
   if (e) return e;
   const RhsDims rd{c->wd.nv, c->wd.no, c->wd.gp};
-  const size_t nv = c->wd.nv, no = c->wd.no;
-  const double* t0 = c->rtab;
-  const RhsTabs tb{t0, t0 + 4 * nv, t0 + 4 * nv + 2 * no, t0 + 4 * nv + 2 * no + g.Ny,
-                   t0 + 4 * nv + 2 * no + g.Ny + 5 * nv};
+  const RhsTabs tb = RhsLayout(g.Ny, c->wd.nv, c->wd.no).at(c->rtab);
   for (int k = 0; k < S.nruns && !e; ++k) {
     const SlabRun& run = S.run[k];
     DnsGeom gs = g;

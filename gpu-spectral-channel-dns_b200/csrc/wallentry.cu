@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(64, 16) k_colloc_fused(const double2* __restri
   auto st = [&](int, int k, double2 v) {
     if (k <= N) line[k] = v * ((k == 0 || k == N) ? 0.5 / N : 1.0 / N);
   };
-  wfft_io<double2, L, 1, false>(line, wtw_of(tab, 0), ld, st, LS);
+  wfft_io<double2, L, 1, false>(line, tab.tw, ld, st, LS);
   __syncwarp();
   for (int k = Ny + lane; k < LB; k += 32) line[k] = cx(0, 0);
   // K-fold integration: (B x)_k = (c_{k-1} x_{k-1} - x_{k+1}) / (2k), (B x)_0 = 0;

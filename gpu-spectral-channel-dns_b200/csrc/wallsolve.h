@@ -99,6 +99,11 @@ void cardinal_rows(int N, int m, int K, int n, double* out);
 // vector f: (B^4 f)_{r+4} = sum_d b4[5r + d/2 + 2] f_{r+4+d}, d = -4,-2,0,2,4;
 // (B^2 f)_{r+2} = sum_d b2[3r + d/2 + 1] f_{r+2+d}, d = -2,0,2.
 void integration_stencils(int N, int n, double* b4, double* b2);
+// the same for rows 4.. of B^3: (B^3 f)_{r+4} = sum_t b3[4r + t] f_{r+4+2t-3}
+void integration_stencil3(int N, int n, double* b3);
+// second and fourth derivatives of T_k, k = 0..N: out[0..3][k] = second at
+// y = 1, fourth at y = 1, second and fourth at y_1 = cos(pi/N)
+void wall_derivatives(int N, double* out);
 
 // Chebyshev coefficients (N+1) from basis unknowns: v or Dirichlet recombination
 void recombine(int eq, int N, const cx* x, cx* a);

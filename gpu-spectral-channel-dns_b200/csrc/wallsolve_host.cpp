@@ -343,6 +343,36 @@ void integration_stencils(int N, int n, double* b4, double* b2) {
   }
 }
 
+void integration_stencil3(int N, int n, double* b3) {
+  std::fill(b3, b3 + (size_t)4 * n, 0.0);
+  const size_t m = (size_t)N + n + 12;
+  for (int k = 0; k <= N; ++k) {
+    Vec e(m, 0.0);
+    e[k] = 1.0;
+    const Vec e3 = int_B_pow(e, 3);
+    for (int r = 0; r < n; ++r) {
+      const int d = k - (r + 4) + 3;
+      if (d >= 0 && d <= 6 && (d & 1) == 0) b3[(size_t)4 * r + d / 2] = e3[r + 4];
+    }
+  }
+}
+
+void wall_derivatives(int N, double* out) {
+  const long double y1 = cosl(3.141592653589793238462643383279502884L / N);
+  for (int p = 0; p < 2; ++p) {
+    // m-th derivatives: T_{k+1} = 2 y T_k + 2 m (T_k, m - 1) - T_{k-1}
+    const long double y = p ? y1 : 1.0L;
+    long double a[5] = {1.0L, 0, 0, 0, 0}, b[5] = {y, 1.0L, 0, 0, 0};
+    for (int k = 0; k <= N; ++k) {
+      out[(size_t)(2 * p) * (N + 1) + k] = (double)a[2];
+      out[(size_t)(2 * p + 1) * (N + 1) + k] = (double)a[4];
+      long double c[5];
+      for (int d = 0; d < 5; ++d) c[d] = 2 * y * b[d] + (d ? 2 * d * b[d - 1] : 0.0L) - a[d];
+      for (int d = 0; d < 5; ++d) { a[d] = b[d]; b[d] = c[d]; }
+    }
+  }
+}
+
 void recombine(int eq, int N, const cx* x, cx* a) {
   const int nb = (eq == EQ_V) ? N - 3 : N - 1;
   auto b = [&](int j) { return (j >= 0 && j < nb) ? x[j] : cx{0, 0}; };

@@ -15,6 +15,14 @@
 #include "fft2.cuh"
 #include "kernels.cuh"
 
+// index range hints (resolve, per compile-time r, which branch of a load or
+// store applies)
+#ifdef __CUDA_ARCH__
+#define YDCT_ASSUME(c) __builtin_assume(c)
+#else
+#define YDCT_ASSUME(c) ((void)0)
+#endif
+
 template <int M> struct DPlan { enum { ok = 0, A = 2, B = 2 }; };
 #define DPLAN(M, RA, RB)                                                                      \
   template <> struct DPlan<M> {                                                               \
@@ -75,6 +83,7 @@ template <typename C, int M, int NL> struct Dct {
   // e[n] = 0 for n0 <= n <= M/2
   template <int N0, class LD> DNS_HD static void pass_a(C* X, int i, LD ld) {
     const int l = i / JH, j = i - l * JH;
+    YDCT_ASSUME(j >= 0 && j < JH);
     C v[RA];
 #pragma unroll
     for (int r = 0; r < RA; ++r) {
@@ -100,6 +109,7 @@ template <typename C, int M, int NL> struct Dct {
   // (some twice, with equal values)
   template <class ST> DNS_HD static void pass_b(const C* X, const C* tw, int i, ST st) {
     const int l = i / SH, s = i - l * SH;
+    YDCT_ASSUME(s >= 0 && s < SH);
     const C* xs = X + s * XP + l * JH;
     const C* xm = X + (s ? RA - s : 0) * XP + l * JH;
     C v[RB];

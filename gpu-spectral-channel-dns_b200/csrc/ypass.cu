@@ -20,7 +20,6 @@
 #include "fftline.cuh"
 #include "kernels.cuh"
 #include "mbar.cuh"
-#include "wfft.cuh"
 #include "ydct.cuh"
 #include "ypass.cuh"
 
@@ -117,60 +116,6 @@ __device__ __noinline__ void ddz_fast(const E* __restrict__ a, E* __restrict__ b
   }
 }
 
-// Second derivative of a Chebyshev series by one warp in one sweep, CH
-// (even) coefficients per lane: b_i = (1 / c_i) sum_{j >= i+2, j - i even}
-// j (j^2 - i^2) a_j (c_0 = 2, else 1), the composition of two ddz_warp
-// steps, as parity-split suffix sums of j a_j and j^3 a_j.  The lane's run
-// is read twice from shared memory rather than held in registers.
-template <int CH>
-__device__ __noinline__ void d2z_fast(const double2* __restrict__ a, double2* __restrict__ b, int N) {
-  static_assert(CH % 2 == 0, "runs of even length");
-  const int lane = threadIdx.x & 31;
-  const int j0 = lane * CH;
-  double t[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // (j a_j, j^3 a_j) x (even, odd j), re / im
-#pragma unroll
-  for (int i = 0; i < CH; ++i) {
-    if (j0 + i < N) {
-      const double2 v = a[j0 + i];
-      const double j = (double)(j0 + i), j3 = j * j * j;
-      const int o = (i & 1) * 4;
-      t[o + 0] += j * v.x;
-      t[o + 1] += j * v.y;
-      t[o + 2] += j3 * v.x;
-      t[o + 3] += j3 * v.y;
-    }
-  }
-  // inclusive suffix sums over the lanes, then those of the lanes above
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const double x = __shfl_down_sync(0xffffffffu, t[k], d);
-      if (lane + d < 32) t[k] += x;
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const double x = __shfl_down_sync(0xffffffffu, t[k], 1);
-    t[k] = lane < 31 ? x : 0.0;
-  }
-#pragma unroll
-  for (int i = CH - 1; i >= 0; --i) {
-    const int jj = j0 + i;
-    if (jj < N) {
-      const double j = (double)jj, j2 = j * j;
-      const int o = (i & 1) * 4;  // j' >= j + 2 of the same parity
-      double2 out = make_double2(t[o + 2] - j2 * t[o + 0], t[o + 3] - j2 * t[o + 1]);
-      if (jj == 0) out = out * 0.5;
-      const double2 v = a[jj];
-      b[jj] = out;
-      t[o + 0] += j * v.x;
-      t[o + 1] += j * v.y;
-      t[o + 2] += j * j2 * v.x;
-      t[o + 3] += j * j2 * v.y;
-    }
-  }
-}
 // lanes' run length for Ny coefficients
 __host__ __device__ constexpr int ddz_run(int Ny) { return 2 * ((Ny + 63) / 64); }
 
@@ -467,7 +412,8 @@ __global__ void __launch_bounds__(256, 3) k_y3(const double2* __restrict__ V, co
 // What bounds it: with whole 3-pass FFTs of the even extensions the pass moved
 // each of 512 values of a line five times through shared memory and spent its
 // issue slots on the redundant half; the two pruned passes move 0.56 of them
-// once.  Measured, FP64: see launch_y3.
+// once.  FP64 256 x 129 x 256 440 -> 301 us, 128 x 65 x 128 65 -> 50; mixed
+// 144 x 55 x 72, a length on the block form before, 126 -> 19.
 template <typename C, int M, int MB>
 __global__ void __launch_bounds__(64, MB) k_y3d(const double2* __restrict__ V, const double2* __restrict__ O,
                                                PencilArr out, DnsGeom g, PhysParams ph, const C* __restrict__ dt,
@@ -621,31 +567,6 @@ __device__ __forceinline__ double2 umul_gl(const double2* X, int k, int N, const
   auto u = [&](int j) {
     double2 r = cget(X, j, N) * ph.U0 + ymul(X, j, N) * ph.U1;
     if (quad) r = r + y2mul(X, j, N) * ph.U2;
-    return r;
-  };
-  double2 r = u(k);
-  if (k == N - 1 || k == N - 2) r = r + u(2 * N - k);
-  return r;
-}
-// the same for X given element-wise by a functor (X(j) for 0 <= j <= N):
-// one interpolant of a combination in place of a combination of interpolants
-template <class F>
-__device__ __forceinline__ double2 umul_fn(F X, int k, int N, const PhysParams& ph) {
-  const double2 z = make_double2(0.0, 0.0);
-  auto xm = [&](int j) { return (j >= 0 && j <= N) ? X(j) : z; };
-  auto ym = [&](int j) {
-    if (j < 0) return z;
-    if (j == 0) return xm(1) * 0.5;
-    return (xm(j - 1) * (j == 1 ? 2.0 : 1.0) + xm(j + 1)) * 0.5;
-  };
-  auto u = [&](int j) {
-    double2 r = xm(j) * ph.U0 + ym(j) * ph.U1;
-    if (ph.U2 != 0.0) {
-      const double2 y2 = (j < 0) ? z
-                         : (j == 0) ? ym(1) * 0.5
-                                    : (ym(j - 1) * (j == 1 ? 2.0 : 1.0) + ym(j + 1)) * 0.5;
-      r = r + y2 * ph.U2;
-    }
     return r;
   };
   double2 r = u(k);
@@ -866,43 +787,94 @@ __global__ void __launch_bounds__(256, 3) k_y1(PencilArr lam, const double2* __r
   }
 }
 
-// Same pass with warp FFTs: warps 0-2 transform one Lamb line each (0 and 1
-// also differentiate theirs), while warp 3 forms D^2 v and D^4 v (two
-// second-derivative sweeps) and warp 4 D^2 omega_y; no block barrier inside
-// the transforms.
-template <typename C, int M>
-__global__ void __launch_bounds__(160, sizeof(C) == 8 ? 6 : 4) k_y1w(PencilArr lam, const double2* __restrict__ V,
+// Same pass with the three lines as pruned DCTs (ydct.cuh) on warps 0 and 1
+// (which then differentiate lambda_x and lambda_y), the parts of the
+// right-hand sides that need the state only on warps 2 and 3 meanwhile.
+//
+// The integrated right-hand side is formed without D^2 v and D^4 v.  From row
+// 4 on, B^4 D^4 v = v and B^4 D^2 v = B^2 v, and
+//   U D^2 v = D^2 (U v) - 2 D (U' v) + U'' v
+// (degree <= N: its interpolant is itself), so with h = dt / (2 Re), gam =
+// alpha dt / 2, P = U v (degree <= N + 2) and Pf its interpolant
+//   g = h v + B^2 [(1 - 2 k^2 h) v - i gam P] + B^3 [2 i gam U' v]
+//       + B^4 [-k^2 (1 - k^2 h) v + i gam k^2 Pf + dt (1.5 N - 0.5 N_p)]
+// (the two U'' terms cancel); for omega_y and the mean modes, from row 2 on,
+//   g = h o + B^2 [(1 - k^2 h) o - i gam (U o)f + i kap (U' v)f + dt (...)].
+// The values at the left-out points take the derivatives of T_k there; H_v
+// takes one derivative, of alpha lambda_x + beta lambda_y.
+//
+// What bounds it: issue slots (7055 warp instructions a pencil at M = 512
+// before, a fifth of them FP64), so vectors carry zero guards instead of
+// bounds checks, and the sums over k are halved between lanes at every
+// step.  4530 instructions; 256 x 129 x 256 mixed 383 -> 299 us, FP64 497 ->
+// 440; 128 x 65 x 128 FP64 107 -> 74; twelve 64 x 49 x 64 mixed 184 -> 115;
+// 144 x 55 x 72 mixed, a length on the block form before, 160 -> 33.
+namespace {
+// Sums over the 16 lanes of a parity of NV values a lane, halved at every
+// step: afterwards the lane holds the sum of value `idx` (idx >= NV: none).
+template <int NV>
+__device__ __forceinline__ double parity_sums(double (&v)[NV], int lane, int& idx) {
+  int n = NV;
+  idx = 0;
+#pragma unroll
+  for (int m = 16; m > 1; m >>= 1) {
+    const int half = (n + 1) / 2;
+    const bool up = lane & m;
+#pragma unroll
+    for (int i = 0; i < (NV + 1) / 2; ++i) {
+      if (i >= half) continue;
+      const double hi = i + half < n ? v[i + half] : 0.0;
+      const double send = up ? v[i] : hi, keep = up ? hi : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+    }
+    if (up) idx += half;
+    n = half;
+  }
+  return v[0];
+}
+// coefficient k of U X and, for k <= N, of its Gauss-Lobatto interpolant
+// (degrees N + 1, N + 2 fold to N - 1, N - 2); X has zeros below 0 and above N
+__device__ __forceinline__ void u_times(const double2* X, int k, int N, const PhysParams& ph, double2& P, double2& Pf) {
+  P = X[k] * ph.U0 + (X[k - 1] * (k == 1 ? 1.0 : 0.5) + X[k + 1] * 0.5) * ph.U1;
+  if (ph.U2 != 0.0)
+    P = P + (X[k - 2] * (k == 2 ? 0.5 : 0.25) + X[k] * (k == 1 ? 0.75 : 0.5) + X[k + 2] * 0.25) * ph.U2;
+  Pf = P;
+  if (k == N - 1) Pf = Pf + X[N] * (0.5 * ph.U1) + X[N - 1] * (0.25 * ph.U2);
+  if (k == N - 2) Pf = Pf + X[N] * (0.25 * ph.U2);
+}
+}  // namespace
+
+template <typename C, int M, int MB>
+__global__ void __launch_bounds__(128, MB) k_y1d(PencilArr lam, const double2* __restrict__ V,
                                             const double2* __restrict__ O, double2* Nvp,
                                             double2* Nop, double2* gv, double2* go, RhsDims rd,
                                             RhsTabs tb, DnsGeom g, PhysParams ph,
-                                            FftTab<C> tabP, int boot, int* status) {
+                                            const C* __restrict__ dct, int boot, int* status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  typedef Dct<C, M, 3> D;
   constexpr int Ny = M / 4 + 1;  // the launcher checks g.Ny, g.Py against M
   constexpr int Py = M / 2 + 1;
   constexpr int N = Ny - 1;
-  const int LB = Ny + 8;
+  constexpr int PS = (Py + 1) & ~1;      // staged Lamb pencil
+  constexpr int GU = 12, VL = Ny + GU;   // zero guards above N (two more below 0 for v and omega)
   Carve cv(smem_raw);
-  double2* Vc = cv.take<double2>(Ny);
-  double2* Oc = cv.take<double2>(Ny);
+  double2* Vc = cv.take<double2>(VL + 2) + 2;
+  double2* Oc = cv.take<double2>(VL + 2) + 2;
   double2* nvc = cv.take<double2>(Ny);
   double2* noc = cv.take<double2>(Ny);
-  double2* D2V = cv.take<double2>(Ny);
-  double2* D4V = cv.take<double2>(Ny);
-  double2* D2O = cv.take<double2>(Ny);
-  double2* red = cv.take<double2>(8);
-  const size_t bytesL = (size_t)3 * wlen<C>(M) * sizeof(C), bytesI = (size_t)4 * LB * 16;
-  unsigned char* region = cv.take<unsigned char>(bytesL > bytesI ? bytesL : bytesI);
-  C* lines = (C*)region;
-  // in the line buffer of warp w < 3, after its transform: the coefficients
-  // of lambda_w, then (w < 2) their derivative; fv and fo later take the
-  // slots of lambda_x, lambda_y element by element
-  constexpr size_t VS = (Ny * 16 + 15) / 16;  // vector slot (double2)
-  static_assert((size_t)2 * VS * 16 <= (size_t)wlen<C>(M) * sizeof(C), "vectors do not fit a line");
-  double2* lx = (double2*)lines;
-  double2* ly = (double2*)(lines + (size_t)wlen<C>(M));
-  double2* lz = (double2*)(lines + (size_t)2 * wlen<C>(M));
-  double2* D1x = lx + VS;
-  double2* D1y = ly + VS;
+  double2* S2 = cv.take<double2>(VL);  // under B^2
+  double2* S4 = cv.take<double2>(VL);  // under B^4 (mean modes: B^2)
+  double2* T2 = cv.take<double2>(VL);  // omega: under B^2
+  double2* red = cv.take<double2>(6);  // right-hand sides at the left-out points: v 1, y_1, -y_1, -1; omega 1, -1
+  double* accA = cv.take<double>(2 * 2 * 10);  // [warp - 2][parity][value]: derivatives of the state there
+  double* accB = cv.take<double>(4 * 2 * 6);   // [warp][parity][value]: the rest there
+  // the staged Lamb pencils, then the coefficients of lambda; the exchange of
+  // the transform, then alpha lambda_x + beta lambda_y and its derivative
+  constexpr size_t LB = sizeof(C) * 3 * PS, LC = (size_t)16 * 3 * Ny, XB = sizeof(C) * D::XN, XD = (size_t)16 * 2 * Ny;
+  C* stg = (C*)cv.take<unsigned char>(LB > LC ? LB : LC);
+  C* X = (C*)cv.take<unsigned char>(XB > XD ? XB : XD);
+  double2 *lx = (double2*)stg, *ly = lx + Ny, *lz = ly + Ny;
+  double2 *q = (double2*)X, *Dq = q + Ny;
 
   const long long p = blockIdx.x;
   int run, kx, kz;
@@ -913,16 +885,14 @@ __global__ void __launch_bounds__(160, sizeof(C) == 8 ? 6 : 4) k_y1w(PencilArr l
   // once per CTA (thread 0, under the copies), shared through shared memory
   __shared__ double pen[5];
 
-  // 1. bulk copies on one barrier: the three Lamb pencils (Py
-  //    values, natural order, at the start of each warp's line: the first
-  //    FFT pass reads them all before it writes the line), state, history
-  const uint32_t lamb = (uint32_t)(((Py + 1) & ~1) * sizeof(C));
+  // 1. bulk copies on one barrier: the three Lamb pencils, state, history
+  const uint32_t lamb = (uint32_t)(PS * sizeof(C));
   __shared__ uint64_t bar;
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
     fence_mbar_init();
     mbar_expect_tx(&bar, 3 * lamb + (boot ? 0u : (uint32_t)(4 * Ny * 16)));
-    for (int f = 0; f < 3; ++f) bulk_g2s(lines + (size_t)f * wlen<C>(M), pencil_ptr<C>(lam, f, p), lamb, &bar);
+    for (int f = 0; f < 3; ++f) bulk_g2s(stg + (size_t)f * PS, pencil_ptr<C>(lam, f, p), lamb, &bar);
     if (!boot) {
       bulk_g2s(Vc, V + p * Ny, (uint32_t)(Ny * 16), &bar);
       bulk_g2s(Oc, O + p * Ny, (uint32_t)(Ny * 16), &bar);
@@ -937,6 +907,12 @@ __global__ void __launch_bounds__(160, sizeof(C) == 8 ? 6 : 4) k_y1w(PencilArr l
     pen[2] = kmn_of(a, b);
     pen[3] = dt;
     pen[4] = dt * 0.5 / Re;
+  } else if (threadIdx.x >= 64 && threadIdx.x < 64 + GU + 2) {
+    const int i = threadIdx.x - 64 - 2;  // -2 .. GU - 1
+    const double2 z2 = make_double2(0.0, 0.0);
+    Vc[i < 0 ? i : Ny + i] = z2;
+    Oc[i < 0 ? i : Ny + i] = z2;
+    if (i >= 0) S4[Ny + i] = T2[Ny + i] = S2[Ny + i] = z2;  // (S2 N + 1, N + 2 written below)
   }
   __syncthreads();
   const double ia = pen[0], ib = pen[1], kmn = pen[2];
@@ -947,135 +923,180 @@ __global__ void __launch_bounds__(160, sizeof(C) == 8 ? 6 : 4) k_y1w(PencilArr l
     }
     return;
   }
-  // 2. transforms, one Lamb line per warp (0: lambda_x, 1: lambda_y,
-  //    2: lambda_z), read from the pencils as even extensions, coefficients
-  //    written to lc, and the warp's own derivative (D lambda_x, D lambda_y);
-  //    warps 3 and 4 build the derivative chains of v and omega_y meanwhile
-  const double sc = 1.0 / (Py - 1);
-  if (warp < 3) {
-    C* wline = lines + (size_t)warp * wlen<C>(M);
-    const C* src = wline;  // staged pencil
-    double2* lf = (double2*)wline;  // coefficients over the consumed lines
-    auto ld = [&](int, int n) -> C { return (n < Py) ? src[n] : src[M - n]; };
-    auto st = [&](int, int k, C val) {
+  const double dt = pen[3], h = pen[4], gam = zero ? 0.0 : ia * dt * 0.5;
+  // 2. warps 0, 1: transforms, derivative; warps 2, 3: the state's part of
+  //    the right-hand sides, its derivatives at the left-out points
+  if (warp < 2) {
+    auto pair = []() { asm volatile("bar.sync 1, 64;" ::: "memory"); };
+    for (int i = threadIdx.x; i < D::IA; i += 64)
+      D::template pass_a<0>(X, i, [&](int l, int n) { return stg[l * PS + n]; });
+    pair();
+    for (int i = threadIdx.x; i < D::IB; i += 64)
+      D::pass_b(X, dct, i, [&](int l, int k, C v) {
+        if (k < Ny) lx[l * Ny + k] = to_d2(v) * (k ? 1.0 / (Py - 1) : 0.5 / (Py - 1));
+      });
+    pair();
+    for (int k = threadIdx.x; k < Ny; k += 64) q[k] = lx[k] * ia + ly[k] * ib;
+    pair();
+    if (warp == 0) ddz_fast<ddz_run(Ny)>(q, Dq, Ny);
+  } else if (!boot) {
+    const double c2v = 1 - 2.0 * kmn * h, c0v = kmn * (1 - kmn * h), c0o = 1 - kmn * h;
+    const double kap = -0.5 * ib * dt;  // tilting weight (source/linear.cpp:147-151)
+    double acc[10];
+#pragma unroll
+    for (int i = 0; i < 10; ++i) acc[i] = 0.0;
+    for (int k = threadIdx.x - 64; k < Ny + 2; k += 64) {
+      const double2 v = Vc[k];
+      double2 P, Pf;
+      u_times(Vc, k, N, ph, P, Pf);
+      S2[k] = make_double2(v.x * c2v + P.y * gam, v.y * c2v - P.x * gam);
       if (k < Ny) {
-        double2 c = to_d2(val) * sc;
-        if (k == 0) c = c * 0.5;
-        lf[k] = c;
+        const double kg = kmn * gam;
+        S4[k] = zero ? v : make_double2(-(v.x * c0v + Pf.y * kg), Pf.x * kg - v.y * c0v);
+        const double2 o = Oc[k];
+        double2 Q, Qf, up = v * ph.U1;
+        u_times(Oc, k, N, ph, Q, Qf);
+        if (ph.U2 != 0.0) {  // U' v, its degree N + 1 folded
+          up = up + (Vc[k - 1] * (k == 1 ? 2.0 : 1.0) + Vc[k + 1]) * ph.U2;
+          if (k == N - 1) up = up + Vc[N] * ph.U2;
+        }
+        const double2 im = up * kap - Qf * gam;
+        T2[k] = zero ? o : make_double2(o.x * c0o - im.y, o.y * c0o + im.x);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const double w = __ldg(tb.tw + t * Ny + k);
+          acc[2 * t] += v.x * w;
+          acc[2 * t + 1] += v.y * w;
+        }
+        const double w = __ldg(tb.tw + k);
+        acc[8] += o.x * w;
+        acc[9] += o.y * w;
       }
-    };
-    wfft_io<C, M, 1, false>(wline, wtw_of(tabP, 0), ld, st);
-    if (warp < 2) ddz_fast<ddz_run(Ny)>(lf, lf + VS, Ny);
-  } else if (!boot && warp == 3) {
-    // D^2 v in one sweep, D^4 v = D^2 (D^2 v)
-    d2z_fast<ddz_run(Ny)>(Vc, D2V, Ny);
-    __syncwarp();
-    d2z_fast<ddz_run(Ny)>(D2V, D4V, Ny);
-  } else if (!boot && warp == 4) {
-    d2z_fast<ddz_run(Ny)>(Oc, D2O, Ny);
+    }
+    int idx;
+    const double sum = parity_sums(acc, lane, idx);
+    if (idx < 10) accA[((warp - 2) * 2 + (lane & 1)) * 10 + idx] = sum;
   }
   __syncthreads();
-  // 3. nonlinear terms (coefficients) -> history; interpolated right-hand sides
-  const double dt = pen[3], gam = ia * dt * 0.5;
-  const double kap = -0.5 * ib * dt;  // tilting weight (source/linear.cpp:147-151)
-  // the CN operators' coefficients
-  const double h = pen[4], c2v = 1 - 2.0 * kmn * h, c0v = kmn * (1 - kmn * h), c0o = 1 - kmn * h;
-  double2* fv = lx;
-  double2* fo = ly;
-  for (int k = threadIdx.x; k < Ny; k += blockDim.x) {
-    double2 hv, ho;
-    if (zero) {
-      hv = lx[k];
-      ho = ly[k];
-    } else {
-      hv = lz[k] * kmn + muli(D1x[k] * ia) + muli(D1y[k] * ib);
-      ho = muli(ly[k] * ia) - muli(lx[k] * ib);
+  // 3. nonlinear terms (coefficients) -> history, and into the right-hand
+  //    sides; sums of these for the left-out points
+  const double dtn = zero ? -dt : dt;
+  double acc[6];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) acc[i] = 0.0;
+  for (int k = threadIdx.x; k < Ny; k += 128) {
+    const double2 x = lx[k], y = ly[k];
+    double2 hv = x, ho = y;
+    if (!zero) {
+      const double2 z = lz[k], d = Dq[k];
+      hv = make_double2(z.x * kmn - d.y, z.y * kmn + d.x);
+      ho = make_double2(x.y * ib - y.y * ia, y.x * ia - x.x * ib);
     }
     Nvp[p * Ny + k] = hv;
     Nop[p * Ny + k] = ho;
     if (boot) continue;
-    double2 a, b;
-    if (zero) {
-      a = Vc[k] + D2V[k] * h - (hv * 1.5 - nvc[k] * 0.5) * dt;
-      b = Oc[k] + D2O[k] * h - (ho * 1.5 - noc[k] * 0.5) * dt;
-    } else {
-      const double2 re = D4V[k] * h + D2V[k] * c2v - Vc[k] * c0v;
-      // U (-gam D^2 v + k^2 gam v) as one interpolant
-      const double2 im = umul_fn([&](int j) { return D2V[j] * (-gam) + Vc[j] * (kmn * gam); }, k, N, ph)
-                         + Vc[k] * (gam * 2.0 * ph.U2);
-      a = re + muli(im) + (hv * 1.5 - nvc[k] * 0.5) * dt;
-      const double2 ro = D2O[k] * h + Oc[k] * c0o;
-      b = ro + muli(umul_gl(Oc, k, N, ph) * (-gam)) + (ho * 1.5 - noc[k] * 0.5) * dt
-          + muli(upmul_gl(Vc, k, N, ph) * kap);
-    }
-    fv[k] = a;
-    fo[k] = b;
+    const double2 s4 = S4[k] + (hv * 1.5 - nvc[k] * 0.5) * dtn;
+    const double2 t2 = T2[k] + (ho * 1.5 - noc[k] * 0.5) * dtn;
+    S4[k] = s4;
+    T2[k] = t2;
+    double2 f = s4;
+    if (ph.U2 != 0.0) f = f + muli(Vc[k]) * (2.0 * gam * ph.U2);
+    const double c = __ldg(tb.cosk + k);
+    acc[0] += f.x;
+    acc[1] += f.y;
+    acc[2] += f.x * c;
+    acc[3] += f.y * c;
+    acc[4] += t2.x;
+    acc[5] += t2.y;
   }
   if (boot) return;
-  __syncthreads();
-  // 4. values at the points the equations leave out and the K-fold
-  //    integrals of fv, fo by their banded stencils (all threads); the
-  //    values by three warps, two sums each: warp 0 fv at y = +-1, warp 2
-  //    fv at y_1, y_{N-1}, warp 1 fo at y = +-1 (omega does not use y_1,
-  //    y_{N-1})
-  if (warp < 3) {
-    const double2* f = (warp == 1) ? fo : fv;
-    const bool inner = warp == 2;
-    double2 sa = make_double2(0.0, 0.0), sb = sa;
-    for (int k = lane; k < Ny; k += 32) {
-      const double2 v = f[k];
-      const double sg = (k & 1) ? -1.0 : 1.0;
-      const double cs = inner ? __ldg(tb.cosk + k) : 1.0;
-      sa = sa + v * cs;
-      sb = sb + v * (sg * cs);
-    }
-    sa = warp_sum(sa);
-    sb = warp_sum(sb);
-    if (lane == 0) {
-      const int ia0 = inner ? 1 : 4 * warp;      // y = 1 or y_1
-      const int ib0 = inner ? 2 : 4 * warp + 3;  // y = -1 or y_{N-1}
-      red[ia0] = sa;
-      red[ib0] = sb;
-    }
+  {
+    int idx;
+    const double sum = parity_sums(acc, lane, idx);
+    if (idx < 6) accB[(warp * 2 + (lane & 1)) * 6 + idx] = sum;
   }
-  auto fget = [&](const double2* f, int k) { return (k >= 0 && k <= N) ? f[k] : make_double2(0.0, 0.0); };
-  constexpr int RPT = (Ny + 2 + 159) / 160;  // rows per thread (n <= Ny + 2, 160 threads)
+  __syncthreads();
+  // 4. right-hand sides at the points the equations leave out (six threads);
+  //    the mean modes are two systems of the omega kind
+  if (threadIdx.x >= 96 && threadIdx.x < 102) {
+    const int i = threadIdx.x - 96, at = i == 1 || i == 2;  // at +-y_1
+    const double sg = (i == 2 || i == 3 || i == 5) ? -1.0 : 1.0;
+    auto sumA = [&](int v) {
+      const double* a = accA + v;
+      return make_double2(a[0] + a[20] + (a[10] + a[30]) * sg, a[1] + a[21] + (a[11] + a[31]) * sg);
+    };
+    const double* a = accB + (i >= 4 ? 4 : 2 * at);
+    double2 f = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) f = f + make_double2(a[12 * w] + a[12 * w + 6] * sg, a[12 * w + 1] + a[12 * w + 7] * sg);
+    if (i >= 4 || zero) {
+      f = f + sumA(i >= 4 ? 8 : 0) * h;
+    } else {
+      const double y = (at ? __ldg(tb.cosk + 1) : 1.0) * sg;
+      const double2 d2 = sumA(4 * at), d4 = sumA(4 * at + 2);
+      f = f + d4 * h + d2 * (1 - 2.0 * kmn * h) - muli(d2) * (gam * (ph.U0 + (ph.U1 + ph.U2 * y) * y));
+    }
+    red[i] = f;
+  }
+  //    and the integrals by their banded stencils (all threads)
+  constexpr int RPT = (Ny + 2 + 127) / 128;  // rows per thread (n <= Ny + 2, 128 threads)
+  const int n2 = rd.nv + 2;
   double2 iv[RPT], io[RPT];
 #pragma unroll
   for (int t = 0; t < RPT; ++t) {
-    const int r = threadIdx.x + t * blockDim.x;
-    iv[t] = make_double2(0.0, 0.0);
-    io[t] = make_double2(0.0, 0.0);
+    const int r = threadIdx.x + t * 128;
+    iv[t] = io[t] = make_double2(0.0, 0.0);
     if (r < rd.nv) {
+      const double* b2 = tb.b2 + r;
+      double w[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) w[d] = __ldg(b2 + d * n2);
+      io[t] = Oc[r + 2] * h;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) io[t] = io[t] + T2[r + 2 * d] * w[d];
       if (zero) {
+        iv[t] = Vc[r + 2] * h;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) iv[t] = iv[t] + fget(fv, r + 2 + 2 * d - 2) * __ldg(tb.b2 + (size_t)d * rd.nv + r);
+        for (int d = 0; d < 3; ++d) iv[t] = iv[t] + S4[r + 2 * d] * w[d];
       } else {
+        iv[t] = Vc[r + 4] * h;
+        const double* b4 = tb.b4 + r;
 #pragma unroll
-        for (int d = 0; d < 5; ++d) iv[t] = iv[t] + fget(fv, r + 4 + 2 * d - 4) * __ldg(tb.b4 + (size_t)d * rd.nv + r);
+        for (int d = 0; d < 5; ++d) iv[t] = iv[t] + S4[r + 2 * d] * __ldg(b4 + d * rd.nv);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) iv[t] = iv[t] + S2[r + 2 + 2 * d] * __ldg(b2 + d * n2 + 2);
+        if (ph.U1 != 0.0 || ph.U2 != 0.0) {
+          double2 s3 = make_double2(0.0, 0.0);
+          const double* b3 = tb.b3 + r;
+#pragma unroll
+          for (int d = 0; d < 4; ++d) {
+            const int k = r + 1 + 2 * d;
+            double2 x = Vc[k] * ph.U1;
+            if (ph.U2 != 0.0) x = x + (Vc[k - 1] * (k == 1 ? 2.0 : 1.0) + Vc[k + 1]) * ph.U2;
+            s3 = s3 + x * __ldg(b3 + d * rd.nv);
+          }
+          iv[t] = iv[t] + muli(s3) * (2.0 * gam);
+        }
       }
-    }
-    if (r < rd.no) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) io[t] = io[t] + fget(fo, r + 2 + 2 * d - 2) * __ldg(tb.b2 + (size_t)d * rd.nv + r);
     }
   }
   __syncthreads();
   // 5. minus the integrated cardinal corrections, out
 #pragma unroll
   for (int t = 0; t < RPT; ++t) {
-    const int r = threadIdx.x + t * blockDim.x;
-    if (r < rd.nv) {
+    const int r = threadIdx.x + t * 128;
+    if (r < rd.nv) {  // as many rows of omega
+      const double c0 = __ldg(tb.bkco + r), cN = __ldg(tb.bkco + rd.no + r);
       double2 v = iv[t];
       if (zero) {
-        v = v - red[0] * __ldg(tb.bkco + r) - red[3] * __ldg(tb.bkco + rd.no + r);
+        v = v - red[0] * c0 - red[3] * cN;
       } else {
 #pragma unroll
-        for (int m = 0; m < 4; ++m) v = v - red[m] * __ldg(tb.bkcv + (size_t)m * rd.nv + r);
+        for (int m = 0; m < 4; ++m) v = v - red[m] * __ldg(tb.bkcv + m * rd.nv + r);
       }
       gv[p * rd.gp + r] = v;
+      go[p * rd.gp + r] = io[t] - red[4] * c0 - red[5] * cN;
     }
-    if (r < rd.no) go[p * rd.gp + r] = io[t] - red[4] * __ldg(tb.bkco + r) - red[7] * __ldg(tb.bkco + rd.no + r);
   }
 }
 
@@ -1176,6 +1197,11 @@ cudaError_t launch_y3(const double2* V, const double2* O, PencilArr out, DnsGeom
 template cudaError_t launch_y3<double2>(const double2*, const double2*, PencilArr, DnsGeom, PhysParams, FftTab<double2>, int*, cudaStream_t, int, bool);
 template cudaError_t launch_y3<float2>(const double2*, const double2*, PencilArr, DnsGeom, PhysParams, FftTab<float2>, int*, cudaStream_t, int, bool);
 
+// CTAs per SM of k_y1d: what the first radix leaves of the registers
+template <typename C, int M> constexpr int y1_ctas() {
+  constexpr int RA = DPlan<M>::A;
+  return sizeof(C) == 8 ? (RA > 24 ? 5 : (RA > 18 ? 6 : 8)) : (RA > 24 ? 3 : 4);
+}
 template <typename C>
 cudaError_t launch_y1(PencilArr lam, const double2* V, const double2* O, double2* Nvp,
                       double2* Nop, double2* gv, double2* go, RhsDims rd, RhsTabs tb, DnsGeom g,
@@ -1187,24 +1213,29 @@ cudaError_t launch_y1(PencilArr lam, const double2* V, const double2* O, double2
   // Py = M/2 + 1 as compile-time constants
   const bool bulk_ok = aligned16(lam.base) && (lam.ps * sizeof(C)) % 16 == 0 &&
                        (lam.fs * sizeof(C)) % 16 == 0 && lam.ps >= ((g.Py + 1) & ~1) && aligned16(V) &&
-                       aligned16(O) && aligned16(Nvp) && aligned16(Nop) && wtw_of(tabP, 0) &&
+                       aligned16(O) && aligned16(Nvp) && aligned16(Nop) && tabP.dt &&
                        g.Ny == tabP.plan.L / 4 + 1 && g.Py == tabP.plan.L / 2 + 1;
-  return with_len_m(tabP.plan.L, [&](auto LL) -> cudaError_t {
-    constexpr int L = decltype(LL)::value;
-    if constexpr (L > 0 && WPlan<L, 1, FftMaxRadix<C>::v>::ok) {
-     if ((any || variant == DNS_Y1_WARP) && bulk_ok) {
+  if ((any || variant == DNS_Y1_WARP) && bulk_ok) {
+    const cudaError_t e = with_len_d(tabP.plan.L, [&](auto MM) -> cudaError_t {
+      constexpr int M = decltype(MM)::value;
+      typedef Dct<C, M, 3> D;
       if (probe) return cudaSuccess;
       auto a = [](size_t b) { return (b + 15) & ~(size_t)15; };
-      const size_t bl = (size_t)3 * wlen<C>(L) * sizeof(C), bi = (size_t)4 * (g.Ny + 8) * 16;
-      const size_t sm = 7 * a((size_t)g.Ny * 16) + a(8 * 16) + a(bl > bi ? bl : bi);
-      cudaFuncSetAttribute(k_y1w<C, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_y1w<C, L><<<(unsigned)g.H, 160, sm, st>>>(lam, V, O, Nvp, Nop, gv, go, rd, tb, g, ph, tabP, boot,
-                                                    status);
+      const size_t lb = sizeof(C) * 3 * ((g.Py + 1) & ~1), lc = (size_t)48 * g.Ny, xb = sizeof(C) * D::XN,
+                   xd = (size_t)32 * g.Ny;
+      // vectors with their guards, sums, staged pencils, exchange (as carved)
+      const size_t sm = (size_t)(7 * g.Ny + 5 * 12 + 4 + 6) * 16 + (40 + 48) * 8 + a(lb > lc ? lb : lc) + a(xb > xd ? xb : xd);
+      auto k = k_y1d<C, M, y1_ctas<C, M>()>;
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      k<<<(unsigned)g.H, 128, sm, st>>>(lam, V, O, Nvp, Nop, gv, go, rd, tb, g, ph, tabP.dt, boot, status);
       return cudaGetLastError();
-     }
-    }
-    if (!any && variant != DNS_Y1_BLOCK) return cudaErrorNotSupported;
-    if (probe) return cudaSuccess;
+    });
+    if (e != cudaErrorNotSupported) return e;
+  }
+  if (!any && variant != DNS_Y1_BLOCK) return cudaErrorNotSupported;
+  if (probe) return cudaSuccess;
+  return with_len_m(tabP.plan.L, [&](auto LL) -> cudaError_t {
+    constexpr int L = decltype(LL)::value;
     const size_t sm = y1_smem(g.Ny, FLine<C, L>::stride(tabP.plan.L), sizeof(C));
     cudaFuncSetAttribute(k_y1<C, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     k_y1<C, L><<<(unsigned)g.H, 256, sm, st>>>(lam, V, O, Nvp, Nop, gv, go, rd, tb, g, ph, tabP, boot);

@@ -26,7 +26,17 @@ struct RhsTabs {
   const double* bkco;  // 2 x no: rows 2.. of B^2 C_m, m = 0, N
   const double* cosk;  // cos(k pi / N), k = 0..N
   const double* b4;    // 5 x nv: [d][r], row r of B^4 restricted to rows 4..: weight of f_{r+4+2d-4}
-  const double* b2;    // 3 x nv: [d][r], row r of B^2 restricted to rows 2..: weight of f_{r+2+2d-2}
+  const double* b2;    // 3 x (nv + 2): [d][r], row r of B^2 restricted to rows 2..: weight of f_{r+2+2d-2}
+  const double* b3;    // 4 x nv: [d][r], row r of B^3 restricted to rows 4..: weight of f_{r+4+2d-3}
+  const double* tw;    // 4 x Ny: second, fourth derivative of T_k at 1, then at y_1
+};
+// their layout in one allocation: offsets of the tables, and the end
+struct RhsLayout {
+  size_t bkcv, bkco, cosk, b4, b2, b3, tw, end;
+  RhsLayout(int Ny, int nv, int no)
+      : bkcv(0), bkco(4 * (size_t)nv), cosk(bkco + 2 * (size_t)no), b4(cosk + Ny), b2(b4 + 5 * (size_t)nv),
+        b3(b2 + 3 * (size_t)(nv + 2)), tw(b3 + 4 * (size_t)nv), end(tw + 4 * (size_t)Ny) {}
+  RhsTabs at(const double* t) const { return RhsTabs{t + bkcv, t + bkco, t + cosk, t + b4, t + b2, t + b3, t + tw}; }
 };
 template <typename C>
 cudaError_t launch_y1(PencilArr lam, const double2* V, const double2* O, double2* Nvp,

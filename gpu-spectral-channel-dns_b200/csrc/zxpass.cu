@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(32 * NW, 3) k_zbt(const __grid_constant__ CUte
     return (kxok && kz >= 0) ? tile[2 * kz + l] : cmk<C>(0.0, 0.0);
   };
   auto st = [&](int l, int k, C v) { wl[(size_t)l * LS + wsw<C>(k)] = v; };
-  wfft_io<C, L, 2, true>(wl, tab.wt[1], ld, st, LS);
+  wfft_io<C, L, 2, true>(wl, tab.wt, ld, st, LS);
   __syncthreads();
   // row side: this thread's kx, flat index i = yl * Pz + zp
   const int kxr = threadIdx.x % TX;
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(32 * NW, 3) k_zft(const __grid_constant__ CUte
   }
   auto ld = [&](int l, int n) -> C { return tile[2 * n + l]; };
   auto st = [&](int l, int k, C v) { wl[(size_t)l * LS + wsw<C>(k)] = v; };
-  wfft_io<C, L, 2, false>(wl, tab.wt[1], ld, st, LS);
+  wfft_io<C, L, 2, false>(wl, tab.wt, ld, st, LS);
   __syncthreads();
   // pencil side: line li = (yl, kxl) of this thread, wavenumbers kz
   constexpr int ZB = 8;
@@ -621,7 +621,7 @@ cudaError_t launch_zb(PencilArr in, RowArr out, int nf, DnsGeom g, FftTab<C> tab
         if constexpr (L > 0 && WPlan<L, 2, FftMaxRadix<C>::v>::ok) {
           constexpr int LS = wlen<C>(L) + 1;
           CUtensorMap tm;
-          if (status && g.Nz == L / 3 * 2 && wtw_of(tab, 1) &&
+          if (status && g.Nz == L / 3 * 2 && tab.wt &&
               (size_t)g.Nz * 16 + 128 <= (size_t)2 * LS * sizeof(C) && pencil_tmap(in, nf, g, sizeof(C), &tm)) {
             if (probe) return cudaSuccess;
             // pencils staged by tensor copies (a y pair per line pair), 8 x 2
@@ -665,7 +665,7 @@ cudaError_t launch_zf(RowArr in, PencilArr out, int nf, DnsGeom g, FftTab<C> tab
         if constexpr (L > 0 && WPlan<L, 2, FftMaxRadix<C>::v>::ok) {
           constexpr int LS = wlen<C>(L) + 1;
           CUtensorMap tm;
-          if (status && g.Nz == L / 3 * 2 && wtw_of(tab, 1) &&
+          if (status && g.Nz == L / 3 * 2 && tab.wt &&
               (size_t)L * 16 + 128 <= (size_t)2 * LS * sizeof(C) && row_tmap(in, nf, g, sizeof(C), &tm)) {
             if (probe) return cudaSuccess;
             // rows staged by tensor copies, 4 x 4 tile

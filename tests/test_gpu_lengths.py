@@ -5,7 +5,8 @@ short in the other two directions put every length through the drop-in
 transforms (FP64, against the oracle: 1e-13 of the largest value, the parity
 bar of the transforms) and through the time step (the mixed form against FP64:
 1e-6 relative after two steps, the bar of the variants; the FP64 streamwise
-pass against its block form, 1e-12).  The short directions leave ragged tiles:
+and wall-normal passes against their block forms: 1e-12, and 1e-11, the step's
+parity bar, where the two forms build the right-hand sides differently).  The short directions leave ragged tiles:
 9 streamwise modes, 17 wall-normal points, 54 span points (no multiple of 4)."""
 import numpy as np
 import pytest
@@ -16,6 +17,7 @@ pytestmark = pytest.mark.gpu
 from oracle import rpcf_oracle as O  # noqa: E402
 
 SPAN = [24, 32, 36, 48, 54, 64, 72, 96, 108, 128, 144, 162, 192, 216, 256, 288, 324, 384, 432, 512, 576, 768]
+WALL = [32, 36, 48, 64, 72, 96, 108, 128, 144, 192, 216, 256, 288, 324, 384, 432, 512, 576, 768]
 
 
 @pytest.fixture(autouse=True)
@@ -51,8 +53,8 @@ def _transform_errors(pkg, mx, my, mz):
     return eb, ef
 
 
-def _state_after(pkg, prec, mx, my, mz, variants=()):
-    c = pkg.Context(pkg.make_params(mx, my, mz, Re=1300.0, Ro=0.1, dt=0.001, precision=prec))
+def _state_after(pkg, prec, mx, my, mz, variants=(), U=(0.5, 0.5, 0.0)):
+    c = pkg.Context(pkg.make_params(mx, my, mz, Re=1300.0, Ro=0.1, dt=0.001, U=U, precision=prec))
     for p, v in variants:
         c.set_variant(p, v)
     c.set_state(*pkg.seeded_state(c.Nx, c.Ny, c.Nz, amplitude=0.05, seed=1))
@@ -85,4 +87,17 @@ def test_stream_length(pkg, L):
     block = _state_after(pkg, pkg.PREC_FP64, L, 54, 32, [(pkg.PASS_X, pkg.X_BLOCK)])
     assert _apart(fused, block) < 1e-12
     e = _step_error(pkg, L, 54, 32, [(pkg.PASS_X, pkg.X_WARP3)])
+    assert e < 1e-6, e
+
+
+@pytest.mark.parametrize("M", WALL)
+def test_wall_length(pkg, M):
+    eb, ef = _transform_errors(pkg, 24, 24, M)
+    assert eb < 1e-13 and ef < 1e-13, (eb, ef)
+    warp, block = [(pkg.PASS_Y3, pkg.Y3_FFT)], [(pkg.PASS_Y3, pkg.Y3_BLOCK)]
+    assert _apart(*(_state_after(pkg, pkg.PREC_FP64, 24, 24, M, v) for v in (warp, block))) < 1e-12
+    warp, block = [(pkg.PASS_Y1, pkg.Y1_WARP)], [(pkg.PASS_Y1, pkg.Y1_BLOCK)]
+    for U in ((0.5, 0.5, 0.0), (1.0, 0.0, -1.0), (0.3, 0.7, -0.4)):
+        assert _apart(*(_state_after(pkg, pkg.PREC_FP64, 24, 24, M, v, U) for v in (warp, block))) < 1e-11, U
+    e = _step_error(pkg, 24, 24, M, [(pkg.PASS_Y3, pkg.Y3_FFT), (pkg.PASS_Y1, pkg.Y1_WARP)])
     assert e < 1e-6, e
