@@ -169,8 +169,8 @@ dns_status ctx_build_wall_solver(dns_ctx* c) {
     if (!err.empty()) return fail(DNS_ERR_SINGULAR, err);
     if (g.nrun > 1) fac.insert(fac.end(), f1.begin(), f1.end());
   }
-  std::vector<double> Q((size_t)7 * wd.no);
-  if (!wall::tilting_table(N, wd.no, c->ph.U1, c->ph.U2, Q.data()))
+  std::vector<double> Q((size_t)7 * WALL_QROWS(wd.no));
+  if (!wall::tilting_table(N, wd.no, c->ph.U1, c->ph.U2, Q.data() + 7 * WALL_QLOW))
     return fail(DNS_ERR_ARG, "tilting table outside its band");
   wd.group_complex = pk.group_complex;
   wd.nslots = (long long)g.Kx * (sl ? sl->s1 - sl->s0 : g.Kh);
@@ -517,7 +517,7 @@ dns_status ctx_create(const dns_params* p, SlabState* slab, dns_ctx** out, int n
   c->wd.delta = wall::base_degree(p->U1, p->U2);
   c->wd.nv = c->wd.no = Ny + c->wd.delta;
   c->wd.gp = c->wd.nv;
-  c->wd.qbytes = (int)((7 * (size_t)c->wd.no * 8 + 15) & ~(size_t)15);
+  c->wd.qbytes = (int)((7 * (size_t)WALL_QROWS(c->wd.no) * 8 + 15) & ~(size_t)15);
   const size_t gn = (size_t)(sl ? sl->np : g.H * nrun) * c->wd.gp;
   if ((e = c->alloc(&c->T0, NN)) || (e = c->alloc(&c->T2, NN)) || (e = c->alloc(&c->T4, NN)) ||
       (e = c->alloc(&c->Ut, Ny)) || (e = c->alloc(&c->dUt, Ny)) || (e = c->alloc(&c->ddUt, Ny)) ||

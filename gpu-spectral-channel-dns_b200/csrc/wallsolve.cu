@@ -45,7 +45,20 @@ __host__ __device__ constexpr int rows_per_chunk(int stg, int entries, int cap) 
   return (stg / (entries * 256)) < cap ? (stg / (entries * 256)) : cap;
 }
 
-__device__ __forceinline__ double2 sel(bool p, double2 a) { return p ? a : make_double2(0.0, 0.0); }
+struct Whole { static constexpr bool full = true; };
+struct Part { static constexpr bool full = false; };
+
+// acc + a b, acc - a b: four fused operations (a product and a sum apart
+// are six)
+__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 acc) {
+  return make_double2(fma(-a.y, b.y, fma(a.x, b.x, acc.x)), fma(a.y, b.x, fma(a.x, b.y, acc.y)));
+}
+__device__ __forceinline__ double2 cfms(double2 a, double2 b, double2 acc) {
+  return make_double2(fma(a.y, b.y, fma(-a.x, b.x, acc.x)), fma(-a.y, b.x, fma(-a.x, b.y, acc.y)));
+}
+__device__ __forceinline__ double2 rfma(double a, double2 b, double2 acc) {
+  return make_double2(fma(a, b.x, acc.x), fma(a, b.y, acc.y));
+}
 
 template <int KLV, int KUV, int KLO, int KUO, int STG>
 struct WallCfg {
@@ -53,30 +66,8 @@ struct WallCfg {
   // rows per ring chunk; the solve keeps two chunks of vector rows in registers
   static constexpr int R0 = rows_per_chunk(STG, E0, 12), R1 = rows_per_chunk(STG, E1, 12);
   static constexpr int R2 = rows_per_chunk(STG, E2, 8), R3 = rows_per_chunk(STG, E3, 12);
-  static_assert(R0 > 0 && R1 > 0 && R2 > 0 && R3 > 0, "stage too small for a row");
+  static_assert(R0 > 0 && R1 > 1 && R2 > 0 && R3 > 0, "stage too small for a row");
 };
-
-// chunk c of a group's stream: byte count and offset (complex values)
-template <class CF>
-__device__ __forceinline__ void chunk_of(int c, const WallDims& wd, uint32_t& bytes, long long& off) {
-  const int n0 = (wd.nv + CF::R0 - 1) / CF::R0, n1 = (wd.nv + CF::R1 - 1) / CF::R1;
-  const int n2 = (wd.no + CF::R2 - 1) / CF::R2;
-  long long base;
-  int r0, rows, E;
-  if (c < n0) {
-    base = 0; E = CF::E0; r0 = c * CF::R0; rows = min(CF::R0, wd.nv - r0);
-  } else if (c < n0 + n1) {
-    base = 16LL * wd.nv * CF::E0; E = CF::E1; r0 = (c - n0) * CF::R1; rows = min(CF::R1, wd.nv - r0);
-  } else if (c < n0 + n1 + n2) {
-    base = 16LL * wd.nv * (CF::E0 + CF::E1); E = CF::E2; r0 = (c - n0 - n1) * CF::R2;
-    rows = min(CF::R2, wd.no - r0);
-  } else {
-    base = 16LL * (wd.nv * (CF::E0 + CF::E1) + wd.no * CF::E2); E = CF::E3;
-    r0 = (c - n0 - n1 - n2) * CF::R3; rows = min(CF::R3, wd.no - r0);
-  }
-  off = base + 16LL * r0 * E;
-  bytes = (uint32_t)(rows * E * 256);
-}
 
 }  // namespace
 
@@ -91,10 +82,10 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
   uint64_t* full = (uint64_t*)smem_raw;
   double2* ring = (double2*)(smem_raw + WALL_HDR);
   double* Qsm = (double*)(smem_raw + WALL_HDR + WALL_NST * WALL_STG);
-  const double* Qs = QSM ? Qsm : Qg;  // tilting table: shared memory or through L1
-  // recombination weights 2k/(k+1), (k-3)/(k-1) of the clamped basis, k <= N
+  const double* Qs = (QSM ? Qsm : Qg) + 7 * WALL_QLOW;  // tilting table: shared memory or through L1
+  // recombination weights of the clamped basis, row by row
   double* rc2 = Qsm + (QSM ? wd.qbytes / 8 : 0);
-  double* rc4 = rc2 + g.Ny;
+  double* rc4 = rc2 + wd.nv;
 
   const int lane = threadIdx.x;
   const int q = lane >> 1, b = lane & 1;
@@ -127,14 +118,25 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
   const int total = nch0 + nch1 + nch2 + nch3;
 
   const uint64_t pol = EF ? l2_evict_first() : 0;
-  auto issue = [&](int c) {
-    uint32_t bytes;
-    long long off;
-    chunk_of<CF>(c, wd, bytes, off);
-    uint64_t* bar = &full[c % WALL_NST];
+  // the group's stream is contiguous: lane 0 walks it phase by phase, ic the
+  // next chunk, irow rows of its phase issued
+  int ic = 0, iph = 0, irow = 0;
+  const double2* isrc = gfac;
+  auto issue = [&]() {
+    const int rows = iph < 2 ? wd.nv : wd.no;
+    const int R = iph == 0 ? CF::R0 : iph == 1 ? CF::R1 : iph == 2 ? CF::R2 : CF::R3;
+    const int E = iph == 0 ? CF::E0 : iph == 1 ? CF::E1 : iph == 2 ? CF::E2 : CF::E3;
+    const int n = min(R, rows - irow);
+    const uint32_t bytes = (uint32_t)(n * E * 256);
+    uint64_t* bar = &full[ic % WALL_NST];
+    double2* dst = ring + (size_t)(ic % WALL_NST) * (WALL_STG / 16);
     mbar_expect_tx(bar, bytes);
-    if (EF) bulk_g2s_hint(ring + (size_t)(c % WALL_NST) * (WALL_STG / 16), gfac + off, bytes, bar, pol);
-    else bulk_g2s(ring + (size_t)(c % WALL_NST) * (WALL_STG / 16), gfac + off, bytes, bar);
+    if (EF) bulk_g2s_hint(dst, isrc, bytes, bar, pol);
+    else bulk_g2s(dst, isrc, bytes, bar);
+    isrc += n * E * 16;
+    irow += n;
+    if (irow == rows) { irow = 0; ++iph; }
+    ++ic;
   };
   // on a timed-out wait: report, let the copies in flight land, leave
   auto abort_at = [&](int c) {
@@ -149,17 +151,17 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
                                       WALL_WAIT_LIMIT, status);
     return __all_sync(0xffffffffu, ok);
   };
-  auto release = [&](int c) {
+  auto release = [&]() {
     __syncwarp();
-    if (lane == 0 && c + WALL_NST < total) {
+    if (lane == 0 && ic < total) {
       fence_proxy_async();
-      issue(c + WALL_NST);
+      issue();
     }
   };
-  // scratch rows (plain loads: the kernel writes them) and right-hand sides
-  auto lds = [&](int i) { return (i >= 0 && i < wd.nv) ? S[32 * i] : z2; };
+  auto chunk_at = [&](int c) { return ring + (size_t)(c % WALL_NST) * (WALL_STG / 16) + q; };
   const double2* gvp = gv + pen * wd.gp;
   const double2* gop = go + pen * wd.gp;
+  const int nv = wd.nv, no = wd.no;
 
   // ---- start: barriers, ring prefetch, tables ----------------------------
   if (lane == 0) {
@@ -168,233 +170,261 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
   }
   __syncwarp();
   if (QSM)
-    for (int k = lane; k < 7 * wd.no; k += 32) Qsm[k] = Qg[k];
-  for (int k = lane; k < g.Ny; k += 32) {
-    rc2[k] = 2.0 * k / (k + 1);
-    rc4[k] = (k >= 4) ? (double)(k - 3) / (double)(k - 1) : 0.0;
+    for (int k = lane; k < WALL_QROWS(no) * 7; k += 32) Qsm[k] = Qg[k];
+  // recombination weights of row i: V_{i+4} = x_{i+4} - 2k/(k+1) x_{i+2} +
+  // (k-3)/(k-1) x_i, k = i + 4, unknowns from N - 3 on are not part of it
+  for (int i = lane; i < nv; i += 32) {
+    const int k = i + 4;
+    rc2[i] = i + 2 < N - 3 ? 2.0 * k / (k + 1) : 0.0;
+    rc4[i] = i < N - 3 ? (double)(k - 3) / (double)(k - 1) : 0.0;
   }
   if (lane == 0)
-    for (int c = 0; c < min(WALL_NST, total); ++c) issue(c);
+    for (int c = 0; c < min(WALL_NST, total); ++c) issue();
   __syncwarp();
+  // the group of the mean modes (two systems of the omega kind)
+  const bool mean = __any_sync(0xffffffffu, zero);
 
+  // Rows go in chunks of the ring; a row's vector element is loaded one chunk
+  // ahead into the register it is consumed from.  Whole chunks run without
+  // conditions between their rows, so that the windows of earlier rows are
+  // renamed registers and not moves; FULL = false is a phase's last chunk.
   int c = 0;
   // ---- v: forward substitution (unit lower band) -------------------------
-  // the right-hand side rows of each chunk are loaded one chunk ahead
   {
     constexpr int R = CF::R0;
-    double2 yw[KLV];
+    double2 yw[KLV], cur[R];
 #pragma unroll
     for (int e = 0; e < KLV; ++e) yw[e] = z2;
-    double2 nxt[R];
 #pragma unroll
-    for (int rr = 0; rr < R; ++rr) nxt[rr] = (active && rr < wd.nv) ? __ldg(gvp + rr) : z2;
-    for (int r0 = 0; r0 < wd.nv; r0 += R, ++c) {
-      double2 cur[R];
-#pragma unroll
-      for (int rr = 0; rr < R; ++rr) {
-        cur[rr] = nxt[rr];
-        const int i = r0 + R + rr;
-        nxt[rr] = (active && i < wd.nv) ? __ldg(gvp + i) : z2;
-      }
-      if (!wait_chunk(c)) { abort_at(c); return; }
-      const double2* ch = ring + (size_t)(c % WALL_NST) * (WALL_STG / 16) + q;
-      const int rows = min(R, wd.nv - r0);
+    for (int rr = 0; rr < R; ++rr) cur[rr] = (active && rr < nv) ? __ldg(gvp + rr) : z2;
+    auto chunk = [&](auto whole, const double2* ch, int r0) {
+      const double2* nx = gvp + r0 + R;
+      double2* Sr = S + 32 * r0;
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
-        if (rr < rows) {
-          const int i = r0 + rr;
-          const double2* Lr = ch + rr * CF::E0 * 16;
-          // the older entries in independent partial sums; the newest
-          // (y_{i-1}) last, so only it is on the row-to-row critical path
-          double2 a0 = cur[rr], a1 = z2;
+        if (!whole.full && r0 + rr >= nv) continue;
+        const double2* Lr = ch + rr * CF::E0 * 16;
+        // the older entries in independent partial sums; the newest
+        // (y_{i-1}) last, so only it is on the row-to-row critical path
+        double2 a0 = cur[rr], a1 = z2;
+        if (whole.full) cur[rr] = (active && r0 + R + rr < nv) ? __ldg(nx + rr) : z2;
 #pragma unroll
-          for (int e = 0; e < KLV - 1; ++e) {
-            if (e & 1) a1 = a1 + cmul(Lr[e * 16], yw[e]);
-            else a0 = a0 - cmul(Lr[e * 16], yw[e]);
-          }
-          const double2 acc = (a0 - a1) - cmul(Lr[(KLV - 1) * 16], yw[KLV - 1]);
-          S[32 * i] = acc;
-#pragma unroll
-          for (int e = 0; e < KLV - 1; ++e) yw[e] = yw[e + 1];
-          yw[KLV - 1] = acc;
+        for (int e = 0; e < KLV - 1; ++e) {
+          if (e & 1) a1 = cfms(Lr[e * 16], yw[e], a1);
+          else a0 = cfms(Lr[e * 16], yw[e], a0);
         }
+        const double2 acc = cfms(Lr[(KLV - 1) * 16], yw[KLV - 1], a0 + a1);
+        Sr[32 * rr] = acc;
+#pragma unroll
+        for (int e = 0; e < KLV - 1; ++e) yw[e] = yw[e + 1];
+        yw[KLV - 1] = acc;
       }
-      release(c);
+    };
+    int r0 = 0;
+    for (; r0 + R <= nv; r0 += R, ++c) {
+      if (!wait_chunk(c)) { abort_at(c); return; }
+      chunk(Whole(), chunk_at(c), r0);
+      release();
+    }
+    if (r0 < nv) {
+      if (!wait_chunk(c)) { abort_at(c); return; }
+      chunk(Part(), chunk_at(c), r0);
+      release();
+      ++c;
     }
   }
   // ---- v: back substitution, recombination, tilting term -----------------
-  // rows descend; a chunk's rows are loaded one chunk ahead.  The tilting
-  // term of row k+1 is written over rows already consumed (k + 1 > i).
+  // rows descend.  The tilting term of row k+1 is written over rows already
+  // consumed (k + 1 > i).
   {
     constexpr int R = CF::R1;
-    double2 xw[KUV];
+    double2 xw[KUV], cur[R];
 #pragma unroll
     for (int e = 0; e < KUV; ++e) xw[e] = z2;
     double2 xd0 = z2, xd1 = z2;
     double2 P[7];  // P[j]: partial tilting sum of row k+1-j, k = next coefficient emitted
 #pragma unroll
     for (int j = 0; j < 7; ++j) P[j] = z2;
-    const int nbv = zero ? N - 1 : N - 3;
     // base-flow degree (KLV = deg U + 4): U' = U1 (degree 1) makes the
     // tilting operator B^2 U1, three diagonals; U' = 0 (degree 0) none
     constexpr int DEG = KLV - 4;
-    auto emit = [&](int k, double2 a) {
-      if (active) V[pen * Ny + k] = a;
+    // coefficient k into the tilting sums, row k + 1 of the term out; the
+    // table has zero rows around it (FIRST: rows below 0 beyond those)
+    auto tilt = [&](int k, double2 a, bool first) {
 #pragma unroll
       for (int j = 0; j < 7; ++j) {
         if (DEG == 0 || (DEG == 1 && (j & 1) == 0)) continue;
         const int r = k + 1 - j;
-        if (r >= 0 && r < wd.no) P[j] = P[j] + a * (QSM ? Qs[7 * r + j] : __ldg(Qs + 7 * r + j));
+        if (!first || r >= 0) P[j] = rfma(QSM ? Qs[7 * r + j] : __ldg(Qs + 7 * r + j), a, P[j]);
       }
-      if (k + 1 < wd.no) S[32 * (k + 1)] = muli(P[0] * kap);
+      if (k + 1 < no) S[32 * (k + 1)] = make_double2(-P[0].y * kap, P[0].x * kap);
 #pragma unroll
       for (int j = 0; j < 6; ++j) P[j] = P[j + 1];
       P[6] = z2;
     };
-    double2 nxt[R];
 #pragma unroll
-    for (int rr = 0; rr < R; ++rr) nxt[rr] = lds(wd.nv - 1 - rr);
-    for (int r0 = 0; r0 < wd.nv; r0 += R, ++c) {
-      double2 cur[R];
-#pragma unroll
-      for (int rr = 0; rr < R; ++rr) {
-        cur[rr] = nxt[rr];
-        nxt[rr] = lds(wd.nv - 1 - (r0 + R + rr));
-      }
-      if (!wait_chunk(c)) { abort_at(c); return; }
-      const double2* ch = ring + (size_t)(c % WALL_NST) * (WALL_STG / 16) + q;
-      const int rows = min(R, wd.nv - r0);
+    for (int rr = 0; rr < R; ++rr) cur[rr] = rr < nv ? S[32 * (nv - 1 - rr)] : z2;
+    double2* Vp = V + pen * Ny + (zero ? 2 : 4);  // row i emits coefficient i + 4, of the mean modes i + 2
+    const int top = zero ? N - 2 : N - 4;         // the last row that emits one
+    auto chunk = [&](auto whole, const double2* ch, int r0) {
+      const int i0 = nv - 1 - r0;
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
-        if (rr < rows) {
-          const int i = wd.nv - 1 - (r0 + rr);
-          const double2* Ur = ch + rr * CF::E1 * 16;
-          const double2 a0 = cur[rr];
-          if (i >= N + 2) S[32 * i] = z2;  // no tilting term above row N+1
-          // independent partial sums; x_{i+1} enters last
-          double2 a1 = cmul(Ur[(KUV + 1) * 16], xd0) + cmul(Ur[(KUV + 2) * 16], xd1);
-          double2 a2 = z2;
+        if (!whole.full && r0 + rr >= nv) continue;
+        const int i = i0 - rr;
+        const double2* Ur = ch + rr * CF::E1 * 16;
+        double2 a0 = cur[rr];
+        if (whole.full) cur[rr] = i >= R ? S[32 * (i - R)] : z2;
+        // independent partial sums; x_{i+1} enters last
+        double2 a1 = z2, a2 = z2;
+        a1 = cfms(Ur[(KUV + 1) * 16], xd0, a1);
+        a2 = cfms(Ur[(KUV + 2) * 16], xd1, a2);
 #pragma unroll
-          for (int e = KUV; e >= 2; --e) {
-            if (e & 1) a1 = a1 + cmul(Ur[e * 16], xw[e - 1]);
-            else a2 = a2 + cmul(Ur[e * 16], xw[e - 1]);
-          }
-          const double2 acc = (a0 - (a1 + a2)) - cmul(Ur[16], xw[0]);
-          const double2 x = cmul(Ur[0], acc);
-          if (i == wd.nv - 1) xd1 = x;
-          if (i == wd.nv - 2) xd0 = x;
-#pragma unroll
-          for (int e = KUV - 1; e >= 1; --e) xw[e] = xw[e - 1];
-          xw[0] = x;
-          if (i < nbv) {
-            if (!zero) {
-              const int k = i + 4;
-              emit(k, sel(i + 4 < nbv, xw[4]) - sel(i + 2 < nbv, xw[2]) * rc2[k] + x * rc4[k]);
-            } else {
-              emit(i + 2, x - sel(i + 2 < nbv, xw[2]));
-            }
-          }
+        for (int e = KUV; e >= 2; --e) {
+          if (e % 3 == 0) a1 = cfms(Ur[e * 16], xw[e - 1], a1);
+          else if (e % 3 == 1) a2 = cfms(Ur[e * 16], xw[e - 1], a2);
+          else a0 = cfms(Ur[e * 16], xw[e - 1], a0);
         }
+        const double2 acc = cfms(Ur[16], xw[0], a0 + (a1 + a2));
+        const double2 x = cmul(Ur[0], acc);
+        // the two unknowns with dense columns
+        if (rr == 0 && r0 == 0) xd1 = x;
+        if (rr == 1 && r0 == 0) xd0 = x;
+#pragma unroll
+        for (int e = KUV - 1; e >= 1; --e) xw[e] = xw[e - 1];
+        xw[0] = x;
+        double w2 = rc2[i], w4 = rc4[i], w0 = i + 4 < N - 3 ? 1.0 : 0.0;
+        if (mean && zero) {
+          w2 = i + 2 < N - 1 ? 1.0 : 0.0;
+          w4 = i < N - 1 ? 1.0 : 0.0;
+          w0 = 0.0;
+        }
+        const double2 a = rfma(w4, x, rfma(-w2, xw[2], xw[4] * w0));
+        if (active && i <= top) Vp[i] = a;
+        tilt(i + 4, a, false);
       }
-      release(c);
+    };
+    int r0 = 0;
+    for (; r0 + R <= nv; r0 += R, ++c) {
+      if (!wait_chunk(c)) { abort_at(c); return; }
+      chunk(Whole(), chunk_at(c), r0);
+      release();
     }
-    if (!zero) {
-      emit(3, xw[3] - xw[1] * 1.5);
-      emit(2, xw[2] - xw[0] * (4.0 / 3.0));
-      emit(1, xw[1]);
-      emit(0, xw[0]);
-    } else {
-      emit(1, make_double2(-xw[1].x, -xw[1].y));
-      emit(0, make_double2(-xw[0].x, -xw[0].y));
+    if (r0 < nv) {
+      if (!wait_chunk(c)) { abort_at(c); return; }
+      chunk(Part(), chunk_at(c), r0);
+      release();
+      ++c;
     }
-    S[0] = muli(P[0] * kap);
+    double2 a[4];
+    a[3] = xw[3] - xw[1] * 1.5;
+    a[2] = xw[2] - xw[0] * (4.0 / 3.0);
+    a[1] = xw[1];
+    a[0] = xw[0];
+    if (zero) {
+      a[1] = make_double2(-xw[1].x, -xw[1].y);
+      a[0] = make_double2(-xw[0].x, -xw[0].y);
+    }
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+      if (active && !(zero && k > 1)) V[pen * Ny + k] = a[k];
+      tilt(k, a[k], true);
+    }
+    S[0] = make_double2(-P[0].y * kap, P[0].x * kap);
   }
   // ---- omega: forward substitution (adds g_o to the tilting term) --------
   {
     constexpr int R = CF::R2;
-    double2 ow[KLO];
+    double2 ow[KLO], gc[R], sc[R];
 #pragma unroll
     for (int e = 0; e < KLO; ++e) ow[e] = z2;
-    double2 gnext[R], snext[R];
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) {
-      gnext[rr] = (active && rr < wd.no) ? __ldg(gop + rr) : z2;
-      snext[rr] = (rr < wd.no) ? lds(rr) : z2;
+      gc[rr] = (active && rr < no) ? __ldg(gop + rr) : z2;
+      sc[rr] = rr < no ? S[32 * rr] : z2;
     }
-    for (int r0 = 0; r0 < wd.no; r0 += R, ++c) {
-      double2 gcur[R], scur[R];
+    auto chunk = [&](auto whole, const double2* ch, int r0) {
+      const double2* nx = gop + r0 + R;
+      double2* Sr = S + 32 * r0;
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
-        gcur[rr] = gnext[rr];
-        scur[rr] = snext[rr];
-        const int i = r0 + R + rr;
-        gnext[rr] = (active && i < wd.no) ? __ldg(gop + i) : z2;
-        snext[rr] = (i < wd.no) ? lds(i) : z2;
-      }
-      if (!wait_chunk(c)) { abort_at(c); return; }
-      const double2* ch = ring + (size_t)(c % WALL_NST) * (WALL_STG / 16) + q;
-      const int rows = min(R, wd.no - r0);
-#pragma unroll
-      for (int rr = 0; rr < R; ++rr) {
-        if (rr < rows) {
-          const int i = r0 + rr;
-          const double2* Lr = ch + rr * CF::E2 * 16;
-          double2 a0 = scur[rr] + gcur[rr], a1 = z2;
-#pragma unroll
-          for (int e = 0; e < KLO - 1; ++e) {
-            if (e & 1) a1 = a1 + cmul(Lr[e * 16], ow[e]);
-            else a0 = a0 - cmul(Lr[e * 16], ow[e]);
-          }
-          const double2 acc = (a0 - a1) - cmul(Lr[(KLO - 1) * 16], ow[KLO - 1]);
-          S[32 * i] = acc;
-#pragma unroll
-          for (int e = 0; e < KLO - 1; ++e) ow[e] = ow[e + 1];
-          ow[KLO - 1] = acc;
+        if (!whole.full && r0 + rr >= no) continue;
+        const double2* Lr = ch + rr * CF::E2 * 16;
+        double2 a0 = sc[rr] + gc[rr];
+        if (whole.full) {
+          const bool more = r0 + R + rr < no;
+          gc[rr] = (active && more) ? __ldg(nx + rr) : z2;
+          sc[rr] = more ? Sr[32 * (R + rr)] : z2;
         }
+        double2 a1 = z2;
+#pragma unroll
+        for (int e = 0; e < KLO - 1; ++e) {
+          if (e & 1) a1 = cfms(Lr[e * 16], ow[e], a1);
+          else a0 = cfms(Lr[e * 16], ow[e], a0);
+        }
+        const double2 acc = cfms(Lr[(KLO - 1) * 16], ow[KLO - 1], a0 + a1);
+        Sr[32 * rr] = acc;
+#pragma unroll
+        for (int e = 0; e < KLO - 1; ++e) ow[e] = ow[e + 1];
+        ow[KLO - 1] = acc;
       }
-      release(c);
+    };
+    int r0 = 0;
+    for (; r0 + R <= no; r0 += R, ++c) {
+      if (!wait_chunk(c)) { abort_at(c); return; }
+      chunk(Whole(), chunk_at(c), r0);
+      release();
+    }
+    if (r0 < no) {
+      if (!wait_chunk(c)) { abort_at(c); return; }
+      chunk(Part(), chunk_at(c), r0);
+      release();
+      ++c;
     }
   }
   // ---- omega: back substitution and recombination ------------------------
   {
     constexpr int R = CF::R3;
-    double2 zw[KUO];
+    double2 zw[KUO], cur[R];
 #pragma unroll
     for (int e = 0; e < KUO; ++e) zw[e] = z2;
     const int nbo = N - 1;
-    double2 nxt[R];
+    double2* Op = O + pen * Ny + 2;
 #pragma unroll
-    for (int rr = 0; rr < R; ++rr) nxt[rr] = (rr < wd.no) ? lds(wd.no - 1 - rr) : z2;
-    for (int r0 = 0; r0 < wd.no; r0 += R, ++c) {
-      double2 cur[R];
-#pragma unroll
-      for (int rr = 0; rr < R; ++rr) {
-        cur[rr] = nxt[rr];
-        nxt[rr] = lds(wd.no - 1 - (r0 + R + rr));
-      }
-      if (!wait_chunk(c)) { abort_at(c); return; }
-      const double2* ch = ring + (size_t)(c % WALL_NST) * (WALL_STG / 16) + q;
-      const int rows = min(R, wd.no - r0);
+    for (int rr = 0; rr < R; ++rr) cur[rr] = rr < no ? S[32 * (no - 1 - rr)] : z2;
+    auto chunk = [&](auto whole, const double2* ch, int r0) {
+      const int i0 = no - 1 - r0;
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
-        if (rr < rows) {
-          const int i = wd.no - 1 - (r0 + rr);
-          const double2* Ur = ch + rr * CF::E3 * 16;
-          double2 a1 = z2, a2 = z2;
+        if (!whole.full && r0 + rr >= no) continue;
+        const int i = i0 - rr;
+        const double2* Ur = ch + rr * CF::E3 * 16;
+        double2 a0 = cur[rr], a1 = z2;
+        if (whole.full) cur[rr] = i >= R ? S[32 * (i - R)] : z2;
 #pragma unroll
-          for (int e = KUO; e >= 2; --e) {
-            if (e & 1) a1 = a1 + cmul(Ur[e * 16], zw[e - 1]);
-            else a2 = a2 + cmul(Ur[e * 16], zw[e - 1]);
-          }
-          const double2 acc = (cur[rr] - (a1 + a2)) - cmul(Ur[16], zw[0]);
-          const double2 x = cmul(Ur[0], acc);
-#pragma unroll
-          for (int e = KUO - 1; e >= 1; --e) zw[e] = zw[e - 1];
-          zw[0] = x;
-          if (i < nbo && active) O[pen * Ny + i + 2] = x - sel(i + 2 < nbo, zw[2]);
+        for (int e = KUO; e >= 2; --e) {
+          if (e & 1) a1 = cfms(Ur[e * 16], zw[e - 1], a1);
+          else a0 = cfms(Ur[e * 16], zw[e - 1], a0);
         }
+        const double2 acc = cfms(Ur[16], zw[0], a0 + a1);
+        const double2 x = cmul(Ur[0], acc);
+#pragma unroll
+        for (int e = KUO - 1; e >= 1; --e) zw[e] = zw[e - 1];
+        zw[0] = x;
+        if (active && i < nbo) Op[i] = rfma(i + 2 < nbo ? -1.0 : 0.0, zw[2], x);
       }
-      release(c);
+    };
+    int r0 = 0;
+    for (; r0 + R <= no; r0 += R, ++c) {
+      if (!wait_chunk(c)) { abort_at(c); return; }
+      chunk(Whole(), chunk_at(c), r0);
+      release();
+    }
+    if (r0 < no) {
+      if (!wait_chunk(c)) { abort_at(c); return; }
+      chunk(Part(), chunk_at(c), r0);
+      release();
+      ++c;
     }
     if (active) {
       O[pen * Ny + 1] = make_double2(-zw[1].x, -zw[1].y);

@@ -3,6 +3,11 @@
 #pragma once
 #include "kernels.cuh"
 
+// rows of the tilting table: zero rows below 0 and above the last, so that
+// the solve reads it without bounds checks
+#define WALL_QLOW 2
+#define WALL_QROWS(no) ((no) + WALL_QLOW + 8)
+
 struct WallDims {
   int nv, no;              // rows of the packed v and omega systems (N + deg U + 1)
   int delta;               // base-flow degree: selects the band instance
