@@ -340,6 +340,14 @@ void default_variants(dns_ctx* c) {
     for (int i = skip; i < 3 && ord[i] >= 0; ++i)
       if (variant_available(c, p, ord[i])) { c->variant[p] = ord[i]; break; }
   }
+  // the solve: more groups than four CTAs per SM take run in one wave with
+  // the small ring, as long as their scratch vectors stay in L2 (us, 3 x 12 KB
+  // / 2 x 8 KB, evict-first: 1041 groups of 33 points 80 / 70, 828 of 49 points
+  // 100 / 85; 1041 of 129 points, 70 MB of scratch, 249 / 297)
+  const long long groups = ((long long)c->g.Kx * (c->slab ? c->slab->s1 - c->slab->s0 : c->g.Kh) + 15) / 16 * c->g.nrun;
+  if (groups > 4 * 148 && groups * 32 * c->wd.nv * 16 <= (40LL << 20) &&
+      variant_available(c, DNS_PASS_Y2, DNS_Y2_RING2_8K_EF))
+    c->variant[DNS_PASS_Y2] = DNS_Y2_RING2_8K_EF;
 }
 // the spanwise variant of the FP64 per-function entries: the context's own
 // in the FP64 form, else the first that the length allows
