@@ -355,9 +355,14 @@ int zvar64(const dns_ctx* c, int pass) {
   return c->P.precision == DNS_PREC_FP64 ? c->variant[pass] : VAR_AUTO;
 }
 
+// streamwise rows of the reference-layout transforms: one field, or as many
+// (up to the six of a getUVW) as 64 MB hold, so that small fields share launches
 dns_status need_scratch(dns_ctx* c) {
   if (c->scratch) return DNS_OK;
-  CK(c->alloc(&c->scratch, (size_t)c->g.Py * c->g.Pz * c->RS));
+  const size_t one = (size_t)c->g.Py * c->g.Pz * c->RS;
+  const int n = (int)std::max<size_t>(1, std::min<size_t>(6, ((size_t)64 << 20) / (one * 16)));
+  CK(c->alloc(&c->scratch, one * n));
+  c->scratch_fields = n;
   return DNS_OK;
 }
 
@@ -677,44 +682,43 @@ dns_status dns_get_state(dns_ctx* c, void* v, void* o, size_t pitch, int where) 
 
 // The AB2 history is held as Chebyshev coefficients; the ABI exchanges it
 // as values at the Gauss-Lobatto points (the reference's rhs_v_p /
-// rhs_omega_y_p), converted here with the no-pad s2p / p2s.
-// (k_cheby_inplace writes whole FFT lines, so the scratch pencils have
-// pitch mz/2 >= the no-pad FFT length.)
-static dns_status history_out(dns_ctx* c, const double2* src, void* dst, size_t pitch, int where) {
-  dns_status s = need_scratch(c);
-  if (s) return s;
-  const size_t w = (size_t)c->g.Ny * 16, ps = (size_t)(c->P.mz / 2);
+// rhs_omega_y_p), converted here with the no-pad s2p / p2s: on device pencils
+// straight between the caller's and the library's, on host pencils through the
+// scratch, member by member of a batch.
+static dns_status history_copy(dns_ctx* c, double2* hist, void* user, size_t pitch, int where, bool out) {
+  const size_t w = (size_t)c->g.Ny * 16;
   if (where != DNS_HOST && where != DNS_DEVICE) return fail(DNS_ERR_ARG, "where must be DNS_HOST or DNS_DEVICE");
   if (pitch < w || pitch % 16) return fail(DNS_ERR_ARG, "pencil pitch must be >= Ny*16 and a multiple of 16");
   const long long H = c->g.H;
-  for (int r = 0; r < c->g.nrun; ++r) {  // a batch: member by member through the scratch
-    CK(cudaMemcpy2DAsync(c->scratch, ps * 16, src + r * H * c->g.Ny, w, w, (size_t)H, cudaMemcpyDeviceToDevice,
-                         c->st));
-    PencilArr a{c->scratch, (long long)ps, 0};
-    CK(launch_cheby_inplace<double2>(a, H, 1, c->g.Ny, c->fy0_d.tab(), c->st));
-    CK(cudaMemcpy2DAsync((char*)dst + (size_t)r * H * pitch, pitch, c->scratch, ps * 16, w, (size_t)H,
-                         kind_of(where, false), c->st));
+  auto convert = [&](double2* h, void* u, long long ups, long long n) {
+    const PencilList lib{{h}, c->g.Ny}, usr{{u}, ups};
+    return launch_cheby(out ? lib : usr, out ? usr : lib, 1, n, out ? 1 : 3, c->g.Ny, c->fy0_d.tab(), false, c->st);
+  };
+  if (where == DNS_DEVICE) {
+    CK(convert(hist, user, (long long)(pitch / 16), H * c->g.nrun));
+  } else {
+    dns_status s = need_scratch(c);
+    if (s) return s;
+    for (int r = 0; r < c->g.nrun; ++r) {
+      double2* h = hist + r * H * c->g.Ny;
+      char* u = (char*)user + (size_t)r * H * pitch;
+      if (out) {
+        CK(convert(h, c->scratch, c->g.Ny, H));
+        CK(cudaMemcpy2DAsync(u, pitch, c->scratch, w, w, (size_t)H, cudaMemcpyDeviceToHost, c->st));
+      } else {
+        CK(cudaMemcpy2DAsync(c->scratch, w, u, pitch, w, (size_t)H, cudaMemcpyHostToDevice, c->st));
+        CK(convert(h, c->scratch, c->g.Ny, H));
+      }
+    }
   }
   CK(cudaStreamSynchronize(c->st));
   return DNS_OK;
 }
+static dns_status history_out(dns_ctx* c, const double2* src, void* dst, size_t pitch, int where) {
+  return history_copy(c, (double2*)src, dst, pitch, where, true);
+}
 static dns_status history_in(dns_ctx* c, double2* dst, const void* src, size_t pitch, int where) {
-  dns_status s = need_scratch(c);
-  if (s) return s;
-  const size_t w = (size_t)c->g.Ny * 16, ps = (size_t)(c->P.mz / 2);
-  if (where != DNS_HOST && where != DNS_DEVICE) return fail(DNS_ERR_ARG, "where must be DNS_HOST or DNS_DEVICE");
-  if (pitch < w || pitch % 16) return fail(DNS_ERR_ARG, "pencil pitch must be >= Ny*16 and a multiple of 16");
-  const long long H = c->g.H;
-  for (int r = 0; r < c->g.nrun; ++r) {
-    CK(cudaMemcpy2DAsync(c->scratch, ps * 16, (const char*)src + (size_t)r * H * pitch, pitch, w, (size_t)H,
-                         kind_of(where, true), c->st));
-    PencilArr a{c->scratch, (long long)ps, 0};
-    CK(launch_cheby_inplace<double2>(a, H, 3, c->g.Ny, c->fy0_d.tab(), c->st));
-    CK(cudaMemcpy2DAsync(dst + r * H * c->g.Ny, w, c->scratch, ps * 16, w, (size_t)H, cudaMemcpyDeviceToDevice,
-                         c->st));
-  }
-  CK(cudaStreamSynchronize(c->st));
-  return DNS_OK;
+  return history_copy(c, dst, (void*)src, pitch, where, false);
 }
 
 dns_status dns_get_history(dns_ctx* c, void* nv, void* no, size_t pitch, int where) {
@@ -990,43 +994,54 @@ static dns_status check_phys_pitch(dns_ctx* c, size_t pitch) {
   return DNS_OK;
 }
 
-dns_status dns_transform_3d_one(dns_ctx* c, int dir, void* phys, size_t pitch, void* spec,
-                                size_t tpitch, int pad) {
-  if (!c || !phys || !spec) return fail(DNS_ERR_ARG, "null argument");
+// nf fields, as many a launch as the scratch holds
+static dns_status transform_fields(dns_ctx* c, int dir, int nf, void* const* phys, size_t pitch, void* const* spec,
+                                   size_t tpitch, int pad) {
   if ((dir != DNS_FORWARD && dir != DNS_BACKWARD) || (pad != DNS_PADDING && pad != DNS_NO_PADDING))
     return fail(DNS_ERR_ARG, "bad direction or padding mode");
+  for (int i = 0; i < nf; ++i)
+    if (!phys[i] || !spec[i]) return fail(DNS_ERR_ARG, "null argument");
   dns_status s;
   if ((s = check_spec_pitch(c, tpitch)) || (s = check_phys_pitch(c, pitch))) return s;
   if ((s = need_scratch(c))) return s;
   CK(cudaSetDevice(c->P.device));
   const DnsGeom& g = c->g;
-  PencilArr sp{spec, (long long)(tpitch / 16), 0};
-  RowArr sr{c->scratch, c->RS, 0};
-  const long long nrows = (long long)g.Py * g.Pz;
-  const long long rps = (long long)(pitch / 8);
-  if (dir == DNS_BACKWARD) {
-    if (pad == DNS_PADDING) CK(launch_cheby_inplace<double2>(sp, g.H, 0, g.Ny, c->fyP_d.tab(), c->st));
-    else CK(launch_cheby_inplace<double2>(sp, g.H, 1, g.Ny, c->fy0_d.tab(), c->st));
-    CK(launch_zb<double2>(sp, sr, 1, g, c->fz_d.tab(), c->st, nullptr, zvar64(c, DNS_PASS_ZB)));
-    CK(launch_x_c2r<double2>(sr, (double*)phys, rps, nrows, g, c->fx_d.tab(), c->st));
-  } else {
-    CK(launch_x_r2c<double2>((const double*)phys, rps, sr, nrows, g, c->fx_d.tab(),
-                             1.0 / g.Px / g.Pz, c->st));
-    CK(launch_zf<double2>(sr, sp, 1, g, c->fz_d.tab(), c->st, nullptr, zvar64(c, DNS_PASS_ZF)));
-    if (pad == DNS_PADDING) CK(launch_cheby_inplace<double2>(sp, g.H, 2, g.Ny, c->fyP_d.tab(), c->st));
-    else CK(launch_cheby_inplace<double2>(sp, g.H, 3, g.Ny, c->fy0_d.tab(), c->st));
+  const long long nrows = (long long)g.Py * g.Pz, rps = (long long)(pitch / 8);
+  const RowArr sr{c->scratch, c->RS, nrows * c->RS};
+  const FftTab<double2> ty = pad == DNS_PADDING ? c->fyP_d.tab() : c->fy0_d.tab();
+  const int mode = (dir == DNS_BACKWARD ? 0 : 2) + (pad == DNS_PADDING ? 0 : 1);
+  for (int f = 0; f < nf; f += c->scratch_fields) {
+    const int n = std::min(nf - f, c->scratch_fields);
+    PencilList sp{{}, (long long)(tpitch / 16)};
+    FieldList ph{};
+    for (int i = 0; i < n; ++i) {
+      sp.f.p[i] = spec[f + i];
+      ph.p[i] = phys[f + i];
+    }
+    // (the no-pad backward pass reads planes beyond the Ny points: the tail of the lines)
+    if (dir == DNS_BACKWARD) {
+      CK(launch_cheby(sp, sp, n, g.H, mode, g.Ny, ty, pad == DNS_NO_PADDING, c->st));
+      CK(launch_zb_fields(sp, sr, n, g, c->fz_d.tab(), c->st, zvar64(c, DNS_PASS_ZB)));
+      CK(launch_x_c2r(sr, ph, n, rps, nrows, g, c->fx_d.tab(), c->st));
+    } else {
+      CK(launch_x_r2c(ph, n, rps, sr, nrows, g, c->fx_d.tab(), 1.0 / g.Px / g.Pz, c->st));
+      CK(launch_zf_fields(sr, sp, n, g, c->fz_d.tab(), c->st, zvar64(c, DNS_PASS_ZF)));
+      CK(launch_cheby(sp, sp, n, g.H, mode, g.Ny, ty, false, c->st));
+    }
   }
   return DNS_OK;
+}
+
+dns_status dns_transform_3d_one(dns_ctx* c, int dir, void* phys, size_t pitch, void* spec,
+                                size_t tpitch, int pad) {
+  if (!c || !phys || !spec) return fail(DNS_ERR_ARG, "null argument");
+  return transform_fields(c, dir, 1, &phys, pitch, &spec, tpitch, pad);
 }
 
 dns_status dns_transform(dns_ctx* c, int dir, int nf, void* const* phys, size_t pitch,
                          void* const* spec, size_t tpitch) {
   if (!c || !phys || !spec || nf < 1 || nf > 6) return fail(DNS_ERR_ARG, "bad arguments");
-  for (int i = 0; i < nf; ++i) {
-    dns_status s = dns_transform_3d_one(c, dir, phys[i], pitch, spec[i], tpitch, DNS_PADDING);
-    if (s) return s;
-  }
-  return DNS_OK;
+  return transform_fields(c, dir, nf, phys, pitch, spec, tpitch, DNS_PADDING);
 }
 
 dns_status dns_cuda_transpose(dns_ctx* c, int dir, void* xyz, size_t pitch, void* zxy, size_t tpitch) {
@@ -1046,10 +1061,10 @@ static dns_status cheby_call(dns_ctx* c, void* zxy, size_t tpitch, int pad, bool
   dns_status s = check_spec_pitch(c, tpitch);
   if (s) return s;
   CK(cudaSetDevice(c->P.device));
-  PencilArr sp{zxy, (long long)(tpitch / 16), 0};
+  const PencilList sp{{zxy}, (long long)(tpitch / 16)};
   const int mode = (s2p ? 0 : 2) + (pad == DNS_PADDING ? 0 : 1);
   const DevFft<double2>& t = (pad == DNS_PADDING) ? c->fyP_d : c->fy0_d;
-  CK(launch_cheby_inplace<double2>(sp, c->g.H, mode, c->g.Ny, t.tab(), c->st));
+  CK(launch_cheby(sp, sp, 1, c->g.H, mode, c->g.Ny, t.tab(), true, c->st));
   return DNS_OK;
 }
 dns_status dns_cheby_s2p(dns_ctx* c, void* zxy, size_t tpitch, int pad) { return cheby_call(c, zxy, tpitch, pad, true); }
@@ -1194,7 +1209,8 @@ cudaError_t enqueue_solve_wall(dns_ctx* c, const double2* bv, const double2* bo,
                                       c->fy0_d.tab(), c->status, c->st);
   if (e == cudaErrorNotSupported) {
     e = launch_colloc_prep(bv, bo, bp, sv, so, ls, pbc, cosk, c->Ut, c->ddUt, g, c->ph, c->st);
-    if (!e) e = launch_cheby_inplace<double2>(PencilArr{sv, ls, 0}, 2 * g.H, 3, g.Ny, c->fy0_d.tab(), c->st);
+    const PencilList lines{{sv, so}, ls};
+    if (!e) e = launch_cheby(lines, lines, 2, g.H, 3, g.Ny, c->fy0_d.tab(), false, c->st);
     if (!e) e = launch_colloc_integrate(sv, so, ls, c->rv, c->ro, c->wd, g, c->st);
   }
   WallDims wd = c->wd;

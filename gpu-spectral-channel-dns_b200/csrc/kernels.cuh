@@ -39,6 +39,17 @@ struct PencilArr {      // generic pencil-major array
   long long fs;         // field stride (elements)
 };
 
+struct FieldList {      // up to six fields, anywhere
+  void* p[6];
+};
+struct PencilList {     // pencil-major fields, anywhere
+  FieldList f;
+  long long ps;         // pencil pitch (elements)
+};
+// field f of either form
+template <typename C> DNS_HD C* field_base(const PencilArr& a, int f) { return (C*)a.base + (long long)f * a.fs; }
+template <typename C> DNS_HD C* field_base(const PencilList& a, int f) { return (C*)a.f.p[f]; }
+
 struct RowArr {         // generic row-major [field][y][zp][kx] array
   void* base;
   long long rs;         // row pitch (elements)

@@ -101,35 +101,35 @@ extern "C" dns_status dns_transform_3d_one_noalloc(dns_ctx* c, int dir, void* ph
   const int S = (int)(DNS_NOALLOC_SCRATCH_BYTES / plane_bytes);
   const long long ps = (long long)(tpitch / 16);
   const long long rps = (long long)(pitch / 8);
-  PencilArr sp{spec, ps, 0};
+  const PencilList sp{{spec}, ps};
   RowArr sr{scr, c->RS, 0};
   auto ck = [&](cudaError_t err) { return err == cudaSuccess ? DNS_OK : fail(DNS_ERR_CUDA, cudaGetErrorString(err)); };
   dns_status st = DNS_OK;
   if (dir == DNS_BACKWARD) {
-    if (pad == DNS_PADDING) st = ck(launch_cheby_inplace<double2>(sp, g.H, 0, g.Ny, c->fyP_d.tab(), c->st));
-    else st = ck(launch_cheby_inplace<double2>(sp, g.H, 1, g.Ny, c->fy0_d.tab(), c->st));
+    if (pad == DNS_PADDING) st = ck(launch_cheby(sp, sp, 1, g.H, 0, g.Ny, c->fyP_d.tab(), false, c->st));
+    else st = ck(launch_cheby(sp, sp, 1, g.H, 1, g.Ny, c->fy0_d.tab(), true, c->st));
     for (int y0 = 0; y0 < g.Py && st == DNS_OK; y0 += S) {
       DnsGeom gs = g;
       gs.Py = (g.Py - y0 < S) ? g.Py - y0 : S;
-      PencilArr slab_in{(double2*)spec + y0, ps, 0};
+      const PencilList slab_in{{(double2*)spec + y0}, ps};
       double* out = (double*)phys + (long long)y0 * g.Pz * rps;
-      st = ck(launch_zb<double2>(slab_in, sr, 1, gs, c->fz_d.tab(), c->st, nullptr));
+      st = ck(launch_zb_fields(slab_in, sr, 1, gs, c->fz_d.tab(), c->st));
       if (st == DNS_OK)
-        st = ck(launch_x_c2r<double2>(sr, out, rps, (long long)gs.Py * g.Pz, gs, c->fx_d.tab(), c->st));
+        st = ck(launch_x_c2r(sr, FieldList{{out}}, 1, rps, (long long)gs.Py * g.Pz, gs, c->fx_d.tab(), c->st));
     }
   } else {
     for (int y0 = 0; y0 < g.Py && st == DNS_OK; y0 += S) {
       DnsGeom gs = g;
       gs.Py = (g.Py - y0 < S) ? g.Py - y0 : S;
       const double* in = (const double*)phys + (long long)y0 * g.Pz * rps;
-      PencilArr slab_out{(double2*)spec + y0, ps, 0};
-      st = ck(launch_x_r2c<double2>(in, rps, sr, (long long)gs.Py * g.Pz, gs, c->fx_d.tab(),
+      const PencilList slab_out{{(double2*)spec + y0}, ps};
+      st = ck(launch_x_r2c(FieldList{{(void*)in}}, 1, rps, sr, (long long)gs.Py * g.Pz, gs, c->fx_d.tab(),
                                      1.0 / g.Px / g.Pz, c->st));
-      if (st == DNS_OK) st = ck(launch_zf<double2>(sr, slab_out, 1, gs, c->fz_d.tab(), c->st, nullptr));
+      if (st == DNS_OK) st = ck(launch_zf_fields(sr, slab_out, 1, gs, c->fz_d.tab(), c->st));
     }
     if (st == DNS_OK) {
-      if (pad == DNS_PADDING) st = ck(launch_cheby_inplace<double2>(sp, g.H, 2, g.Ny, c->fyP_d.tab(), c->st));
-      else st = ck(launch_cheby_inplace<double2>(sp, g.H, 3, g.Ny, c->fy0_d.tab(), c->st));
+      if (pad == DNS_PADDING) st = ck(launch_cheby(sp, sp, 1, g.H, 2, g.Ny, c->fyP_d.tab(), false, c->st));
+      else st = ck(launch_cheby(sp, sp, 1, g.H, 3, g.Ny, c->fy0_d.tab(), false, c->st));
     }
   }
   return st;

@@ -29,6 +29,8 @@ template <int M> struct DPlan { enum { ok = 0, A = 2, B = 2 }; };
     enum { ok = 1, A = RA, B = RB };                                                          \
     static_assert(RA * RB == M && RA % 2 == 0 && RB % 2 == 0 && M % 4 == 0, "plan");          \
   };
+DPLAN(16, 4, 4)
+DPLAN(24, 6, 4)
 DPLAN(32, 8, 4)
 DPLAN(36, 6, 6)
 DPLAN(48, 8, 6)
@@ -53,12 +55,15 @@ DPLAN(768, 32, 24)
   X(32) X(36) X(48) X(64) X(72) X(96) X(108) X(128) X(144) X(192) X(216) X(256) X(288) X(324) X(384) X(432) \
   X(512) X(576) X(768)
 
+// lengths of the no-padding transforms only
+#define DPLAN_SHORT(X) X(16) X(24)
+
 // pass-B twiddles W_M^{j s}, j = 1..RB/2, s = 0..RA/2, stored [j - 1][s]
 template <typename C> int dtw_table(int M, std::vector<C>& out) {
   int ra = 0, rb = 0;
 #define DCASE(n) \
   case n: ra = DPlan<n>::A; rb = DPlan<n>::B; break;
-  switch (M) { DPLAN_LENGTHS(DCASE) default: return -1; }
+  switch (M) { DPLAN_SHORT(DCASE) DPLAN_LENGTHS(DCASE) default: return -1; }
 #undef DCASE
   const long double PI = 3.141592653589793238462643383279502884L;
   const int sh = ra / 2 + 1;

@@ -137,59 +137,77 @@ __device__ __forceinline__ C* pencil_ptr(const PencilArr& a, int f, long long p)
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Reference-layout in-place Chebyshev transforms (drop-in cheby_s2p/p2s)
+// Reference-layout Chebyshev transforms (drop-in cheby_s2p/p2s)
 // mode 0: s2p pad (FFT length mz), 1: s2p no-pad (mz/2),
 // mode 2: p2s pad (mz), 3: p2s no-pad (mz/2).
 // ---------------------------------------------------------------------------
-template <typename C>
-__global__ void k_cheby_inplace(PencilArr arr, long long npencils, int mode, int Ny,
-                                FftTab<C> tab, int PB) {
+__global__ void k_cheby(PencilList in, PencilList out, long long npencils, int mode, int Ny, FftTab<double2> tab,
+                        int PB, int nout) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* lines = (C*)smem_raw;
-  const int L = tab.plan.L;
+  double2* lines = (double2*)smem_raw;
+  const int L = tab.plan.L, H = L / 2;
   const long long p0 = (long long)blockIdx.x * PB;
-  const int P = (mode == 2) ? L / 2 + 1 : Ny;  // p2s input points
   for (int w = threadIdx.x; w < PB * L; w += blockDim.x) {
     const int b = w / L;
     const int n = w - b * L;
     const long long p = p0 + b;
-    C val = cmk<C>(0.0, 0.0);
+    double2 val = make_double2(0.0, 0.0);
     if (p < npencils) {
-      const C* src = pencil_ptr<C>(arr, 0, p);
+      const double2* src = field_base<double2>(in, blockIdx.y) + p * in.ps;
+      const int m = n <= H ? n : L - n;  // even extension
       if (mode == 0) {
-        const int nzl = Ny - 1;
-        if (n == 0) val = src[0];
-        else if (n <= nzl) val = src[n] * (decltype(val.x))0.5;
-        else if (n >= L - nzl) val = src[L - n] * (decltype(val.x))0.5;
+        if (m < Ny) val = src[m] * (m ? 0.5 : 1.0);
       } else if (mode == 1) {
-        const int nzl = Ny - 1;
-        if (n == 0) val = src[0];
-        else if (n < nzl) val = src[n] * (decltype(val.x))0.5;
-        else if (n == nzl) val = src[n];
-        else val = src[L - n] * (decltype(val.x))0.5;
+        val = src[m] * (m && m < H ? 0.5 : 1.0);
       } else {
-        const int Pm = (mode == 2) ? P : Ny;
-        val = (n < Pm) ? src[n] : src[L - n];
+        val = src[m];
       }
     }
     lines[(size_t)b * L + tab.drev[n]] = val;
   }
-  fft_batch<C, false>(lines, PB, L, tab.plan, tab.tw);
-  for (int w = threadIdx.x; w < PB * L; w += blockDim.x) {
-    const int b = w / L;
-    const int k = w - b * L;
+  fft_batch<double2, false>(lines, PB, L, tab.plan, tab.tw);
+  for (int w = threadIdx.x; w < PB * nout; w += blockDim.x) {
+    const int b = w / nout;
+    const int k = w - b * nout;
     const long long p = p0 + b;
     if (p >= npencils) continue;
-    C v = lines[(size_t)b * L + k];
-    if (mode >= 2) {
-      const int Pm = L / 2 + 1;
-      if (k < Pm) {
-        v = v * (decltype(v.x))(1.0 / (Pm - 1));
-        if (k == 0 || k == Pm - 1) v = v * (decltype(v.x))0.5;
-      }
-    }
-    pencil_ptr<C>(arr, 0, p)[k] = v;
+    double2 v = lines[(size_t)b * L + k];
+    if (mode >= 2 && k <= H) v = v * (k && k < H ? 1.0 / H : 0.5 / H);
+    (field_base<double2>(out, blockIdx.y) + p * out.ps)[k] = v;
   }
+}
+
+// Same transforms by pruned DCTs (ydct.cuh), six pencils per CTA of two
+// warps; pass A reads the pencils and pass B stores them straight from and to
+// global memory, with a block barrier in between (in place: every input is
+// read before any output is stored).  MODE 3 = 2.  Three fields of 384 x 384 x
+// 512 to points 923 -> 146 us, three of 192 x 192 x 256 to coefficients 130 ->
+// 28, against one barrier and one trip through shared memory per radix 4.
+template <int M, int MODE, int MB>
+__global__ void __launch_bounds__(64, MB) k_cheby_dct(PencilList in, PencilList out, long long npencils, int tail,
+                                                      const double2* __restrict__ dt) {
+  typedef Dct<double2, M, 6> D;
+  constexpr int H = M / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* X = (double2*)smem_raw;
+  const long long p0 = (long long)blockIdx.x * 6;
+  const int np = (int)min(6LL, npencils - p0);
+  const double2* src = field_base<double2>(in, blockIdx.y) + p0 * in.ps;
+  for (int i = threadIdx.x; i < D::IA; i += 64)
+    D::template pass_a<MODE == 0 ? M / 4 + 1 : 0>(X, i, [&](int l, int n) {
+      const double2 v = l < np ? src[l * in.ps + n] : make_double2(0.0, 0.0);
+      if (MODE >= 2) return v;
+      return v * (n && (MODE == 0 || n < H) ? 0.5 : 1.0);
+    });
+  __syncthreads();
+  double2* dst = field_base<double2>(out, blockIdx.y) + p0 * out.ps;
+  for (int i = threadIdx.x; i < D::IB; i += 64)
+    D::pass_b(X, dt, i, [&](int l, int k, double2 v) {
+      if (l >= np) return;
+      double2* d = dst + l * out.ps;
+      if (tail && k && k < H) d[M - k] = v;
+      d[k] = MODE < 2 ? v : v * (k && k < H ? 1.0 / H : 0.5 / H);
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -1113,20 +1131,40 @@ size_t y1_smem(int Ny, int lsP, size_t csz) {
   size_t bp = (size_t)3 * lsP * csz, bi = (size_t)4 * (Ny + 8) * 16;
   return s + a(bp > bi ? bp : bi);
 }
-template <typename C>
-cudaError_t launch_cheby_inplace(PencilArr arr, long long npencils, int mode, int Ny,
-                                 FftTab<C> tab, cudaStream_t st) {
+#define DNS_DCASE(n) case n: return f(std::integral_constant<int, n>());
+template <typename F> cudaError_t with_len_d(int M, F&& f) {
+  switch (M) { DPLAN_LENGTHS(DNS_DCASE) }
+  return cudaErrorNotSupported;
+}
+template <typename F> cudaError_t with_len_cheby(int M, F&& f) {
+  switch (M) { DPLAN_SHORT(DNS_DCASE) DPLAN_LENGTHS(DNS_DCASE) }
+  return cudaErrorNotSupported;
+}
+cudaError_t launch_cheby(PencilList in, PencilList out, int nf, long long npencils, int mode, int Ny,
+                         FftTab<double2> tab, bool tail, cudaStream_t st) {
   const int L = tab.plan.L;
-  int PB = (int)(32768 / ((size_t)L * sizeof(C)));
-  if (PB < 1) PB = 1;
-  if (PB > 8) PB = 8;
-  const size_t sm = (size_t)PB * L * sizeof(C);
-  cudaFuncSetAttribute(k_cheby_inplace<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  const long long nb = (npencils + PB - 1) / PB;
-  k_cheby_inplace<C><<<(unsigned)nb, 256, sm, st>>>(arr, npencils, mode, Ny, tab, PB);
+  // the pruned DCT takes the zeros above Ny = L/4 + 1 as known
+  if (tab.dt && (mode != 0 || Ny == L / 4 + 1)) {
+    const cudaError_t e = with_len_cheby(L, [&](auto MM) -> cudaError_t {
+      constexpr int M = decltype(MM)::value;
+      typedef Dct<double2, M, 6> D;
+      constexpr int MB = D::RA > 24 ? 4 : (D::RA > 18 ? 6 : 8);
+      auto k = mode == 0 ? k_cheby_dct<M, 0, MB> : mode == 1 ? k_cheby_dct<M, 1, MB> : k_cheby_dct<M, 2, MB>;
+      const size_t sm = sizeof(double2) * D::XN;
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      k<<<dim3((unsigned)((npencils + 5) / 6), nf), 64, sm, st>>>(in, out, npencils, tail, tab.dt);
+      return cudaGetLastError();
+    });
+    if (e != cudaErrorNotSupported) return e;
+  }
+  int PB = (int)(32768 / ((size_t)L * 16));
+  PB = PB < 1 ? 1 : (PB > 8 ? 8 : PB);
+  const size_t sm = (size_t)PB * L * 16;
+  cudaFuncSetAttribute(k_cheby, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_cheby<<<dim3((unsigned)((npencils + PB - 1) / PB), nf), 256, sm, st>>>(in, out, npencils, mode, Ny, tab, PB,
+                                                                           tail ? L : L / 2 + 1);
   return cudaGetLastError();
 }
-template cudaError_t launch_cheby_inplace<double2>(PencilArr, long long, int, int, FftTab<double2>, cudaStream_t);
 
 cudaError_t launch_get_uvw(double2* const f[6], long long ps, DnsGeom g, PhysParams ph,
                            cudaStream_t st) {
@@ -1153,12 +1191,6 @@ cudaError_t launch_solve_eq(const double2* inv, double2* rhs, long long ps, int 
   cudaFuncSetAttribute(k_solve_eq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_solve_eq<<<(unsigned)npencils, 256, sm, st>>>(inv, rhs, ps, N, npencils);
   return cudaGetLastError();
-}
-
-#define DNS_DCASE(n) case n: return f(std::integral_constant<int, n>());
-template <typename F> cudaError_t with_len_d(int M, F&& f) {
-  switch (M) { DPLAN_LENGTHS(DNS_DCASE) }
-  return cudaErrorNotSupported;
 }
 
 template <typename C>

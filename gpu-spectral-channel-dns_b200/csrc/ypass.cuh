@@ -2,9 +2,13 @@
 #pragma once
 #include "kernels.cuh"
 
-template <typename C>
-cudaError_t launch_cheby_inplace(PencilArr arr, long long npencils, int mode, int Ny,
-                                 FftTab<C> tab, cudaStream_t st);
+// Chebyshev transforms of nf reference-layout fields (FP64), npencils each,
+// from in to out (the same pencils, or others).  mode 0: s2p pad (tab: length
+// mz), 1: s2p no-pad (mz/2), 2: p2s pad (mz), 3: p2s no-pad (mz/2).  tail:
+// fill the whole line of the FFT length, as the reference's in-place
+// transforms do, instead of the points or coefficients alone.
+cudaError_t launch_cheby(PencilList in, PencilList out, int nf, long long npencils, int mode, int Ny,
+                         FftTab<double2> tab, bool tail, cudaStream_t st);
 cudaError_t launch_get_uvw(double2* const f[6], long long ps, DnsGeom g, PhysParams ph,
                            cudaStream_t st);
 cudaError_t launch_rhs_nonlinear(double2* lx, double2* ly, const double2* lz, long long ps,

@@ -95,8 +95,8 @@ __device__ __forceinline__ void zpass_b(C* v, const C* buf, const C* __restrict_
 }
 
 // spanwise inverse: pencils [f][kz Kx + kx][y] -> rows [f][y][zp][kx]
-template <typename C, int L, int TX, int TY, int NT, int MB>
-__global__ void __launch_bounds__(NT, MB) k_zb2(PencilArr in, RowArr out, DnsGeom g, const C* __restrict__ tw) {
+template <typename C, int L, int TX, int TY, int NT, int MB, class PA>
+__global__ void __launch_bounds__(NT, MB) k_zb2(PA in, RowArr out, DnsGeom g, const C* __restrict__ tw) {
   constexpr int RA = ZPlan<L>::A, RB = ZPlan<L>::B, NL = TX * TY;
   constexpr int Nz = L / 3 * 2, hz = Nz / 2;  // the launcher checks g.Nz
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(NT, MB) k_zb2(PencilArr in, RowArr out, DnsGeo
     const int kx = kx0 + li / TY, y = y0 + li % TY;
     // the streamwise Nyquist column (kx = Kx - 1) and rows beyond Py are zero
     const bool ok = kx < Kx - 1 && y < Py;
-    const C* src = (const C*)in.base + (long long)f * in.fs + (long long)kx * in.ps + y + (long long)j * kzs;
+    const C* src = field_base<C>(in, f) + (long long)kx * in.ps + y + (long long)j * kzs;
     C v[RA];
 #pragma unroll
     for (int r = 0; r < RA; ++r) {
@@ -141,8 +141,8 @@ __global__ void __launch_bounds__(NT, MB) k_zb2(PencilArr in, RowArr out, DnsGeo
 
 // spanwise forward: rows [f][y][zp][kx] -> pencils [f][kz Kx + kx][y], the
 // Nz kept wavenumbers
-template <typename C, int L, int TX, int TY, int NT, int MB>
-__global__ void __launch_bounds__(NT, MB) k_zf2(RowArr in, PencilArr out, DnsGeom g, const C* __restrict__ tw) {
+template <typename C, int L, int TX, int TY, int NT, int MB, class PA>
+__global__ void __launch_bounds__(NT, MB) k_zf2(RowArr in, PA out, DnsGeom g, const C* __restrict__ tw) {
   constexpr int RA = ZPlan<L>::A, RB = ZPlan<L>::B, NL = TX * TY;
   constexpr int Nz = L / 3 * 2, hz = Nz / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(NT, MB) k_zf2(RowArr in, PencilArr out, DnsGeo
     zpass_b<C, RA, RB, NL, false>(v, buf, tw, li, k);
     const int kx = kx0 + li / TY, y = y0 + li % TY;
     if (kx < Kx && y < Py) {
-      C* dst = (C*)out.base + (long long)f * out.fs + (long long)kx * out.ps + y + (long long)k * kzs;
+      C* dst = field_base<C>(out, f) + (long long)kx * out.ps + y + (long long)k * kzs;
 #pragma unroll
       for (int r = 0; r < RB; ++r) {
         const int n = k + r * RA;  // kept: n <= Nz/2 and n > L - Nz/2

@@ -23,6 +23,7 @@
 
 #include "mbar.cuh"
 #include "wfft.cuh"
+#include "xline.cuh"
 #include "xpass.cuh"
 #include "zpass.cuh"
 #include "zxpass.cuh"
@@ -580,28 +581,28 @@ template <typename F> cudaError_t with_len_z(int L, F&& f) {
   switch (L) { ZPLAN_LENGTHS(DNS_ZCASE) }
   return cudaErrorNotSupported;
 }
-template <typename C>
-cudaError_t launch_zb2(PencilArr in, RowArr out, int nf, DnsGeom g, FftTab<C> tab, cudaStream_t st, bool probe) {
+template <typename C, class PA>
+cudaError_t launch_zb2(PA in, RowArr out, int nf, DnsGeom g, FftTab<C> tab, cudaStream_t st, bool probe) {
   return with_len_z(g.Pz, [&](auto LL) -> cudaError_t {
     constexpr int L = decltype(LL)::value;
     typedef ZTwo<C, L> T;
     if (!tab.zt || g.Nz != L / 3 * 2) return cudaErrorNotSupported;
     if (probe) return cudaSuccess;
-    auto k = k_zb2<C, L, T::TX, T::TY, T::NT, T::MB>;
+    auto k = k_zb2<C, L, T::TX, T::TY, T::NT, T::MB, PA>;
     const size_t sm = (size_t)L * T::TX * T::TY * sizeof(C);
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     k<<<dim3((g.Kx + T::TX - 1) / T::TX, (g.Py + T::TY - 1) / T::TY, nf), T::NT, sm, st>>>(in, out, g, tab.zt);
     return cudaGetLastError();
   });
 }
-template <typename C>
-cudaError_t launch_zf2(RowArr in, PencilArr out, int nf, DnsGeom g, FftTab<C> tab, cudaStream_t st, bool probe) {
+template <typename C, class PA>
+cudaError_t launch_zf2(RowArr in, PA out, int nf, DnsGeom g, FftTab<C> tab, cudaStream_t st, bool probe) {
   return with_len_z(g.Pz, [&](auto LL) -> cudaError_t {
     constexpr int L = decltype(LL)::value;
     typedef ZTwo<C, L> T;
     if (!tab.zt || g.Nz != L / 3 * 2) return cudaErrorNotSupported;
     if (probe) return cudaSuccess;
-    auto k = k_zf2<C, L, T::TX, T::TY, T::NT, T::MB>;
+    auto k = k_zf2<C, L, T::TX, T::TY, T::NT, T::MB, PA>;
     const size_t sm = (size_t)L * T::TX * T::TY * sizeof(C);
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     k<<<dim3((g.Kx + T::TX - 1) / T::TX, (g.Py + T::TY - 1) / T::TY, nf), T::NT, sm, st>>>(in, out, g, tab.zt);
@@ -758,23 +759,81 @@ cudaError_t launch_x_fused(RowArr in, RowArr out, DnsGeom g, FftTab<C> tab, cons
     return cudaGetLastError();
   });
 }
-template <typename C>
-cudaError_t launch_x_c2r(RowArr in, T_of<C>* outr, long long rps, long long nrows, DnsGeom g,
-                         FftTab<C> tab, cudaStream_t st) {
+// Streamwise lines of nf fields.  Lengths with a plan take the two-butterfly
+// form (us, before / after: three fields of 384 x 384 x 512 to points 1119 /
+// 345, three of 192 x 192 x 256 to modes 163 / 59), other lengths one launch a
+// field of the runtime-length form.
+cudaError_t launch_x_c2r(RowArr in, FieldList out, int nf, long long rps, long long nrows, DnsGeom g,
+                         FftTab<double2> tab, cudaStream_t st) {
+  if (tab.zt && g.Nx / 2 == g.Px / 3) {
+    const cudaError_t e = with_len_z(g.Px, [&](auto LL) -> cudaError_t {
+      constexpr int L = decltype(LL)::value;
+      typedef XLine<L> P;
+      const size_t sm = (size_t)P::NL * P::LS * 16;
+      k_c2r2<L><<<dim3((unsigned)((nrows + 2 * P::NL - 1) / (2 * P::NL)), nf), 64, sm, st>>>(in, out, rps, nrows, tab.zt);
+      return cudaGetLastError();
+    });
+    if (e != cudaErrorNotSupported) return e;
+  }
   const int RB = 4;
-  const size_t sm = (size_t)(RB / 2) * g.Px * sizeof(C);
-  cudaFuncSetAttribute(k_x_c2r<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_x_c2r<C><<<(unsigned)((nrows + RB - 1) / RB), 256, sm, st>>>(in, outr, rps, nrows, g, tab, RB);
+  const size_t sm = (size_t)(RB / 2) * g.Px * 16;
+  cudaFuncSetAttribute(k_x_c2r<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  for (int f = 0; f < nf; ++f) {
+    const RowArr rf{(double2*)in.base + (long long)f * in.fs, in.rs, 0};
+    k_x_c2r<double2><<<(unsigned)((nrows + RB - 1) / RB), 256, sm, st>>>(rf, (double*)out.p[f], rps, nrows, g, tab, RB);
+  }
   return cudaGetLastError();
 }
-template <typename C>
-cudaError_t launch_x_r2c(const T_of<C>* inr, long long rps, RowArr out, long long nrows,
-                         DnsGeom g, FftTab<C> tab, double scale, cudaStream_t st) {
+cudaError_t launch_x_r2c(FieldList in, int nf, long long rps, RowArr out, long long nrows, DnsGeom g,
+                         FftTab<double2> tab, double scale, cudaStream_t st) {
+  if (tab.zt) {
+    const cudaError_t e = with_len_z(g.Px, [&](auto LL) -> cudaError_t {
+      constexpr int L = decltype(LL)::value;
+      typedef XLine<L> P;
+      const size_t sm = (size_t)P::NL * P::LS * 16;
+      k_r2c2<L><<<dim3((unsigned)((nrows + 2 * P::NL - 1) / (2 * P::NL)), nf), 64, sm, st>>>(in, rps, out, nrows, g.Kx,
+                                                                                          scale, tab.zt);
+      return cudaGetLastError();
+    });
+    if (e != cudaErrorNotSupported) return e;
+  }
   const int RB = 4;
-  const size_t sm = (size_t)(RB / 2) * g.Px * sizeof(C);
-  cudaFuncSetAttribute(k_x_r2c<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_x_r2c<C><<<(unsigned)((nrows + RB - 1) / RB), 256, sm, st>>>(inr, rps, out, nrows, g, tab, RB, scale);
+  const size_t sm = (size_t)(RB / 2) * g.Px * 16;
+  cudaFuncSetAttribute(k_x_r2c<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  for (int f = 0; f < nf; ++f) {
+    const RowArr rf{(double2*)out.base + (long long)f * out.fs, out.rs, 0};
+    k_x_r2c<double2><<<(unsigned)((nrows + RB - 1) / RB), 256, sm, st>>>((const double*)in.p[f], rps, rf, nrows, g, tab,
+                                                                         RB, scale);
+  }
   return cudaGetLastError();
+}
+// Spanwise passes of nf reference-layout fields (FP64), rows field by field
+cudaError_t launch_zb_fields(PencilList in, RowArr out, int nf, DnsGeom g, FftTab<double2> tab, cudaStream_t st,
+                             int variant) {
+  if (variant == VAR_AUTO || variant == DNS_Z_WARP) {
+    const cudaError_t e = launch_zb2<double2>(in, out, nf, g, tab, st, false);
+    if (e != cudaErrorNotSupported) return e;
+  }
+  for (int f = 0; f < nf; ++f) {
+    const cudaError_t e = launch_zb<double2>(PencilArr{in.f.p[f], in.ps, 0},
+                                             RowArr{(double2*)out.base + (long long)f * out.fs, out.rs, 0}, 1, g, tab, st,
+                                             nullptr, variant, false);
+    if (e) return e;
+  }
+  return cudaSuccess;
+}
+cudaError_t launch_zf_fields(RowArr in, PencilList out, int nf, DnsGeom g, FftTab<double2> tab, cudaStream_t st,
+                             int variant) {
+  if (variant == VAR_AUTO || variant == DNS_Z_WARP) {
+    const cudaError_t e = launch_zf2<double2>(in, out, nf, g, tab, st, false);
+    if (e != cudaErrorNotSupported) return e;
+  }
+  for (int f = 0; f < nf; ++f) {
+    const cudaError_t e = launch_zf<double2>(RowArr{(double2*)in.base + (long long)f * in.fs, in.rs, 0},
+                                             PencilArr{out.f.p[f], out.ps, 0}, 1, g, tab, st, nullptr, variant, false);
+    if (e) return e;
+  }
+  return cudaSuccess;
 }
 cudaError_t launch_lamb_rows(const double* const in6[6], double* const out3[3], long long rps,
                              long long nrows, DnsGeom g, const double* Uy, double Ro,
@@ -791,10 +850,6 @@ cudaError_t launch_lamb_rows(const double* const in6[6], double* const out3[3], 
   template cudaError_t launch_zb<C>(PencilArr, RowArr, int, DnsGeom, FftTab<C>, cudaStream_t, int*, int, bool); \
   template cudaError_t launch_zf<C>(RowArr, PencilArr, int, DnsGeom, FftTab<C>, cudaStream_t, int*, int, bool); \
   template cudaError_t launch_x_fused<C>(RowArr, RowArr, DnsGeom, FftTab<C>, const double*,       \
-                                         double, int*, cudaStream_t, int, bool, const double*);   \
-  template cudaError_t launch_x_c2r<C>(RowArr, T_of<C>*, long long, long long, DnsGeom,           \
-                                       FftTab<C>, cudaStream_t);                                  \
-  template cudaError_t launch_x_r2c<C>(const T_of<C>*, long long, RowArr, long long, DnsGeom,     \
-                                       FftTab<C>, double, cudaStream_t);
+                                         double, int*, cudaStream_t, int, bool, const double*);
 INST_Z(double2)
 INST_Z(float2)

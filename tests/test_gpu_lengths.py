@@ -101,3 +101,47 @@ def test_wall_length(pkg, M):
         assert _apart(*(_state_after(pkg, pkg.PREC_FP64, 24, 24, M, v, U) for v in (warp, block))) < 1e-11, U
     e = _step_error(pkg, 24, 24, M, [(pkg.PASS_Y3, pkg.Y3_FFT), (pkg.PASS_Y1, pkg.Y1_WARP)])
     assert e < 1e-6, e
+
+
+@pytest.mark.parametrize("M", WALL)
+def test_cheby_whole_line(pkg, M):
+    """dns_cheby_s2p / p2s fill the FFT's whole line, as the reference does in place."""
+    sz = O.Sizes(24, 24, M)
+    r = np.random.default_rng(M)
+    c = pkg.Context(pkg.make_params(24, 24, M, Re=1300.0, dt=0.001))
+    for pad in (pkg.PADDING, pkg.NO_PADDING):
+        line = M if pad == pkg.PADDING else M // 2
+        for f, ref in ((c.cheby_s2p, O.cheby_s2p), (c.cheby_p2s, O.cheby_p2s)):
+            S = r.standard_normal((sz.ny, sz.hnx, M)) + 1j * r.standard_normal((sz.ny, sz.hnx, M))
+            t = torch.from_numpy(S).cuda()
+            torch.cuda.synchronize()
+            f(t.data_ptr(), M * 16, pad)
+            c.synchronize()
+            got, exp = t.cpu().numpy(), ref(S, M, pad == pkg.PADDING)
+            assert np.abs(got[..., :line] - exp[..., :line]).max() < 1e-13 * np.abs(exp[..., :line]).max()
+            assert np.array_equal(got[..., line:], S[..., line:])
+    c.close()
+
+
+@pytest.mark.parametrize("mx,my,mz", [(24, 24, 32), (96, 192, 256)])
+def test_six_fields_equal_one_by_one(pkg, mx, my, mz):
+    """dns_transform shares launches between fields (the second grid's rows
+    fill the workspace with two): bit for bit the fields one by one."""
+    sz = O.Sizes(mx, my, mz)
+    pitch = (mx // 2 + 1) * 16
+    g = torch.Generator(device="cuda").manual_seed(5)
+    c = pkg.Context(pkg.make_params(mx, my, mz, Re=1300.0, dt=0.001))
+    spec = [torch.randn(sz.ny, sz.hnx, mz, dtype=torch.complex128, device="cuda", generator=g) for _ in range(6)]
+    out = []
+    for together in (True, False):
+        s = [t.clone() for t in spec]
+        p = [torch.zeros(sz.pz, my, pitch // 8, dtype=torch.float64, device="cuda") for _ in s]
+        torch.cuda.synchronize()
+        for d in (pkg.BACKWARD, pkg.FORWARD):
+            groups = [range(6)] if together else [[i] for i in range(6)]
+            for i in groups:
+                c.transform(d, [p[k].data_ptr() for k in i], pitch, [s[k].data_ptr() for k in i], mz * 16)
+        c.synchronize()
+        out.append([t.cpu().numpy()[..., :mx] for t in p] + [t.cpu().numpy()[..., :sz.pz] for t in s])
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+    c.close()
