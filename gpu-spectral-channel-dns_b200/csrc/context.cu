@@ -60,12 +60,14 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
     std::memcpy(h.data() + at, p, bytes);
     return at;
   };
+  std::vector<double2> W(L);
   std::vector<C> tw(L);
   std::vector<short> dr(L);
   const long double PI = 3.141592653589793238462643383279502884L;
   for (int j = 0; j < L; ++j) {
     const long double a = -2.0L * PI * (long double)j / (long double)L;
-    tw[j] = cmk<C>((double)cosl(a), (double)sinl(a));
+    W[j] = make_double2((double)cosl(a), (double)sinl(a));
+    tw[j] = from_d2<C>(W[j]);
     dr[j] = (short)fft_digitrev(f.plan, j);
   }
   const size_t otw = put(tw.data(), sizeof(C) * L), odr = put(dr.data(), sizeof(short) * L);
@@ -79,8 +81,8 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
   for (int i = 0; i < 4; ++i) {
     if (i < 2 && !f32) continue;
     const int n = i == 0 ? wtw_table_any<C, 2>(L, t)
-                : i == 1 ? xtw_table<C>(L, t)
-                : i == 2 ? ztw_table<C>(L, t) : dtw_table<C>(L, t);
+                : i == 1 ? xtw_table<C>(L, W.data(), t)
+                : i == 2 ? ztw_table<C>(L, W.data(), t) : dtw_table<C>(L, W.data(), t);
     if (n > 0) off[i] = put(t.data(), sizeof(C) * n);
   }
   cudaError_t e = cudaMalloc(&f.mem, h.size());
@@ -530,6 +532,7 @@ dns_status ctx_create(const dns_params* p, SlabState* slab, dns_ctx** out, int n
   c->wd.delta = wall::base_degree(p->U1, p->U2);
   c->wd.nv = c->wd.no = Ny + c->wd.delta;
   c->wd.gp = c->wd.nv;
+  c->wd.xp = Ny;
   c->wd.qbytes = (int)((7 * (size_t)WALL_QROWS(c->wd.no) * 8 + 15) & ~(size_t)15);
   const size_t gn = (size_t)(sl ? sl->np : g.H * nrun) * c->wd.gp;
   if ((e = c->alloc(&c->T0, NN)) || (e = c->alloc(&c->T2, NN)) || (e = c->alloc(&c->T4, NN)) ||
@@ -1192,35 +1195,38 @@ dns_status dns_check_state(dns_ctx* c) {
 }
 
 namespace {
-// The solve-only sequence on the device: right-hand sides bv, bo (pitch bp,
-// either may stand for a zero system) -> solutions into ov, oo (pitch op).
+// The solve-only sequence on the device: right-hand sides bv, bo (pitch bp;
+// null: that system is left alone, where the length allows it, else
+// cudaErrorNotSupported and nothing launched) -> solutions into ov, oo (pitch op).
 // Point values and their DCT-I go through the transform buffer F6, which the
 // banded solve then takes as its scratch.
 cudaError_t enqueue_solve_wall(dns_ctx* c, const double2* bv, const double2* bo, long long bp,
-                               double2* Xv, double2* Xo, double2* pbc, double2* ov, double2* oo,
-                               long long op) {
+                               double2* pbc, double2* ov, double2* oo, long long op, int sys = 3) {
   const DnsGeom& g = c->g;
   const long long ls = c->P.mz / 2;  // no-padding DCT-I length 2N
   double2* sv = (double2*)c->F6;
   double2* so = sv + g.H * ls;
-  const double* cosk = c->rtab + RhsLayout(g.Ny, c->wd.nv, c->wd.no).cosk;
-  // one kernel where the DCT length has a warp plan, else three
-  cudaError_t e = launch_colloc_fused(bv, bo, bp, pbc, cosk, c->Ut, c->ddUt, c->rv, c->ro, c->wd, g, c->ph,
-                                      c->fy0_d.tab(), c->status, c->st);
+  const RhsTabs tb = RhsLayout(g.Ny, c->wd.nv, c->wd.no).at(c->rtab);
+  // one kernel where the DCT length has a plan, else three (for both systems:
+  // the caller stages a zero one)
+  cudaError_t e = launch_colloc_fused(bv, bo, bp, pbc, c->Ut, c->ddUt, c->rv, c->ro, c->wd, tb, g, c->ph,
+                                      c->fy0_d.tab(), c->st);
   if (e == cudaErrorNotSupported) {
-    e = launch_colloc_prep(bv, bo, bp, sv, so, ls, pbc, cosk, c->Ut, c->ddUt, g, c->ph, c->st);
+    if (!bv || !bo) return e;
+    e = launch_colloc_prep(bv, bo, bp, sv, so, ls, pbc, tb.cosk, c->Ut, c->ddUt, g, c->ph, c->st);
     const PencilList lines{{sv, so}, ls};
     if (!e) e = launch_cheby(lines, lines, 2, g.H, 3, g.Ny, c->fy0_d.tab(), false, c->st);
     if (!e) e = launch_colloc_integrate(sv, so, ls, c->rv, c->ro, c->wd, g, c->st);
   }
   WallDims wd = c->wd;
   wd.tilt = 0;
-  if (!e) e = launch_wall_solve(c->wfac, Xv, Xo, c->rv, c->ro, c->wQ, (double2*)c->F6, wd, g, c->ph,
-                                c->status, c->st, c->variant[DNS_PASS_Y2]);
+  wd.sys = sys & ((bv ? 1 : 0) | (bo ? 2 : 0));
+  wd.xp = op;
+  if (!e) e = launch_wall_solve(c->wfac, ov, oo, c->rv, c->ro, c->wQ, (double2*)c->F6, wd, g, c->ph,
+                                c->status, c->st, c->variant[DNS_PASS_Y2], pbc);
   if (e == cudaErrorNotSupported)
-    e = launch_wall_solve(c->wfac, Xv, Xo, c->rv, c->ro, c->wQ, (double2*)c->F6, wd, g, c->ph, c->status, c->st,
-                          DNS_Y2_RING2_8K_EF);
-  if (!e) e = launch_colloc_finish(Xv, Xo, pbc, ov, oo, op, g, c->st);
+    e = launch_wall_solve(c->wfac, ov, oo, c->rv, c->ro, c->wQ, (double2*)c->F6, wd, g, c->ph, c->status, c->st,
+                          DNS_Y2_RING2_8K_EF, pbc);
   return e;
 }
 }  // namespace
@@ -1252,7 +1258,7 @@ dns_status dns_solve_wall(dns_ctx* c, void* v, void* omega, size_t tpitch, int w
       cudaGraph_t gr;
       CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
       cudaError_t e = enqueue_solve_wall(c, (const double2*)v, (const double2*)omega, (long long)(tpitch / 16),
-                                         Xv, Xo, pbc, (double2*)v, (double2*)omega, (long long)(tpitch / 16));
+                                         pbc, (double2*)v, (double2*)omega, (long long)(tpitch / 16));
       cudaError_t e2 = cudaStreamEndCapture(c->st, &gr);
       if (e) return fail(DNS_ERR_CUDA, std::string("solve capture: ") + cudaGetErrorString(e));
       CK(e2);
@@ -1265,18 +1271,26 @@ dns_status dns_solve_wall(dns_ctx* c, void* v, void* omega, size_t tpitch, int w
     CK(cudaGraphLaunch(c->solve_graph, c->st));
     return check_status(c);
   }
-  // host buffers, or one system only: staged through Xv, Xo (pitch Ny); a
-  // missing system is solved for a zero right-hand side and not written
+  if (where == DNS_DEVICE) {  // one system: straight from and to the caller's pencils
+    const cudaError_t e = enqueue_solve_wall(c, (const double2*)v, (const double2*)omega, (long long)(tpitch / 16),
+                                             pbc, (double2*)v, (double2*)omega, (long long)(tpitch / 16));
+    if (e == cudaSuccess) return check_status(c);
+    if (e != cudaErrorNotSupported) CK(e);
+  }
+  // host buffers, or one system only of a length without a plan: staged
+  // through Xv, Xo (pitch Ny); a missing system is prepared from a zero
+  // right-hand side and not solved
   if (v) CK(cudaMemcpy2DAsync(Xv, row, v, tpitch, row, g.H, kind_of(where, true), c->st));
   else CK(cudaMemsetAsync(Xv, 0, hn * 16, c->st));
   if (omega) CK(cudaMemcpy2DAsync(Xo, row, omega, tpitch, row, g.H, kind_of(where, true), c->st));
   else CK(cudaMemsetAsync(Xo, 0, hn * 16, c->st));
   if (where == DNS_HOST) {
-    CK(enqueue_solve_wall(c, Xv, Xo, g.Ny, Xv, Xo, pbc, Xv, Xo, g.Ny));
+    CK(enqueue_solve_wall(c, Xv, Xo, g.Ny, pbc, Xv, Xo, g.Ny));
     if (v) CK(cudaMemcpy2DAsync(v, tpitch, Xv, row, row, g.H, cudaMemcpyDeviceToHost, c->st));
     if (omega) CK(cudaMemcpy2DAsync(omega, tpitch, Xo, row, row, g.H, cudaMemcpyDeviceToHost, c->st));
   } else {
-    CK(enqueue_solve_wall(c, Xv, Xo, g.Ny, Xv, Xo, pbc, (double2*)v, (double2*)omega, (long long)(tpitch / 16)));
+    CK(enqueue_solve_wall(c, Xv, Xo, g.Ny, pbc, (double2*)v, (double2*)omega, (long long)(tpitch / 16),
+                          (v ? 1 : 0) | (omega ? 2 : 0)));
   }
   return check_status(c);
 }

@@ -13,13 +13,17 @@
 // The fused time step does not use these kernels: it forms the same right-
 // hand sides in Chebyshev coefficient space inside its y1 pass.  Here each
 // pencil's right-hand side is the reference's collocation form, evaluated on
-// the GPU: one CTA per pencil, one warp per collocation row, lanes over the
-// Chebyshev index (coalesced rows of the T tables), FP64 throughout.
+// the GPU, FP64 throughout: in coefficient space (derivatives by sweeps,
+// products with U and U' as interpolants) and one DCT-I to the points
+// (k_rhs_dct), or, for lengths without a DCT plan, as products with the T
+// tables, one warp per collocation row.
 #include <algorithm>
 #include <string>
 
 #include "../../include/dns_b200.h"
 #include "context_impl.cuh"
+#include "ycoef.cuh"
+#include "ydct.cuh"
 
 namespace {
 
@@ -121,6 +125,90 @@ __global__ void k_rhs_omega(double2* ro, const double2* no, const double2* nop, 
   }
 }
 
+// Both right-hand sides of a pencil through one DCT-I over the Gauss-Lobatto
+// points (even extension of length L = 2 N): four pencils per CTA, a warp
+// each for the coefficients.  OMEGA = false: k_rhs_v, true: k_rhs_omega.
+//
+// What bounds it: the T-table form reads three Ny x Ny tables through L1 for
+// every pencil, 2 Ny^2 products each; here a pencil's vectors are read and
+// written once.  128 x 65 x 128, v / omega_y: 202 / 221 -> 36 / 30 us.
+template <int L, bool OMEGA>
+__global__ void __launch_bounds__(128) k_rhs_dct(double2* x, double2* xp, const double2* nl, const double2* nlp,
+                                                 const double2* vn1, const double2* vn, long long ps, DnsGeom g,
+                                                 PhysParams ph, const double2* __restrict__ dt) {
+  typedef Dct<double2, L, 4> D;
+  constexpr int N = L / 2, Ny = N + 1, VS = Ny + 4;  // two zeros on either side
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double2* A = (double2*)smem_raw + (size_t)warp * 3 * VS + 2;  // v or omega
+  double2* B = A + VS;                                          // D^2 v, or the sum of the two v
+  double2* F = B + VS;                                          // D^4 v or D^2 omega, then the right-hand side
+  double2* X = (double2*)smem_raw + (size_t)4 * 3 * VS;
+  const long long p0 = (long long)blockIdx.x * 4, p = p0 + warp;
+  const double2 z2 = make_double2(0.0, 0.0);
+  if (lane < 2) A[lane - 2] = A[Ny + lane] = B[lane - 2] = B[Ny + lane] = z2;
+  if (p < g.H) {
+    const int kx = (int)(p % g.Kx), kz = (int)(p / g.Kx);
+    for (int n = lane; n < Ny; n += 32) {
+      const double2 v = x[p * ps + n];
+      A[n] = v;
+      if (OMEGA) B[n] = vn[p * ps + n] + vn1[p * ps + n];
+      else if (p) xp[p * ps + n] = v;
+    }
+    __syncwarp();
+    double ia, ib;
+    wavenumbers(kx, kz, g.Nz, ph.aphi, ph.beta, ia, ib);
+    const double kmn = kmn_of(ia, ib), h = ph.dt * 0.5 / ph.Re, gam = ia * ph.dt * 0.5;
+    constexpr int CH = ddz_run(Ny);
+    if (OMEGA) {
+      d2z_fast<CH>(A, F, Ny);
+      __syncwarp();
+      const double a0 = 1 - kmn * h, kap = -0.5 * ib * ph.dt;
+      for (int k = lane; k < Ny; k += 32) {
+        double2 P, Pf;
+        u_times(A, k, N, ph, P, Pf);
+        F[k] = F[k] * h + A[k] * a0 + muli(up_times(B, k, N, ph) * kap - Pf * gam);
+      }
+    } else {
+      d2z_fast<CH>(A, B, Ny);
+      __syncwarp();
+      d2z_fast<CH>(B, F, Ny);
+      __syncwarp();
+      const double a2 = 1 - 2.0 * kmn * h, a0 = kmn * (1 - kmn * h);
+      for (int k = lane; k < Ny; k += 32) {
+        const double2 v = A[k], d2 = B[k];
+        F[k] = F[k] * h + d2 * a2 - v * a0 + muli(v) * (2.0 * gam * ph.U2);
+        B[k] = v * kmn - d2;  // under i gam U
+      }
+      __syncwarp();
+      for (int k = lane; k < Ny; k += 32) {
+        double2 P, Pf;
+        u_times(B, k, N, ph, P, Pf);
+        F[k] = F[k] + muli(Pf) * gam;
+      }
+    }
+  } else {
+    for (int n = lane; n < Ny; n += 32) F[n] = z2;
+  }
+  __syncthreads();
+  const double2* F0 = (const double2*)smem_raw + 2 + 2 * VS;
+  for (int i = threadIdx.x; i < D::IA; i += 128)
+    D::template pass_a<0>(X, i, [&](int l, int n) { return F0[l * 3 * VS + n] * (n && n < N ? 0.5 : 1.0); });
+  __syncthreads();
+  // point r goes to row r + 2 (v, r = 2..N-2) or r + 1 (omega, r = 1..N-1);
+  // the wall rows are zero
+  constexpr int OFF = OMEGA ? 1 : 2;
+  for (int i = threadIdx.x; i < D::IB; i += 128)
+    D::pass_b(X, dt, i, [&](int l, int r, double2 f) {
+      const long long q = p0 + l;
+      if (q >= g.H || q == 0) return;
+      double2* row = x + q * ps;
+      if (r >= OFF && r <= N - OFF)
+        row[r + OFF] = f + (nl[q * ps + r] * 1.5 - nlp[q * ps + r] * 0.5) * ph.dt;
+      if (r < 2 * OFF) row[r] = z2;
+    });
+}
+
 // the mean modes u0 (block 0) and w0 (block 1): rows 2..N of
 // (T0 + dt/(2 Re) T2) x - dt (1.5 lambda - 0.5 lambda_p) at r = i - 1;
 // rows 0, 1 (Dirichlet) zero
@@ -193,6 +281,21 @@ dns_status staged(dns_ctx* c, Stage* f, int n, size_t tpitch, int where, F launc
   return DNS_OK;
 }
 
+template <bool OMEGA>
+cudaError_t launch_rhs_dct(dns_ctx* c, double2* x, double2* xp, const double2* nl, const double2* nlp,
+                           const double2* vn1, const double2* vn, long long ps) {
+  const FftTab<double2> tab = c->fy0_d.tab();
+  if (!tab.dt || c->g.Ny != tab.plan.L / 2 + 1) return cudaErrorNotSupported;
+  return with_len_cheby(tab.plan.L, [&](auto LL) -> cudaError_t {
+    constexpr int L = decltype(LL)::value;
+    auto k = k_rhs_dct<L, OMEGA>;
+    const size_t sm = (size_t)(4 * 3 * (L / 2 + 5) + Dct<double2, L, 4>::XN) * 16;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k<<<(unsigned)((c->g.H + 3) / 4), 128, sm, c->st>>>(x, xp, nl, nlp, vn1, vn, ps, c->g, c->ph, tab.dt);
+    return cudaGetLastError();
+  });
+}
+
 unsigned threads_for(int Ny) { return (unsigned)std::min(256, std::max(64, (Ny + 31) / 32 * 32)); }
 
 }  // namespace
@@ -208,6 +311,8 @@ dns_status dns_rhs_v(dns_ctx* c, void* rhs_v, void* rhs_v_p, const void* nv, con
   const PhysParams ph = c->ph;
   const size_t sm = (size_t)g.Ny * 16;
   return staged(c, f, 4, tpitch, where, [&](double2** q, long long ps) {
+    const cudaError_t e = launch_rhs_dct<false>(c, q[0], q[1], q[2], q[3], nullptr, nullptr, ps);
+    if (e != cudaErrorNotSupported) return e;
     k_rhs_v<<<(unsigned)g.H, threads_for(g.Ny), sm, c->st>>>(q[0], q[1], q[2], q[3], ps, c->T0, c->T2,
                                                             c->T4, c->Ut, c->ddUt, g, ph);
     return cudaGetLastError();
@@ -224,6 +329,8 @@ dns_status dns_rhs_omega(dns_ctx* c, void* rhs_omega, const void* nomega, const 
   const PhysParams ph = c->ph;
   const size_t sm = (size_t)2 * g.Ny * 16;
   return staged(c, f, 5, tpitch, where, [&](double2** q, long long ps) {
+    const cudaError_t e = launch_rhs_dct<true>(c, q[0], nullptr, q[1], q[2], q[3], q[4], ps);
+    if (e != cudaErrorNotSupported) return e;
     k_rhs_omega<<<(unsigned)g.H, threads_for(g.Ny), sm, c->st>>>(q[0], q[1], q[2], q[3], q[4], ps,
                                                                 c->T0, c->T2, c->Ut, c->dUt, g, ph);
     return cudaGetLastError();

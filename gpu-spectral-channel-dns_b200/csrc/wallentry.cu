@@ -18,7 +18,8 @@
 //   3. rows K .. K+n-1 of the K-fold Chebyshev integral (K = 4 for v, 2
 //      otherwise), the input of the banded solve, which then runs without
 //      the tilting term;
-//   4. x = the banded solution + p, written over the right-hand side.
+//   4. x = the banded solution + p, written over the right-hand side by the
+//      solve itself.
 // A p is evaluated from the operator rows of the reference's matrices:
 //   v:     Re part  (1 + k^2 dt/Re) p'' - k^2 (1 + k^2 dt/(2Re)) p   (p'''' = 0)
 //          Im part  a dt/2 U p'' - (k^2 a dt/2 U + a dt/2 U'') p
@@ -29,9 +30,8 @@
 #include <type_traits>
 
 #include "kernels.cuh"
-#include "mbar.cuh"
 #include "wallsolve_dev.cuh"
-#include "wfft.cuh"
+#include "ydct.cuh"
 
 namespace {
 
@@ -149,22 +149,6 @@ __global__ void __launch_bounds__(128) k_colloc_integrate(const double2* __restr
   for (int r = threadIdx.x; r < no; r += blockDim.x) go[p * gp + r] = (2 + r < LB) ? ao[2 + r] : cx(0, 0);
 }
 
-// 4. x = banded solution + wall polynomial, into the caller's pencils
-__global__ void __launch_bounds__(256) k_colloc_finish(const double2* __restrict__ Xv,
-                                                       const double2* __restrict__ Xo,
-                                                       const double2* __restrict__ pbc, double2* ov,
-                                                       double2* oo, long long op, int Ny, long long H) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= H * Ny) return;
-  const long long p = i / Ny;
-  const int k = (int)(i - p * Ny);
-  double2 a = Xv[i], b = Xo[i];
-  if (k < 4) a = a + pbc[p * 6 + k];
-  if (k < 2) b = b + pbc[p * 6 + 4 + k];
-  if (ov) ov[p * op + k] = a;
-  if (oo) oo[p * op + k] = b;
-}
-
 // any non-finite real or imaginary part in a or b sets *flag
 __global__ void __launch_bounds__(256) k_nonfinite(const double2* __restrict__ a,
                                                    const double2* __restrict__ b, long long n,
@@ -178,144 +162,136 @@ __global__ void __launch_bounds__(256) k_nonfinite(const double2* __restrict__ a
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flag, 1);
 }
 
-// 1-3 fused, one CTA per pencil, one warp per system (0: v, 1: omega_y):
-// the point values of step 2 are formed in the first pass of a warp FFT of
-// the even extension (the DCT-I over the Gauss-Lobatto points, length
-// L = 2N), its coefficients written over the consumed line, and the K-fold
-// integration runs in place of the line (two halves as ping-pong buffers).
-// Compile-time L = 2 (Ny - 1); the launcher falls back to the three kernels
-// above for lengths without a warp plan.
+// 1-3 fused: four lines (a system of a pencil each) per CTA of two warps.  A
+// warp forms the wall polynomial and the point values of two lines from the
+// right-hand sides in global memory, the DCT-I over the Gauss-Lobatto points is
+// a pruned one (ydct.cuh, even extension of length L = 2 N), and the K-fold
+// integral its banded stencils.  A missing system has no lines.
+//
+// What bounds it: the whole FFT of each even extension (three passes of twice
+// the points) and four integration sweeps kept a call on shared memory; now a
+// value crosses it twice.  384 x 193 x 384: 555 -> 451 us, and the
+// 140 us of a last kernel that added the wall polynomial are gone.
 template <int L>
-__global__ void __launch_bounds__(64, 16) k_colloc_fused(const double2* __restrict__ bv, const double2* __restrict__ bo,
-                                                     long long bp, double2* pbc, const double* __restrict__ cosk,
-                                                     const double* __restrict__ Ut, const double* __restrict__ ddUt,
-                                                     double2* gv, double2* go, int nv, int no, long long gp,
-                                                     DnsGeom g, PhysParams ph, FftTab<double2> tab, int* status) {
-  constexpr int N = L / 2, Ny = N + 1, LB = Ny + 8;
-  constexpr int LS = (wlen<double2>(L) > 2 * LB) ? wlen<double2>(L) : 2 * LB;  // line stride
-  static_assert(LS - Ny >= Ny, "the staged right-hand side lies above the point values");
+__global__ void __launch_bounds__(64, 6) k_colloc_dct(const double2* __restrict__ bv, const double2* __restrict__ bo,
+                                                      long long bp, double2* pbc, const double* __restrict__ Ut,
+                                                      const double* __restrict__ ddUt, double2* gv, double2* go, int nv,
+                                                      int no, long long gp, RhsTabs tb, DnsGeom g, PhysParams ph,
+                                                      const double2* __restrict__ dt) {
+  typedef Dct<double2, L, 4> D;
+  constexpr int N = L / 2, Ny = N + 1, VS = Ny + 12;  // zeros above N for the stencils
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ uint64_t bars[2];
+  double2* F = (double2*)smem_raw;  // point values, then coefficients
+  double2* X = F + 4 * VS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double2* line = (double2*)smem_raw + (size_t)warp * LS;
-  const long long p = blockIdx.x;
-  const int kx = (int)(p % g.Kx), kz = (int)(p / g.Kx);
-  const bool zero = p == 0;
-  // this warp's right-hand side (Ny point values) by one bulk copy into the
-  // top of its line, above the point values the next loop writes (the
-  // launcher checks the 16-byte alignment)
-  const double2* b = line + (LS - Ny);
-  {
-    uint64_t* bar = &bars[warp];
-    if (lane == 0) {
-      mbar_init(bar, 1);
-      fence_mbar_init();
-      mbar_expect_tx(bar, (uint32_t)(Ny * 16));
-      bulk_g2s(line + (LS - Ny), (warp ? bo : bv) + p * bp, (uint32_t)(Ny * 16), bar);
-    }
-    __syncwarp();
-    if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar, 0, ph.wait_limit, status))) {
-      if (lane == 0) {
-        atomicOr(status, 1);
-        mbar_wait_bounded(bar, 0, DNS_WAIT_LIMIT, nullptr);  // let the copy land before leaving
-      }
-      return;
-    }
+  const bool both = bv && bo;
+  const long long nlines = both ? 2 * g.H : g.H, l0 = (long long)blockIdx.x * 4;
+  // both lines' right-hand sides first, every load in flight: rows m + 2 (v)
+  // or m + 1 (omega and the mean modes) at point m
+  constexpr int KP = (Ny + 31) / 32;
+  double2 row[2][KP], wall[2][4];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const long long gl = min(l0 + 2 * warp + u, nlines - 1);
+    const long long p = both ? gl >> 1 : gl;
+    const bool om = both ? (gl & 1) : !bv;
+    const double2* b = (om ? bo : bv) + p * bp;
+    const int off = om || p == 0 ? 1 : 2;
+#pragma unroll
+    for (int i = 0; i < KP; ++i) row[u][i] = b[min(lane + 32 * i + off, N)];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) wall[u][i] = b[i];
   }
-  // wall polynomial (every lane; rows 0..3 of the right-hand side)
-  double2 pc0, pc1, pc2 = cx(0, 0), pc3 = cx(0, 0);
+  // the wavenumbers of both lines at once (lane u: line u): FP64 divisions
+  double la, lb;
   {
-    const double2 r0 = b[0], r1 = b[1];
-    const double2 e = (r0 + r1) * 0.5, o = (r0 - r1) * 0.5;
-    pc0 = e;
-    pc1 = o;
-    if (warp == 0 && !zero) {
-      const double2 r2 = b[2], r3 = b[3];
-      pc2 = (r2 - r3) * 0.125;
-      pc3 = ((r2 + r3) * 0.5 - o) * 0.125;
+    const long long gl = min(l0 + 2 * warp + (lane & 1), nlines - 1);
+    const long long p = both ? gl >> 1 : gl;
+    wavenumbers((int)(p % g.Kx), (int)(p / g.Kx), g.Nz, ph.aphi, ph.beta, la, lb);
+  }
+  const double h = ph.dt * 0.5 / ph.Re;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const double ia = __shfl_sync(0xffffffffu, la, u), ib = __shfl_sync(0xffffffffu, lb, u);
+    const long long gl = l0 + 2 * warp + u;
+    double2* f = F + (2 * warp + u) * VS;
+    if (gl >= nlines) {
+      for (int m = lane; m < Ny; m += 32) f[m] = cx(0, 0);
+      continue;
+    }
+    const long long p = both ? gl >> 1 : gl;
+    const bool om = both ? (gl & 1) : !bv, zero = p == 0;
+    // wall polynomial (rows 0..3 of the right-hand side)
+    const double2 e = (wall[u][0] + wall[u][1]) * 0.5, o = (wall[u][0] - wall[u][1]) * 0.5;
+    double2 pc0 = e, pc1 = o, pc2 = cx(0, 0), pc3 = cx(0, 0);
+    if (!om && !zero) {
+      pc2 = (wall[u][2] - wall[u][3]) * 0.125;
+      pc3 = ((wall[u][2] + wall[u][3]) * 0.5 - o) * 0.125;
       pc0 = e - pc2;
       pc1 = o - pc3;
     }
     if (lane == 0) {
-      if (warp == 0) {
-        pbc[p * 6 + 0] = pc0; pbc[p * 6 + 1] = pc1; pbc[p * 6 + 2] = pc2; pbc[p * 6 + 3] = pc3;
+      double2* q = pbc + p * 6 + (om ? 4 : 0);
+      q[0] = pc0;
+      q[1] = pc1;
+      if (!om) { q[2] = pc2; q[3] = pc3; }
+    }
+    const double kmn = ia * ia + ib * ib;
+    const double cv2 = 1 + 2.0 * kmn * h, co0 = 1 + kmn * h, cv0 = kmn * co0, ah = ia * ph.dt * 0.5;
+    // point value m of the interior right-hand side minus A p, zero where the
+    // equation has no row
+#pragma unroll
+    for (int i = 0; i < KP; ++i) {
+      const int m = lane + 32 * i;
+      if (m > N) break;
+      const double y = __ldg(tb.cosk + m);
+      double2 v = cx(0, 0);
+      if (zero || om) {
+        if (m >= 1 && m <= N - 1) {
+          const double2 P0 = pc0 + pc1 * y;
+          v = zero ? row[u][i] - P0 : row[u][i] - (P0 * co0 + muli(P0 * (ah * __ldg(Ut + m))));
+        }
+      } else if (m >= 2 && m <= N - 2) {
+        const double2 P0 = pc0 + pc1 * y + pc2 * (2 * y * y - 1) + pc3 * (y * (4 * y * y - 3));
+        const double2 P2 = pc2 * 4.0 + pc3 * (24.0 * y);
+        const double U = __ldg(Ut + m), ddU = __ldg(ddUt + m);
+        const double2 re = P2 * cv2 - P0 * cv0;
+        const double2 im = P2 * (ah * U) - P0 * (kmn * ah * U + ah * ddU);
+        v = row[u][i] - (re + muli(im));
+      }
+      f[m] = v;
+    }
+  }
+  for (int i = threadIdx.x; i < 4 * 12; i += 64) F[i / 12 * VS + Ny + i % 12] = cx(0, 0);
+  __syncthreads();
+  for (int i = threadIdx.x; i < D::IA; i += 64)
+    D::template pass_a<0>(X, i, [&](int l, int n) { return F[l * VS + n]; });
+  __syncthreads();
+  for (int i = threadIdx.x; i < D::IB; i += 64)
+    D::pass_b(X, dt, i, [&](int l, int k, double2 v) { F[l * VS + k] = v * (k && k < N ? 1.0 / N : 0.5 / N); });
+  __syncthreads();
+  // rows K .. K+n-1 of the K-fold integral (K = 4 for v, 2 otherwise)
+#pragma unroll 1
+  for (int u = 0; u < 2; ++u) {
+    const long long gl = l0 + 2 * warp + u;
+    if (gl >= nlines) return;
+    const long long p = both ? gl >> 1 : gl;
+    const bool om = both ? (gl & 1) : !bv, four = !om && p != 0;
+    const double2* f = F + (2 * warp + u) * VS;
+    double2* out = (om ? go : gv) + p * gp;
+#pragma unroll 2
+    for (int r = lane; r < nv; r += 32) {  // (as many rows of omega)
+      double2 v = cx(0, 0);
+      if (four) {
+#pragma unroll
+        for (int d = 0; d < 5; ++d) v = v + f[r + 2 * d] * __ldg(tb.b4 + d * nv + r);
       } else {
-        pbc[p * 6 + 4] = pc0; pbc[p * 6 + 5] = pc1;
-      }
-    }
-  }
-  double ia, ib;
-  wavenumbers(kx, kz, g.Nz, ph.aphi, ph.beta, ia, ib);
-  const double kmn = ia * ia + ib * ib, dt = ph.dt, Re = ph.Re;
-  // the operator's constants (the same expressions as the three-kernel path)
-  const double cv2 = 1 + kmn * dt / Re, cv0 = kmn * (1 + kmn * dt * 0.5 / Re), co0 = 1 + kmn * dt * 0.5 / Re;
-  const double ah = ia * dt * 0.5;
-  // point value m of the interior right-hand side minus A p (zero where the
-  // equation has no row), staged at line[m] in natural order: the FFT's
-  // first pass reads them all before it writes the line
-  for (int m = lane; m <= N; m += 32) {
-    const double y = __ldg(cosk + m);
-    double2 f = cx(0, 0);
-    if (zero || warp == 1) {
-      if (m >= 1 && m <= N - 1) {
-        const double2 P0 = pc0 + pc1 * y;
-        f = zero ? b[m + 1] - P0 : b[m + 1] - (P0 * co0 + muli(P0 * (ah * __ldg(Ut + m))));
-      }
-    } else if (m >= 2 && m <= N - 2) {
-      const double2 P0 = pc0 + pc1 * y + pc2 * (2 * y * y - 1) + pc3 * (y * (4 * y * y - 3));
-      const double2 P2 = pc2 * 4.0 + pc3 * (24.0 * y);
-      const double U = __ldg(Ut + m), ddU = __ldg(ddUt + m);
-      const double2 re = P2 * cv2 - P0 * cv0;
-      const double2 im = P2 * (ah * U) - P0 * (kmn * ah * U + ah * ddU);
-      f = b[m + 2] - (re + muli(im));
-    }
-    line[m] = f;
-  }
-  __syncwarp();
-  // DCT-I: FFT of the even extension; coefficient k = value / N, halved at
-  // k = 0 and k = N, written over the line (its last pass read it all)
-  auto ld = [&](int, int n) -> double2 { return line[n <= N ? n : L - n]; };
-  auto st = [&](int, int k, double2 v) {
-    if (k <= N) line[k] = v * ((k == 0 || k == N) ? 0.5 / N : 1.0 / N);
-  };
-  wfft_io<double2, L, 1, false>(line, tab.tw, ld, st, LS);
-  __syncwarp();
-  for (int k = Ny + lane; k < LB; k += 32) line[k] = cx(0, 0);
-  // K-fold integration: (B x)_k = (c_{k-1} x_{k-1} - x_{k+1}) / (2k), (B x)_0 = 0;
-  // each lane keeps the weights 1 / (2k) of its elements k = lane + 32 i
-  // (the divisions once, not once per sweep)
-  const int K = (warp == 0 && !zero) ? 4 : 2;
-  constexpr int KPL = (LB + 31) / 32;
-  double w2k[KPL];
 #pragma unroll
-  for (int i = 0; i < KPL; ++i) {
-    const int k = lane + 32 * i;
-    w2k[i] = k >= 1 ? 1.0 / (2.0 * k) : 0.0;
-  }
-  double2* x = line;
-  double2* yb = line + LB;
-  for (int it = 0; it < K; ++it) {
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < KPL; ++i) {
-      const int k = lane + 32 * i;
-      if (k >= LB) break;
-      double2 r = cx(0, 0);
-      if (k >= 1) {
-        const double2 xm = x[k - 1] * (k == 1 ? 2.0 : 1.0);
-        const double2 xp = (k + 1 < LB) ? x[k + 1] : cx(0, 0);
-        r = (xm - xp) * w2k[i];
+        for (int d = 0; d < 3; ++d) v = v + f[r + 2 * d] * __ldg(tb.b2 + d * (nv + 2) + r);
       }
-      yb[k] = r;
+      out[r] = v;
     }
-    double2* t = x;
-    x = yb;
-    yb = t;
   }
-  __syncwarp();
-  double2* out = (warp ? go : gv) + p * gp;
-  const int n = warp ? no : nv;
-  for (int r = lane; r < n; r += 32) out[r] = (K + r < LB) ? x[K + r] : cx(0, 0);
 }
 
 }  // namespace
@@ -351,39 +327,19 @@ cudaError_t launch_colloc_integrate(const double2* cv, const double2* co, long l
   return cudaGetLastError();
 }
 
-cudaError_t launch_colloc_finish(const double2* Xv, const double2* Xo, const double2* pbc,
-                                 double2* ov, double2* oo, long long op, const DnsGeom& g,
-                                 cudaStream_t st) {
-  const long long n = g.H * g.Ny;
-  k_colloc_finish<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(Xv, Xo, pbc, ov, oo, op, g.Ny, g.H);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_colloc_fused(const double2* bv, const double2* bo, long long bp, double2* pbc,
-                                const double* cosk, const double* Ut, const double* ddUt, double2* gv,
-                                double2* go, const WallDims& wd, const DnsGeom& g, const PhysParams& ph,
-                                FftTab<double2> tab, int* status, cudaStream_t st) {
-  auto go1 = [&](auto LL) -> cudaError_t {
+                                const double* Ut, const double* ddUt, double2* gv, double2* go, const WallDims& wd,
+                                const RhsTabs& tb, const DnsGeom& g, const PhysParams& ph, FftTab<double2> tab,
+                                cudaStream_t st) {
+  if (!tab.dt || g.Ny != tab.plan.L / 2 + 1 || wd.nv != wd.no) return cudaErrorNotSupported;
+  return with_len_cheby(tab.plan.L, [&](auto LL) -> cudaError_t {
     constexpr int L = decltype(LL)::value;
-    if constexpr (WPlan<L, 1, FftMaxRadix<double2>::v>::ok) {
-      if (tab.plan.L != L || g.Ny != L / 2 + 1 || !tab.tw || !status || !aligned16(bv) || !aligned16(bo))
-        return cudaErrorNotSupported;
-      constexpr int LB = L / 2 + 9;
-      constexpr int LS = (wlen<double2>(L) > 2 * LB) ? wlen<double2>(L) : 2 * LB;
-      const size_t sm = (size_t)2 * LS * 16;
-      cudaFuncSetAttribute(k_colloc_fused<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_colloc_fused<L><<<(unsigned)g.H, 64, sm, st>>>(bv, bo, bp, pbc, cosk, Ut, ddUt, gv, go, wd.nv, wd.no,
-                                                       wd.gp, g, ph, tab, status);
-      return cudaGetLastError();
-    }
-    return cudaErrorNotSupported;
-  };
-  switch (tab.plan.L) {
-    case 128: return go1(std::integral_constant<int, 128>());
-    case 256: return go1(std::integral_constant<int, 256>());
-    case 384: return go1(std::integral_constant<int, 384>());
-    case 512: return go1(std::integral_constant<int, 512>());
-    case 768: return go1(std::integral_constant<int, 768>());
-  }
-  return cudaErrorNotSupported;
+    const size_t sm = (size_t)(4 * (L / 2 + 13) + Dct<double2, L, 4>::XN) * 16;
+    const long long nlines = bv && bo ? 2 * g.H : g.H;
+    auto k = k_colloc_dct<L>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k<<<(unsigned)((nlines + 3) / 4), 64, sm, st>>>(bv, bo, bp, pbc, Ut, ddUt, gv, go, wd.nv, wd.no, wd.gp, tb, g, ph,
+                                                    tab.dt);
+    return cudaGetLastError();
+  });
 }

@@ -18,7 +18,8 @@
 //
 // Inputs from the y1 kernel: g_v, g_o (rows K.. of the integrated
 // collocation right-hand sides, the v^n part of the tilting term included).
-// Outputs: V, O (Chebyshev coefficients of v^{n+1}, omega_y^{n+1}).
+// Outputs: V, O (Chebyshev coefficients of v^{n+1}, omega_y^{n+1}); the
+// solve-only entry adds its wall polynomials (pbc) to the lowest ones.
 #include "kernels.cuh"
 #include "mbar.cuh"
 #include "wallsolve_dev.cuh"
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
                                                    double2* O, const double2* __restrict__ gv,
                                                    const double2* __restrict__ go,
                                                    const double* __restrict__ Qg, double2* Sw,
-                                                   WallDims wd, DnsGeom g, PhysParams ph, int* status) {
+                                                   const double2* __restrict__ pbc, WallDims wd, DnsGeom g, PhysParams ph, int* status) {
   typedef WallCfg<KLV, KUV, KLO, KUO, WALL_STG> CF;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* full = (uint64_t*)smem_raw;
@@ -115,13 +116,14 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
   const double2* gfac = fac + (long long)blockIdx.x * wd.group_complex;
   const int nch0 = (wd.nv + CF::R0 - 1) / CF::R0, nch1 = (wd.nv + CF::R1 - 1) / CF::R1;
   const int nch2 = (wd.no + CF::R2 - 1) / CF::R2, nch3 = (wd.no + CF::R3 - 1) / CF::R3;
-  const int total = nch0 + nch1 + nch2 + nch3;
+  const bool dov = wd.sys & 1, doo = wd.sys & 2;
+  const int total = (dov ? nch0 + nch1 : 0) + (doo ? nch2 + nch3 : 0);
 
   const uint64_t pol = EF ? l2_evict_first() : 0;
   // the group's stream is contiguous: lane 0 walks it phase by phase, ic the
   // next chunk, irow rows of its phase issued
-  int ic = 0, iph = 0, irow = 0;
-  const double2* isrc = gfac;
+  int ic = 0, iph = dov ? 0 : 2, irow = 0;
+  const double2* isrc = gfac + (dov ? 0 : 16LL * wd.nv * (CF::E0 + CF::E1));
   auto issue = [&]() {
     const int rows = iph < 2 ? wd.nv : wd.no;
     const int R = iph == 0 ? CF::R0 : iph == 1 ? CF::R1 : iph == 2 ? CF::R2 : CF::R3;
@@ -190,7 +192,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
   // renamed registers and not moves; FULL = false is a phase's last chunk.
   int c = 0;
   // ---- v: forward substitution (unit lower band) -------------------------
-  {
+  if (dov) {
     constexpr int R = CF::R0;
     double2 yw[KLV], cur[R];
 #pragma unroll
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
   // ---- v: back substitution, recombination, tilting term -----------------
   // rows descend.  The tilting term of row k+1 is written over rows already
   // consumed (k + 1 > i).
-  {
+  if (dov) {
     constexpr int R = CF::R1;
     double2 xw[KUV], cur[R];
 #pragma unroll
@@ -264,7 +266,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
     };
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) cur[rr] = rr < nv ? S[32 * (nv - 1 - rr)] : z2;
-    double2* Vp = V + pen * Ny + (zero ? 2 : 4);  // row i emits coefficient i + 4, of the mean modes i + 2
+    double2* Vp = V + pen * wd.xp + (zero ? 2 : 4);  // row i emits coefficient i + 4, of the mean modes i + 2
     const int top = zero ? N - 2 : N - 4;         // the last row that emits one
     auto chunk = [&](auto whole, const double2* ch, int r0) {
       const int i0 = nv - 1 - r0;
@@ -327,11 +329,12 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
     }
 #pragma unroll
     for (int k = 3; k >= 0; --k) {
-      if (active && !(zero && k > 1)) V[pen * Ny + k] = a[k];
+      if (active && !(zero && k > 1)) V[pen * wd.xp + k] = pbc ? a[k] + pbc[pen * 6 + k] : a[k];
       tilt(k, a[k], true);
     }
     S[0] = make_double2(-P[0].y * kap, P[0].x * kap);
   }
+  if (!doo) return;
   // ---- omega: forward substitution (adds g_o to the tilting term) --------
   {
     constexpr int R = CF::R2;
@@ -341,7 +344,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) {
       gc[rr] = (active && rr < no) ? __ldg(gop + rr) : z2;
-      sc[rr] = rr < no ? S[32 * rr] : z2;
+      sc[rr] = dov && rr < no ? S[32 * rr] : z2;
     }
     auto chunk = [&](auto whole, const double2* ch, int r0) {
       const double2* nx = gop + r0 + R;
@@ -354,7 +357,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
         if (whole.full) {
           const bool more = r0 + R + rr < no;
           gc[rr] = (active && more) ? __ldg(nx + rr) : z2;
-          sc[rr] = more ? Sr[32 * (R + rr)] : z2;
+          sc[rr] = dov && more ? Sr[32 * (R + rr)] : z2;
         }
         double2 a1 = z2;
 #pragma unroll
@@ -389,7 +392,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
 #pragma unroll
     for (int e = 0; e < KUO; ++e) zw[e] = z2;
     const int nbo = N - 1;
-    double2* Op = O + pen * Ny + 2;
+    double2* Op = O + pen * wd.xp + 2;
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) cur[rr] = rr < no ? S[32 * (no - 1 - rr)] : z2;
     auto chunk = [&](auto whole, const double2* ch, int r0) {
@@ -427,8 +430,9 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
       ++c;
     }
     if (active) {
-      O[pen * Ny + 1] = make_double2(-zw[1].x, -zw[1].y);
-      O[pen * Ny + 0] = make_double2(-zw[0].x, -zw[0].y);
+      const double2 a1 = make_double2(-zw[1].x, -zw[1].y), a0 = make_double2(-zw[0].x, -zw[0].y);
+      O[pen * wd.xp + 1] = pbc ? a1 + pbc[pen * 6 + 5] : a1;
+      O[pen * wd.xp + 0] = pbc ? a0 + pbc[pen * 6 + 4] : a0;
     }
   }
 }
@@ -449,26 +453,26 @@ bool wall_band_of(int delta, int* klv, int* kuv, int* klo, int* kuo) {
 
 template <int A, int B, int C, int D, int VAR>
 static cudaError_t launch_inst(const double2* fac, double2* V, double2* O, const double2* gv,
-                               const double2* go, const double* Q, double2* Sw, const WallDims& wd,
-                               const DnsGeom& g, const PhysParams& ph, int* status, cudaStream_t st) {
+                               const double2* go, const double* Q, double2* Sw, const double2* pbc,
+                               const WallDims& wd, const DnsGeom& g, const PhysParams& ph, int* status, cudaStream_t st) {
   constexpr WallVar v = kWallVar[VAR];
   auto k = k_wall_solve<A, B, C, D, v.nst, v.stg, v.qsm, v.ef>;
   const size_t sm = wall_smem_bytes(wd, VAR);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e) return e;
-  k<<<(unsigned)wd.ngroups, 32, sm, st>>>(fac, V, O, gv, go, Q, Sw, wd, g, ph, status);
+  k<<<(unsigned)wd.ngroups, 32, sm, st>>>(fac, V, O, gv, go, Q, Sw, pbc, wd, g, ph, status);
   return cudaGetLastError();
 }
 
 template <int A, int B, int C, int D>
 static cudaError_t launch_var(int variant, const double2* fac, double2* V, double2* O, const double2* gv,
-                              const double2* go, const double* Q, double2* Sw, const WallDims& wd,
-                              const DnsGeom& g, const PhysParams& ph, int* status, cudaStream_t st) {
+                              const double2* go, const double* Q, double2* Sw, const double2* pbc,
+                              const WallDims& wd, const DnsGeom& g, const PhysParams& ph, int* status, cudaStream_t st) {
   switch (variant) {
-    case 0: return launch_inst<A, B, C, D, 0>(fac, V, O, gv, go, Q, Sw, wd, g, ph, status, st);
-    case 1: return launch_inst<A, B, C, D, 1>(fac, V, O, gv, go, Q, Sw, wd, g, ph, status, st);
-    case 2: return launch_inst<A, B, C, D, 2>(fac, V, O, gv, go, Q, Sw, wd, g, ph, status, st);
-    case 3: return launch_inst<A, B, C, D, 3>(fac, V, O, gv, go, Q, Sw, wd, g, ph, status, st);
+    case 0: return launch_inst<A, B, C, D, 0>(fac, V, O, gv, go, Q, Sw, pbc, wd, g, ph, status, st);
+    case 1: return launch_inst<A, B, C, D, 1>(fac, V, O, gv, go, Q, Sw, pbc, wd, g, ph, status, st);
+    case 2: return launch_inst<A, B, C, D, 2>(fac, V, O, gv, go, Q, Sw, pbc, wd, g, ph, status, st);
+    case 3: return launch_inst<A, B, C, D, 3>(fac, V, O, gv, go, Q, Sw, pbc, wd, g, ph, status, st);
   }
   return cudaErrorNotSupported;
 }
@@ -476,13 +480,13 @@ static cudaError_t launch_var(int variant, const double2* fac, double2* V, doubl
 cudaError_t launch_wall_solve(const double2* fac, double2* V, double2* O, const double2* gv,
                               const double2* go, const double* Q, double2* Sw, const WallDims& wd,
                               const DnsGeom& g, const PhysParams& ph, int* status, cudaStream_t st,
-                              int variant) {
+                              int variant, const double2* pbc) {
   if (variant < 0 || variant >= DNS_WALL_VARIANTS) return cudaErrorNotSupported;
   if (wall_smem_bytes(wd, variant) > 227 * 1024) return cudaErrorNotSupported;
   switch (wd.delta) {
-    case 0: return launch_var<4, 8, 2, 4>(variant, fac, V, O, gv, go, Q, Sw, wd, g, ph, status, st);
-    case 1: return launch_var<5, 9, 3, 6>(variant, fac, V, O, gv, go, Q, Sw, wd, g, ph, status, st);
-    case 2: return launch_var<6, 10, 4, 8>(variant, fac, V, O, gv, go, Q, Sw, wd, g, ph, status, st);
+    case 0: return launch_var<4, 8, 2, 4>(variant, fac, V, O, gv, go, Q, Sw, pbc, wd, g, ph, status, st);
+    case 1: return launch_var<5, 9, 3, 6>(variant, fac, V, O, gv, go, Q, Sw, pbc, wd, g, ph, status, st);
+    case 2: return launch_var<6, 10, 4, 8>(variant, fac, V, O, gv, go, Q, Sw, pbc, wd, g, ph, status, st);
   }
   return cudaErrorInvalidValue;
 }

@@ -88,16 +88,27 @@ XPLAN(768, 8, 8, 4, 6, 12, 8)
   X(324) X(384) X(432) X(512) X(576) X(768)
 
 // FP32 twiddles: the inverse plan's passes, then the forward plan's (FP64
-// passes take W_L^j and products)
-template <typename C> int xtw_table(int L, std::vector<C>& out) {
+// passes take W_L^j and products); W: the table W_L^j, j < L
+template <typename C, int... Rs> void xtw_fill(Radices<Rs...>, int L, const double2* W, C* out) {
+  const int rs[] = {Rs...};
+  int ns = 1;
+  for (int i = 0; i < (int)sizeof...(Rs); ++i) {
+    const int R = rs[i];
+    if (ns > 1)
+      for (int r = 1; r < R; ++r)
+        for (int k = 0; k < ns; ++k) *out++ = from_d2<C>(W[r * k * (L / (ns * R))]);
+    ns *= R;
+  }
+}
+template <typename C> int xtw_table(int L, const double2* W, std::vector<C>& out) {
   switch (L) {
 #define XCASE(n)                                                    \
   case n: {                                                         \
     typedef XPlan<n, FftMaxRadix<C>::v> P;                          \
     const int ni = wtw_size(typename P::INV()), nf = wtw_size(typename P::FWD()); \
     out.resize((size_t)(ni + nf));                                  \
-    wtw_fill_radices<C, n, 1>(typename P::INV(), out.data());       \
-    wtw_fill_radices<C, n, 1>(typename P::FWD(), out.data() + ni);  \
+    xtw_fill(typename P::INV(), n, W, out.data());                  \
+    xtw_fill(typename P::FWD(), n, W, out.data() + ni);             \
     return ni + nf;                                                 \
   }
     XPLAN_LENGTHS(XCASE)

@@ -9,7 +9,7 @@
 // the whole FFT (9 of 16 and 17 of 32 at M = 512), at the FFT's accuracy: no
 // prefix sums, no division by sines.
 #pragma once
-#include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "fft2.cuh"
@@ -58,21 +58,18 @@ DPLAN(768, 32, 24)
 // lengths of the no-padding transforms only
 #define DPLAN_SHORT(X) X(16) X(24)
 
-// pass-B twiddles W_M^{j s}, j = 1..RB/2, s = 0..RA/2, stored [j - 1][s]
-template <typename C> int dtw_table(int M, std::vector<C>& out) {
+// pass-B twiddles W_M^{j s}, j = 1..RB/2, s = 0..RA/2, stored [j - 1][s]; W:
+// the table W_M^j, j < M
+template <typename C> int dtw_table(int M, const double2* W, std::vector<C>& out) {
   int ra = 0, rb = 0;
 #define DCASE(n) \
   case n: ra = DPlan<n>::A; rb = DPlan<n>::B; break;
   switch (M) { DPLAN_SHORT(DCASE) DPLAN_LENGTHS(DCASE) default: return -1; }
 #undef DCASE
-  const long double PI = 3.141592653589793238462643383279502884L;
   const int sh = ra / 2 + 1;
   out.resize((size_t)(rb / 2) * sh);
   for (int j = 1; j <= rb / 2; ++j)
-    for (int s = 0; s < sh; ++s) {
-      const long double a = -2.0L * PI * (long double)(j * s) / (long double)M;
-      out[(size_t)(j - 1) * sh + s] = cmk<C>((double)cosl(a), (double)sinl(a));
-    }
+    for (int s = 0; s < sh; ++s) out[(size_t)(j - 1) * sh + s] = from_d2<C>(W[j * s]);
   return (int)out.size();
 }
 
@@ -134,3 +131,15 @@ template <typename C, int M, int NL> struct Dct {
     }
   }
 };
+
+#define YDCT_CASE(n) case n: return f(std::integral_constant<int, n>());
+// the lengths of the time step, and with the short ones of small no-padding
+// transforms; cudaErrorNotSupported for others
+template <typename F> cudaError_t with_len_d(int M, F&& f) {
+  switch (M) { DPLAN_LENGTHS(YDCT_CASE) }
+  return cudaErrorNotSupported;
+}
+template <typename F> cudaError_t with_len_cheby(int M, F&& f) {
+  switch (M) { DPLAN_SHORT(YDCT_CASE) DPLAN_LENGTHS(YDCT_CASE) }
+  return cudaErrorNotSupported;
+}

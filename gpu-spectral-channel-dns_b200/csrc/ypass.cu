@@ -20,6 +20,7 @@
 #include "fftline.cuh"
 #include "kernels.cuh"
 #include "mbar.cuh"
+#include "ycoef.cuh"
 #include "ydct.cuh"
 #include "ypass.cuh"
 
@@ -115,9 +116,6 @@ __device__ __noinline__ void ddz_fast(const E* __restrict__ a, E* __restrict__ b
     else re = re + v[i] * f;
   }
 }
-
-// lanes' run length for Ny coefficients
-__host__ __device__ constexpr int ddz_run(int Ny) { return 2 * ((Ny + 63) / 64); }
 
 // even extension for the padded s2p (cheby_pre_s2p_pad): e[0] = c0,
 // e[k] = e[M-k] = c_k/2 for 1 <= k <= Ny-1, zero otherwise; M = 4(Ny-1).
@@ -850,16 +848,6 @@ __device__ __forceinline__ double parity_sums(double (&v)[NV], int lane, int& id
   }
   return v[0];
 }
-// coefficient k of U X and, for k <= N, of its Gauss-Lobatto interpolant
-// (degrees N + 1, N + 2 fold to N - 1, N - 2); X has zeros below 0 and above N
-__device__ __forceinline__ void u_times(const double2* X, int k, int N, const PhysParams& ph, double2& P, double2& Pf) {
-  P = X[k] * ph.U0 + (X[k - 1] * (k == 1 ? 1.0 : 0.5) + X[k + 1] * 0.5) * ph.U1;
-  if (ph.U2 != 0.0)
-    P = P + (X[k - 2] * (k == 2 ? 0.5 : 0.25) + X[k] * (k == 1 ? 0.75 : 0.5) + X[k + 2] * 0.25) * ph.U2;
-  Pf = P;
-  if (k == N - 1) Pf = Pf + X[N] * (0.5 * ph.U1) + X[N - 1] * (0.25 * ph.U2);
-  if (k == N - 2) Pf = Pf + X[N] * (0.25 * ph.U2);
-}
 }  // namespace
 
 template <typename C, int M, int MB>
@@ -972,13 +960,9 @@ __global__ void __launch_bounds__(128, MB) k_y1d(PencilArr lam, const double2* _
         const double kg = kmn * gam;
         S4[k] = zero ? v : make_double2(-(v.x * c0v + Pf.y * kg), Pf.x * kg - v.y * c0v);
         const double2 o = Oc[k];
-        double2 Q, Qf, up = v * ph.U1;
+        double2 Q, Qf;
         u_times(Oc, k, N, ph, Q, Qf);
-        if (ph.U2 != 0.0) {  // U' v, its degree N + 1 folded
-          up = up + (Vc[k - 1] * (k == 1 ? 2.0 : 1.0) + Vc[k + 1]) * ph.U2;
-          if (k == N - 1) up = up + Vc[N] * ph.U2;
-        }
-        const double2 im = up * kap - Qf * gam;
+        const double2 im = up_times(Vc, k, N, ph) * kap - Qf * gam;
         T2[k] = zero ? o : make_double2(o.x * c0o - im.y, o.y * c0o + im.x);
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
@@ -1130,15 +1114,6 @@ size_t y1_smem(int Ny, int lsP, size_t csz) {
   size_t s = a((size_t)3 * Ny * 16) + a((size_t)2 * Ny * 16) + 10 * a((size_t)Ny * 16) + a(8 * 16);
   size_t bp = (size_t)3 * lsP * csz, bi = (size_t)4 * (Ny + 8) * 16;
   return s + a(bp > bi ? bp : bi);
-}
-#define DNS_DCASE(n) case n: return f(std::integral_constant<int, n>());
-template <typename F> cudaError_t with_len_d(int M, F&& f) {
-  switch (M) { DPLAN_LENGTHS(DNS_DCASE) }
-  return cudaErrorNotSupported;
-}
-template <typename F> cudaError_t with_len_cheby(int M, F&& f) {
-  switch (M) { DPLAN_SHORT(DNS_DCASE) DPLAN_LENGTHS(DNS_DCASE) }
-  return cudaErrorNotSupported;
 }
 cudaError_t launch_cheby(PencilList in, PencilList out, int nf, long long npencils, int mode, int Ny,
                          FftTab<double2> tab, bool tail, cudaStream_t st) {

@@ -16,7 +16,6 @@
 // a clock and SM was the bound.  TY elements of a pencil and TX of a row are
 // the contiguous runs, whole 32-byte sectors on both sides.
 #pragma once
-#include <cmath>
 #include <vector>
 
 #include "fft2.cuh"
@@ -54,20 +53,17 @@ ZPLAN(768, 32, 24)
   X(24) X(32) X(36) X(48) X(54) X(64) X(72) X(96) X(108) X(128) X(144) X(162) X(192) X(216) X(256) X(288) \
   X(324) X(384) X(432) X(512) X(576) X(768)
 
-// Pass-B twiddles W_L^{r k}, r = 1..RB-1, k < RA, stored [r - 1][k].
-template <typename C> int ztw_table(int L, std::vector<C>& out) {
+// Pass-B twiddles W_L^{r k}, r = 1..RB-1, k < RA, stored [r - 1][k]; W: the
+// table W_L^j, j < L
+template <typename C> int ztw_table(int L, const double2* W, std::vector<C>& out) {
   int ra = 0, rb = 0;
 #define ZCASE(n) \
   case n: ra = ZPlan<n>::A; rb = ZPlan<n>::B; break;
   switch (L) { ZPLAN_LENGTHS(ZCASE) default: return -1; }
 #undef ZCASE
-  const long double PI = 3.141592653589793238462643383279502884L;
   out.resize((size_t)(rb - 1) * ra);
   for (int r = 1; r < rb; ++r)
-    for (int k = 0; k < ra; ++k) {
-      const long double a = -2.0L * PI * (long double)(r * k) / (long double)L;
-      out[(size_t)(r - 1) * ra + k] = cmk<C>((double)cosl(a), (double)sinl(a));
-    }
+    for (int k = 0; k < ra; ++k) out[(size_t)(r - 1) * ra + k] = from_d2<C>(W[r * k]);
   return (int)out.size();
 }
 

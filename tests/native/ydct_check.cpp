@@ -17,7 +17,9 @@ template <typename C, int M, int NL, int N0> double check() {
   std::vector<C> e(NL * (H + 1)), X(D::XN, cmk<C>(1e30, 1e30)), out(NL * (H + 1), cmk<C>(1e30, 1e30)), tw;
   for (int l = 0; l < NL; ++l)
     for (int n = 0; n <= H; ++n) e[l * (H + 1) + n] = (N0 && n >= N0) ? cmk<C>(0.0, 0.0) : cmk<C>(nd(rng), nd(rng));
-  dtw_table<C>(M, tw);
+  std::vector<double2> W(M);
+  for (int j = 0; j < M; ++j) W[j] = make_double2((double)cosl(-2 * PI * j / M), (double)sinl(-2 * PI * j / M));
+  dtw_table<C>(M, W.data(), tw);
   for (int i = 0; i < D::IA; ++i)
     D::template pass_a<N0>(X.data(), i, [&](int l, int n) { return e[l * (H + 1) + n]; });
   for (int i = 0; i < D::IB; ++i)
@@ -46,6 +48,7 @@ template <typename C, int M, int NL, int N0> double check() {
          check<double2, M, 1, 0>());
 
 int main() {
+  DPLAN_SHORT(CASE)
   DPLAN_LENGTHS(CASE)
   return 0;
 }

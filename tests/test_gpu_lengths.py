@@ -145,3 +145,22 @@ def test_six_fields_equal_one_by_one(pkg, mx, my, mz):
         out.append([t.cpu().numpy()[..., :mx] for t in p] + [t.cpu().numpy()[..., :sz.pz] for t in s])
     assert all(np.array_equal(a, b) for a, b in zip(*out))
     c.close()
+
+
+@pytest.mark.parametrize("M", [36, 64, 108, 128, 256])
+def test_solve_one_system(pkg, M):
+    """dns_solve_wall of one system (36, 108: no DCT plan for 2 (Ny - 1) points)
+    equals that system of a call with both, bit for bit, and leaves no other."""
+    sz = O.Sizes(24, 24, M)
+    g = torch.Generator(device="cuda").manual_seed(M)
+    b = [torch.randn(sz.ny, sz.hnx, M, dtype=torch.complex128, device="cuda", generator=g) for _ in range(2)]
+    c = pkg.Context(pkg.make_params(24, 24, M, Re=1300.0, dt=0.001))
+    both, one = [t.clone() for t in b], [t.clone() for t in b]
+    torch.cuda.synchronize()
+    c.solve_wall(both[0].data_ptr(), both[1].data_ptr(), M * 16)
+    c.solve_wall(one[0].data_ptr(), None, M * 16)
+    c.solve_wall(None, one[1].data_ptr(), M * 16)
+    for x, y, z in zip(both, one, b):
+        assert torch.equal(x, y)
+        assert torch.equal(x[..., sz.nz:], z[..., sz.nz:])
+    c.close()
