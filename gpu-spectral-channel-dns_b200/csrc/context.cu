@@ -71,18 +71,16 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
     dr[j] = (short)fft_digitrev(f.plan, j);
   }
   const size_t otw = put(tw.data(), sizeof(C) * L), odr = put(dr.data(), sizeof(short) * L);
-  // twiddle tables where the length has a plan: FP32 warp FFTs (two lines
-  // per warp) and the fused streamwise form, both precisions the two-pass
+  // twiddle tables where the length has a plan: FP32 the fused streamwise form, both precisions the two-pass
   // spanwise form and the pruned DCT
   const bool f32 = std::is_same<C, float2>::value;
   const size_t none = ~(size_t)0;
-  size_t off[4] = {none, none, none, none};
+  size_t off[3] = {none, none, none};
   std::vector<C> t;
-  for (int i = 0; i < 4; ++i) {
-    if (i < 2 && !f32) continue;
-    const int n = i == 0 ? wtw_table_any<C, 2>(L, t)
-                : i == 1 ? xtw_table<C>(L, W.data(), t)
-                : i == 2 ? ztw_table<C>(L, W.data(), t) : dtw_table<C>(L, W.data(), t);
+  for (int i = 0; i < 3; ++i) {
+    if (i < 1 && !f32) continue;
+    const int n = i == 0 ? xtw_table<C>(L, W.data(), t)
+                : i == 1 ? ztw_table<C>(L, W.data(), t) : dtw_table<C>(L, W.data(), t);
     if (n > 0) off[i] = put(t.data(), sizeof(C) * n);
   }
   cudaError_t e = cudaMalloc(&f.mem, h.size());
@@ -91,10 +89,9 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
   auto at = [&](size_t o) { return o == none ? nullptr : (C*)(f.mem + o); };
   f.tw = at(otw);
   f.drev = (short*)(f.mem + odr);
-  f.wt = at(off[0]);
-  f.xt = at(off[1]);
-  f.zt = at(off[2]);
-  f.dt = at(off[3]);
+  f.xt = at(off[0]);
+  f.zt = at(off[1]);
+  f.dt = at(off[2]);
   return cudaSuccess;
 }
 template <typename C> void free_fft(DevFft<C>& f) {
@@ -330,11 +327,12 @@ void default_variants(dns_ctx* c) {
       {DNS_Y3_FFT, DNS_Y3_BLOCK, -1}, {DNS_Y1_WARP, DNS_Y1_BLOCK, -1},
       {DNS_Z_WARP, DNS_Z_BLOCK, -1}, {DNS_Z_WARP, DNS_Z_BLOCK, -1},
       {DNS_Y2_RING3_12K_EF, DNS_Y2_RING2_8K_EF, -1}, {DNS_X_WARP3, DNS_X_BLOCK, -1}};
-  // FP32 spanwise lines: the tensor-staged tiles win once a tile is large
-  // (inverse / forward, us: 384 x 384 x 512 229 / 123 against 273 / 131;
-  // 192 x 192 x 256 41 / 24 against 41 / 23; four 144 x 144 x 256 106 / 51
-  // against 85 / 43)
-  const bool z2 = mixed && c->g.Pz < 256;
+  // FP32 spanwise lines: tensor-staged tiles from 144 points on, where pass A
+  // keeps most lanes of a warp busy (inverse + forward, us: 384 x 384 x 512 195
+  // + 115 against 263 + 132; two 96 x 288 x 256 50 + 33 against 60 + 34; four
+  // 144 x 144 x 256 66 + 41 against 71 + 43; twelve 96 x 96 x 192 72 + 41 against
+  // 70 + 42)
+  const bool z2 = mixed && c->g.Pz < 144;
   for (int p = 0; p < DNS_NUM_PASSES; ++p) {
     const int* ord = mixed ? order_mixed[p] : order_fp64[p];
     c->variant[p] = ord[0];

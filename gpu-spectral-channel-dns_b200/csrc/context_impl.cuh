@@ -13,13 +13,12 @@ template <typename C> struct DevFft {
   unsigned char* mem = nullptr;  // holds the tables below
   C* tw = nullptr;
   short* drev = nullptr;
-  C *wt = nullptr, *dt = nullptr, *xt = nullptr, *zt = nullptr;
+  C *dt = nullptr, *xt = nullptr, *zt = nullptr;
   FftTab<C> tab() const {
     FftTab<C> t;
     t.plan = plan;
     t.tw = tw;
     t.drev = drev;
-    t.wt = wt;
     t.dt = dt;
     t.xt = xt;
     t.zt = zt;

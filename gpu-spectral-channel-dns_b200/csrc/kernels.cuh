@@ -20,7 +20,6 @@ template <typename C> struct FftTab {
   FftPlan plan;
   const C* tw;          // W_L^j, j < L
   const short* drev;    // digit-reversed position of natural index n
-  const C* wt;          // FP32 warp-FFT twiddles of the plan with two lines per warp
   const C* dt;          // twiddles of the pruned DCT (ydct.cuh), null for lengths without one
   const C* xt;          // FP32 twiddles of the fused streamwise form (xpass.cuh)
   const C* zt;          // twiddles of the two-pass spanwise form (zpass.cuh), null for lengths without one

@@ -1,5 +1,8 @@
-// Warp-synchronous line FFT: one warp transforms NL lines of length L held
-// in shared memory, with no block-wide barrier.
+// Index arithmetic of warp-synchronous line FFTs: one warp transforms lines of
+// length L held in shared memory, with no block-wide barrier.  The padded
+// layout and the store check below carry the streamwise lines (xpass.cuh,
+// xline.cuh); WPass and the plans are the same passes for NL lines at once,
+// run lane by lane on the host as the reference form of that arithmetic.
 //
 // Each pass is a Stockham autosort step (as in fft2.cuh): with Ns = product
 // of the previous radices, butterfly j in [0, L/R) reads x[j + r L/R],
@@ -255,105 +258,3 @@ template <typename C, int L, int NL> int wtw_table(std::vector<C>& out) {
     return -1;
   }
 }
-// runtime length: the lengths that have warp plans
-template <typename C, int NL> int wtw_table_any(int L, std::vector<C>& out) {
-  switch (L) {
-    case 48: return wtw_table<C, 48, NL>(out);
-    case 96: return wtw_table<C, 96, NL>(out);
-    case 144: return wtw_table<C, 144, NL>(out);
-    case 128: return wtw_table<C, 128, NL>(out);
-    case 192: return wtw_table<C, 192, NL>(out);
-    case 256: return wtw_table<C, 256, NL>(out);
-    case 384: return wtw_table<C, 384, NL>(out);
-    case 512: return wtw_table<C, 512, NL>(out);
-    case 768: return wtw_table<C, 768, NL>(out);
-  }
-  return -1;
-}
-
-#ifdef __CUDACC__
-template <typename C, int L, int NL, bool INV, int R, int Ns>
-__device__ __forceinline__ void wfft_pass(C* buf, int ls, const C* __restrict__ tw, int lane) {
-  typedef WPass<C, L, NL, INV, R, Ns> P;
-  C v[P::B][R];
-#pragma unroll
-  for (int q = 0; q < P::B; ++q)
-    if (P::on(lane, q)) P::load(buf, ls, tw, lane, q, v[q]);
-  __syncwarp();
-#pragma unroll
-  for (int q = 0; q < P::B; ++q)
-    if (P::on(lane, q)) P::store(buf, ls, lane, q, v[q]);
-  __syncwarp();
-}
-
-template <typename C, int L, int NL, bool INV, int Ns, int R, int... Rest>
-struct WRun {
-  __device__ __forceinline__ static void go(C* buf, int ls, const C* tw, int lane) {
-    wfft_pass<C, L, NL, INV, R, Ns>(buf, ls, tw, lane);
-    WRun<C, L, NL, INV, Ns * R, Rest...>::go(buf, ls, tw, lane);
-  }
-};
-template <typename C, int L, int NL, bool INV, int Ns, int R>
-struct WRun<C, L, NL, INV, Ns, R> {
-  __device__ __forceinline__ static void go(C* buf, int ls, const C* tw, int lane) {
-    wfft_pass<C, L, NL, INV, R, Ns>(buf, ls, tw, lane);
-  }
-};
-template <typename C, int L, int NL, bool INV, typename RS> struct WDo;
-template <typename C, int L, int NL, bool INV, int... Rs>
-struct WDo<C, L, NL, INV, Radices<Rs...>> {
-  __device__ __forceinline__ static void go(C* buf, int ls, const C* tw, int lane) {
-    WRun<C, L, NL, INV, 1, Rs...>::go(buf, ls, tw, lane);
-  }
-};
-
-// Variant with the input and output fused into the first and last passes:
-// the first pass reads ld(line, n), the last hands st(line, k, value) every
-// output; buf (NL lines, ls >= wlen(L) apart) holds the intermediate passes only.
-template <typename C, int L, int NL, bool INV, int Ns, bool FIRST, int R, int... Rest>
-struct WRunIO {
-  template <class LD, class ST>
-  __device__ __forceinline__ static void go(C* buf, int ls, const C* tw, int lane, LD& ld, ST& st) {
-    typedef WPass<C, L, NL, INV, R, Ns> P;
-    constexpr bool LAST = sizeof...(Rest) == 0;
-    C v[P::B][R];
-#pragma unroll
-    for (int q = 0; q < P::B; ++q) {
-      if (!P::on(lane, q)) continue;
-      if constexpr (FIRST) P::template load_fn<LD>(ld, lane, q, v[q]);
-      else P::load(buf, ls, tw, lane, q, v[q]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < P::B; ++q) {
-      if (!P::on(lane, q)) continue;
-      if constexpr (LAST) P::template store_fn<ST>(st, lane, q, v[q]);
-      else P::store(buf, ls, lane, q, v[q]);
-    }
-    __syncwarp();
-    if constexpr (!LAST) WRunIO<C, L, NL, INV, Ns * R, false, Rest...>::go(buf, ls, tw, lane, ld, st);
-  }
-};
-template <typename C, int L, int NL, bool INV, typename RS> struct WDoIO;
-template <typename C, int L, int NL, bool INV, int... Rs>
-struct WDoIO<C, L, NL, INV, Radices<Rs...>> {
-  template <class LD, class ST>
-  __device__ __forceinline__ static void go(C* buf, int ls, const C* tw, int lane, LD& ld, ST& st) {
-    WRunIO<C, L, NL, INV, 1, true, Rs...>::go(buf, ls, tw, lane, ld, st);
-  }
-};
-template <typename C, int L, int NL, bool INV, class LD, class ST>
-__device__ __forceinline__ void wfft_io(C* buf, const C* __restrict__ tw, LD ld, ST st, int ls = wlen<C>(L)) {
-  WDoIO<C, L, NL, INV, typename WPlan<L, NL, FftMaxRadix<C>::v>::R>::go(buf, ls, tw, threadIdx.x & 31, ld, st);
-}
-
-// Transform the NL lines at buf (line stride ls >= wlen(L), positions wsw(i)) by
-// the calling warp.  The lines must have been written by this warp (or be
-// visible to it after a barrier); a __syncwarp is taken first.
-// tw: the plan's twiddle table (FP32, wtw_table) or W_L^j, j < L (FP64).
-template <typename C, int L, int NL, bool INV>
-__device__ __forceinline__ void wfft(C* buf, const C* __restrict__ tw, int ls = wlen<C>(L)) {
-  __syncwarp();
-  WDo<C, L, NL, INV, typename WPlan<L, NL, FftMaxRadix<C>::v>::R>::go(buf, ls, tw, threadIdx.x & 31);
-}
-#endif

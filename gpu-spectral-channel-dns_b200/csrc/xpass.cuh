@@ -19,7 +19,7 @@
 // transfers of each inverse line (store, Lamb read, write, read).  Measured
 // at 384 x 384 x 512 against the form with the Lamb vector between two whole
 // transforms: FP32 356 -> 294 us, FP64 987 -> 623; 192 x 192 x 256 FP64
-// 125 -> 99; 128 x 128 x 128 FP64, a length without a plan before, 96 -> 25.
+// 125 -> 82; 128 x 128 x 128 FP64, a length without a plan before, 96 -> 25.
 #pragma once
 #include "kernels.cuh"
 #include "mbar.cuh"
@@ -28,6 +28,9 @@
 // RF and the other radices (inverse: PRE..., RF; forward: RF, PRE...), rows
 // per CTA and warps.  A row pair's 2 L/RF butterflies fit the CTA's threads;
 // three pairs of RF complex values stay in registers (RF <= 18 FP32, 9 FP64).
+// Chosen by measurement where that leaves a choice (us, FP64 192: 8 with 24 82,
+// with 6, 4 99; 216: 9 with 24 128, with 6, 4 152; 144: 8 with 18 105, 9 with
+// 16 124; FP32 96: 8 with 12 95, 4 with 24 115; 128: eight rows 60, four 64).
 template <int L, int MAXR> struct XPlan { enum { ok = 0 }; };
 #define XPLAN(L, MAXR, RF_, NR_, NW_, ...)                                \
   template <> struct XPlan<L, MAXR> {                                     \
@@ -42,11 +45,11 @@ XPLAN(32, 16, 4, 8, 3, 8)
 XPLAN(36, 16, 6, 8, 3, 6)
 XPLAN(48, 16, 4, 8, 3, 12)
 XPLAN(54, 16, 6, 8, 3, 9)
-XPLAN(64, 16, 4, 8, 3, 16)
+XPLAN(64, 16, 8, 8, 3, 8)
 XPLAN(72, 16, 4, 8, 3, 18)
-XPLAN(96, 16, 4, 8, 3, 24)
+XPLAN(96, 16, 8, 8, 3, 12)
 XPLAN(108, 16, 6, 8, 3, 18)
-XPLAN(128, 16, 8, 4, 3, 16)
+XPLAN(128, 16, 8, 8, 3, 16)
 XPLAN(144, 16, 6, 4, 3, 24)
 XPLAN(162, 16, 9, 4, 3, 18)
 XPLAN(192, 16, 8, 4, 3, 24)
@@ -70,10 +73,10 @@ XPLAN(72, 8, 6, 8, 3, 12)
 XPLAN(96, 8, 8, 8, 3, 12)
 XPLAN(108, 8, 9, 8, 3, 12)
 XPLAN(128, 8, 8, 4, 3, 16)
-XPLAN(144, 8, 9, 4, 3, 16)
+XPLAN(144, 8, 8, 4, 3, 18)
 XPLAN(162, 8, 9, 4, 3, 18)
-XPLAN(192, 8, 8, 4, 3, 6, 4)
-XPLAN(216, 8, 9, 4, 3, 6, 4)
+XPLAN(192, 8, 8, 4, 3, 24)
+XPLAN(216, 8, 9, 4, 3, 24)
 XPLAN(256, 8, 8, 2, 3, 8, 4)
 XPLAN(288, 8, 9, 2, 3, 8, 4)
 XPLAN(324, 8, 9, 2, 3, 6, 6)

@@ -90,7 +90,9 @@ __device__ __forceinline__ void zpass_b(C* v, const C* buf, const C* __restrict_
   Codelet<RB, INV, C>::run(v);
 }
 
-// spanwise inverse: pencils [f][kz Kx + kx][y] -> rows [f][y][zp][kx]
+// spanwise inverse: pencils [f][kz Kx + kx][y] -> rows [f][y][zp][kx].  The
+// streamwise Nyquist column (kx = Kx - 1) is zero and no streamwise pass reads
+// it: it is left out.
 template <typename C, int L, int TX, int TY, int NT, int MB, class PA>
 __global__ void __launch_bounds__(NT, MB) k_zb2(PA in, RowArr out, DnsGeom g, const C* __restrict__ tw) {
   constexpr int RA = ZPlan<L>::A, RB = ZPlan<L>::B, NL = TX * TY;
@@ -103,7 +105,6 @@ __global__ void __launch_bounds__(NT, MB) k_zb2(PA in, RowArr out, DnsGeom g, co
   for (int t = threadIdx.x; t < NL * RB; t += NT) {
     const int li = t % NL, j = t / NL;  // li = kxl TY + yl: TY neighbours of a pencil
     const int kx = kx0 + li / TY, y = y0 + li % TY;
-    // the streamwise Nyquist column (kx = Kx - 1) and rows beyond Py are zero
     const bool ok = kx < Kx - 1 && y < Py;
     const C* src = field_base<C>(in, f) + (long long)kx * in.ps + y + (long long)j * kzs;
     C v[RA];
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(NT, MB) k_zb2(PA in, RowArr out, DnsGeom g, co
     C v[RB];
     zpass_b<C, RA, RB, NL, true>(v, buf, tw, li, k);
     const int kx = kx0 + li / TY, y = y0 + li % TY;
-    if (kx < Kx && y < Py) {
+    if (kx < Kx - 1 && y < Py) {
       C* dst = (C*)out.base + (long long)f * out.fs + ((long long)y * L + k) * out.rs + kx;
 #pragma unroll
       for (int r = 0; r < RB; ++r) dst[(long long)(r * RA) * out.rs] = v[r];

@@ -22,7 +22,6 @@
 #include <type_traits>
 
 #include "mbar.cuh"
-#include "wfft.cuh"
 #include "xline.cuh"
 #include "xpass.cuh"
 #include "zpass.cuh"
@@ -125,65 +124,59 @@ __global__ void __launch_bounds__(256, 3) k_zf(RowArr in, PencilArr out, DnsGeom
   }
 }
 
-// Same spanwise passes in FP32 with warp FFTs on tensor-staged tiles: a TX x TY
-// tile of 16 lines (streamwise modes x wall-normal points), NW warps with
-// 16/NW lines each, no block barrier inside the transforms; the tiles (k_zbt
-// 8 x 2, k_zft 4 x 4) are chosen for their row side.
-//
-// Index arithmetic: on the pencil side a thread keeps one line (its kx and
-// y) and walks the spanwise wavenumbers kz = t/16 + 16 m; on the row side it
-// keeps one kx and walks the flat (y, zp) index of the tile's rows, whose
-// global offset is i * rs from the tile's first row.  Both walks are strided
-// by a constant, so an element costs one multiply-add of its address.
-namespace {
-template <typename C, int L, int TX, int TY, int NT>
-struct SpanTile {
-  static constexpr int NL = TX * TY;
-  static constexpr int LS = wlen<C>(L) + 1;  // odd line stride: the 16 lines of a position fall in distinct banks
-  static constexpr int KS = NT / NL;         // kz stride of the pencil-side walk
-  static constexpr int IS = NT / TX;         // (y, zp) stride of the row-side walk
-  static_assert(NT % NL == 0 && NT % TX == 0, "tile does not divide the block");
+// Same spanwise passes in FP32 on tensor-staged tiles of 16 lines (streamwise
+// modes x wall-normal points), eight warps with a pair of lines each: a warp
+// loads its pair by tiled 4-D copies into its own part of shared memory (the
+// box's innermost extent is the pair, 16 bytes), takes pass A of the plan from
+// there (every input is read before an output is stored) and pass B, shared by
+// the CTA, stores the lines straight to global memory.  Element pos of line l
+// of a pair sits at 2 (pos + pos / RA) + l: the lanes of pass A, RA apart, and
+// those of pass B, which take the 16 lines of a position (pairs WS apart), fall
+// in distinct banks.  384 x 384 x 512, inverse / forward: 195 / 115 us, against
+// 230 / 124 with both passes by the warp and the tile's rows or pencils written
+// from shared memory in a third.
+template <typename C, int L> struct ZStage {
+  static constexpr int RA = ZPlan<L>::A, RB = ZPlan<L>::B;
+  static constexpr int raw = 2 * RB * (RA + 1);
+  static constexpr int WS = raw + (18 - raw % 16) % 16;  // 2 mod 16
+  static constexpr bool ok = ZPlan<L>::ok && RB <= 16 && sizeof(C) == 8;
+  // the staged values (n per line) from the first 128-byte boundary on
+  static constexpr bool fits(int n) { return n * 16 + 128 <= WS * 8; }
 };
-}  // namespace
-
-// Inverse pass with the pencils staged by the tensor-memory accelerator: warp w owns lines 2w, 2w+1 (one kx, two consecutive y) and
-// loads their Nz spanwise values with one tiled 4-D copy (box y 2 x kx 1 x
-// kz Nz x field 1, 4 KB at Nz = 256) into its own line buffer; the first FFT
-// pass reads them there (padding, Nyquist and streamwise-Nyquist zeros
-// applied in the read) before it writes the lines.  Rows beyond Py and
-// columns beyond Kx read as the copy's zero fill.  No per-element global
-// loads, no L1 dependence.
-template <typename C, int L, int NW, int TX, int TY>
-__global__ void __launch_bounds__(32 * NW, 3) k_zbt(const __grid_constant__ CUtensorMap tin, RowArr out,
-                                                 DnsGeom g, FftTab<C> tab, int* status) {
-  typedef SpanTile<C, L, TX, TY, 32 * NW> ST;
-  constexpr int NL = ST::NL, LS = ST::LS, Pz = L;
-  static_assert(NL == 2 * NW && TY % 2 == 0 && ST::KS > 0, "two lines per warp, a y pair each");
-  extern __shared__ __align__(16) unsigned char smem_raw[];  // the tile is rounded up to 128 bytes
-  __shared__ uint64_t bars[NW];
-  C* lines = (C*)smem_raw;
-  constexpr int Nz = L / 3 * 2;  // my / 3 * 2 (the launcher checks g.Nz)
-  constexpr int hz = Nz / 2;
-  const int Kx = g.Kx, Py = g.Py;
-  const int kx0 = blockIdx.x * TX;
-  const int y0 = blockIdx.y * TY;
-  const int f = blockIdx.z;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int li0 = 2 * warp;                       // lines (kxl, yl0), (kxl, yl0 + 1)
-  const int kxl = li0 / TY, yl0 = li0 % TY;
-  C* wl = lines + (size_t)li0 * LS;
-  // the staged values [kz][y pair] at the first 128-byte boundary of the warp's lines
-  C* tile = (C*)(((uintptr_t)wl + 127) & ~(uintptr_t)127);
-  uint64_t* bar = bars + warp;
-  if (lane == 0) {
-    mbar_init(bar, 1);
-    fence_mbar_init();
-    mbar_expect_tx(bar, (uint32_t)(2 * Nz * sizeof(C)));
-    tma_load_4d(tile, &tin, y0 + yl0, kx0 + kxl, 0, f, bar);
+namespace {
+template <typename C, int L, bool INV, class LD>
+__device__ __forceinline__ void zstage_a(C* wl, int lane, LD ld) {
+  typedef ZStage<C, L> Z;
+  C v[Z::RA];
+  const int l = lane & 1, j = lane >> 1;
+  if (j < Z::RB) {
+    WFFT_ASSUME(j >= 0 && j < Z::RB);
+#pragma unroll
+    for (int r = 0; r < Z::RA; ++r) v[r] = ld(l, j + r * Z::RB);
+    Codelet<Z::RA, INV, C>::run(v);
   }
   __syncwarp();
-  // a wait that runs out is reported and waited once more (bounded); the
-  // warp then goes on, so that every warp reaches the block barriers
+  if (j < Z::RB) {
+    C* o = wl + 2 * j * (Z::RA + 1) + l;
+#pragma unroll
+    for (int r = 0; r < Z::RA; ++r) o[2 * r] = v[r];
+  }
+}
+template <typename C, int L, bool INV>
+__device__ __forceinline__ void zstage_b(C* v, const C* line, const C* __restrict__ tw, int k) {
+  typedef ZStage<C, L> Z;
+#pragma unroll
+  for (int r = 0; r < Z::RB; ++r) v[r] = line[2 * (k + r * (Z::RA + 1))];
+#pragma unroll
+  for (int r = 1; r < Z::RB; ++r) {
+    const C w = tw[(r - 1) * Z::RA + k];
+    v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
+  }
+  Codelet<Z::RB, INV, C>::run(v);
+}
+// a wait that runs out is reported and waited once more (bounded); the warp
+// then goes on, so that every warp reaches the block barriers
+__device__ __forceinline__ void zstage_wait(uint64_t* bar, int lane, int* status) {
   if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar, 0, 1LL << 31, status))) {
     if (lane == 0) {
       atomicOr(status, 1);
@@ -191,107 +184,98 @@ __global__ void __launch_bounds__(32 * NW, 3) k_zbt(const __grid_constant__ CUte
     }
     __syncwarp();
   }
-  // the streamwise Nyquist column (kx = Kx - 1) stays zero
-  const bool kxok = kx0 + kxl < Kx - 1;
-  auto ld = [&](int l, int n) -> C {
-    const int kz = (n < hz) ? n : (n > Pz - hz ? n - (Pz - Nz) : -1);
-    return (kxok && kz >= 0) ? tile[2 * kz + l] : cmk<C>(0.0, 0.0);
-  };
-  auto st = [&](int l, int k, C v) { wl[(size_t)l * LS + wsw<C>(k)] = v; };
-  wfft_io<C, L, 2, true>(wl, tab.wt, ld, st, LS);
+}
+}  // namespace
+
+// Inverse pass, 8 x 2 tile (64-byte runs on the row side): warp w owns kx0 + w
+// and two consecutive y (box y 2 x kx 1 x kz Nz x field 1, 4 KB at Nz = 256).
+// Rows beyond Py read as the copy's zero fill; the streamwise Nyquist column
+// (kx = Kx - 1) is zero and not read later: it is left out.
+template <typename C, int L>
+__global__ void __launch_bounds__(256, 3) k_zbt(const __grid_constant__ CUtensorMap tin, RowArr out,
+                                                DnsGeom g, const C* __restrict__ tw, int* status) {
+  typedef ZStage<C, L> Z;
+  constexpr int Nz = L / 3 * 2, hz = Nz / 2;  // my / 3 * 2 (the launcher checks g.Nz)
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint64_t bars[8];
+  C* lines = (C*)smem_raw;
+  const int kx0 = blockIdx.x * 8, y0 = blockIdx.y * 2, f = blockIdx.z;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  C* wl = lines + (size_t)warp * Z::WS;
+  const C* tile = (const C*)(((uintptr_t)wl + 127) & ~(uintptr_t)127);  // [kz][y pair]
+  if (lane == 0) {
+    mbar_init(bars + warp, 1);
+    fence_mbar_init();
+    mbar_expect_tx(bars + warp, (uint32_t)(2 * Nz * sizeof(C)));
+    tma_load_4d((void*)tile, &tin, y0, kx0 + warp, 0, f, bars + warp);
+  }
+  __syncwarp();
+  zstage_wait(bars + warp, lane, status);
+  zstage_a<C, L, true>(wl, lane, [&](int l, int n) -> C {
+    if (n < hz) return tile[2 * n + l];
+    if (n > L - hz) return tile[2 * (n - (L - Nz)) + l];
+    return cmk<C>(0.0, 0.0);
+  });
   __syncthreads();
-  // row side: this thread's kx, flat index i = yl * Pz + zp
-  const int kxr = threadIdx.x % TX;
-  const int kx = kx0 + kxr;
-  if (kx >= Kx || y0 >= Py) return;
-  const int ni = min(TY, Py - y0) * Pz;
-  C* rowb = prow<C>(out, f, (long long)y0 * Pz) + kx;
-  const C* lb = lines + kxr * TY * LS;
-  constexpr int ZB = 8;
-  for (int i0 = threadIdx.x / TX; i0 < ni; i0 += ZB * ST::IS) {
-    C v[ZB];
+  for (int t = threadIdx.x; t < 16 * Z::RA; t += 256) {
+    const int kxl = t & 7, yl = (t >> 3) & 1, k = t >> 4;
+    const int kx = kx0 + kxl, y = y0 + yl;
+    C v[Z::RB];
+    zstage_b<C, L, true>(v, lines + (size_t)kxl * Z::WS + yl, tw, k);
+    if (kx < g.Kx - 1 && y < g.Py) {
+      C* dst = prow<C>(out, f, (long long)y * L + k) + kx;
 #pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int i = i0 + u * ST::IS;
-      const int yl = i / Pz, zp = i - yl * Pz;
-      v[u] = (i < ni) ? lb[yl * LS + wsw<C>(zp)] : cmk<C>(0.0, 0.0);
-    }
-#pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int i = i0 + u * ST::IS;
-      if (i < ni) rowb[(long long)i * out.rs] = v[u];
+      for (int r = 0; r < Z::RB; ++r) dst[(long long)(r * Z::RA) * out.rs] = v[r];
     }
   }
 }
 
-// Forward pass with the rows staged by tensor copies: lines are
-// numbered y-major (li = yl * 4 + kxl), warp w owns lines 2w, 2w+1 (one y,
-// a kx pair) and loads their Pz values with two tiled 4-D copies (box kx 2
-// x zp Pz/2 x y 1 x field 1) into its own line buffer, [zp][kx pair]; the
-// first FFT pass reads them there.  Rows beyond Py and columns beyond Kx
-// read as the copy's zero fill.
-template <typename C, int L, int NW>
-__global__ void __launch_bounds__(32 * NW, 3) k_zft(const __grid_constant__ CUtensorMap tin, PencilArr out,
-                                                    DnsGeom g, FftTab<C> tab, int* status) {
-  constexpr int TX = 4, TY = 4;
-  typedef SpanTile<C, L, TX, TY, 32 * NW> ST;
-  constexpr int NL = ST::NL, LS = ST::LS, Pz = L;
-  static_assert(NL == 2 * NW && Pz % 2 == 0, "two lines per warp, a kx pair each");
-  extern __shared__ __align__(16) unsigned char smem_raw[];  // the tile is rounded up to 128 bytes
-  __shared__ uint64_t bars[NW];
+// Forward pass, 4 x 4 tile (32-byte runs on the pencil side): warp w owns y0 +
+// w / 2 and a kx pair, two copies (box kx 2 x zp Pz/2 x y 1 x field 1).  Rows
+// beyond Py and columns beyond Kx read as the copy's zero fill.
+template <typename C, int L>
+__global__ void __launch_bounds__(256, 3) k_zft(const __grid_constant__ CUtensorMap tin, PencilArr out,
+                                                DnsGeom g, const C* __restrict__ tw, int* status) {
+  typedef ZStage<C, L> Z;
+  constexpr int Nz = L / 3 * 2, hz = Nz / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint64_t bars[8];
   C* lines = (C*)smem_raw;
-  constexpr int Nz = L / 3 * 2;  // my / 3 * 2 (the launcher checks g.Nz)
-  constexpr int hz = Nz / 2;
   const int Kx = g.Kx, Py = g.Py;
-  const int kx0 = blockIdx.x * TX;
-  const int y0 = blockIdx.y * TY;
-  const int f = blockIdx.z;
+  const int kx0 = blockIdx.x * 4, y0 = blockIdx.y * 4, f = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int li0 = 2 * warp;
-  const int yl = li0 / TX, kxl0 = li0 % TX;
-  C* wl = lines + (size_t)li0 * LS;
-  C* tile = (C*)(((uintptr_t)wl + 127) & ~(uintptr_t)127);
-  uint64_t* bar = bars + warp;
+  C* wl = lines + (size_t)warp * Z::WS;
+  C* tile = (C*)(((uintptr_t)wl + 127) & ~(uintptr_t)127);  // [zp][kx pair]
   if (lane == 0) {
-    mbar_init(bar, 1);
+    mbar_init(bars + warp, 1);
     fence_mbar_init();
-    mbar_expect_tx(bar, (uint32_t)(2 * Pz * sizeof(C)));
-    tma_load_4d(tile, &tin, kx0 + kxl0, 0, y0 + yl, f, bar);
-    tma_load_4d(tile + Pz, &tin, kx0 + kxl0, Pz / 2, y0 + yl, f, bar);
+    mbar_expect_tx(bars + warp, (uint32_t)(2 * L * sizeof(C)));
+    const int x = kx0 + 2 * (warp & 1), y = y0 + (warp >> 1);
+    tma_load_4d(tile, &tin, x, 0, y, f, bars + warp);
+    tma_load_4d(tile + L, &tin, x, L / 2, y, f, bars + warp);
   }
   __syncwarp();
-  // a wait that runs out is reported and waited once more (bounded); the
-  // warp then goes on, so that every warp reaches the block barriers
-  if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar, 0, 1LL << 31, status))) {
-    if (lane == 0) {
-      atomicOr(status, 1);
-      mbar_wait_bounded(bar, 0, 1LL << 31, nullptr);
-    }
-    __syncwarp();
-  }
-  auto ld = [&](int l, int n) -> C { return tile[2 * n + l]; };
-  auto st = [&](int l, int k, C v) { wl[(size_t)l * LS + wsw<C>(k)] = v; };
-  wfft_io<C, L, 2, false>(wl, tab.wt, ld, st, LS);
+  zstage_wait(bars + warp, lane, status);
+  zstage_a<C, L, false>(wl, lane, [&](int l, int n) -> C { return tile[2 * n + l]; });
   __syncthreads();
-  // pencil side: line li = (yl, kxl) of this thread, wavenumbers kz
-  constexpr int ZB = 8;
-  const int li = threadIdx.x % NL;
-  const int kx = kx0 + li % TX, y = y0 + li / TX;
-  if (kx >= Kx || y >= Py) return;
-  const C* lsrc = lines + li * LS;
-  C* dst = ppen<C>(out, f, kx) + y;
   const long long kzs = (long long)Kx * out.ps;
-  for (int kz0 = threadIdx.x / NL; kz0 < Nz; kz0 += ZB * ST::KS) {
-    C v[ZB];
+  for (int t = threadIdx.x; t < 16 * Z::RA; t += 256) {
+    const int yl = t & 3, kxl = (t >> 2) & 3, k = t >> 4;
+    const int kx = kx0 + kxl, y = y0 + yl;
+    C v[Z::RB];
+    zstage_b<C, L, false>(v, lines + (size_t)(2 * yl + (kxl >> 1)) * Z::WS + (kxl & 1), tw, k);
+    if (kx < Kx && y < Py) {
+      C* dst = ppen<C>(out, f, kx) + y + (long long)k * kzs;
 #pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int kz = kz0 + u * ST::KS;
-      v[u] = (kz < Nz) ? lsrc[wsw<C>(kz <= hz ? kz : kz + (Pz - Nz))] : cmk<C>(0.0, 0.0);
-    }
-#pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int kz = kz0 + u * ST::KS;
-      if (kz < Nz) dst[kz * kzs] = v[u];
+      for (int r = 0; r < Z::RB; ++r) {
+        const int n = k + r * Z::RA;  // kept: n <= Nz/2 and n > L - Nz/2
+        if (r * Z::RA <= hz) {
+          if (n <= hz) dst[(long long)(r * Z::RA) * kzs] = v[r];
+        }
+        if (r * Z::RA + Z::RA - 1 > L - Nz + hz) {
+          if (n > L - Nz + hz) dst[(long long)(r * Z::RA - (L - Nz)) * kzs] = v[r];
+        }
+      }
     }
   }
 }
@@ -566,14 +550,16 @@ bool row_tmap(const RowArr& in, int nf, const DnsGeom& g, size_t esz, CUtensorMa
 // (inverse / forward, us): FP64 4 x 2 lines on 128 threads, three CTAs per SM
 // 466 / 240, four CTAs (no registers to keep a radix-24 butterfly's loads in
 // flight) 511 / 246, 4 x 4 lines on 256 threads 476 / 246; at 192 x 192 x 256
-// 4 x 4 lines on 128 threads 64 / 36, 4 x 2 on 64 96 / 50, 8 x 2 71 / 34.
+// 4 x 4 lines on 128 threads 64 / 36, 4 x 2 on 64 96 / 50, 8 x 2 71 / 34; at
+// 256 x 256 x 256 4 x 2 lines, four CTAs 97 / 50, three 98 / 52, 4 x 4 on 128
+// threads 104 / 58.
 // FP32 at 384: 4 x 4 lines on 256 threads 270 / 130, on 128 288 / 150, 8 x 4
-// 293 / 138 (the tensor-staged form 230 / 124 comes first there).
+// 293 / 138 (the tensor-staged form, 195 / 115, comes first there).
 template <typename C, int L> struct ZTwo {
   enum {
     TX = 4, TY = (sizeof(C) == 8 || L <= 192) ? 4 : 2,
     NT = (sizeof(C) == 8 && L >= 256) ? 256 : 128,
-    MB = sizeof(C) == 8 ? 2 : (L <= 192 ? 4 : (ZPlan<L>::A > 24 ? 2 : 3))
+    MB = sizeof(C) == 8 ? 2 : (ZPlan<L>::A <= 18 ? 4 : (ZPlan<L>::A > 24 ? 2 : 3))
   };
 };
 #define DNS_ZCASE(n) case n: return f(std::integral_constant<int, n>());
@@ -591,7 +577,7 @@ cudaError_t launch_zb2(PA in, RowArr out, int nf, DnsGeom g, FftTab<C> tab, cuda
     auto k = k_zb2<C, L, T::TX, T::TY, T::NT, T::MB, PA>;
     const size_t sm = (size_t)L * T::TX * T::TY * sizeof(C);
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k<<<dim3((g.Kx + T::TX - 1) / T::TX, (g.Py + T::TY - 1) / T::TY, nf), T::NT, sm, st>>>(in, out, g, tab.zt);
+    k<<<dim3((g.Kx - 1 + T::TX - 1) / T::TX, (g.Py + T::TY - 1) / T::TY, nf), T::NT, sm, st>>>(in, out, g, tab.zt);
     return cudaGetLastError();
   });
 }
@@ -617,20 +603,17 @@ cudaError_t launch_zb(PencilArr in, RowArr out, int nf, DnsGeom g, FftTab<C> tab
   const bool any = variant == VAR_AUTO;
   if constexpr (sizeof(C) == 8) {
     if (any || variant == DNS_Z_TENSOR_COPY) {
-      const cudaError_t e = with_len_xz(g.Pz, [&](auto LL) -> cudaError_t {
+      const cudaError_t e = with_len_z(g.Pz, [&](auto LL) -> cudaError_t {
         constexpr int L = decltype(LL)::value;
-        if constexpr (L > 0 && WPlan<L, 2, FftMaxRadix<C>::v>::ok) {
-          constexpr int LS = wlen<C>(L) + 1;
+        typedef ZStage<C, L> Z;
+        if constexpr (Z::ok && Z::fits(L / 3 * 2)) {
           CUtensorMap tm;
-          if (status && g.Nz == L / 3 * 2 && tab.wt &&
-              (size_t)g.Nz * 16 + 128 <= (size_t)2 * LS * sizeof(C) && pencil_tmap(in, nf, g, sizeof(C), &tm)) {
+          if (status && g.Nz == L / 3 * 2 && tab.zt && pencil_tmap(in, nf, g, sizeof(C), &tm)) {
             if (probe) return cudaSuccess;
-            // pencils staged by tensor copies (a y pair per line pair), 8 x 2
-            // tile: 64-byte runs on the row side
-            const size_t sm = ((size_t)16 * LS) * sizeof(C);
-            cudaFuncSetAttribute(k_zbt<C, L, 8, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            dim3 grid((g.Kx + 7) / 8, (g.Py + 1) / 2, nf);
-            k_zbt<C, L, 8, 8, 2><<<grid, 256, sm, st>>>(tm, out, g, tab, status);
+            const size_t sm = (size_t)8 * Z::WS * sizeof(C);
+            cudaFuncSetAttribute(k_zbt<C, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            dim3 grid((g.Kx - 1 + 7) / 8, (g.Py + 1) / 2, nf);
+            k_zbt<C, L><<<grid, 256, sm, st>>>(tm, out, g, tab.zt, status);
             return cudaGetLastError();
           }
         }
@@ -661,19 +644,17 @@ cudaError_t launch_zf(RowArr in, PencilArr out, int nf, DnsGeom g, FftTab<C> tab
   const bool any = variant == VAR_AUTO;
   if constexpr (sizeof(C) == 8) {
     if (any || variant == DNS_Z_TENSOR_COPY) {
-      const cudaError_t e = with_len_xz(g.Pz, [&](auto LL) -> cudaError_t {
+      const cudaError_t e = with_len_z(g.Pz, [&](auto LL) -> cudaError_t {
         constexpr int L = decltype(LL)::value;
-        if constexpr (L > 0 && WPlan<L, 2, FftMaxRadix<C>::v>::ok) {
-          constexpr int LS = wlen<C>(L) + 1;
+        typedef ZStage<C, L> Z;
+        if constexpr (Z::ok && Z::fits(L)) {
           CUtensorMap tm;
-          if (status && g.Nz == L / 3 * 2 && tab.wt &&
-              (size_t)L * 16 + 128 <= (size_t)2 * LS * sizeof(C) && row_tmap(in, nf, g, sizeof(C), &tm)) {
+          if (status && g.Nz == L / 3 * 2 && tab.zt && row_tmap(in, nf, g, sizeof(C), &tm)) {
             if (probe) return cudaSuccess;
-            // rows staged by tensor copies, 4 x 4 tile
-            const size_t sm = ((size_t)16 * LS) * sizeof(C);
-            cudaFuncSetAttribute(k_zft<C, L, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            const size_t sm = (size_t)8 * Z::WS * sizeof(C);
+            cudaFuncSetAttribute(k_zft<C, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             dim3 grid((g.Kx + 3) / 4, (g.Py + 3) / 4, nf);
-            k_zft<C, L, 8><<<grid, 256, sm, st>>>(tm, out, g, tab, status);
+            k_zft<C, L><<<grid, 256, sm, st>>>(tm, out, g, tab.zt, status);
             return cudaGetLastError();
           }
         }
@@ -698,11 +679,11 @@ cudaError_t launch_zf(RowArr in, PencilArr out, int nf, DnsGeom g, FftTab<C> tab
   });
 }
 // CTAs per SM that k_x2 is compiled for, measured at 384 (FP32 / FP64, us):
-// five 294 / 623, four 312 / 642; FP32 at 216: seven 33.1, five 34.7.  Radix 18
-// in the middle needs the registers of four.
+// five 294 / 623, four 312 / 642; FP32 at 216: seven 33.1, five 34.7; at 96 ten
+// 95, seven 99.  Radix 18 in the middle needs the registers of four.
 template <typename C, int L> constexpr int x2_ctas() {
   typedef XPlan<L, FftMaxRadix<C>::v> P;
-  return P::NW > 3 ? (L > 576 ? 1 : 2) : (P::RF > 16 ? 4 : (sizeof(C) == 8 && L < 256 ? 7 : 5));
+  return P::NW > 3 ? (L > 576 ? 1 : 2) : (P::RF > 16 ? 4 : sizeof(C) == 16 || L >= 256 ? 5 : L > 96 ? 7 : 10);
 }
 template <typename C, int L, int SC>
 cudaError_t launch_x2(RowArr in, RowArr out, DnsGeom g, FftTab<C> tab, const double* Uy, double Ro, int* status,
