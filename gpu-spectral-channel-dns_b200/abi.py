@@ -40,6 +40,8 @@ PASS_Y3, PASS_Y1, PASS_ZB, PASS_ZF, PASS_Y2, PASS_X, NUM_PASSES, MAX_VARIANTS = 
 Y3_FFT, Y3_TENSOR, Y3_BLOCK = 0, 1, 2
 Y1_WARP, Y1_BLOCK = 0, 1
 Z_TENSOR_COPY, Z_WARP, Z_BLOCK = 0, 1, 2
+Y2_RING2_24K_EF, Y2_RING2_18K_EF, Y2_RING2_12K_EF, Y2_RING2_16K_EF = 0, 1, 2, 3
+# earlier names of the same values
 Y2_RING3_12K, Y2_RING3_12K_EF, Y2_RING2_8K_EF, Y2_RING3_8K_EF = 0, 1, 2, 3
 X_WARP3, X_WARP6, X_BLOCK = 0, 1, 2
 # names of the tunable passes and their variants (bench and test reports)
@@ -50,8 +52,8 @@ VARIANT_NAMES = {
     PASS_Y1: {Y1_WARP: "warp_fft", Y1_BLOCK: "block_fft"},
     PASS_ZB: {Z_TENSOR_COPY: "warp_fft_tensor_copy", Z_WARP: "warp_fft", Z_BLOCK: "block_fft"},
     PASS_ZF: {Z_TENSOR_COPY: "warp_fft_tensor_copy", Z_WARP: "warp_fft", Z_BLOCK: "block_fft"},
-    PASS_Y2: {Y2_RING3_12K: "ring_3x12k", Y2_RING3_12K_EF: "ring_3x12k_evict_first",
-              Y2_RING2_8K_EF: "ring_2x8k_evict_first", Y2_RING3_8K_EF: "ring_3x8k_evict_first"},
+    PASS_Y2: {Y2_RING2_24K_EF: "ring_2x24k", Y2_RING2_18K_EF: "ring_2x18k",
+              Y2_RING2_12K_EF: "ring_2x12k", Y2_RING2_16K_EF: "ring_2x16k"},
     PASS_X: {X_WARP3: "warp_fft_3_warps", X_WARP6: "warp_fft_6_warps", X_BLOCK: "block_fft"},
 }
 

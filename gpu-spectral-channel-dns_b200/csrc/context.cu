@@ -178,7 +178,7 @@ dns_status ctx_build_wall_solver(dns_ctx* c) {
     wd.groups_per_run = wd.ngroups;
     wd.ngroups *= g.nrun;
   }
-  if (wall_smem_bytes(wd, DNS_Y2_RING2_8K_EF) > 227 * 1024) return fail(DNS_ERR_ARG, "Ny too large for the wall solve");
+  if (wall_smem_bytes(wd, DNS_Y2_RING2_12K_EF) > 227 * 1024) return fail(DNS_ERR_ARG, "Ny too large for the wall solve");
   if (wall_scratch_complex(wd) * 16 > c->F6_bytes)
     return fail(DNS_ERR_ARG, "wall solve scratch does not fit the transform buffer");
   CK(c->alloc(&c->wfac, fac.size()));
@@ -255,7 +255,7 @@ cudaError_t enqueue_pipeline(dns_ctx* c, int boot, const DevFft<C>& fz, const De
   if (!boot)
     if ((e = var(DNS_PASS_Y2, [&](int v) {
            return launch_wall_solve(c->wfac, b.V, b.O, c->rv, c->ro, c->wQ, (double2*)c->F6, c->wd, g, c->ph,
-                                    c->status, c->st, v == VAR_AUTO ? DNS_Y2_RING2_8K_EF : v);
+                                    c->status, c->st, v == VAR_AUTO ? DNS_Y2_RING2_12K_EF : v);
          })))
       return e;
   mark();
@@ -322,11 +322,11 @@ void default_variants(dns_ctx* c) {
   static const int order_mixed[DNS_NUM_PASSES][3] = {
       {DNS_Y3_FFT, DNS_Y3_BLOCK, -1}, {DNS_Y1_WARP, DNS_Y1_BLOCK, -1},
       {DNS_Z_TENSOR_COPY, DNS_Z_WARP, DNS_Z_BLOCK}, {DNS_Z_TENSOR_COPY, DNS_Z_WARP, DNS_Z_BLOCK},
-      {DNS_Y2_RING3_12K_EF, DNS_Y2_RING2_8K_EF, -1}, {DNS_X_WARP3, DNS_X_BLOCK, -1}};
+      {DNS_Y2_RING2_18K_EF, DNS_Y2_RING2_12K_EF, -1}, {DNS_X_WARP3, DNS_X_BLOCK, -1}};
   static const int order_fp64[DNS_NUM_PASSES][3] = {
       {DNS_Y3_FFT, DNS_Y3_BLOCK, -1}, {DNS_Y1_WARP, DNS_Y1_BLOCK, -1},
       {DNS_Z_WARP, DNS_Z_BLOCK, -1}, {DNS_Z_WARP, DNS_Z_BLOCK, -1},
-      {DNS_Y2_RING3_12K_EF, DNS_Y2_RING2_8K_EF, -1}, {DNS_X_WARP3, DNS_X_BLOCK, -1}};
+      {DNS_Y2_RING2_18K_EF, DNS_Y2_RING2_12K_EF, -1}, {DNS_X_WARP3, DNS_X_BLOCK, -1}};
   // FP32 spanwise lines: tensor-staged tiles from 144 points on, where pass A
   // keeps most lanes of a warp busy (inverse + forward, us: 384 x 384 x 512 195
   // + 115 against 263 + 132; two 96 x 288 x 256 50 + 33 against 60 + 34; four
@@ -340,14 +340,19 @@ void default_variants(dns_ctx* c) {
     for (int i = skip; i < 3 && ord[i] >= 0; ++i)
       if (variant_available(c, p, ord[i])) { c->variant[p] = ord[i]; break; }
   }
-  // the solve: more groups than four CTAs per SM take run in one wave with
-  // the small ring, as long as their scratch vectors stay in L2 (us, 3 x 12 KB
-  // / 2 x 8 KB, evict-first: 1041 groups of 33 points 80 / 70, 828 of 49 points
-  // 100 / 85; 1041 of 129 points, 70 MB of scratch, 249 / 297)
+  // The solve (us, 2 x 24 / 2 x 18 / 2 x 12 / 2 x 16 KB): up to three groups per
+  // SM the most rows per stage (116 groups of 33 points 28 / 29 / 31 / 27, 265 of
+  // 65 points 50 / 58 / 66 / 57, 169 of 55 points 38 / 43 / 45 / 41); beyond, one
+  // wave of small rings as long as the scratch vectors stay in L2 (828 of 49
+  // points 97 / 102 / 80 / 90, 1041 of 33 points 73 / 74 / 67 / 79), else the
+  // largest that leaves four CTAs per SM and no fifth (1041 of 129 points 263 /
+  // 239 / 287 / 286, five of 2 x 16 KB; 2329 of 193 points 857 / 874 / 977 / 815).
   const long long groups = ((long long)c->g.Kx * (c->slab ? c->slab->s1 - c->slab->s0 : c->g.Kh) + 15) / 16 * c->g.nrun;
-  if (groups > 4 * 148 && groups * 32 * c->wd.nv * 16 <= (40LL << 20) &&
-      variant_available(c, DNS_PASS_Y2, DNS_Y2_RING2_8K_EF))
-    c->variant[DNS_PASS_Y2] = DNS_Y2_RING2_8K_EF;
+  const int ring = groups <= 3 * 148                                      ? DNS_Y2_RING2_24K_EF
+                   : groups * 32 * c->wd.nv * 16 <= (40LL << 20)          ? DNS_Y2_RING2_12K_EF
+                   : wall_smem_bytes(c->wd, DNS_Y2_RING2_16K_EF) > 45 * 1024 ? DNS_Y2_RING2_16K_EF
+                                                                            : DNS_Y2_RING2_18K_EF;
+  if (variant_available(c, DNS_PASS_Y2, ring)) c->variant[DNS_PASS_Y2] = ring;
 }
 // the spanwise variant of the FP64 per-function entries: the context's own
 // in the FP64 form, else the first that the length allows
@@ -1224,7 +1229,7 @@ cudaError_t enqueue_solve_wall(dns_ctx* c, const double2* bv, const double2* bo,
                                 c->status, c->st, c->variant[DNS_PASS_Y2], pbc);
   if (e == cudaErrorNotSupported)
     e = launch_wall_solve(c->wfac, ov, oo, c->rv, c->ro, c->wQ, (double2*)c->F6, wd, g, c->ph, c->status, c->st,
-                          DNS_Y2_RING2_8K_EF, pbc);
+                          DNS_Y2_RING2_12K_EF, pbc);
   return e;
 }
 }  // namespace

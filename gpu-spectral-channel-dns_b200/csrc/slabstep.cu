@@ -187,7 +187,7 @@ cudaError_t part_y1(dns_ctx* c, int boot, const void* recv) {
                           c->st, c->variant[DNS_PASS_Y2]);
     if (e == cudaErrorNotSupported)
       e = launch_wall_solve(c->wfac, c->V, c->O, c->rv, c->ro, c->wQ, (double2*)c->F6, c->wd, g, c->ph,
-                            c->status, c->st, DNS_Y2_RING2_8K_EF);
+                            c->status, c->st, DNS_Y2_RING2_12K_EF);
   }
   return e;
 }

@@ -30,24 +30,20 @@ namespace {
 
 constexpr int WALL_HDR = 128;        // mbarriers
 
-// Variants (the solve's tunable block shape): ring stages, bytes per stage,
-// whether the tilting table sits in shared memory (else read through L1),
-// and whether the factor stream is read with the L2 evict-first policy (the
-// scratch vectors then stay in L2).  Smaller rings leave room for more CTAs
-// per SM.
+// Variants (the solve's tunable block shape): ring stages, bytes per stage
+// and whether the tilting table sits in shared memory (else read through L1).
+// The factor stream is read with the L2 evict-first policy (the scratch vectors
+// then stay in L2).  More rows per stage hide the scratch loads of a warp, a
+// smaller ring leaves room for more CTAs per SM.
 struct WallVar {
   int nst, stg;
-  bool qsm, ef;
+  bool qsm;
 };
-constexpr WallVar kWallVar[DNS_WALL_VARIANTS] = {
-    {3, 12288, true, false}, {3, 12288, true, true}, {2, 8192, false, true}, {3, 8192, false, true}};
+constexpr WallVar kWallVar[DNS_WALL_VARIANTS] = {{2, 24576, true}, {2, 18432, true}, {2, 12288, false}, {2, 16384, true}};
 
 __host__ __device__ constexpr int rows_per_chunk(int stg, int entries, int cap) {
   return (stg / (entries * 256)) < cap ? (stg / (entries * 256)) : cap;
 }
-
-struct Whole { static constexpr bool full = true; };
-struct Part { static constexpr bool full = false; };
 
 // acc + a b, acc - a b: four fused operations (a product and a sum apart
 // are six)
@@ -64,15 +60,15 @@ __device__ __forceinline__ double2 rfma(double a, double2 b, double2 acc) {
 template <int KLV, int KUV, int KLO, int KUO, int STG>
 struct WallCfg {
   static constexpr int E0 = KLV, E1 = 1 + KUV + 2, E2 = KLO, E3 = 1 + KUO;
-  // rows per ring chunk; the solve keeps two chunks of vector rows in registers
-  static constexpr int R0 = rows_per_chunk(STG, E0, 12), R1 = rows_per_chunk(STG, E1, 12);
-  static constexpr int R2 = rows_per_chunk(STG, E2, 8), R3 = rows_per_chunk(STG, E3, 12);
+  // rows per ring chunk; the solve keeps a chunk of vector rows in registers
+  static constexpr int R0 = rows_per_chunk(STG, E0, WALL_ROWS), R1 = rows_per_chunk(STG, E1, WALL_ROWS);
+  static constexpr int R2 = rows_per_chunk(STG, E2, WALL_ROWS), R3 = rows_per_chunk(STG, E3, WALL_ROWS);
   static_assert(R0 > 0 && R1 > 1 && R2 > 0 && R3 > 0, "stage too small for a row");
 };
 
 }  // namespace
 
-template <int KLV, int KUV, int KLO, int KUO, int WALL_NST, int WALL_STG, bool QSM, bool EF>
+template <int KLV, int KUV, int KLO, int KUO, int WALL_NST, int WALL_STG, bool QSM>
 __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ fac, double2* V,
                                                    double2* O, const double2* __restrict__ gv,
                                                    const double2* __restrict__ go,
@@ -86,7 +82,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
   const double* Qs = (QSM ? Qsm : Qg) + 7 * WALL_QLOW;  // tilting table: shared memory or through L1
   // recombination weights of the clamped basis, row by row
   double* rc2 = Qsm + (QSM ? wd.qbytes / 8 : 0);
-  double* rc4 = rc2 + wd.nv;
+  double* rc4 = rc2 + wd.nv + WALL_ROWS;
 
   const int lane = threadIdx.x;
   const int q = lane >> 1, b = lane & 1;
@@ -119,22 +115,28 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
   const bool dov = wd.sys & 1, doo = wd.sys & 2;
   const int total = (dov ? nch0 + nch1 : 0) + (doo ? nch2 + nch3 : 0);
 
-  const uint64_t pol = EF ? l2_evict_first() : 0;
+  const uint64_t pol = l2_evict_first();
   // the group's stream is contiguous: lane 0 walks it phase by phase, ic the
-  // next chunk, irow rows of its phase issued
+  // next chunk, irow rows of its phase issued.  Rows ascend in phases 0 and 2,
+  // whose last chunk may be short; they descend in phases 1 and 3, whose first
+  // one may be, its rows at the end of the stage.
+  const int n1 = (wd.nv - 1) % CF::R1 + 1, n3 = (wd.no - 1) % CF::R3 + 1;
   int ic = 0, iph = dov ? 0 : 2, irow = 0;
   const double2* isrc = gfac + (dov ? 0 : 16LL * wd.nv * (CF::E0 + CF::E1));
   auto issue = [&]() {
     const int rows = iph < 2 ? wd.nv : wd.no;
     const int R = iph == 0 ? CF::R0 : iph == 1 ? CF::R1 : iph == 2 ? CF::R2 : CF::R3;
     const int E = iph == 0 ? CF::E0 : iph == 1 ? CF::E1 : iph == 2 ? CF::E2 : CF::E3;
-    const int n = min(R, rows - irow);
-    const uint32_t bytes = (uint32_t)(n * E * 256);
+    int n = min(R, rows - irow);
     uint64_t* bar = &full[ic % WALL_NST];
     double2* dst = ring + (size_t)(ic % WALL_NST) * (WALL_STG / 16);
+    if ((iph & 1) && irow == 0) {
+      n = iph == 1 ? n1 : n3;
+      dst += (R - n) * E * 16;
+    }
+    const uint32_t bytes = (uint32_t)(n * E * 256);
     mbar_expect_tx(bar, bytes);
-    if (EF) bulk_g2s_hint(dst, isrc, bytes, bar, pol);
-    else bulk_g2s(dst, isrc, bytes, bar);
+    bulk_g2s_hint(dst, isrc, bytes, bar, pol);
     isrc += n * E * 16;
     irow += n;
     if (irow == rows) { irow = 0; ++iph; }
@@ -161,6 +163,14 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
     }
   };
   auto chunk_at = [&](int c) { return ring + (size_t)(c % WALL_NST) * (WALL_STG / 16) + q; };
+  // zeros before the rows of a descending phase's short first chunk: those rows,
+  // above the last, then come out as zeros
+  auto zero_rows = [&](int c, int n) {
+    double2* z = ring + (size_t)(c % WALL_NST) * (WALL_STG / 16);
+    for (int k = lane; k < n * 16; k += 32) z[k] = z2;
+    fence_proxy_async();
+    __syncwarp();
+  };
   const double2* gvp = gv + pen * wd.gp;
   const double2* gop = go + pen * wd.gp;
   const int nv = wd.nv, no = wd.no;
@@ -175,7 +185,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
     for (int k = lane; k < WALL_QROWS(no) * 7; k += 32) Qsm[k] = Qg[k];
   // recombination weights of row i: V_{i+4} = x_{i+4} - 2k/(k+1) x_{i+2} +
   // (k-3)/(k-1) x_i, k = i + 4, unknowns from N - 3 on are not part of it
-  for (int i = lane; i < nv; i += 32) {
+  for (int i = lane; i < nv + WALL_ROWS; i += 32) {
     const int k = i + 4;
     rc2[i] = i + 2 < N - 3 ? 2.0 * k / (k + 1) : 0.0;
     rc4[i] = i < N - 3 ? (double)(k - 3) / (double)(k - 1) : 0.0;
@@ -187,9 +197,12 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
   const bool mean = __any_sync(0xffffffffu, zero);
 
   // Rows go in chunks of the ring; a row's vector element is loaded one chunk
-  // ahead into the register it is consumed from.  Whole chunks run without
-  // conditions between their rows, so that the windows of earlier rows are
-  // renamed registers and not moves; FULL = false is a phase's last chunk.
+  // ahead into the register it is consumed from.  Every chunk runs the same
+  // code without conditions between its rows, so that the windows of earlier
+  // rows are renamed registers and not moves: rows beyond a phase's last are
+  // computed and not stored (ascending) or come first as zeros (descending).
+  // One body per phase: a warp is alone on its scheduler, and a grid of few
+  // groups spends a third of its time fetching instructions.
   int c = 0;
   // ---- v: forward substitution (unit lower band) -------------------------
   if (dov) {
@@ -199,40 +212,32 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
     for (int e = 0; e < KLV; ++e) yw[e] = z2;
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) cur[rr] = (active && rr < nv) ? __ldg(gvp + rr) : z2;
-    auto chunk = [&](auto whole, const double2* ch, int r0) {
+    auto chunk = [&](const double2* ch, int r0) {
       const double2* nx = gvp + r0 + R;
       double2* Sr = S + 32 * r0;
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
-        if (!whole.full && r0 + rr >= nv) continue;
         const double2* Lr = ch + rr * CF::E0 * 16;
         // the older entries in independent partial sums; the newest
         // (y_{i-1}) last, so only it is on the row-to-row critical path
         double2 a0 = cur[rr], a1 = z2;
-        if (whole.full) cur[rr] = (active && r0 + R + rr < nv) ? __ldg(nx + rr) : z2;
+        cur[rr] = (active && r0 + R + rr < nv) ? __ldg(nx + rr) : z2;
 #pragma unroll
         for (int e = 0; e < KLV - 1; ++e) {
           if (e & 1) a1 = cfms(Lr[e * 16], yw[e], a1);
           else a0 = cfms(Lr[e * 16], yw[e], a0);
         }
         const double2 acc = cfms(Lr[(KLV - 1) * 16], yw[KLV - 1], a0 + a1);
-        Sr[32 * rr] = acc;
+        if (r0 + rr < nv) Sr[32 * rr] = acc;
 #pragma unroll
         for (int e = 0; e < KLV - 1; ++e) yw[e] = yw[e + 1];
         yw[KLV - 1] = acc;
       }
     };
-    int r0 = 0;
-    for (; r0 + R <= nv; r0 += R, ++c) {
+    for (int r0 = 0; r0 < nv; r0 += R, ++c) {
       if (!wait_chunk(c)) { abort_at(c); return; }
-      chunk(Whole(), chunk_at(c), r0);
+      chunk(chunk_at(c), r0);
       release();
-    }
-    if (r0 < nv) {
-      if (!wait_chunk(c)) { abort_at(c); return; }
-      chunk(Part(), chunk_at(c), r0);
-      release();
-      ++c;
     }
   }
   // ---- v: back substitution, recombination, tilting term -----------------
@@ -265,18 +270,19 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
       P[6] = z2;
     };
 #pragma unroll
-    for (int rr = 0; rr < R; ++rr) cur[rr] = rr < nv ? S[32 * (nv - 1 - rr)] : z2;
+    for (int rr = 0; rr < R; ++rr) {
+      const int i = nch1 * R - 1 - rr;
+      cur[rr] = i < nv ? S[32 * i] : z2;
+    }
     double2* Vp = V + pen * wd.xp + (zero ? 2 : 4);  // row i emits coefficient i + 4, of the mean modes i + 2
     const int top = zero ? N - 2 : N - 4;         // the last row that emits one
-    auto chunk = [&](auto whole, const double2* ch, int r0) {
-      const int i0 = nv - 1 - r0;
+    auto chunk = [&](const double2* ch, int i0) {
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
-        if (!whole.full && r0 + rr >= nv) continue;
         const int i = i0 - rr;
         const double2* Ur = ch + rr * CF::E1 * 16;
         double2 a0 = cur[rr];
-        if (whole.full) cur[rr] = i >= R ? S[32 * (i - R)] : z2;
+        cur[rr] = i >= R ? S[32 * (i - R)] : z2;
         // independent partial sums; x_{i+1} enters last
         double2 a1 = z2, a2 = z2;
         a1 = cfms(Ur[(KUV + 1) * 16], xd0, a1);
@@ -289,9 +295,10 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
         }
         const double2 acc = cfms(Ur[16], xw[0], a0 + (a1 + a2));
         const double2 x = cmul(Ur[0], acc);
-        // the two unknowns with dense columns
-        if (rr == 0 && r0 == 0) xd1 = x;
-        if (rr == 1 && r0 == 0) xd0 = x;
+        if (i >= nv - 2) {  // the two unknowns with dense columns
+          if (i == nv - 1) xd1 = x;
+          if (i == nv - 2) xd0 = x;
+        }
 #pragma unroll
         for (int e = KUV - 1; e >= 1; --e) xw[e] = xw[e - 1];
         xw[0] = x;
@@ -306,17 +313,11 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
         tilt(i + 4, a, false);
       }
     };
-    int r0 = 0;
-    for (; r0 + R <= nv; r0 += R, ++c) {
+    for (int i0 = nch1 * R - 1; i0 >= 0; i0 -= R, ++c) {
       if (!wait_chunk(c)) { abort_at(c); return; }
-      chunk(Whole(), chunk_at(c), r0);
+      if (i0 >= nv) zero_rows(c, (R - n1) * CF::E1);
+      chunk(chunk_at(c), i0);
       release();
-    }
-    if (r0 < nv) {
-      if (!wait_chunk(c)) { abort_at(c); return; }
-      chunk(Part(), chunk_at(c), r0);
-      release();
-      ++c;
     }
     double2 a[4];
     a[3] = xw[3] - xw[1] * 1.5;
@@ -346,19 +347,16 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
       gc[rr] = (active && rr < no) ? __ldg(gop + rr) : z2;
       sc[rr] = dov && rr < no ? S[32 * rr] : z2;
     }
-    auto chunk = [&](auto whole, const double2* ch, int r0) {
+    auto chunk = [&](const double2* ch, int r0) {
       const double2* nx = gop + r0 + R;
       double2* Sr = S + 32 * r0;
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
-        if (!whole.full && r0 + rr >= no) continue;
         const double2* Lr = ch + rr * CF::E2 * 16;
         double2 a0 = sc[rr] + gc[rr];
-        if (whole.full) {
-          const bool more = r0 + R + rr < no;
-          gc[rr] = (active && more) ? __ldg(nx + rr) : z2;
-          sc[rr] = dov && more ? Sr[32 * (R + rr)] : z2;
-        }
+        const bool more = r0 + R + rr < no;
+        gc[rr] = (active && more) ? __ldg(nx + rr) : z2;
+        sc[rr] = dov && more ? Sr[32 * (R + rr)] : z2;
         double2 a1 = z2;
 #pragma unroll
         for (int e = 0; e < KLO - 1; ++e) {
@@ -366,23 +364,16 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
           else a0 = cfms(Lr[e * 16], ow[e], a0);
         }
         const double2 acc = cfms(Lr[(KLO - 1) * 16], ow[KLO - 1], a0 + a1);
-        Sr[32 * rr] = acc;
+        if (r0 + rr < no) Sr[32 * rr] = acc;
 #pragma unroll
         for (int e = 0; e < KLO - 1; ++e) ow[e] = ow[e + 1];
         ow[KLO - 1] = acc;
       }
     };
-    int r0 = 0;
-    for (; r0 + R <= no; r0 += R, ++c) {
+    for (int r0 = 0; r0 < no; r0 += R, ++c) {
       if (!wait_chunk(c)) { abort_at(c); return; }
-      chunk(Whole(), chunk_at(c), r0);
+      chunk(chunk_at(c), r0);
       release();
-    }
-    if (r0 < no) {
-      if (!wait_chunk(c)) { abort_at(c); return; }
-      chunk(Part(), chunk_at(c), r0);
-      release();
-      ++c;
     }
   }
   // ---- omega: back substitution and recombination ------------------------
@@ -394,16 +385,17 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
     const int nbo = N - 1;
     double2* Op = O + pen * wd.xp + 2;
 #pragma unroll
-    for (int rr = 0; rr < R; ++rr) cur[rr] = rr < no ? S[32 * (no - 1 - rr)] : z2;
-    auto chunk = [&](auto whole, const double2* ch, int r0) {
-      const int i0 = no - 1 - r0;
+    for (int rr = 0; rr < R; ++rr) {
+      const int i = nch3 * R - 1 - rr;
+      cur[rr] = i < no ? S[32 * i] : z2;
+    }
+    auto chunk = [&](const double2* ch, int i0) {
 #pragma unroll
       for (int rr = 0; rr < R; ++rr) {
-        if (!whole.full && r0 + rr >= no) continue;
         const int i = i0 - rr;
         const double2* Ur = ch + rr * CF::E3 * 16;
         double2 a0 = cur[rr], a1 = z2;
-        if (whole.full) cur[rr] = i >= R ? S[32 * (i - R)] : z2;
+        cur[rr] = i >= R ? S[32 * (i - R)] : z2;
 #pragma unroll
         for (int e = KUO; e >= 2; --e) {
           if (e & 1) a1 = cfms(Ur[e * 16], zw[e - 1], a1);
@@ -417,17 +409,11 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
         if (active && i < nbo) Op[i] = rfma(i + 2 < nbo ? -1.0 : 0.0, zw[2], x);
       }
     };
-    int r0 = 0;
-    for (; r0 + R <= no; r0 += R, ++c) {
+    for (int i0 = nch3 * R - 1; i0 >= 0; i0 -= R, ++c) {
       if (!wait_chunk(c)) { abort_at(c); return; }
-      chunk(Whole(), chunk_at(c), r0);
+      if (i0 >= no) zero_rows(c, (R - n3) * CF::E3);
+      chunk(chunk_at(c), i0);
       release();
-    }
-    if (r0 < no) {
-      if (!wait_chunk(c)) { abort_at(c); return; }
-      chunk(Part(), chunk_at(c), r0);
-      release();
-      ++c;
     }
     if (active) {
       const double2 a1 = make_double2(-zw[1].x, -zw[1].y), a0 = make_double2(-zw[0].x, -zw[0].y);
@@ -439,7 +425,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
 
 size_t wall_smem_bytes(const WallDims& wd, int variant) {
   const WallVar& v = kWallVar[variant];
-  return (size_t)WALL_HDR + (size_t)v.nst * v.stg + (v.qsm ? wd.qbytes : 0) + (size_t)2 * (wd.nv + 2) * 8;
+  return (size_t)WALL_HDR + (size_t)v.nst * v.stg + (v.qsm ? wd.qbytes : 0) + (size_t)2 * (wd.nv + WALL_ROWS) * 8;
 }
 size_t wall_scratch_complex(const WallDims& wd) { return (size_t)wd.ngroups * 32 * wd.nv; }
 
@@ -456,7 +442,7 @@ static cudaError_t launch_inst(const double2* fac, double2* V, double2* O, const
                                const double2* go, const double* Q, double2* Sw, const double2* pbc,
                                const WallDims& wd, const DnsGeom& g, const PhysParams& ph, int* status, cudaStream_t st) {
   constexpr WallVar v = kWallVar[VAR];
-  auto k = k_wall_solve<A, B, C, D, v.nst, v.stg, v.qsm, v.ef>;
+  auto k = k_wall_solve<A, B, C, D, v.nst, v.stg, v.qsm>;
   const size_t sm = wall_smem_bytes(wd, VAR);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e) return e;

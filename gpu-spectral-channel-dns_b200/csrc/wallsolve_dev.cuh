@@ -7,7 +7,8 @@
 // rows of the tilting table: zero rows below 0 and above the last, so that
 // the solve reads it without bounds checks
 #define WALL_QLOW 2
-#define WALL_QROWS(no) ((no) + WALL_QLOW + 8)
+#define WALL_ROWS 12  // most rows of a ring chunk
+#define WALL_QROWS(no) ((no) + WALL_QLOW + 8 + WALL_ROWS)
 
 struct WallDims {
   int nv, no;              // rows of the packed v and omega systems (N + deg U + 1)

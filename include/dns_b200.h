@@ -211,11 +211,12 @@ dns_status dns_set_wait_limit(dns_ctx* ctx, long long cycles);
  *     warps, two lines each) for lengths with warp plans, DNS_X_BLOCK (block
  *     FFT, every grid).
  *   DNS_PASS_Y2: the banded wall-normal solves; the block shape of the
- *     factor stream (ring stages x bytes per stage; the tilting table in
- *     shared memory or read through L1; the stream read with the L2
- *     evict-first policy or not): DNS_Y2_RING3_12K (table in shared memory),
- *     DNS_Y2_RING3_12K_EF (the same, evict-first), DNS_Y2_RING2_8K_EF,
- *     DNS_Y2_RING3_8K_EF.
+ *     factor stream (ring stages x bytes per stage, read with the L2
+ *     evict-first policy): DNS_Y2_RING2_24K_EF, DNS_Y2_RING2_18K_EF,
+ *     DNS_Y2_RING2_12K_EF (the tilting table read through L1, else in shared
+ *     memory), DNS_Y2_RING2_16K_EF.  DNS_Y2_RING3_12K, DNS_Y2_RING3_12K_EF,
+ *     DNS_Y2_RING2_8K_EF and DNS_Y2_RING3_8K_EF are earlier names of the same
+ *     values.
  * dns_set_variant fails with DNS_ERR_ARG for a variant this context cannot
  * run.  dns_autotune times every available variant of every tunable pass
  * inside whole steps on this context's buffers and grid (state and AB2
@@ -237,6 +238,7 @@ enum {
 enum { DNS_Y3_FFT = 0, DNS_Y3_TENSOR = 1, DNS_Y3_BLOCK = 2 };
 enum { DNS_Y1_WARP = 0, DNS_Y1_BLOCK = 1 };
 enum { DNS_Z_TENSOR_COPY = 0, DNS_Z_WARP = 1, DNS_Z_BLOCK = 2 };
+enum { DNS_Y2_RING2_24K_EF = 0, DNS_Y2_RING2_18K_EF = 1, DNS_Y2_RING2_12K_EF = 2, DNS_Y2_RING2_16K_EF = 3 };
 enum { DNS_Y2_RING3_12K = 0, DNS_Y2_RING3_12K_EF = 1, DNS_Y2_RING2_8K_EF = 2, DNS_Y2_RING3_8K_EF = 3 };
 enum { DNS_X_WARP3 = 0, DNS_X_WARP6 = 1, DNS_X_BLOCK = 2 };
 dns_status dns_set_variant(dns_ctx* ctx, int pass, int variant);
