@@ -12,11 +12,11 @@
 //                                  (reference-layout op; the time step solves
 //                                  the banded systems of wallsolve.cu)
 //
-// The Chebyshev transforms are DCT-I evaluated as complex FFTs of the even
-// extension, as the reference does with cuFFT, but in shared memory with the
-// project's own FFT (fft.cuh).  Collocation-point values of v, v'', v'''',
-// omega, omega'' (the reference's T0/T2/T4 matrix products) are obtained the
-// same way: coefficient-space derivatives, then the no-pad DCT.
+// The Chebyshev transforms are DCT-I of complex series.  Lengths 2^a 3^b with a
+// plan run the FFT of the even extension with its mirrored half left out, on two
+// register butterflies and one exchange (ydct.cuh: k_y3d, k_y1d, k_cheby_dct);
+// other lengths the block-wide FFT of the whole extension (fft2.cuh, fft.cuh:
+// k_y3, k_y1, k_cheby).
 #include "fftline.cuh"
 #include "kernels.cuh"
 #include "mbar.cuh"
@@ -822,8 +822,8 @@ __global__ void __launch_bounds__(256, 3) k_y1(PencilArr lam, const double2* __r
 // What bounds it: issue slots (7055 warp instructions a pencil at M = 512
 // before, a fifth of them FP64), so vectors carry zero guards instead of
 // bounds checks, and the sums over k are halved between lanes at every
-// step.  4530 instructions; 256 x 129 x 256 mixed 383 -> 299 us, FP64 497 ->
-// 440; 128 x 65 x 128 FP64 107 -> 74; twelve 64 x 49 x 64 mixed 184 -> 115;
+// step.  4530 instructions; 256 x 129 x 256 mixed 383 -> 278 us, FP64 497 ->
+// 432; 128 x 65 x 128 FP64 107 -> 63; twelve 64 x 49 x 64 mixed 184 -> 114;
 // 144 x 55 x 72 mixed, a length on the block form before, 160 -> 33.
 namespace {
 // Sums over the 16 lanes of a parity of NV values a lane, halved at every
@@ -1204,10 +1204,14 @@ cudaError_t launch_y3(const double2* V, const double2* O, PencilArr out, DnsGeom
 template cudaError_t launch_y3<double2>(const double2*, const double2*, PencilArr, DnsGeom, PhysParams, FftTab<double2>, int*, cudaStream_t, int, bool);
 template cudaError_t launch_y3<float2>(const double2*, const double2*, PencilArr, DnsGeom, PhysParams, FftTab<float2>, int*, cudaStream_t, int, bool);
 
-// CTAs per SM of k_y1d: what the first radix leaves of the registers
+// CTAs per SM of k_y1d, by the first radix (its registers). The kernel waits at
+// barriers between short phases, so one more resident CTA is worth a few spilled
+// words: with 5 | 6 | 8 (FP32) and 3 | 4 | 4 (FP64) CTAs 84x33x84 took 31.0 us
+// (now 25.4), 128x65x128 74.6 (63.4), mixed 256x129x256 300 (277), FP64
+// 256x129x256 442 (432); one CTA more again, 10 in FP32, 5 % slower.
 template <typename C, int M> constexpr int y1_ctas() {
   constexpr int RA = DPlan<M>::A;
-  return sizeof(C) == 8 ? (RA > 24 ? 5 : (RA > 18 ? 6 : 8)) : (RA > 24 ? 3 : 4);
+  return sizeof(C) == 8 ? (RA > 24 ? 7 : (RA > 18 ? 8 : 9)) : (RA > 24 ? 4 : (RA > 16 ? 5 : 7));
 }
 template <typename C>
 cudaError_t launch_y1(PencilArr lam, const double2* V, const double2* O, double2* Nvp,
