@@ -365,12 +365,28 @@ int zvar64(const dns_ctx* c, int pass) {
 dns_status need_scratch(dns_ctx* c) {
   if (c->scratch) return DNS_OK;
   const size_t one = (size_t)c->g.Py * c->g.Pz * c->RS;
-  const int n = (int)std::max<size_t>(1, std::min<size_t>(6, ((size_t)64 << 20) / (one * 16)));
-  CK(c->alloc(&c->scratch, one * n));
+  int n = (int)std::max<size_t>(1, std::min<size_t>(6, ((size_t)64 << 20) / (one * 16)));
+  if (n > 1 && c->alloc(&c->scratch, one * n)) {  // a device that is nearly full: one field
+    cudaGetLastError();
+    c->bytes -= one * n * 16;
+    c->scratch = nullptr;
+    n = 1;
+  }
+  if (!c->scratch) CK(c->alloc(&c->scratch, one));
   c->scratch_fields = n;
   return DNS_OK;
 }
 
+// device or managed memory, aligned for complex loads: a pointer that a kernel
+// can take where copies would take, or refuse, any
+bool kernel_ptr(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return aligned16(p) && (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged);
+}
 cudaMemcpyKind kind_of(int where, bool to_device) {
   if (where == DNS_DEVICE) return cudaMemcpyDeviceToDevice;
   return to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
@@ -689,8 +705,8 @@ dns_status dns_get_state(dns_ctx* c, void* v, void* o, size_t pitch, int where) 
 // The AB2 history is held as Chebyshev coefficients; the ABI exchanges it
 // as values at the Gauss-Lobatto points (the reference's rhs_v_p /
 // rhs_omega_y_p), converted here with the no-pad s2p / p2s: on device pencils
-// straight between the caller's and the library's, on host pencils through the
-// scratch, member by member of a batch.
+// straight between the caller's and the library's (where the pointer is one
+// that a kernel can take), else through the scratch, member by member of a batch.
 static dns_status history_copy(dns_ctx* c, double2* hist, void* user, size_t pitch, int where, bool out) {
   const size_t w = (size_t)c->g.Ny * 16;
   if (where != DNS_HOST && where != DNS_DEVICE) return fail(DNS_ERR_ARG, "where must be DNS_HOST or DNS_DEVICE");
@@ -700,7 +716,7 @@ static dns_status history_copy(dns_ctx* c, double2* hist, void* user, size_t pit
     const PencilList lib{{h}, c->g.Ny}, usr{{u}, ups};
     return launch_cheby(out ? lib : usr, out ? usr : lib, 1, n, out ? 1 : 3, c->g.Ny, c->fy0_d.tab(), false, c->st);
   };
-  if (where == DNS_DEVICE) {
+  if (where == DNS_DEVICE && kernel_ptr(user)) {
     CK(convert(hist, user, (long long)(pitch / 16), H * c->g.nrun));
   } else {
     dns_status s = need_scratch(c);
@@ -710,9 +726,9 @@ static dns_status history_copy(dns_ctx* c, double2* hist, void* user, size_t pit
       char* u = (char*)user + (size_t)r * H * pitch;
       if (out) {
         CK(convert(h, c->scratch, c->g.Ny, H));
-        CK(cudaMemcpy2DAsync(u, pitch, c->scratch, w, w, (size_t)H, cudaMemcpyDeviceToHost, c->st));
+        CK(cudaMemcpy2DAsync(u, pitch, c->scratch, w, w, (size_t)H, kind_of(where, false), c->st));
       } else {
-        CK(cudaMemcpy2DAsync(c->scratch, w, u, pitch, w, (size_t)H, cudaMemcpyHostToDevice, c->st));
+        CK(cudaMemcpy2DAsync(c->scratch, w, u, pitch, w, (size_t)H, kind_of(where, true), c->st));
         CK(convert(h, c->scratch, c->g.Ny, H));
       }
     }
@@ -1274,13 +1290,13 @@ dns_status dns_solve_wall(dns_ctx* c, void* v, void* omega, size_t tpitch, int w
     CK(cudaGraphLaunch(c->solve_graph, c->st));
     return check_status(c);
   }
-  if (where == DNS_DEVICE) {  // one system: straight from and to the caller's pencils
+  if (where == DNS_DEVICE && kernel_ptr(v ? v : omega)) {  // one system: straight from and to the caller's pencils
     const cudaError_t e = enqueue_solve_wall(c, (const double2*)v, (const double2*)omega, (long long)(tpitch / 16),
                                              pbc, (double2*)v, (double2*)omega, (long long)(tpitch / 16));
     if (e == cudaSuccess) return check_status(c);
     if (e != cudaErrorNotSupported) CK(e);
   }
-  // host buffers, or one system only of a length without a plan: staged
+  // host buffers, or one system only that the line above leaves: staged
   // through Xv, Xo (pitch Ny); a missing system is prepared from a zero
   // right-hand side and not solved
   if (v) CK(cudaMemcpy2DAsync(Xv, row, v, tpitch, row, g.H, kind_of(where, true), c->st));

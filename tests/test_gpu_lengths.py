@@ -164,3 +164,30 @@ def test_solve_one_system(pkg, M):
         assert torch.equal(x, y)
         assert torch.equal(x[..., sz.nz:], z[..., sz.nz:])
     c.close()
+
+
+@pytest.mark.parametrize("mz", [128, 108])  # a wall-normal length with a plan, one without
+@pytest.mark.parametrize("offset", [0, 8])
+def test_history_on_device_pointers(pkg, mz, offset):
+    """The AB2 history to and from device pencils of a wider pitch, 16- and 8-byte
+    aligned, against the host form: the same kernel on the same values."""
+    c = pkg.Context(pkg.make_params(24, 24, mz, Re=1300.0, dt=0.001))
+    r = np.random.default_rng(3)
+    V, W = (r.standard_normal(c.shape) + 1j * r.standard_normal(c.shape) for _ in range(2))
+    c.set_history(V, W)
+    hv, ho = c.get_history()
+    H, Ny = int(np.prod(c.shape[:-1])), c.shape[-1]
+    row = 2 * Ny + 6  # doubles per pencil
+    buf = [torch.zeros(H * row + 1, dtype=torch.float64, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    ptr = [b.data_ptr() + offset for b in buf]
+    view = [b[offset // 8:offset // 8 + H * row].view(H, row)[:, :2 * Ny] for b in buf]
+    c._call("dns_get_history", ptr[0], ptr[1], row * 8, pkg.DEVICE)
+    for a, b in zip(view, (hv, ho)):
+        assert np.array_equal(a.cpu().numpy(), np.ascontiguousarray(b).view(np.float64).reshape(H, 2 * Ny))
+    c.set_history(W, V)
+    c._call("dns_set_history", ptr[0], ptr[1], row * 8, pkg.DEVICE)
+    c2 = pkg.Context(pkg.make_params(24, 24, mz, Re=1300.0, dt=0.001))
+    c2.set_history(hv, ho)
+    for a, b in zip(c.get_history(), c2.get_history()):
+        assert np.array_equal(a, b)
