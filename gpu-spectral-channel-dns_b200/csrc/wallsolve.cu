@@ -12,8 +12,8 @@
 // slots side by side), and are streamed through a shared-memory ring with
 // cp.async.bulk and mbarriers.  Each lane keeps its intermediate solution
 // and tilting term in one column of a global scratch of the group (rows
-// interleaved over the lanes, L2-resident, read two ring chunks ahead into
-// registers), so that a CTA needs only the ring and two small tables in
+// interleaved over the lanes, L2-resident, one ring chunk of rows in
+// registers ahead of the recurrence), so that a CTA needs only the ring and two small tables in
 // shared memory and several CTAs share an SM.
 //
 // Inputs from the y1 kernel: g_v, g_o (rows K.. of the integrated

@@ -193,23 +193,24 @@ dns_status dns_set_wait_limit(dns_ctx* ctx, long long cycles);
  * context starts with the first variant, in the order listed below, that it
  * can run (the tensor-core y3 only by choice or by the autotuner).
  *   DNS_PASS_Y3: the backward wall-normal pass (getUVW + padded s2p)
- *     DNS_Y3_FFT     warp-synchronous FFTs of the even extensions, two lines
- *                    per warp (lengths with a warp plan);
+ *     DNS_Y3_FFT     DCT-I by a pruned FFT of the even extension, two register
+ *                    butterflies per line (lengths 2^a 3^b with a plan);
  *     DNS_Y3_TENSOR  batched 3xTF32 Chebyshev products on the tensor cores
  *                    (tcgen05, FP32 accumulation): mixed form, Ny = 129;
  *     DNS_Y3_BLOCK   block-wide FFT (every grid).
  *   DNS_PASS_Y1: the forward wall-normal pass (p2s, nonlinear terms,
- *     right-hand sides): DNS_Y1_WARP (one warp per Lamb line, lengths with a
- *     warp plan) or DNS_Y1_BLOCK (every grid).
+ *     right-hand sides): DNS_Y1_WARP (the same DCT-I, right-hand sides by
+ *     integrated stencils, 128 threads per pencil) or DNS_Y1_BLOCK (every grid).
  *   DNS_PASS_ZB, DNS_PASS_ZF: the spanwise inverse / forward passes:
- *     DNS_Z_TENSOR_COPY  warp FFTs on tiles staged by tensor copies (mixed
- *                        form, Nz <= 256);
- *     DNS_Z_WARP         warp FFTs on tiles gathered through L1;
+ *     DNS_Z_TENSOR_COPY  two butterflies per line on tiles staged by tensor
+ *                        copies (mixed form, Nz <= 256);
+ *     DNS_Z_WARP         two butterflies per line, straight from and to global
+ *                        memory;
  *     DNS_Z_BLOCK        block-wide FFT (every grid).
- *   DNS_PASS_X: the streamwise pass (C2R, Lamb vector, R2C) on four rows
- *     per CTA: DNS_X_WARP3 (three warps, four lines each), DNS_X_WARP6 (six
- *     warps, two lines each) for lengths with warp plans, DNS_X_BLOCK (block
- *     FFT, every grid).
+ *   DNS_PASS_X: the streamwise pass (C2R, Lamb vector, R2C), two rows per
+ *     FFT line, two or three register butterflies per line: DNS_X_WARP3 (two
+ *     to eight rows per CTA by length), DNS_X_WARP6 (twice the rows and warps;
+ *     at 48, 96, 144, 192 and 384 points), DNS_X_BLOCK (block FFT, every grid).
  *   DNS_PASS_Y2: the banded wall-normal solves; the block shape of the
  *     factor stream (ring stages x bytes per stage, read with the L2
  *     evict-first policy): DNS_Y2_RING2_24K_EF, DNS_Y2_RING2_18K_EF,
@@ -278,7 +279,9 @@ dns_status dns_transform_3d_one_noalloc(dns_ctx* ctx, int dir, void* phys, size_
                                         size_t tpitch, int pad);
 /* transform (source/transform.cu:321-351): BACKWARD on six fields
  * (u, v, w, omega_x, omega_y, omega_z), FORWARD on three (lamb_z, lamb_y,
- * lamb_x order of the reference is immaterial). */
+ * lamb_x order of the reference is immaterial).  As many fields at a time as a
+ * row buffer of 64 MB holds (at least one) share each launch; the buffer is
+ * allocated on first use. */
 dns_status dns_transform(dns_ctx* ctx, int dir, int nfields, void* const* phys, size_t pitch,
                          void* const* spec, size_t tpitch);
 /* cuda_transpose (source/transpose.cu:115-166); xyz is complex. */
@@ -316,9 +319,10 @@ dns_status dns_solve_eq(dns_ctx* ctx, const void* inv, void* rhs, int N, size_t 
  * solves v before it forms the omega_y right-hand side).  where = DNS_HOST
  * or DNS_DEVICE.  Synchronous; allocates its vectors (2 H Ny + 6 H complex)
  * on first use.  On device pencils with both systems the whole sequence
- * (right-hand-side preparation, DCT-I, integration, the banded solve of all
- * pencils in one launch, the wall polynomial added back) is one CUDA graph,
- * captured on the first call with those buffers and launched on each. */
+ * (one kernel for the right-hand sides, their DCT-I and the integration, one
+ * for the banded solves, which adds the wall polynomial) is one CUDA graph,
+ * captured on the first call with those buffers and launched on each.  With
+ * one of the pointers NULL only the other system is prepared and solved. */
 dns_status dns_solve_wall(dns_ctx* ctx, void* v, void* omega, size_t tpitch, int where);
 /* No counterpart in the reference.  Residual of solved systems: b the
  * collocation right-hand sides as dns_solve_wall takes them, x the
