@@ -211,8 +211,9 @@ __global__ void __launch_bounds__(128) k_rhs_dct(double2* x, double2* xp, const 
 
 // the mean modes u0 (block 0) and w0 (block 1): rows 2..N of
 // (T0 + dt/(2 Re) T2) x - dt (1.5 lambda - 0.5 lambda_p) at r = i - 1;
-// rows 0, 1 (Dirichlet) zero
-__global__ void k_rhs_mean(double2* u0, const double2* lx, const double2* lxp, double2* w0,
+// rows 0, 1 (Dirichlet) zero.  Two pencils, each in place, so two blocks: a warp
+// a row at a time, as many warps as there are rows or fit (a row is one latency).
+__global__ void __launch_bounds__(1024) k_rhs_mean(double2* u0, const double2* lx, const double2* lxp, double2* w0,
                            const double2* lz, const double2* lzp, int Ny, const double* T0,
                            const double* T2, double Re, double dt) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -361,7 +362,7 @@ dns_status dns_rhs_mean(dns_ctx* c, void* u0, const void* lambx0, const void* la
     for (int i = 0; i < 6; ++i) q[i] = (double2*)src[i];
   }
   if (!e) {
-    k_rhs_mean<<<2, threads_for(Ny), vb, c->st>>>(q[0], q[1], q[2], q[3], q[4], q[5], Ny, c->T0, c->T2,
+    k_rhs_mean<<<2, std::min(1024, 32 * Ny), vb, c->st>>>(q[0], q[1], q[2], q[3], q[4], q[5], Ny, c->T0, c->T2,
                                                 c->ph.Re, c->ph.dt);
     e = cudaGetLastError();
   }
