@@ -163,17 +163,21 @@ __global__ void __launch_bounds__(256) k_nonfinite(const double2* __restrict__ a
 }
 
 // 1-3 fused: four lines (a system of a pencil each) per CTA of two warps.  A
-// warp forms the wall polynomial and the point values of two lines from the
-// right-hand sides in global memory, the DCT-I over the Gauss-Lobatto points is
+// warp forms the wall polynomial and the point values of two lines of one system
+// from the right-hand sides in global memory, the DCT-I over the Gauss-Lobatto points is
 // a pruned one (ydct.cuh, even extension of length L = 2 N), and the K-fold
 // integral its banded stencils.  A missing system has no lines.
 //
 // What bounds it: the whole FFT of each even extension (three passes of twice
 // the points) and four integration sweeps kept a call on shared memory; now a
-// value crosses it twice.  384 x 193 x 384: 555 -> 451 us, and the
-// 140 us of a last kernel that added the wall polynomial are gone.
+// value crosses it twice, and what is left is latency: 45 % of a warp's cycles
+// wait for L1, the tables among it, so two lines share each table value and
+// eight CTAs an SM (six with 32-point butterflies; six, seven, eight, ten at 384:
+// 451, 433, 423, 487 us before the sharing).  384 x 193 x 384: 555 -> 347 us,
+// and the 140 us of a last kernel that added the wall polynomial are gone.
 template <int L>
-__global__ void __launch_bounds__(64, 6) k_colloc_dct(const double2* __restrict__ bv, const double2* __restrict__ bo,
+__global__ void __launch_bounds__(64, DPlan<L>::A > 24 ? 6 : 8)
+                                         k_colloc_dct(const double2* __restrict__ bv, const double2* __restrict__ bo,
                                                       long long bp, double2* pbc, const double* __restrict__ Ut,
                                                       const double* __restrict__ ddUt, double2* gv, double2* go, int nv,
                                                       int no, long long gp, RhsTabs tb, DnsGeom g, PhysParams ph,
@@ -186,15 +190,16 @@ __global__ void __launch_bounds__(64, 6) k_colloc_dct(const double2* __restrict_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool both = bv && bo;
   const long long nlines = both ? 2 * g.H : g.H, l0 = (long long)blockIdx.x * 4;
-  // both lines' right-hand sides first, every load in flight: rows m + 2 (v)
-  // or m + 1 (omega and the mean modes) at point m
+  // a warp's lines: l0 + warp + 2 u, of one system, so that they share what is
+  // read from the tables.  Both right-hand sides first, every load in flight:
+  // rows m + 2 (v) or m + 1 (omega and the mean modes) at point m
   constexpr int KP = (Ny + 31) / 32;
+  const bool om = both ? (warp & 1) : !bv;
   double2 row[2][KP], wall[2][4];
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    const long long gl = min(l0 + 2 * warp + u, nlines - 1);
+    const long long gl = min(l0 + warp + 2 * u, nlines - (both ? 2 - warp : 1));
     const long long p = both ? gl >> 1 : gl;
-    const bool om = both ? (gl & 1) : !bv;
     const double2* b = (om ? bo : bv) + p * bp;
     const int off = om || p == 0 ? 1 : 2;
 #pragma unroll
@@ -205,61 +210,64 @@ __global__ void __launch_bounds__(64, 6) k_colloc_dct(const double2* __restrict_
   // the wavenumbers of both lines at once (lane u: line u): FP64 divisions
   double la, lb;
   {
-    const long long gl = min(l0 + 2 * warp + (lane & 1), nlines - 1);
+    const long long gl = min(l0 + warp + 2 * (lane & 1), nlines - 1);
     const long long p = both ? gl >> 1 : gl;
     wavenumbers((int)(p % g.Kx), (int)(p / g.Kx), g.Nz, ph.aphi, ph.beta, la, lb);
   }
   const double h = ph.dt * 0.5 / ph.Re;
+  double2 pc[2][4];
+  double k2[2], ah[2];
+  bool live[2], zero[2];
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     const double ia = __shfl_sync(0xffffffffu, la, u), ib = __shfl_sync(0xffffffffu, lb, u);
-    const long long gl = l0 + 2 * warp + u;
-    double2* f = F + (2 * warp + u) * VS;
-    if (gl >= nlines) {
-      for (int m = lane; m < Ny; m += 32) f[m] = cx(0, 0);
-      continue;
-    }
-    const long long p = both ? gl >> 1 : gl;
-    const bool om = both ? (gl & 1) : !bv, zero = p == 0;
+    const long long gl = l0 + warp + 2 * u, p = both ? gl >> 1 : gl;
+    live[u] = gl < nlines;
+    zero[u] = p == 0;
+    k2[u] = ia * ia + ib * ib;
+    ah[u] = ia * ph.dt * 0.5;
     // wall polynomial (rows 0..3 of the right-hand side)
     const double2 e = (wall[u][0] + wall[u][1]) * 0.5, o = (wall[u][0] - wall[u][1]) * 0.5;
-    double2 pc0 = e, pc1 = o, pc2 = cx(0, 0), pc3 = cx(0, 0);
-    if (!om && !zero) {
-      pc2 = (wall[u][2] - wall[u][3]) * 0.125;
-      pc3 = ((wall[u][2] + wall[u][3]) * 0.5 - o) * 0.125;
-      pc0 = e - pc2;
-      pc1 = o - pc3;
+    pc[u][0] = e;
+    pc[u][1] = o;
+    pc[u][2] = pc[u][3] = cx(0, 0);
+    if (!om && !zero[u]) {
+      pc[u][2] = (wall[u][2] - wall[u][3]) * 0.125;
+      pc[u][3] = ((wall[u][2] + wall[u][3]) * 0.5 - o) * 0.125;
+      pc[u][0] = e - pc[u][2];
+      pc[u][1] = o - pc[u][3];
     }
-    if (lane == 0) {
+    if (lane == 0 && live[u]) {
       double2* q = pbc + p * 6 + (om ? 4 : 0);
-      q[0] = pc0;
-      q[1] = pc1;
-      if (!om) { q[2] = pc2; q[3] = pc3; }
+      q[0] = pc[u][0];
+      q[1] = pc[u][1];
+      if (!om) { q[2] = pc[u][2]; q[3] = pc[u][3]; }
     }
-    const double kmn = ia * ia + ib * ib;
-    const double cv2 = 1 + 2.0 * kmn * h, co0 = 1 + kmn * h, cv0 = kmn * co0, ah = ia * ph.dt * 0.5;
-    // point value m of the interior right-hand side minus A p, zero where the
-    // equation has no row
+  }
+  // point value m of the interior right-hand side minus A p, zero where the
+  // equation has no row
 #pragma unroll
-    for (int i = 0; i < KP; ++i) {
-      const int m = lane + 32 * i;
-      if (m > N) break;
-      const double y = __ldg(tb.cosk + m);
+  for (int i = 0; i < KP; ++i) {
+    const int m = lane + 32 * i;
+    if (m > N) break;
+    const double y = __ldg(tb.cosk + m), U = __ldg(Ut + m), ddU = om ? 0.0 : __ldg(ddUt + m);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
       double2 v = cx(0, 0);
-      if (zero || om) {
+      if (om || zero[u]) {
         if (m >= 1 && m <= N - 1) {
-          const double2 P0 = pc0 + pc1 * y;
-          v = zero ? row[u][i] - P0 : row[u][i] - (P0 * co0 + muli(P0 * (ah * __ldg(Ut + m))));
+          const double2 P0 = pc[u][0] + pc[u][1] * y;
+          v = zero[u] ? row[u][i] - P0 : row[u][i] - (P0 * (1 + k2[u] * h) + muli(P0 * (ah[u] * U)));
         }
       } else if (m >= 2 && m <= N - 2) {
-        const double2 P0 = pc0 + pc1 * y + pc2 * (2 * y * y - 1) + pc3 * (y * (4 * y * y - 3));
-        const double2 P2 = pc2 * 4.0 + pc3 * (24.0 * y);
-        const double U = __ldg(Ut + m), ddU = __ldg(ddUt + m);
+        const double2 P0 = pc[u][0] + pc[u][1] * y + pc[u][2] * (2 * y * y - 1) + pc[u][3] * (y * (4 * y * y - 3));
+        const double2 P2 = pc[u][2] * 4.0 + pc[u][3] * (24.0 * y);
+        const double cv2 = 1 + 2.0 * k2[u] * h, cv0 = k2[u] * (1 + k2[u] * h);
         const double2 re = P2 * cv2 - P0 * cv0;
-        const double2 im = P2 * (ah * U) - P0 * (kmn * ah * U + ah * ddU);
+        const double2 im = P2 * (ah[u] * U) - P0 * (k2[u] * ah[u] * U + ah[u] * ddU);
         v = row[u][i] - (re + muli(im));
       }
-      f[m] = v;
+      F[(warp + 2 * u) * VS + m] = live[u] ? v : cx(0, 0);
     }
   }
   for (int i = threadIdx.x; i < 4 * 12; i += 64) F[i / 12 * VS + Ny + i % 12] = cx(0, 0);
@@ -271,25 +279,39 @@ __global__ void __launch_bounds__(64, 6) k_colloc_dct(const double2* __restrict_
     D::pass_b(X, dt, i, [&](int l, int k, double2 v) { F[l * VS + k] = v * (k && k < N ? 1.0 / N : 0.5 / N); });
   __syncthreads();
   // rows K .. K+n-1 of the K-fold integral (K = 4 for v, 2 otherwise)
-#pragma unroll 1
-  for (int u = 0; u < 2; ++u) {
-    const long long gl = l0 + 2 * warp + u;
-    if (gl >= nlines) return;
-    const long long p = both ? gl >> 1 : gl;
-    const bool om = both ? (gl & 1) : !bv, four = !om && p != 0;
-    const double2* f = F + (2 * warp + u) * VS;
-    double2* out = (om ? go : gv) + p * gp;
+  const double2 *f0 = F + warp * VS, *f1 = f0 + 2 * VS;
+  double2* out = (om ? go : gv) + (both ? l0 >> 1 : l0 + warp) * gp;
+  const long long step = (both ? 1 : 2) * gp;  // to the warp's second line
+  if (om) {
 #pragma unroll 2
     for (int r = lane; r < nv; r += 32) {  // (as many rows of omega)
-      double2 v = cx(0, 0);
-      if (four) {
+      double2 v0 = cx(0, 0), v1 = cx(0, 0);
 #pragma unroll
-        for (int d = 0; d < 5; ++d) v = v + f[r + 2 * d] * __ldg(tb.b4 + d * nv + r);
-      } else {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) v = v + f[r + 2 * d] * __ldg(tb.b2 + d * (nv + 2) + r);
+      for (int d = 0; d < 3; ++d) {
+        const double w = __ldg(tb.b2 + d * (nv + 2) + r);
+        v0 = v0 + f0[r + 2 * d] * w;
+        v1 = v1 + f1[r + 2 * d] * w;
       }
-      out[r] = v;
+      if (live[0]) out[r] = v0;
+      if (live[1]) out[step + r] = v1;
+    }
+  } else {
+#pragma unroll 2
+    for (int r = lane; r < nv; r += 32) {
+      double2 v0 = cx(0, 0), v1 = cx(0, 0);
+#pragma unroll
+      for (int d = 0; d < 5; ++d) {
+        const double w = __ldg(tb.b4 + d * nv + r);
+        v0 = v0 + f0[r + 2 * d] * w;
+        v1 = v1 + f1[r + 2 * d] * w;
+      }
+      if (zero[0]) {  // the mean modes: two-fold
+        v0 = cx(0, 0);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v0 = v0 + f0[r + 2 * d] * __ldg(tb.b2 + d * (nv + 2) + r);
+      }
+      if (live[0]) out[r] = v0;
+      if (live[1]) out[step + r] = v1;
     }
   }
 }
