@@ -67,6 +67,23 @@ template <typename C> int ztw_table(int L, const double2* W, std::vector<C>& out
   return (int)out.size();
 }
 
+// The tensor-staged FP32 form (k_zbt, k_zft): a warp's pair of lines.  Element
+// pos of line l sits at 2 (pos + pos / RA) + l, a pair is WS elements; before
+// that the values, [n][line], lie from the pair's first 128-byte boundary on.
+// Tiled copies need destinations on 128-byte boundaries and boxes of at most 256
+// rows: a line up to 256 points comes in one copy, a longer one in two halves
+// where the second starts on such a boundary (L a multiple of 16).
+template <typename C, int L> struct ZStage {
+  static constexpr int RA = ZPlan<L>::A, RB = ZPlan<L>::B;
+  static constexpr int raw = 2 * RB * (RA + 1);
+  static constexpr int WS = raw + (18 - raw % 16) % 16;  // 2 mod 16
+  static constexpr bool ok = ZPlan<L>::ok && RB <= 16 && sizeof(C) == 8;
+  static constexpr bool fits(int n) { return n * 16 + 128 <= WS * 8; }
+  static constexpr int ROWS = L <= 256 ? L : L / 2;  // of a forward copy
+  static constexpr bool copies_ok = ROWS <= 256 && L % ROWS == 0 && (ROWS == L || ROWS * 2 * sizeof(C) % 128 == 0);
+};
+
+#ifdef __CUDACC__
 // butterfly (line li, j) of pass A after its inputs: the RA-point transform,
 // outputs to positions j RA + r
 template <typename C, int RA, int NL, bool INV>
@@ -178,3 +195,4 @@ __global__ void __launch_bounds__(NT, MB) k_zf2(RowArr in, PA out, DnsGeom g, co
     }
   }
 }
+#endif

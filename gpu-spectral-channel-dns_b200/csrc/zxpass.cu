@@ -134,15 +134,7 @@ __global__ void __launch_bounds__(256, 3) k_zf(RowArr in, PencilArr out, DnsGeom
 // those of pass B, which take the 16 lines of a position (pairs WS apart), fall
 // in distinct banks.  384 x 384 x 512, inverse / forward: 195 / 115 us, against
 // 230 / 124 with both passes by the warp and the tile's rows or pencils written
-// from shared memory in a third.
-template <typename C, int L> struct ZStage {
-  static constexpr int RA = ZPlan<L>::A, RB = ZPlan<L>::B;
-  static constexpr int raw = 2 * RB * (RA + 1);
-  static constexpr int WS = raw + (18 - raw % 16) % 16;  // 2 mod 16
-  static constexpr bool ok = ZPlan<L>::ok && RB <= 16 && sizeof(C) == 8;
-  // the staged values (n per line) from the first 128-byte boundary on
-  static constexpr bool fits(int n) { return n * 16 + 128 <= WS * 8; }
-};
+// from shared memory in a third.  The tile: ZStage (zpass.cuh).
 namespace {
 template <typename C, int L, bool INV, class LD>
 __device__ __forceinline__ void zstage_a(C* wl, int lane, LD ld) {
@@ -231,12 +223,14 @@ __global__ void __launch_bounds__(256, 3) k_zbt(const __grid_constant__ CUtensor
 }
 
 // Forward pass, 4 x 4 tile (32-byte runs on the pencil side): warp w owns y0 +
-// w / 2 and a kx pair, two copies (box kx 2 x zp Pz/2 x y 1 x field 1).  Rows
-// beyond Py and columns beyond Kx read as the copy's zero fill.
+// w / 2 and a kx pair, one copy of the whole line up to 256 points, two of its
+// halves beyond (box kx 2 x zp ROWS x y 1 x field 1).  Rows beyond Py and columns
+// beyond Kx read as the copy's zero fill.
 template <typename C, int L>
 __global__ void __launch_bounds__(256, 3) k_zft(const __grid_constant__ CUtensorMap tin, PencilArr out,
                                                 DnsGeom g, const C* __restrict__ tw, int* status) {
   typedef ZStage<C, L> Z;
+  static_assert(Z::copies_ok, "a copy's destination is 128-byte aligned");
   constexpr int Nz = L / 3 * 2, hz = Nz / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint64_t bars[8];
@@ -251,8 +245,8 @@ __global__ void __launch_bounds__(256, 3) k_zft(const __grid_constant__ CUtensor
     fence_mbar_init();
     mbar_expect_tx(bars + warp, (uint32_t)(2 * L * sizeof(C)));
     const int x = kx0 + 2 * (warp & 1), y = y0 + (warp >> 1);
-    tma_load_4d(tile, &tin, x, 0, y, f, bars + warp);
-    tma_load_4d(tile + L, &tin, x, L / 2, y, f, bars + warp);
+#pragma unroll
+    for (int z = 0; z < L; z += Z::ROWS) tma_load_4d(tile + 2 * z, &tin, x, z, y, f, bars + warp);
   }
   __syncwarp();
   zstage_wait(bars + warp, lane, status);
@@ -529,16 +523,15 @@ bool pencil_tmap(const PencilArr& in, int nf, const DnsGeom& g, size_t esz, CUte
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// 4-D map (kx, zp, y, field) over 8-byte row elements, box 2 x Pz/2 x 1 x 1
-bool row_tmap(const RowArr& in, int nf, const DnsGeom& g, size_t esz, CUtensorMap* m) {
+// 4-D map (kx, zp, y, field) over 8-byte row elements, box 2 x rows x 1 x 1
+bool row_tmap(const RowArr& in, int nf, const DnsGeom& g, size_t esz, int rows, CUtensorMap* m) {
   PFN_cuTensorMapEncodeTiled_v12000 enc = tmap_encoder();
-  if (!enc || esz != 8 || !aligned16(in.base) || (in.rs * esz) % 16 || (in.fs * esz) % 16 || g.Pz % 2 ||
-      g.Pz / 2 > 256)
+  if (!enc || esz != 8 || !aligned16(in.base) || (in.rs * esz) % 16 || (in.fs * esz) % 16 || g.Pz % rows || rows > 256)
     return false;
   const cuuint64_t dims[4] = {(cuuint64_t)g.Kx, (cuuint64_t)g.Pz, (cuuint64_t)g.Py, (cuuint64_t)nf};
   const cuuint64_t strides[3] = {(cuuint64_t)(in.rs * esz), (cuuint64_t)((long long)g.Pz * in.rs * esz),
                                  (cuuint64_t)(in.fs * esz)};
-  const cuuint32_t box[4] = {2, (cuuint32_t)(g.Pz / 2), 1, 1};
+  const cuuint32_t box[4] = {2, (cuuint32_t)rows, 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, in.base, dims, strides, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -647,9 +640,9 @@ cudaError_t launch_zf(RowArr in, PencilArr out, int nf, DnsGeom g, FftTab<C> tab
       const cudaError_t e = with_len_z(g.Pz, [&](auto LL) -> cudaError_t {
         constexpr int L = decltype(LL)::value;
         typedef ZStage<C, L> Z;
-        if constexpr (Z::ok && Z::fits(L)) {
+        if constexpr (Z::ok && Z::fits(L) && Z::copies_ok) {
           CUtensorMap tm;
-          if (status && g.Nz == L / 3 * 2 && tab.zt && row_tmap(in, nf, g, sizeof(C), &tm)) {
+          if (status && g.Nz == L / 3 * 2 && tab.zt && row_tmap(in, nf, g, sizeof(C), Z::ROWS, &tm)) {
             if (probe) return cudaSuccess;
             const size_t sm = (size_t)8 * Z::WS * sizeof(C);
             cudaFuncSetAttribute(k_zft<C, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
