@@ -2,6 +2,59 @@
 #pragma once
 #include "kernels.cuh"
 
+// Sums over the 16 lanes of a parity of NV values a lane, the values halved
+// between a lane and its partner at every step (masks 16, 8, 4, 2; 11 exchanges
+// for ten values instead of 40).  Where an odd count is halved the upper lane
+// gets one fewer, so that some lanes end with none.
+template <int NV> struct ParitySums {
+  enum { HALF = (NV + 1) / 2 };
+  // a step on n values, the first (n + 1) / 2 to the lower lane: v keeps the
+  // lane's own, send goes to the partner
+  DNS_HD static void split(double (&v)[NV], double (&send)[HALF], int n, bool up) {
+    const int half = (n + 1) / 2;
+#pragma unroll
+    for (int i = 0; i < HALF; ++i) {
+      if (i >= half) continue;
+      const double hi = i + half < n ? v[i + half] : 0.0;
+      send[i] = up ? v[i] : hi;
+      v[i] = up ? hi : v[i];
+    }
+  }
+  // the value whose sum the lane ends with, NV: none
+  DNS_HD static int slot(int lane) {
+    int idx = 0, cnt = NV;  // this lane's values idx .. idx + cnt - 1
+#pragma unroll
+    for (int m = 16, n = NV; m > 1; m >>= 1) {
+      const int half = (n + 1) / 2;
+      if (lane & m) {
+        idx += half;
+        cnt -= half;
+      } else if (cnt > half) {
+        cnt = half;
+      }
+      n = half;
+    }
+    return cnt > 0 ? idx : (int)NV;
+  }
+#ifdef __CUDACC__
+  __device__ __forceinline__ static double run(double (&v)[NV], int lane) {
+    int n = NV;
+#pragma unroll
+    for (int m = 16; m > 1; m >>= 1) {
+      double send[HALF];
+      split(v, send, n, lane & m);
+      n = (n + 1) / 2;
+#pragma unroll
+      for (int i = 0; i < HALF; ++i)
+        if (i < n) v[i] += __shfl_xor_sync(0xffffffffu, send[i], m);
+    }
+    return v[0];
+  }
+#endif
+};
+
+#ifdef __CUDACC__
+
 // run length of a lane for Ny coefficients (even: the parity of each of its
 // elements is known at compile time)
 __host__ __device__ constexpr int ddz_run(int Ny) { return 2 * ((Ny + 63) / 64); }
@@ -80,3 +133,4 @@ __device__ __noinline__ void d2z_fast(const double2* __restrict__ a, double2* __
     }
   }
 }
+#endif

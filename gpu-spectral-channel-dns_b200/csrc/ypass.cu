@@ -825,31 +825,6 @@ __global__ void __launch_bounds__(256, 3) k_y1(PencilArr lam, const double2* __r
 // step.  4530 instructions; 256 x 129 x 256 mixed 383 -> 278 us, FP64 497 ->
 // 432; 128 x 65 x 128 FP64 107 -> 63; twelve 64 x 49 x 64 mixed 184 -> 114;
 // 144 x 55 x 72 mixed, a length on the block form before, 160 -> 33.
-namespace {
-// Sums over the 16 lanes of a parity of NV values a lane, halved at every
-// step: afterwards the lane holds the sum of value `idx` (idx >= NV: none).
-template <int NV>
-__device__ __forceinline__ double parity_sums(double (&v)[NV], int lane, int& idx) {
-  int n = NV;
-  idx = 0;
-#pragma unroll
-  for (int m = 16; m > 1; m >>= 1) {
-    const int half = (n + 1) / 2;
-    const bool up = lane & m;
-#pragma unroll
-    for (int i = 0; i < (NV + 1) / 2; ++i) {
-      if (i >= half) continue;
-      const double hi = i + half < n ? v[i + half] : 0.0;
-      const double send = up ? v[i] : hi, keep = up ? hi : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
-    }
-    if (up) idx += half;
-    n = half;
-  }
-  return v[0];
-}
-}  // namespace
-
 template <typename C, int M, int MB>
 __global__ void __launch_bounds__(128, MB) k_y1d(PencilArr lam, const double2* __restrict__ V,
                                             const double2* __restrict__ O, double2* Nvp,
@@ -975,8 +950,8 @@ __global__ void __launch_bounds__(128, MB) k_y1d(PencilArr lam, const double2* _
         acc[9] += o.y * w;
       }
     }
-    int idx;
-    const double sum = parity_sums(acc, lane, idx);
+    const double sum = ParitySums<10>::run(acc, lane);
+    const int idx = ParitySums<10>::slot(lane);
     if (idx < 10) accA[((warp - 2) * 2 + (lane & 1)) * 10 + idx] = sum;
   }
   __syncthreads();
@@ -1013,8 +988,8 @@ __global__ void __launch_bounds__(128, MB) k_y1d(PencilArr lam, const double2* _
   }
   if (boot) return;
   {
-    int idx;
-    const double sum = parity_sums(acc, lane, idx);
+    const double sum = ParitySums<6>::run(acc, lane);
+    const int idx = ParitySums<6>::slot(lane);
     if (idx < 6) accB[(warp * 2 + (lane & 1)) * 6 + idx] = sum;
   }
   __syncthreads();
