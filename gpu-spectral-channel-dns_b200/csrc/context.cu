@@ -377,15 +377,15 @@ dns_status need_scratch(dns_ctx* c) {
   return DNS_OK;
 }
 
-// device or managed memory, aligned for complex loads: a pointer that a kernel
-// can take where copies would take, or refuse, any
-bool kernel_ptr(const void* p) {
+// a pointer that a kernel of this context can take where copies would take, or
+// refuse, any
+bool kernel_ptr(const dns_ctx* c, const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return aligned16(p) && (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged);
+  return kernel_memory(p, a, c->P.device);
 }
 cudaMemcpyKind kind_of(int where, bool to_device) {
   if (where == DNS_DEVICE) return cudaMemcpyDeviceToDevice;
@@ -716,7 +716,7 @@ static dns_status history_copy(dns_ctx* c, double2* hist, void* user, size_t pit
     const PencilList lib{{h}, c->g.Ny}, usr{{u}, ups};
     return launch_cheby(out ? lib : usr, out ? usr : lib, 1, n, out ? 1 : 3, c->g.Ny, c->fy0_d.tab(), false, c->st);
   };
-  if (where == DNS_DEVICE && kernel_ptr(user)) {
+  if (where == DNS_DEVICE && kernel_ptr(c, user)) {
     CK(convert(hist, user, (long long)(pitch / 16), H * c->g.nrun));
   } else {
     dns_status s = need_scratch(c);
@@ -1290,7 +1290,8 @@ dns_status dns_solve_wall(dns_ctx* c, void* v, void* omega, size_t tpitch, int w
     CK(cudaGraphLaunch(c->solve_graph, c->st));
     return check_status(c);
   }
-  if (where == DNS_DEVICE && kernel_ptr(v ? v : omega)) {  // one system: straight from and to the caller's pencils
+  const bool direct = where == DNS_DEVICE && kernel_ptr(c, v ? v : omega);
+  if (direct) {  // one system: straight from and to the caller's pencils
     const cudaError_t e = enqueue_solve_wall(c, (const double2*)v, (const double2*)omega, (long long)(tpitch / 16),
                                              pbc, (double2*)v, (double2*)omega, (long long)(tpitch / 16));
     if (e == cudaSuccess) return check_status(c);
@@ -1303,13 +1304,13 @@ dns_status dns_solve_wall(dns_ctx* c, void* v, void* omega, size_t tpitch, int w
   else CK(cudaMemsetAsync(Xv, 0, hn * 16, c->st));
   if (omega) CK(cudaMemcpy2DAsync(Xo, row, omega, tpitch, row, g.H, kind_of(where, true), c->st));
   else CK(cudaMemsetAsync(Xo, 0, hn * 16, c->st));
-  if (where == DNS_HOST) {
-    CK(enqueue_solve_wall(c, Xv, Xo, g.Ny, pbc, Xv, Xo, g.Ny));
-    if (v) CK(cudaMemcpy2DAsync(v, tpitch, Xv, row, row, g.H, cudaMemcpyDeviceToHost, c->st));
-    if (omega) CK(cudaMemcpy2DAsync(omega, tpitch, Xo, row, row, g.H, cudaMemcpyDeviceToHost, c->st));
+  const int sys = (v ? 1 : 0) | (omega ? 2 : 0);
+  if (direct) {
+    CK(enqueue_solve_wall(c, Xv, Xo, g.Ny, pbc, (double2*)v, (double2*)omega, (long long)(tpitch / 16), sys));
   } else {
-    CK(enqueue_solve_wall(c, Xv, Xo, g.Ny, pbc, (double2*)v, (double2*)omega, (long long)(tpitch / 16),
-                          (v ? 1 : 0) | (omega ? 2 : 0)));
+    CK(enqueue_solve_wall(c, Xv, Xo, g.Ny, pbc, Xv, Xo, g.Ny, sys));
+    if (v) CK(cudaMemcpy2DAsync(v, tpitch, Xv, row, row, g.H, kind_of(where, false), c->st));
+    if (omega) CK(cudaMemcpy2DAsync(omega, tpitch, Xo, row, row, g.H, kind_of(where, false), c->st));
   }
   return check_status(c);
 }

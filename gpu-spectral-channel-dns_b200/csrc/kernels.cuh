@@ -72,5 +72,11 @@ DNS_HD double run_dt(const PhysParams& ph, int r) { return ph.runs ? ph.runs[3 *
 
 // 16-byte alignment of a device pointer (bulk-copy sources)
 inline bool aligned16(const void* p) { return ((unsigned long long)p & 15ull) == 0; }
+// whether a kernel on device dev can take p for complex loads, a the runtime's
+// attributes of p: dev's own or managed memory.  Another device's memory is for
+// copies only (without peer access a kernel faults on it), as is the host's.
+inline bool kernel_memory(const void* p, const cudaPointerAttributes& a, int dev) {
+  return aligned16(p) && ((a.type == cudaMemoryTypeDevice && a.device == dev) || a.type == cudaMemoryTypeManaged);
+}
 
 #define DNS_CHECK_LAUNCH() do { cudaError_t e__ = cudaGetLastError(); if (e__ != cudaSuccess) return e__; } while (0)
