@@ -58,6 +58,14 @@ DPLAN(768, 32, 24)
 // lengths of the no-padding transforms only
 #define DPLAN_SHORT(X) X(16) X(24)
 
+// Elements of the derivatives in getUVW.  The mixed form rounds the state to
+// FP32 first at the lengths below, where it always did; at the others the sweeps
+// are FP64, as in the block form, and only the six fields are rounded.
+template <typename C, int M> struct Y3Form {
+  static constexpr bool fp32 = sizeof(C) == 8 && (M == 128 || M == 192 || M == 256 || M == 384 || M == 512 || M == 768);
+  typedef typename std::conditional<fp32, float2, double2>::type E;
+};
+
 // pass-B twiddles W_M^{j s}, j = 1..RB/2, s = 0..RA/2, stored [j - 1][s]; W:
 // the table W_M^j, j < M
 template <typename C> int dtw_table(int M, const double2* W, std::vector<C>& out) {

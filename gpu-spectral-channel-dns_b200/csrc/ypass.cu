@@ -429,7 +429,8 @@ __global__ void __launch_bounds__(256, 3) k_y3(const double2* __restrict__ V, co
 // each of 512 values of a line five times through shared memory and spent its
 // issue slots on the redundant half; the two pruned passes move 0.56 of them
 // once.  FP64 256 x 129 x 256 440 -> 301 us, 128 x 65 x 128 65 -> 50; mixed
-// 144 x 55 x 72, a length on the block form before, 126 -> 19.
+// 144 x 55 x 72, a length on the block form before, 126 -> 21 (19 with the
+// derivatives in FP32, which that length never had).
 template <typename C, int M, int MB>
 __global__ void __launch_bounds__(64, MB) k_y3d(const double2* __restrict__ V, const double2* __restrict__ O,
                                                PencilArr out, DnsGeom g, PhysParams ph, const C* __restrict__ dt,
@@ -437,8 +438,7 @@ __global__ void __launch_bounds__(64, MB) k_y3d(const double2* __restrict__ V, c
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typedef Dct<C, M, 6> D;
   constexpr int Ny = M / 4 + 1, Py = M / 2 + 1;  // the launcher checks g.Ny, g.Py against M
-  // derivatives in double2, or float2 where they feed FP32 transforms only
-  typedef typename std::conditional<sizeof(C) == 8, float2, double2>::type E;
+  typedef typename Y3Form<C, M>::E E;  // of the derivatives
   typedef T_of<E> S;
   constexpr int FS = (Ny + 1) & ~1;  // field stride
   C* fld = (C*)smem_raw;             // six fields
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(64, MB) k_y3d(const double2* __restrict__ V, c
   // derivatives from D^2 w, D oz (source/velocity.cu:90-170).  The mean
   // mode holds u0, w0 in (w, oz): u = w, v = oz, omega_x = D oz, omega_y = -D w.
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if constexpr (sizeof(C) == 8) {
+  if constexpr (sizeof(E) == 8) {
     // to FP32 in place: element n of the FP32 copy lies below element n of
     // the FP64 vector, so the conversion runs in one pass per warp
     const double2* src = warp ? oz : w;
@@ -1156,7 +1156,7 @@ cudaError_t launch_y3(const double2* V, const double2* O, PencilArr out, DnsGeom
       typedef Dct<C, M, 6> D;
       if (probe) return cudaSuccess;
       constexpr int FS = (M / 4 + 2) & ~1;
-      constexpr size_t es = sizeof(C) == 8 ? 8 : 16, vec = (size_t)FS * (2 * 16 + 3 * es), ex = D::XN * sizeof(C);
+      constexpr size_t es = sizeof(typename Y3Form<C, M>::E), vec = (size_t)FS * (2 * 16 + 3 * es), ex = D::XN * sizeof(C);
       const size_t sm = (size_t)6 * FS * sizeof(C) + (vec > ex ? vec : ex);
       constexpr int MB = sizeof(C) == 8 ? (D::RA > 18 ? 8 : 12) : (D::RA > 24 ? 4 : (D::RA > 18 ? 6 : 8));
       auto k = k_y3d<C, M, MB>;
