@@ -71,14 +71,12 @@ template <typename C> cudaError_t make_fft(int L, DevFft<C>& f) {
     dr[j] = (short)fft_digitrev(f.plan, j);
   }
   const size_t otw = put(tw.data(), sizeof(C) * L), odr = put(dr.data(), sizeof(short) * L);
-  // twiddle tables where the length has a plan: FP32 the fused streamwise form, both precisions the two-pass
-  // spanwise form and the pruned DCT
-  const bool f32 = std::is_same<C, float2>::value;
+  // twiddle tables where the length has a plan: the fused streamwise form, the two-pass spanwise form and the
+  // pruned DCT
   const size_t none = ~(size_t)0;
   size_t off[3] = {none, none, none};
   std::vector<C> t;
   for (int i = 0; i < 3; ++i) {
-    if (i < 1 && !f32) continue;
     const int n = i == 0 ? xtw_table<C>(L, W.data(), t)
                 : i == 1 ? ztw_table<C>(L, W.data(), t) : dtw_table<C>(L, W.data(), t);
     if (n > 0) off[i] = put(t.data(), sizeof(C) * n);

@@ -21,7 +21,7 @@ template <typename C> struct FftTab {
   const C* tw;          // W_L^j, j < L
   const short* drev;    // digit-reversed position of natural index n
   const C* dt;          // twiddles of the pruned DCT (ydct.cuh), null for lengths without one
-  const C* xt;          // FP32 twiddles of the fused streamwise form (xpass.cuh)
+  const C* xt;          // twiddles of the fused streamwise form (xpass.cuh), null for lengths without one
   const C* zt;          // twiddles of the two-pass spanwise form (zpass.cuh), null for lengths without one
 };
 

@@ -22,8 +22,10 @@
 // 125 -> 82; 128 x 128 x 128 FP64, a length without a plan before, 96 -> 25.
 #pragma once
 #include "kernels.cuh"
-#include "mbar.cuh"
 #include "wfft.cuh"
+#ifdef __CUDACC__
+#include "mbar.cuh"
+#endif
 
 // RF and the other radices (inverse: PRE..., RF; forward: RF, PRE...), rows
 // per CTA and warps.  A row pair's 2 L/RF butterflies fit the CTA's threads;
@@ -90,8 +92,11 @@ XPLAN(768, 8, 8, 4, 6, 12, 8)
   X(24) X(32) X(36) X(48) X(54) X(64) X(72) X(96) X(108) X(128) X(144) X(162) X(192) X(216) X(256) X(288) \
   X(324) X(384) X(432) X(512) X(576) X(768)
 
-// FP32 twiddles: the inverse plan's passes, then the forward plan's (FP64
-// passes take W_L^j and products); W: the table W_L^j, j < L
+// Twiddles: the inverse plan's passes, then the forward plan's, every value
+// rounded from W, the table W_L^j, j < L.  FP64 products w, w^2, w^3, ... would
+// save loads, but their error grows with the radix: rms error of a forward line
+// (1e-16) 4.6 by products and 1.8 from the table at 192, 5.1 and 2.0 at 216, 3.0
+// and 1.9 at 384; 384 x 384 x 512 634 -> 646 us, 192 x 192 x 256 84 -> 87.
 template <typename C, int... Rs> void xtw_fill(Radices<Rs...>, int L, const double2* W, C* out) {
   const int rs[] = {Rs...};
   int ns = 1;
@@ -140,14 +145,8 @@ template <typename C, int L, int R, int Ns, int TWO, bool INV> struct XPass {
   // the twiddles w[1..R-1] of butterfly j
   DNS_HD static void weights(const C* tw, int j, C* w) {
     const int k = j % Ns;
-    if constexpr (FftMaxRadix<C>::v == 8) {
-      w[1] = tw[k * (L / (Ns * R))];
 #pragma unroll
-      for (int r = 2; r < R; ++r) w[r] = cmul(w[r - 1], w[1]);
-    } else {
-#pragma unroll
-      for (int r = 1; r < R; ++r) w[r] = tw[TWO + (r - 1) * Ns + k];
-    }
+    for (int r = 1; r < R; ++r) w[r] = tw[TWO + (r - 1) * Ns + k];
   }
   DNS_HD static void run(C* v, const C* w) {
     if constexpr (Ns > 1) {
@@ -374,7 +373,7 @@ __global__ void __launch_bounds__(32 * SC * XPlan<L, FftMaxRadix<C>::v>::NW, MB)
 #pragma unroll 1
     for (int b = 0; b < FPW; b += NLF) {
       auto atb = [&](int l) { return at(b + l); };
-      const C* twf = FftMaxRadix<C>::v == 8 ? tw : tw + wtw_size(typename P::INV());
+      const C* twf = tw + wtw_size(typename P::INV());
       XDo<C, L, NLF, false, RF, 0, false, 0, typename P::PRE>::go(
           twf, lane, atb, 0, [](int kk) { return kk <= hx || kk >= L - hx; });
     }

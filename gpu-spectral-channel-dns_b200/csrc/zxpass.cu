@@ -688,7 +688,7 @@ cudaError_t launch_x2(RowArr in, RowArr out, DnsGeom g, FftTab<C> tab, const dou
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   const long long nrows = (long long)g.Py * g.Pz * g.nrun;
   k<<<(unsigned)((nrows + NR - 1) / NR), 32 * SC * P::NW, sm, st>>>(
-      in, out, g, FftMaxRadix<C>::v == 8 ? tab.tw : tab.xt, Uy, Ro, runs, status);
+      in, out, g, tab.xt, Uy, Ro, runs, status);
   return cudaGetLastError();
 }
 #define DNS_XCASE(n) case n: return f(std::integral_constant<int, n>());
@@ -707,7 +707,7 @@ cudaError_t launch_x_fused(RowArr in, RowArr out, DnsGeom g, FftTab<C> tab, cons
   const int sr = (g.Nx / 2 + 7) / 8 * 8;
   const bool ok = g.Pz % 2 == 0 && g.Nx / 2 == g.Px / 3 && in.rs >= sr && (in.rs * sizeof(C)) % 16 == 0 &&
                   (in.fs * sizeof(C)) % 16 == 0 && aligned16(in.base) && status && nrows < (1LL << 31) &&
-                  (sizeof(C) == 16 || tab.xt);
+                  tab.xt;
   if (ok && (any || variant == DNS_X_WARP3 || variant == DNS_X_WARP6)) {
     const cudaError_t e = with_len_x(g.Px, [&](auto LL) -> cudaError_t {
       constexpr int L = decltype(LL)::value;
