@@ -1014,7 +1014,7 @@ static dns_status check_phys_pitch(dns_ctx* c, size_t pitch) {
   return DNS_OK;
 }
 
-// nf fields, as many a launch as the scratch holds
+// nf fields, as many a launch as the scratch holds; one by one where they share memory
 static dns_status transform_fields(dns_ctx* c, int dir, int nf, void* const* phys, size_t pitch, void* const* spec,
                                    size_t tpitch, int pad) {
   if ((dir != DNS_FORWARD && dir != DNS_BACKWARD) || (pad != DNS_PADDING && pad != DNS_NO_PADDING))
@@ -1030,8 +1030,14 @@ static dns_status transform_fields(dns_ctx* c, int dir, int nf, void* const* phy
   const RowArr sr{c->scratch, c->RS, nrows * c->RS};
   const FftTab<double2> ty = pad == DNS_PADDING ? c->fyP_d.tab() : c->fy0_d.tab();
   const int mode = (dir == DNS_BACKWARD ? 0 : 2) + (pad == DNS_PADDING ? 0 : 1);
-  for (int f = 0; f < nf; f += c->scratch_fields) {
-    const int n = std::min(nf - f, c->scratch_fields);
+  PitchedBytes pb[6], sb[6];
+  for (int i = 0; i < nf; ++i) {
+    pb[i] = PitchedBytes{phys[i], nrows, (long long)g.Px * 8, (long long)pitch};
+    sb[i] = PitchedBytes{spec[i], g.H, (long long)c->P.mz * 16, (long long)tpitch};
+  }
+  const int share = fields_apart(dir == DNS_FORWARD, nf, pb, sb) ? c->scratch_fields : 1;
+  for (int f = 0; f < nf; f += share) {
+    const int n = std::min(nf - f, share);
     PencilList sp{{}, (long long)(tpitch / 16)};
     FieldList ph{};
     for (int i = 0; i < n; ++i) {

@@ -78,5 +78,30 @@ inline bool aligned16(const void* p) { return ((unsigned long long)p & 15ull) ==
 inline bool kernel_memory(const void* p, const cudaPointerAttributes& a, int dev) {
   return aligned16(p) && ((a.type == cudaMemoryTypeDevice && a.device == dev) || a.type == cudaMemoryTypeManaged);
 }
+// n rows of w bytes, pitch bytes apart
+struct PitchedBytes {
+  const void* p;
+  long long n, w, pitch;
+  const char* end() const { return (const char*)p + (n - 1) * pitch + w; }
+};
+// whether two of them share a byte (those of one pitch may interleave their rows)
+inline bool rows_overlap(const PitchedBytes& a, const PitchedBytes& b) {
+  if ((const char*)a.p >= b.end() || (const char*)b.p >= a.end()) return false;
+  if (a.pitch != b.pitch) return true;
+  const long long d = ((const char*)b.p - (const char*)a.p) % a.pitch, r = d < 0 ? d + a.pitch : d;
+  return r < a.w || a.pitch - r < b.w;
+}
+// whether the fields of one transform call can share launches: no field's output
+// lies in another's input or output.  Fields that do go one by one, in order.
+inline bool fields_apart(bool forward, int nf, const PitchedBytes* phys, const PitchedBytes* spec) {
+  for (int i = 0; i < nf; ++i)
+    for (int j = 0; j < nf; ++j) {
+      if (i == j) continue;
+      // (the pencils are overwritten in both directions)
+      if (rows_overlap(spec[i], phys[j]) || (i < j && rows_overlap(spec[i], spec[j]))) return false;
+      if (!forward && i < j && rows_overlap(phys[i], phys[j])) return false;
+    }
+  return true;
+}
 
 #define DNS_CHECK_LAUNCH() do { cudaError_t e__ = cudaGetLastError(); if (e__ != cudaSuccess) return e__; } while (0)
