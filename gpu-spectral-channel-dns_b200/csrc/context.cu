@@ -358,20 +358,22 @@ int zvar64(const dns_ctx* c, int pass) {
   return c->P.precision == DNS_PREC_FP64 ? c->variant[pass] : VAR_AUTO;
 }
 
-// streamwise rows of the reference-layout transforms: one field, or as many
-// (up to the six of a getUVW) as 64 MB hold, so that small fields share launches
-dns_status need_scratch(dns_ctx* c) {
-  if (c->scratch) return DNS_OK;
+// streamwise rows of the reference-layout transforms, allocated when a call first
+// needs them and kept: one field's for a call of one field, for a call of several
+// as many fields' (up to the six of a getUVW) as 64 MB hold, so that small fields
+// share launches.  fields: how many *rows hold.
+dns_status need_rows(dns_ctx* c, int nf, double2** rows, int* fields) {
   const size_t one = (size_t)c->g.Py * c->g.Pz * c->RS;
-  int n = (int)std::max<size_t>(1, std::min<size_t>(6, ((size_t)64 << 20) / (one * 16)));
-  if (n > 1 && c->alloc(&c->scratch, one * n)) {  // a device that is nearly full: one field
-    cudaGetLastError();
+  const int n = (int)std::max<size_t>(1, std::min<size_t>(6, ((size_t)64 << 20) / (one * 16)));
+  if (nf > 1 && n > 1 && !c->rows_n && !c->rows_tight && c->alloc(&c->rows_n, one * n)) {
+    cudaGetLastError();  // a device that is nearly full: one field at a time, from now on
     c->bytes -= one * n * 16;
-    c->scratch = nullptr;
-    n = 1;
+    c->rows_n = nullptr;
+    c->rows_tight = true;
   }
-  if (!c->scratch) CK(c->alloc(&c->scratch, one));
-  c->scratch_fields = n;
+  if (!c->rows_n && !c->rows_1) CK(c->alloc(&c->rows_1, one));
+  *rows = c->rows_n ? c->rows_n : c->rows_1;
+  *fields = c->rows_n ? n : 1;
   return DNS_OK;
 }
 
@@ -622,7 +624,7 @@ dns_status dns_destroy(dns_ctx* c) {
   free_fft(c->fz_d); free_fft(c->fx_d); free_fft(c->fyP_d); free_fft(c->fy0_d);
   free_fft(c->fz_f); free_fft(c->fx_f); free_fft(c->fyP_f);
   void* ptrs[] = {c->T0, c->T2, c->T4, c->Ut, c->dUt, c->ddUt, c->Uy, c->V, c->O, c->Nvp,
-                  c->Nop, c->rv, c->ro, c->wfac, c->wQ, c->rtab, c->F6, c->G6, c->scratch, c->solve_io, c->rhs_io, c->nl_io, c->eq_io, c->probe, c->status,
+                  c->Nop, c->rv, c->ro, c->wfac, c->wQ, c->rtab, c->F6, c->G6, c->rows_1, c->rows_n, c->solve_io, c->rhs_io, c->nl_io, c->eq_io, c->probe, c->status,
                   c->y3tc_tab};
   for (void* q : ptrs) cudaFree(q);
   if (c->slab) cudaFree(c->slab->A);
@@ -704,7 +706,7 @@ dns_status dns_get_state(dns_ctx* c, void* v, void* o, size_t pitch, int where) 
 // as values at the Gauss-Lobatto points (the reference's rhs_v_p /
 // rhs_omega_y_p), converted here with the no-pad s2p / p2s: on device pencils
 // straight between the caller's and the library's (where the pointer is one
-// that a kernel can take), else through the scratch, member by member of a batch.
+// that a kernel can take), else through the transform buffer, member by member of a batch.
 static dns_status history_copy(dns_ctx* c, double2* hist, void* user, size_t pitch, int where, bool out) {
   const size_t w = (size_t)c->g.Ny * 16;
   if (where != DNS_HOST && where != DNS_DEVICE) return fail(DNS_ERR_ARG, "where must be DNS_HOST or DNS_DEVICE");
@@ -717,17 +719,16 @@ static dns_status history_copy(dns_ctx* c, double2* hist, void* user, size_t pit
   if (where == DNS_DEVICE && kernel_ptr(c, user)) {
     CK(convert(hist, user, (long long)(pitch / 16), H * c->g.nrun));
   } else {
-    dns_status s = need_scratch(c);
-    if (s) return s;
+    double2* tmp = (double2*)c->F6;  // (six fields of wider pencils; free between steps)
     for (int r = 0; r < c->g.nrun; ++r) {
       double2* h = hist + r * H * c->g.Ny;
       char* u = (char*)user + (size_t)r * H * pitch;
       if (out) {
-        CK(convert(h, c->scratch, c->g.Ny, H));
-        CK(cudaMemcpy2DAsync(u, pitch, c->scratch, w, w, (size_t)H, kind_of(where, false), c->st));
+        CK(convert(h, tmp, c->g.Ny, H));
+        CK(cudaMemcpy2DAsync(u, pitch, tmp, w, w, (size_t)H, kind_of(where, false), c->st));
       } else {
-        CK(cudaMemcpy2DAsync(c->scratch, w, u, pitch, w, (size_t)H, kind_of(where, true), c->st));
-        CK(convert(h, c->scratch, c->g.Ny, H));
+        CK(cudaMemcpy2DAsync(tmp, w, u, pitch, w, (size_t)H, kind_of(where, true), c->st));
+        CK(convert(h, tmp, c->g.Ny, H));
       }
     }
   }
@@ -1014,7 +1015,7 @@ static dns_status check_phys_pitch(dns_ctx* c, size_t pitch) {
   return DNS_OK;
 }
 
-// nf fields, as many a launch as the scratch holds; one by one where they share memory
+// nf fields, as many a launch as the row buffer holds; one by one where they share memory
 static dns_status transform_fields(dns_ctx* c, int dir, int nf, void* const* phys, size_t pitch, void* const* spec,
                                    size_t tpitch, int pad) {
   if ((dir != DNS_FORWARD && dir != DNS_BACKWARD) || (pad != DNS_PADDING && pad != DNS_NO_PADDING))
@@ -1023,11 +1024,13 @@ static dns_status transform_fields(dns_ctx* c, int dir, int nf, void* const* phy
     if (!phys[i] || !spec[i]) return fail(DNS_ERR_ARG, "null argument");
   dns_status s;
   if ((s = check_spec_pitch(c, tpitch)) || (s = check_phys_pitch(c, pitch))) return s;
-  if ((s = need_scratch(c))) return s;
   CK(cudaSetDevice(c->P.device));
+  double2* rows;
+  int share;
+  if ((s = need_rows(c, nf, &rows, &share))) return s;
   const DnsGeom& g = c->g;
   const long long nrows = (long long)g.Py * g.Pz, rps = (long long)(pitch / 8);
-  const RowArr sr{c->scratch, c->RS, nrows * c->RS};
+  const RowArr sr{rows, c->RS, nrows * c->RS};
   const FftTab<double2> ty = pad == DNS_PADDING ? c->fyP_d.tab() : c->fy0_d.tab();
   const int mode = (dir == DNS_BACKWARD ? 0 : 2) + (pad == DNS_PADDING ? 0 : 1);
   PitchedBytes pb[6], sb[6];
@@ -1035,7 +1038,7 @@ static dns_status transform_fields(dns_ctx* c, int dir, int nf, void* const* phy
     pb[i] = PitchedBytes{phys[i], nrows, (long long)g.Px * 8, (long long)pitch};
     sb[i] = PitchedBytes{spec[i], g.H, (long long)c->P.mz * 16, (long long)tpitch};
   }
-  const int share = fields_apart(dir == DNS_FORWARD, nf, pb, sb) ? c->scratch_fields : 1;
+  if (!fields_apart(dir == DNS_FORWARD, nf, pb, sb)) share = 1;
   for (int f = 0; f < nf; f += share) {
     const int n = std::min(nf - f, share);
     PencilList sp{{}, (long long)(tpitch / 16)};

@@ -67,8 +67,8 @@ struct dns_ctx {
   void* F6 = nullptr;  // also the wall solve's scratch (free while it runs)
   void* G6 = nullptr;
   size_t F6_bytes = 0;
-  double2* scratch = nullptr;   // rows of scratch_fields fields (reference-layout transforms)
-  int scratch_fields = 0;
+  double2 *rows_1 = nullptr, *rows_n = nullptr;  // rows of one, of several fields (reference-layout transforms)
+  bool rows_tight = false;                        // the latter did not fit the device
   double2* solve_io = nullptr;  // solve-only entry: both systems' vectors + wall polynomials
   double2* rhs_io = nullptr;    // right-hand-side drop-ins: host staging (6 H Ny)
   double2* nl_io = nullptr;     // dns_nonlinear: state in, nonlinear terms out (4 H Ny)

@@ -280,8 +280,9 @@ dns_status dns_transform_3d_one_noalloc(dns_ctx* ctx, int dir, void* phys, size_
 /* transform (source/transform.cu:321-351): BACKWARD on six fields
  * (u, v, w, omega_x, omega_y, omega_z), FORWARD on three (lamb_z, lamb_y,
  * lamb_x order of the reference is immaterial).  As many fields at a time as a
- * row buffer of 64 MB holds (at least one) share each launch; the buffer is
- * allocated on first use. */
+ * row buffer of 64 MB holds (at least one) share each launch, unless fields
+ * share memory: those go one by one, in order.  The buffer is allocated by the
+ * first call of more than one field (a call of one field: that field's rows). */
 dns_status dns_transform(dns_ctx* ctx, int dir, int nfields, void* const* phys, size_t pitch,
                          void* const* spec, size_t tpitch);
 /* cuda_transpose (source/transpose.cu:115-166); xyz is complex. */
