@@ -385,12 +385,8 @@ def run_one(args):
     if args.variant:
         # fixed variants, no timing of candidates: under a profiler the
         # autotuner's event times mean nothing
-        by_name = {pkg.PASS_NAMES[p]: (p, {n: v for v, n in pkg.VARIANT_NAMES[p].items()})
-                   for p in range(pkg.NUM_PASSES)}
         for item in args.variant:
-            pname, vname = item.split("=")
-            p, names = by_name[pname]
-            ctx.set_variant(p, names[vname])
+            ctx.set_variant(*pkg.variant_by_name(*item.split("=")))
     else:
         ctx.autotune()
     variant = {pkg.PASS_NAMES[p]: pkg.VARIANT_NAMES[p][ctx.get_variant(p)] for p in range(pkg.NUM_PASSES)}

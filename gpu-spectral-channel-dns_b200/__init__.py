@@ -11,7 +11,7 @@ from .abi import (  # noqa: F401
     PASS_Y3, PASS_Y1, PASS_ZB, PASS_ZF, PASS_Y2, PASS_X, X_WARP3, X_WARP6, X_BLOCK, NUM_PASSES, MAX_VARIANTS, Y3_FFT, Y3_TENSOR, Y3_BLOCK,
     Y1_WARP, Y1_BLOCK, Z_TENSOR_COPY, Z_WARP, Z_BLOCK, Y2_RING3_12K, Y2_RING3_12K_EF, Y2_RING2_8K_EF, Y2_RING3_8K_EF,
     Y2_RING2_24K_EF, Y2_RING2_18K_EF, Y2_RING2_12K_EF, Y2_RING2_16K_EF,
-    PASS_NAMES, VARIANT_NAMES, SlabContext, SLAB_Y3, SLAB_XZ, SLAB_Y1, SLAB_V, SLAB_OMEGA, SLAB_NV,
+    PASS_NAMES, VARIANT_NAMES, OLD_VARIANT_NAMES, variant_by_name, SlabContext, SLAB_Y3, SLAB_XZ, SLAB_Y1, SLAB_V, SLAB_OMEGA, SLAB_NV,
     SLAB_NOMEGA,
 )
 from .seed import seeded_state  # noqa: F401

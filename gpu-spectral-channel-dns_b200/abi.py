@@ -41,7 +41,8 @@ Y3_FFT, Y3_TENSOR, Y3_BLOCK = 0, 1, 2
 Y1_WARP, Y1_BLOCK = 0, 1
 Z_TENSOR_COPY, Z_WARP, Z_BLOCK = 0, 1, 2
 Y2_RING2_24K_EF, Y2_RING2_18K_EF, Y2_RING2_12K_EF, Y2_RING2_16K_EF = 0, 1, 2, 3
-# earlier names of the same values
+# earlier names of the same values, deprecated: the ring shape each of them names
+# is no longer compiled, and they select 2 x 24, 2 x 18, 2 x 12 and 2 x 16 KB
 Y2_RING3_12K, Y2_RING3_12K_EF, Y2_RING2_8K_EF, Y2_RING3_8K_EF = 0, 1, 2, 3
 X_WARP3, X_WARP6, X_BLOCK = 0, 1, 2
 # names of the tunable passes and their variants (bench and test reports)
@@ -56,6 +57,20 @@ VARIANT_NAMES = {
               Y2_RING2_12K_EF: "ring_2x12k", Y2_RING2_16K_EF: "ring_2x16k"},
     PASS_X: {X_WARP3: "warp_fft_3_warps", X_WARP6: "warp_fft_6_warps", X_BLOCK: "block_fft"},
 }
+# earlier report names, still understood
+OLD_VARIANT_NAMES = {
+    PASS_Y2: {"ring_3x12k": Y2_RING3_12K, "ring_3x12k_evict_first": Y2_RING3_12K_EF,
+              "ring_2x8k_evict_first": Y2_RING2_8K_EF, "ring_3x8k_evict_first": Y2_RING3_8K_EF},
+}
+
+
+def variant_by_name(pass_name, variant_name):
+    """(pass, variant) of their report names (PASS_NAMES, VARIANT_NAMES or an
+    earlier name); KeyError for others."""
+    p = {n: k for k, n in PASS_NAMES.items()}[pass_name]
+    names = dict(OLD_VARIANT_NAMES.get(p, {}), **{n: v for v, n in VARIANT_NAMES[p].items()})
+    return p, names[variant_name]
+
 
 SLAB_PENCILS, SLAB_PLANES = 0, 1
 SLAB_Y3, SLAB_XZ, SLAB_Y1 = 0, 1, 2

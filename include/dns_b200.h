@@ -215,9 +215,10 @@ dns_status dns_set_wait_limit(dns_ctx* ctx, long long cycles);
  *     factor stream (ring stages x bytes per stage, read with the L2
  *     evict-first policy): DNS_Y2_RING2_24K_EF, DNS_Y2_RING2_18K_EF,
  *     DNS_Y2_RING2_12K_EF (the tilting table read through L1, else in shared
- *     memory), DNS_Y2_RING2_16K_EF.  DNS_Y2_RING3_12K, DNS_Y2_RING3_12K_EF,
- *     DNS_Y2_RING2_8K_EF and DNS_Y2_RING3_8K_EF are earlier names of the same
- *     values.
+ *     memory), DNS_Y2_RING2_16K_EF.  Deprecated names of the same values, whose
+ *     shapes are no longer compiled: DNS_Y2_RING3_12K (selects 2 x 24 KB),
+ *     DNS_Y2_RING3_12K_EF (2 x 18 KB), DNS_Y2_RING2_8K_EF (2 x 12 KB, the
+ *     smallest) and DNS_Y2_RING3_8K_EF (2 x 16 KB).
  * dns_set_variant fails with DNS_ERR_ARG for a variant this context cannot
  * run.  dns_autotune times every available variant of every tunable pass
  * inside whole steps on this context's buffers and grid (state and AB2
