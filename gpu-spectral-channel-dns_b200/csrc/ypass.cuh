@@ -1,4 +1,4 @@
-// Launchers of the wall-normal pass kernels (ypass.cu).
+// Launchers of the wall-normal pass kernels (ystep.cuh; the drop-ins ypass.cu).
 #pragma once
 #include "kernels.cuh"
 

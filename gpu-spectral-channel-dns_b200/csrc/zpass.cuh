@@ -16,6 +16,7 @@
 // a clock and SM was the bound.  TY elements of a pencil and TX of a row are
 // the contiguous runs, whole 32-byte sectors on both sides.
 #pragma once
+#include <type_traits>
 #include <vector>
 
 #include "fft2.cuh"
@@ -194,5 +195,55 @@ __global__ void __launch_bounds__(NT, MB) k_zf2(RowArr in, PA out, DnsGeom g, co
       }
     }
   }
+}
+
+// Tiles of the two-pass forms, measured at 384 x 384 x 512
+// (inverse / forward, us): FP64 4 x 2 lines on 128 threads, three CTAs per SM
+// 466 / 240, four CTAs (no registers to keep a radix-24 butterfly's loads in
+// flight) 511 / 246, 4 x 4 lines on 256 threads 476 / 246; at 192 x 192 x 256
+// 4 x 4 lines on 128 threads 64 / 36, 4 x 2 on 64 96 / 50, 8 x 2 71 / 34; at
+// 256 x 256 x 256 4 x 2 lines, four CTAs 97 / 50, three 98 / 52, 4 x 4 on 128
+// threads 104 / 58.
+// FP32 at 384: 4 x 4 lines on 256 threads 270 / 130, on 128 288 / 150, 8 x 4
+// 293 / 138 (the tensor-staged form, 195 / 115, comes first there).
+template <typename C, int L> struct ZTwo {
+  enum {
+    TX = 4, TY = (sizeof(C) == 8 || L <= 192) ? 4 : 2,
+    NT = (sizeof(C) == 8 && L >= 256) ? 256 : 128,
+    MB = sizeof(C) == 8 ? 2 : (ZPlan<L>::A <= 18 ? 4 : (ZPlan<L>::A > 24 ? 2 : 3))
+  };
+};
+#define DNS_ZCASE(n) case n: return f(std::integral_constant<int, n>());
+template <typename F> cudaError_t with_len_z(int L, F&& f) {
+  switch (L) { ZPLAN_LENGTHS(DNS_ZCASE) }
+  return cudaErrorNotSupported;
+}
+template <typename C, class PA>
+cudaError_t launch_zb2(PA in, RowArr out, int nf, DnsGeom g, FftTab<C> tab, cudaStream_t st, bool probe) {
+  return with_len_z(g.Pz, [&](auto LL) -> cudaError_t {
+    constexpr int L = decltype(LL)::value;
+    typedef ZTwo<C, L> T;
+    if (!tab.zt || g.Nz != L / 3 * 2) return cudaErrorNotSupported;
+    if (probe) return cudaSuccess;
+    auto k = k_zb2<C, L, T::TX, T::TY, T::NT, T::MB, PA>;
+    const size_t sm = (size_t)L * T::TX * T::TY * sizeof(C);
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k<<<dim3((g.Kx - 1 + T::TX - 1) / T::TX, (g.Py + T::TY - 1) / T::TY, nf), T::NT, sm, st>>>(in, out, g, tab.zt);
+    return cudaGetLastError();
+  });
+}
+template <typename C, class PA>
+cudaError_t launch_zf2(RowArr in, PA out, int nf, DnsGeom g, FftTab<C> tab, cudaStream_t st, bool probe) {
+  return with_len_z(g.Pz, [&](auto LL) -> cudaError_t {
+    constexpr int L = decltype(LL)::value;
+    typedef ZTwo<C, L> T;
+    if (!tab.zt || g.Nz != L / 3 * 2) return cudaErrorNotSupported;
+    if (probe) return cudaSuccess;
+    auto k = k_zf2<C, L, T::TX, T::TY, T::NT, T::MB, PA>;
+    const size_t sm = (size_t)L * T::TX * T::TY * sizeof(C);
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k<<<dim3((g.Kx + T::TX - 1) / T::TX, (g.Py + T::TY - 1) / T::TY, nf), T::NT, sm, st>>>(in, out, g, tab.zt);
+    return cudaGetLastError();
+  });
 }
 #endif

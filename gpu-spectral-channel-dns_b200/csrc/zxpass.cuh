@@ -1,4 +1,4 @@
-// Launchers of the spanwise / streamwise pass kernels (zxpass.cu).
+// Launchers of the spanwise / streamwise pass kernels (zxstep.cuh; the drop-ins zxpass.cu).
 #pragma once
 #include "kernels.cuh"
 
