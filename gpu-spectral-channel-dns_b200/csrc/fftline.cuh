@@ -11,11 +11,10 @@
 #include "fft2.cuh"
 #include "kernels.cuh"
 
-// lengths instantiated per use: streamwise / spanwise lines, padded and
-// unpadded Chebyshev extensions (2 (Py-1) = mz and 2 (Ny-1) = mz/2)
+// lengths instantiated per use: streamwise / spanwise lines, padded Chebyshev
+// extensions (2 (Py-1) = mz)
 #define FFT_XZ_LENGTHS(X) X(48) X(96) X(144) X(192) X(288) X(384) X(576)
 #define FFT_M_LENGTHS(X) X(128) X(192) X(256) X(384) X(512) X(768)
-#define FFT_M0_LENGTHS(X) X(64) X(96) X(128) X(192) X(256) X(384)
 
 template <typename C, int L>
 struct FLine {
@@ -40,7 +39,4 @@ template <typename F> cudaError_t with_len_xz(int L, F&& f) {
 }
 template <typename F> cudaError_t with_len_m(int L, F&& f) {
   switch (L) { FFT_M_LENGTHS(DNS_LCASE) default: return f(std::integral_constant<int, 0>()); }
-}
-template <typename F> cudaError_t with_len_m0(int L, F&& f) {
-  switch (L) { FFT_M0_LENGTHS(DNS_LCASE) default: return f(std::integral_constant<int, 0>()); }
 }

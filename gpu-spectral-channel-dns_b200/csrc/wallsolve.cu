@@ -45,11 +45,7 @@ __host__ __device__ constexpr int rows_per_chunk(int stg, int entries, int cap) 
   return (stg / (entries * 256)) < cap ? (stg / (entries * 256)) : cap;
 }
 
-// acc + a b, acc - a b: four fused operations (a product and a sum apart
-// are six)
-__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 acc) {
-  return make_double2(fma(-a.y, b.y, fma(a.x, b.x, acc.x)), fma(a.y, b.x, fma(a.x, b.y, acc.y)));
-}
+// acc - a b: four fused operations (a product and a sum apart are six)
 __device__ __forceinline__ double2 cfms(double2 a, double2 b, double2 acc) {
   return make_double2(fma(a.y, b.y, fma(-a.x, b.x, acc.x)), fma(-a.y, b.x, fma(-a.x, b.y, acc.y)));
 }
@@ -103,7 +99,7 @@ __global__ void __launch_bounds__(32) k_wall_solve(const double2* __restrict__ f
   double ia, ib;
   wavenumbers(kx, kz, g.Nz, ph.aphi, ph.beta, ia, ib);
   const double kap = (zero || !wd.tilt) ? 0.0 : -0.5 * ib * run_dt(ph, run);  // tilting weight of this pencil
-  const int N = g.Ny - 1, Ny = g.Ny;
+  const int N = g.Ny - 1;
   // this lane's vector (right-hand side, intermediate solution, tilting
   // term) in the group's scratch, rows interleaved over the 32 lanes: a
   // row of the warp is one contiguous 512-byte access

@@ -1,8 +1,9 @@
 // Index arithmetic of warp-synchronous line FFTs: one warp transforms lines of
 // length L held in shared memory, with no block-wide barrier.  The padded
-// layout and the store check below carry the streamwise lines (xpass.cuh,
-// xline.cuh); WPass and the plans are the same passes for NL lines at once,
-// run lane by lane on the host as the reference form of that arithmetic.
+// layout, the store check and the table offsets below carry the streamwise lines
+// (xpass.cuh, xline.cuh; tests/native/xpass_check.cpp runs those on the host).  No
+// kernel runs WPass and its plans any more: the same passes for NL lines at once,
+// kept as the reference form that tests/native/wfft_check.cpp runs lane by lane.
 //
 // Each pass is a Stockham autosort step (as in fft2.cuh): with Ns = product
 // of the previous radices, butterfly j in [0, L/R) reads x[j + r L/R],
@@ -116,8 +117,8 @@ constexpr bool wlin_store(int M, int NB, int Ns, int R) {
 
 // FP32 twiddles: one table per plan, pass by pass (passes with Ns > 1), the
 // (R - 1) Ns values W_L^{r k L/(Ns R)}, r = 1..R-1, k < Ns, stored [r][k]:
-// the lanes of a pass (consecutive k) read consecutive entries.  FP64 passes
-// use W_L^j, j < L, and a product recurrence instead.
+// the lanes of a pass (consecutive k) read consecutive entries.  (xpass.cuh has
+// such tables in both precisions; WPass in FP64 uses W_L^j, j < L, and products.)
 template <int... Rs> constexpr int wtw_offset(Radices<Rs...>, int Ns) {
   const int rs[] = {Rs...};
   int off = 0, ns = 1;

@@ -18,8 +18,8 @@
 // memory at 128 bytes a clock and SM; fusing the middle removes four of the
 // transfers of each inverse line (store, Lamb read, write, read).  Measured
 // at 384 x 384 x 512 against the form with the Lamb vector between two whole
-// transforms: FP32 356 -> 294 us, FP64 987 -> 623; 192 x 192 x 256 FP64
-// 125 -> 82; 128 x 128 x 128 FP64, a length without a plan before, 96 -> 25.
+// transforms: FP32 356 -> 298 us, FP64 987 -> 644; 192 x 192 x 256 FP64
+// 125 -> 86; 128 x 128 x 128 FP64, a length without a plan before, 96 -> 29.
 #pragma once
 #include "kernels.cuh"
 #include "wfft.cuh"
@@ -30,9 +30,10 @@
 // RF and the other radices (inverse: PRE..., RF; forward: RF, PRE...), rows
 // per CTA and warps.  A row pair's 2 L/RF butterflies fit the CTA's threads;
 // three pairs of RF complex values stay in registers (RF <= 18 FP32, 9 FP64).
-// Chosen by measurement where that leaves a choice (us, FP64 192: 8 with 24 82,
-// with 6, 4 99; 216: 9 with 24 128, with 6, 4 152; 144: 8 with 18 105, 9 with
-// 16 124; FP32 96: 8 with 12 95, 4 with 24 115; 128: eight rows 60, four 64).
+// Chosen by measurement where that leaves a choice (us; FP64 with 256 points along
+// the wall normal, 192: 8 with 24 86, with 6, 4 105; 216: 9 with 24 134, with 6, 4
+// 158; 144: 8 with 18 61, 9 with 16 73; FP32 96: 8 with 12 95, 4 with 24 115; 128:
+// eight rows 60, four 64).
 template <int L, int MAXR> struct XPlan { enum { ok = 0 }; };
 #define XPLAN(L, MAXR, RF_, NR_, NW_, ...)                                \
   template <> struct XPlan<L, MAXR> {                                     \
@@ -96,7 +97,7 @@ XPLAN(768, 8, 8, 4, 6, 12, 8)
 // rounded from W, the table W_L^j, j < L.  FP64 products w, w^2, w^3, ... would
 // save loads, but their error grows with the radix: rms error of a forward line
 // (1e-16) 4.6 by products and 1.8 from the table at 192, 5.1 and 2.0 at 216, 3.0
-// and 1.9 at 384; 384 x 384 x 512 634 -> 646 us, 192 x 192 x 256 84 -> 87.
+// and 1.9 at 384; 384 x 384 x 512 634 -> 644 us, 192 x 192 x 256 84 -> 86.
 template <typename C, int... Rs> void xtw_fill(Radices<Rs...>, int L, const double2* W, C* out) {
   const int rs[] = {Rs...};
   int ns = 1;

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(64, MB) k_y3d(const double2* __restrict__ V, c
                                                int* status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typedef Dct<C, M, 6> D;
-  constexpr int Ny = M / 4 + 1, Py = M / 2 + 1;  // the launcher checks g.Ny, g.Py against M
+  constexpr int Ny = M / 4 + 1;  // the launcher checks g.Ny, g.Py against M
   typedef typename Y3Form<C, M>::E E;  // of the derivatives
   typedef T_of<E> S;
   constexpr int FS = (Ny + 1) & ~1;  // field stride

@@ -500,7 +500,7 @@ cudaError_t launch_zf(RowArr in, PencilArr out, int nf, DnsGeom g, FftTab<C> tab
   });
 }
 // CTAs per SM that k_x2 is compiled for, measured at 384 (FP32 / FP64, us):
-// five 294 / 623, four 312 / 642; FP32 at 216: seven 33.1, five 34.7; at 96 ten
+// five 298 / 644, four 312 / 659; FP32 at 216: seven 33.1, five 34.7; at 96 ten
 // 95, seven 99.  Radix 18 in the middle needs the registers of four.
 template <typename C, int L> constexpr int x2_ctas() {
   typedef XPlan<L, FftMaxRadix<C>::v> P;
