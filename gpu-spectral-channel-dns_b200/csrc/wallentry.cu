@@ -170,10 +170,10 @@ __global__ void __launch_bounds__(256) k_nonfinite(const double2* __restrict__ a
 //
 // What bounds it: the whole FFT of each even extension (three passes of twice
 // the points) and four integration sweeps kept a call on shared memory; now a
-// value crosses it twice, and what is left is latency: 45 % of a warp's cycles
-// wait for L1, the tables among it, so two lines share each table value and
-// eight CTAs an SM (six with 32-point butterflies; six, seven, eight, ten at 384:
-// 451, 433, 423, 487 us before the sharing).  384 x 193 x 384: 555 -> 347 us,
+// value crosses it twice.  45 % of a warp's cycles then waited for L1, the tables
+// among it, so two lines share each table value (23 % now, the L1 data pipe at 70 %)
+// and eight CTAs an SM (six with 32-point butterflies; six, seven, eight, ten at
+// 384: 451, 433, 423, 487 us before the sharing).  384 x 193 x 384: 555 -> 347 us,
 // and the 140 us of a last kernel that added the wall polynomial are gone.
 template <int L>
 __global__ void __launch_bounds__(64, DPlan<L>::A > 24 ? 6 : 8)

@@ -194,7 +194,9 @@ dns_status dns_set_wait_limit(dns_ctx* ctx, long long cycles);
  * can run (the tensor-core y3 only by choice or by the autotuner).
  *   DNS_PASS_Y3: the backward wall-normal pass (getUVW + padded s2p)
  *     DNS_Y3_FFT     DCT-I by a pruned FFT of the even extension, two register
- *                    butterflies per line (lengths 2^a 3^b with a plan);
+ *                    butterflies per line (lengths 2^a 3^b with a plan; in the
+ *                    mixed form the derivatives of getUVW are FP32 at mz = 128,
+ *                    192, 256, 384, 512 and 768, FP64 at other lengths);
  *     DNS_Y3_TENSOR  batched 3xTF32 Chebyshev products on the tensor cores
  *                    (tcgen05, FP32 accumulation): mixed form, Ny = 129;
  *     DNS_Y3_BLOCK   block-wide FFT (every grid).
