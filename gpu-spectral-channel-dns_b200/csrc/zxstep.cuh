@@ -272,8 +272,7 @@ __global__ void __launch_bounds__(256, 3) k_zft(const __grid_constant__ CUtensor
 // fused streamwise pass: 6 half-spectra rows -> physical -> Lamb vector with
 // the rotation term -> 3 half-spectra rows, x 1/(Px Pz).
 // Input fields u, v(span), w(wall), omega_x, omega_y, omega_z; output
-// lambda_x, lambda_y(span), lambda_z(wall).  RB rows per CTA (even, rows of
-// one wall-normal plane).
+// lambda_x, lambda_y(span), lambda_z(wall).  Two rows per CTA.
 // ---------------------------------------------------------------------------
 template <typename C, int L>
 __global__ void __launch_bounds__(256, 3) k_x_fused(RowArr in, RowArr out, DnsGeom g, FftTab<C> tab,
@@ -291,8 +290,10 @@ __global__ void __launch_bounds__(256, 3) k_x_fused(RowArr in, RowArr out, DnsGe
   const int hx = g.Nx / 2;
   const int ls = FL::stride(Px);
   C* z = (C*)smem_raw;  // 6 lines (9 for the runtime-length FFT)
-  const long long r0 = (long long)blockIdx.x * 2;
-  const long long nrows = (long long)g.Py * g.Pz * g.nrun;  // a batch: members' rows one after another
+  // a batch: members' rows one after another, pairs within a member
+  const long long pr = (long long)g.Py * g.Pz, np = (pr + 1) / 2;
+  const int run = (int)(blockIdx.x / np);
+  const long long r0 = run * pr + 2 * (blockIdx.x - run * np), nrows = (run + 1) * pr;
   for (int t = threadIdx.x; t < 2 * 3 * Px; t += blockDim.x) {
     const int rl = t / (3 * Px);
     const int rem = t - rl * 3 * Px;
@@ -310,12 +311,10 @@ __global__ void __launch_bounds__(256, 3) k_x_fused(RowArr in, RowArr out, DnsGe
     z[(size_t)(rl * 3 + q) * ls + FL::in_pos(tab, n)] = zz;
   }
   FL::template fft<true>(z, 6, ls, tab);
-  // both rows lie in one wall-normal plane of one member
-  const long long pr = (long long)g.Py * g.Pz;
-  const int run = (int)(r0 / pr);
   const T ro = (T)(runs ? runs[3 * run + 1] : Ro);
-  const int y = (int)((r0 - run * pr) / g.Pz);
-  const T Ub = (T)Uy[y < g.Py ? y : 0];
+  T Ub[2];  // of each row's plane: with an odd number of rows a plane the two may differ
+#pragma unroll
+  for (int rl = 0; rl < 2; ++rl) Ub[rl] = (T)Uy[(int)((min(r0 + rl, nrows - 1) - run * pr) / g.Pz)];
   for (int j = threadIdx.x; j < Px; j += blockDim.x) {
     const int op = FL::out_pos(j);
     T lz[2];
@@ -328,7 +327,7 @@ __global__ void __launch_bounds__(256, 3) k_x_fused(RowArr in, RowArr out, DnsGe
       const T u = z0.x, v = z0.y, ox = z1.x, oy = z1.y, w = z2.x, oz = z2.y;
       A[rl].x = oz * v - oy * w - ro * w;
       A[rl].y = ox * w - oz * u;
-      lz[rl] = oy * u - ox * v + ro * (u + Ub);
+      lz[rl] = oy * u - ox * v + ro * (u + Ub[rl]);
     }
     if (L > 0) {  // natural order: write in place
       z[(size_t)0 * ls + op] = A[0];
@@ -556,8 +555,8 @@ cudaError_t launch_x_fused(RowArr in, RowArr out, DnsGeom g, FftTab<C> tab, cons
     constexpr int L = decltype(LL)::value;
     const size_t sm = (size_t)(L > 0 ? 6 : 9) * FLine<C, L>::stride(g.Px) * sizeof(C);
     cudaFuncSetAttribute(k_x_fused<C, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    // Pz is even: row pairs share a plane
-    k_x_fused<C, L><<<(unsigned)((nrows + 1) / 2), 256, sm, st>>>(in, out, g, tab, Uy, Ro, runs);
+    const long long pairs = ((long long)g.Py * g.Pz + 1) / 2 * g.nrun;
+    k_x_fused<C, L><<<(unsigned)pairs, 256, sm, st>>>(in, out, g, tab, Uy, Ro, runs);
     return cudaGetLastError();
   });
 }
