@@ -30,9 +30,9 @@ __global__ void k_x_c2r(RowArr in, T_of<C>* outr, long long rps, long long nrows
     C v = cmk<C>(0.0, 0.0);
     if (ra < nrows) {
       const C* a = prow<C>(in, 0, ra);
+      // a last row without a neighbour is its own: the real part is its points
       const C* b = (rb < nrows) ? prow<C>(in, 0, rb) : a;
       v = pack_c2r<C>(a, b, n, Px, hx);
-      if (rb >= nrows) v.y = 0;
     }
     z[(size_t)q * Px + tab.drev[n]] = v;
   }

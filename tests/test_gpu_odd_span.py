@@ -2,7 +2,9 @@
 streamwise transform may lie in different planes, in a batch of different members.
 
 The FP64 step against the oracle at the parity bar of the step, 1e-11, after two
-steps; a batch bit for bit its members as separate contexts."""
+steps; a batch bit for bit its members as separate contexts; the reference-layout
+transforms at theirs, 1e-13 of the largest value (486 and 27 points: streamwise
+lengths without a plan)."""
 import numpy as np
 import pytest
 
@@ -54,3 +56,28 @@ def test_batch_equals_members(pkg):
         assert all(np.array_equal(got[i][k], x) for i, x in enumerate(c.get_state())), k
         c.close()
     b.close()
+
+
+@pytest.mark.parametrize("mx,my,mz", [(24, 27, 32), (27, 27, 32), (486, 27, 16), (48, 81, 64)])
+def test_transform_matches_oracle(pkg, mx, my, mz):
+    sz = O.Sizes(mx, my, mz)
+    r = np.random.default_rng(mx + my)
+    S = np.zeros((sz.ny, sz.hnx, mz), dtype=np.complex128)
+    S[..., :sz.nz] = r.standard_normal((sz.ny, sz.hnx, sz.nz)) + 1j * r.standard_normal((sz.ny, sz.hnx, sz.nz))
+    pitch = (mx // 2 + 1) * 16
+    c = pkg.Context(pkg.make_params(mx, my, mz, Re=1300.0, dt=0.001))
+    spec = torch.from_numpy(S).cuda()
+    phys = torch.zeros(sz.pz, my, pitch // 8, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    c.transform_3d_one(pkg.BACKWARD, phys.data_ptr(), pitch, spec.data_ptr(), mz * 16)
+    c.synchronize()
+    ref = O.transform_backward(S, sz)
+    assert np.abs(phys.cpu().numpy()[..., :mx] - ref).max() < 1e-13 * np.abs(ref).max()
+    P = r.standard_normal((sz.pz, my, mx))
+    phys[..., :mx] = torch.from_numpy(P)
+    torch.cuda.synchronize()
+    c.transform_3d_one(pkg.FORWARD, phys.data_ptr(), pitch, spec.data_ptr(), mz * 16)
+    c.synchronize()
+    ref = O.transform_forward(P, sz)[..., :sz.pz]
+    assert np.abs(spec.cpu().numpy()[..., :sz.pz] - ref).max() < 1e-13 * np.abs(ref).max()
+    c.close()
