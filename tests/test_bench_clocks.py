@@ -24,7 +24,10 @@ def test_short_region_is_sampled(tmp_path, monkeypatch):
     exe.write_text(FAKE.format(python=sys.executable))
     exe.chmod(exe.stat().st_mode | stat.S_IXUSR)
     monkeypatch.setenv("PATH", str(tmp_path) + os.pathsep + os.environ["PATH"])
-    with bench.ClockSampler(0) as s:
-        time.sleep(0.025)
-    got = s.summary()
+    for _ in range(3):  # a busy host may hold the stand-in up for a whole region
+        with bench.ClockSampler(0) as s:
+            time.sleep(0.025)
+        got = s.summary()
+        if got.get("samples"):
+            break
     assert got.get("samples", 0) >= 1 and got["sm_mhz"] == 1965.0 and got["reasons"] == ["sw_power_cap"], got
